@@ -25,6 +25,16 @@ cudaMemPool_t device_pool(int device) {
   return pools[device];
 }
 
+uint64_t pool_unused() {
+  int device = 0;
+  KG_CUDA(cudaGetDevice(&device));
+  cudaMemPool_t pool = device_pool(device);
+  uint64_t reserved = 0, used = 0;
+  KG_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+  KG_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  return reserved > used ? reserved - used : 0;
+}
+
 thread_local bool g_stage_pageable = false;
 
 namespace {

@@ -95,9 +95,23 @@ void trace_slow_alloc(size_t bytes, double ms);
 // CuPy process may use) has its threshold changed.
 cudaMemPool_t device_pool(int device);
 
+// Bytes the library's pool on the current device holds and no buffer uses.
+uint64_t pool_unused();
+
 // Allocation failures injected for tests (kg_diag_fail_allocations): after `n` more
 // allocations every allocation fails as out of memory, until the count is reset.
 extern std::atomic<uint64_t> g_allocs_left;
+
+// The bytes asked of the pool for `bytes`: from 1 MB on rounded up to an eighth of the
+// power of two below (at most 64 MB more). Calls on inputs of slightly different sizes then
+// ask for the same blocks in the same order and find them free; unrounded, a pool with
+// little to spare moves memory to fit them, which stalls the host for 10 to 240 ms.
+inline size_t pool_bytes(size_t bytes) {
+  if (bytes < (1u << 20)) return bytes;
+  size_t unit = 1u << 17;
+  while (unit < (64u << 20) && unit * 16 <= bytes) unit <<= 1;
+  return (bytes + unit - 1) / unit * unit;
+}
 
 // A device allocation, stream-ordered (cudaMallocFromPoolAsync on the library's pool /
 // cudaFreeAsync).
@@ -142,11 +156,11 @@ struct DeviceBuffer {
     KG_CUDA(cudaGetDevice(&device));
     cudaMemPool_t pool = device_pool(device);
     if (!trace_on()) {
-      KG_CUDA(cudaMallocFromPoolAsync((void**)&ptr, n * sizeof(T), pool, s));
+      KG_CUDA(cudaMallocFromPoolAsync((void**)&ptr, pool_bytes(n * sizeof(T)), pool, s));
       return;
     }
     auto t0 = std::chrono::steady_clock::now();
-    KG_CUDA(cudaMallocFromPoolAsync((void**)&ptr, n * sizeof(T), pool, s));
+    KG_CUDA(cudaMallocFromPoolAsync((void**)&ptr, pool_bytes(n * sizeof(T)), pool, s));
     double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     if (ms > 2.0) trace_slow_alloc(n * sizeof(T), ms);
   }

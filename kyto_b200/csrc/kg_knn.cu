@@ -364,14 +364,21 @@ __global__ void key_bounds_kernel(const unsigned long long* key, uint64_t count,
 // The bounded scan of the exact search (qrows, list_tiles, list_lb2, list_stride,
 // list_sorted of sp): rows by k-means part (about 1,024 rows a part); bounds with
 // skipping when `skip`, else the same lists without bounds. Returns false (sp untouched)
-// when the lists would not fit the sort's 32-bit sizes or `max_bytes` of scratch.
+// when the lists would not fit the sort's 32-bit sizes or memory: twice their scratch
+// unused in the library's pool, or three times free on the device (asked for only then:
+// cudaMemGetInfo takes 0.1 to 1.8 ms).
 bool bounded_scan(const float* x, uint64_t n, uint32_t width, uint32_t d, const double* mean,
-                  double scale, double max_norm, uint32_t qblock, bool skip, uint64_t max_bytes,
-                  ScanPlan& sp, cudaStream_t s, Trace& trace) {
+                  double scale, double max_norm, uint32_t qblock, bool skip, ScanPlan& sp,
+                  cudaStream_t s, Trace& trace) {
   const uint64_t n_blocks = (n + qblock - 1) / qblock;
   const uint32_t n_tiles = (uint32_t)((n + kTile - 1) / kTile);
   const uint64_t entries = n_blocks * n_tiles;
-  if (entries > (uint64_t)INT32_MAX || entries * 28 > max_bytes) return false;
+  if (entries > (uint64_t)INT32_MAX) return false;
+  if (entries * 28 > pool_unused() / 2) {
+    size_t free_b = 0, total_b = 0;
+    KG_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if (entries * 28 > free_b / 3) return false;
+  }
   Clusters cl;
   const uint32_t parts = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(n / 1024, 1), 4096);
   cluster_rows(x, n, width, d, parts, 5, 131072, cl, s);
@@ -1281,11 +1288,8 @@ void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t 
       const std::string order = ord ? ord : "bounded";
       bool listed = false;
       if (order != "morton") {
-        size_t free_b = 0, total_b = 0;
-        KG_CUDA(cudaMemGetInfo(&free_b, &total_b));
         listed = bounded_scan(x, n, width, d, mean.ptr, scale, std::sqrt(h_largest),
-                              filter_query_block(kind), order != "cluster", free_b / 3, sp, s,
-                              trace);
+                              filter_query_block(kind), order != "cluster", sp, s, trace);
       }
       if (!listed) spatial_order(x, n, width, d, mean.ptr, lo_hi.ptr, sp.qrows, s);
       trace.mark("scan order");

@@ -13,6 +13,7 @@
 #include <cstdlib>
 #include <fstream>
 #include <memory>
+#include <map>
 #include <mutex>
 #include <sstream>
 #include <vector>
@@ -319,12 +320,20 @@ bool tune_store(const std::string& path, const std::string& gpu, const std::stri
 }
 
 std::string tune_gpu_name() {
+  // Asked for once a device: cudaGetDeviceProperties takes 2.5 to 40 ms on some hosts, and
+  // every search needs the name.
+  static std::mutex mu;
+  static std::map<int, std::string> names;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return "unknown";
+  std::lock_guard<std::mutex> lock(mu);
+  const auto known = names.find(dev);
+  if (known != names.end()) return known->second;
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return "unknown";
-  return std::string(prop.name) + "/sm_" + std::to_string(prop.major) +
-         std::to_string(prop.minor) + "/" + std::to_string(prop.multiProcessorCount) + " SMs";
+  return names[dev] = std::string(prop.name) + "/sm_" + std::to_string(prop.major) +
+                      std::to_string(prop.minor) + "/" +
+                      std::to_string(prop.multiProcessorCount) + " SMs";
 }
 
 }  // namespace kg
