@@ -23,6 +23,7 @@ __device__ __forceinline__ double rcp_approx(double v) {
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
   return r;
 }
+
 __device__ __forceinline__ float rcp_approx(float v) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
@@ -33,73 +34,40 @@ __device__ __forceinline__ float sqrt_approx(float v) {
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
   return r;
 }
-__device__ __forceinline__ float rsqrt_approx(float v) {
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-  return r;
-}
-// t = sign(z) / (|z| + sqrt(1 + z^2)).
-__device__ __forceinline__ float small_tangent(float z) {
-  const float t = rcp_approx(fabsf(z) + sqrt_approx(fmaf(z, z, 1.0f)));
-  return z >= 0.0f ? t : -t;
+
+// 1/sqrt(x) for x in [1, 2] to f64: an f32 start and two Newton steps.
+__device__ __forceinline__ double rsqrt_12(double x) {
+  double y = (double)rsqrtf((float)x);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const double e = fma(-x * y, y, 1.0);
+    y = fma(0.5 * y, e, y);
+  }
+  return y;
 }
 
 constexpr int kJacobiThreads = 256;  // 32 pairs of 8 lanes
-constexpr int kJacobiLd = kW + 2;    // a column's stride: 16-byte aligned
 
 struct JacobiShared {
-  double a[kW][kJacobiLd];  // by column: the matrix, then U diag(sigma)
-  double norms[kW];         // squared norms while rotating, then norms
+  double a[kW][kW + 1];  // by column: the matrix, then U diag(sigma)
+  double norms[kW];
   double red[32];
   uint32_t order[kW];
 };
 
-// A column's rows of one of its 8 lanes: 16 x + 2 lane and the row after it (a 16-byte
-// access whose 8 lanes cover 128 bytes: free of bank conflicts whatever the columns).
-struct JacobiRows {
-  double2 v[kW / 16];
-  __device__ __forceinline__ void load(const double* col, uint32_t lane) {
-#pragma unroll
-    for (int x = 0; x < (int)kW / 16; ++x)
-      v[x] = *reinterpret_cast<const double2*>(col + 16 * x + 2 * lane);
-  }
-  __device__ __forceinline__ void store(double* col, uint32_t lane) const {
-#pragma unroll
-    for (int x = 0; x < (int)kW / 16; ++x)
-      *reinterpret_cast<double2*>(col + 16 * x + 2 * lane) = v[x];
-  }
-  __device__ __forceinline__ double dot(const JacobiRows& o) const {
-    double p = 0.0, q = 0.0;
-#pragma unroll
-    for (int x = 0; x < (int)kW / 16; ++x) {
-      p = fma(v[x].x, o.v[x].x, p);
-      q = fma(v[x].y, o.v[x].y, q);
-    }
-    p += q;
-#pragma unroll
-    for (int o8 = 4; o8; o8 >>= 1) p += __shfl_xor_sync(0xFFFFFFFFu, p, o8);
-    return p;
-  }
-};
-
-// Hestenes' one-sided Jacobi on the w columns of the w x w matrix sh.a (everything past
-// them zero, w <= 64): pairs orthogonal to 1e-15 of their norms; sh.a becomes U diag(sigma)
-// / 2^e, sh.norms its column norms, sh.order the columns by descending norm (ties to the
-// lower column), sigma[] the singular values in that order. Returns 0, or 1 if 60 sweeps
-// did not converge. All threads of the CTA (at least 256) call it; the first 256 work.
+// Hestenes' one-sided Jacobi on the w columns of the w x w matrix sh.a (rows w .. 63 zero,
+// w <= 64): a round-robin tournament, pairs orthogonal to 1e-15 of their norms; sh.a
+// becomes U diag(sigma) / 2^e, sh.norms its column norms, sh.order the columns by
+// descending norm (ties to the lower column), sigma[] the singular values in that order.
+// Returns 0, or 1 if 60 sweeps did not converge. All threads of the CTA (at least 256)
+// call it; the first 256 work.
 //
-// A block's 60 columns take 10 to 12 sweeps, so a round of 32 disjoint pairs is
-// everything. A pair is 8 lanes of 8 rows. The sweep's order halves the columns again and
-// again: at span h, column i of the lower half of each 2h columns meets the h columns of
-// the upper half in turn, staying in registers while those pass through shared memory (one
-// column read and written a round instead of two). The squared norms follow the rotations
-// (al - t ga, be + t ga; summed afresh every sweep), so a round has one dot product. The
-// angle comes from f32 approximations (the pair keeps a 2^-20th of its product, which the
-// next sweep takes); c = 1 / sqrt(1 + t^2) and s = c t hold c^2 + s^2 = 1 to f64.
-// Latency bounds it: a round is a chain of a shared-memory read, the dot product and three
-// shuffles, the angle, the update and a barrier, about 880 cycles (a warp a pair with
-// three dot products and IEEE division, square root and hypot: 3,900; eight lanes a pair
-// with both columns passing through shared memory: 1,400).
+// A block's 60 columns take about 10 sweeps of 59 rounds, so the round is everything: a
+// pair is 8 lanes of 8 rows (three dot products, three shuffle steps), the rotation's
+// angle comes from 20-bit approximations (the pair's remaining product is a 2^-20th of
+// it, which the next sweeps take; c and s keep c^2 + s^2 = 1 to f64), and a round is one
+// barrier of 8 warps. One warp a pair with IEEE division, square root and hypot took 1.27
+// ms a block of 60 columns (about 3,900 cycles a round).
 __device__ int jacobi_square(JacobiShared& sh, uint32_t w, double* sigma) {
   const uint32_t lane = threadIdx.x & 7u, pair = threadIdx.x >> 3;
   const bool work = threadIdx.x < kJacobiThreads;
@@ -119,75 +87,59 @@ __device__ int jacobi_square(JacobiShared& sh, uint32_t w, double* sigma) {
       sh.a[x / kW][x % kW] = ldexp(sh.a[x / kW][x % kW], -e);
   __syncthreads();
 
-  const uint32_t span = w <= 16 ? 16 : w <= 32 ? 32 : 64;  // columns taking part
-  const bool mine = work && pair < span / 2;
+  const uint32_t players = (w + 1) & ~1u, turns = players - 1;
+  const bool mine = work && pair < players / 2;
   int sweep = 0;
   for (; sweep < 60; ++sweep) {
-    if (work) {
-      for (uint32_t c = pair; c < span; c += kJacobiThreads / 8) {
-        JacobiRows r;
-        r.load(sh.a[c], lane);
-        const double n = r.dot(r);
-        if (lane == 0) sh.norms[c] = n;
-      }
-    }
-    __syncthreads();
     int rotated = 0;
-    for (uint32_t h = span / 2; h; h >>= 1) {
-      const uint32_t i = pair & (h - 1), base = mine ? (pair & ~(h - 1)) * 2 : 0;
-      JacobiRows u;
-      double al = 0.0;
-      if (work) {
-        u.load(sh.a[base + i], lane);
-        al = sh.norms[base + i];
-      }
-      for (uint32_t t = 0; t < h; ++t) {
-        if (work) {  // whole warps
-          const uint32_t j = base + h + ((i + t) & (h - 1));
-          JacobiRows v;
-          v.load(sh.a[j], lane);
-          const double be = sh.norms[j];
-          const double ga = u.dot(v);
-          if (mine && al > 0.0 && be > 0.0 && ga * ga > 1e-30 * (al * be)) {
-            const double gap = be - al;
-            const float z = 0.5f * (float)gap * rcp_approx((float)ga);
-            float tf = small_tangent(z);
-            double tn = (double)tf;
-            double y = (double)rsqrt_approx(fmaf(tf, tf, 1.0f));
-            if (!(fabsf(z) < 1e8f)) {
-              // Columns of very different norms, or products past f32's range:
-              // t = 1 / (2 zeta).
-              const double zeta = 0.5 * gap * rcp_approx(ga);
-              tn = fabs(zeta) > 1e8 ? rcp_approx(2.0 * zeta) : (double)small_tangent((float)zeta);
-              y = (double)rsqrt_approx(fmaf((float)tn, (float)tn, 1.0f));
-            }
-            // 1 / sqrt(1 + t^2) from its f32 approximation by one third-order step.
-            const double x1 = fma(tn, tn, 1.0);
-            const double er = fma(-x1 * y, y, 1.0);
-            const double c = fma(y * er, fma(er, 0.375, 0.5), y), s = c * tn;
-#pragma unroll
-            for (int x = 0; x < (int)kW / 16; ++x) {
-              const double2 p = u.v[x], q = v.v[x];
-              u.v[x].x = fma(c, p.x, -(s * q.x));
-              u.v[x].y = fma(c, p.y, -(s * q.y));
-              v.v[x].x = fma(s, p.x, c * q.x);
-              v.v[x].y = fma(s, p.y, c * q.y);
-            }
-            v.store(sh.a[j], lane);
-            if (lane == 0) sh.norms[j] = fma(tn, ga, be);
-            al = fma(-tn, ga, al);
-            rotated = 1;
-          }
+    // Positions 1 .. players - 1 turn; player 0 stays. Pair p meets positions p and
+    // players - 1 - p.
+    uint32_t pi = pair == 0 ? 0 : pair - 1, pj = players - 2 - (mine ? pair : 0);
+    for (uint32_t r = 0; r < turns; ++r) {
+      if (work) {  // whole warps
+        uint32_t i = pair == 0 ? 0 : pi + 1, j = pj + 1;
+        if (i > j) {
+          const uint32_t t = i;
+          i = j;
+          j = t;
         }
-        // Spans of up to four pairs pass their columns inside one warp.
-        if (h > 4)
-          __syncthreads();
-        else
-          __syncwarp();
-      }
-      if (mine) {
-        u.store(sh.a[base + i], lane);
-        if (lane == 0) sh.norms[base + i] = al;
+        const bool live = mine && j < w;
+        double* ai = sh.a[live ? i : 0];
+        double* aj = sh.a[live ? j : 0];
+        double u[kW / 8], v[kW / 8];
+        double al = 0.0, be = 0.0, ga = 0.0;
+#pragma unroll
+        for (int x = 0; x < (int)kW / 8; ++x) {
+          u[x] = ai[lane + 8 * x];
+          v[x] = aj[lane + 8 * x];
+          al = fma(u[x], u[x], al);
+          be = fma(v[x], v[x], be);
+          ga = fma(u[x], v[x], ga);
+        }
+#pragma unroll
+        for (int o = 4; o; o >>= 1) {
+          al += __shfl_xor_sync(0xFFFFFFFFu, al, o);
+          be += __shfl_xor_sync(0xFFFFFFFFu, be, o);
+          ga += __shfl_xor_sync(0xFFFFFFFFu, ga, o);
+        }
+        if (live && al > 0.0 && be > 0.0 && ga * ga > 1e-30 * (al * be)) {
+          const double zeta = 0.5 * (be - al) * rcp_approx(ga);
+          // t = sign(zeta) / (|zeta| + sqrt(1 + zeta^2)), and 1 / (2 zeta) far out (columns
+          // of very different norms: past f32's range).
+          const float z = (float)zeta;
+          const float tf = rcp_approx(fabsf(z) + sqrt_approx(fmaf(z, z, 1.0f)));
+          const double t = fabs(zeta) > 1e8 ? rcp_approx(2.0 * zeta)
+                                            : (double)(z >= 0.0f ? tf : -tf);
+          const double c = rsqrt_12(fma(t, t, 1.0)), s = c * t;
+#pragma unroll
+          for (int x = 0; x < (int)kW / 8; ++x) {
+            ai[lane + 8 * x] = fma(c, u[x], -(s * v[x]));
+            aj[lane + 8 * x] = fma(s, u[x], c * v[x]);
+          }
+          rotated = 1;
+        }
+        if (++pi == turns) pi = 0;
+        if (++pj == turns) pj = 0;
       }
       __syncthreads();
     }
@@ -195,10 +147,12 @@ __device__ int jacobi_square(JacobiShared& sh, uint32_t w, double* sigma) {
   }
   if (work) {
     for (uint32_t c = pair; c < kW; c += kJacobiThreads / 8) {
-      JacobiRows r;
-      r.load(sh.a[c], lane);
-      const double n = r.dot(r);
-      if (lane == 0) sh.norms[c] = sqrt(n);
+      double ss = 0.0;
+#pragma unroll
+      for (int x = 0; x < (int)kW / 8; ++x) ss = fma(sh.a[c][lane + 8 * x], sh.a[c][lane + 8 * x], ss);
+#pragma unroll
+      for (int o = 4; o; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+      if (lane == 0) sh.norms[c] = sqrt(ss);
     }
   }
   __syncthreads();
@@ -250,16 +204,10 @@ struct XbShared {
 // as zeros) into sh.rows.
 __device__ __forceinline__ void stage_rows(XbShared& sh, const double* a, uint32_t g, uint32_t w,
                                            uint32_t r0, uint32_t r1) {
-  const uint32_t r = threadIdx.x % kXbRows, c0 = threadIdx.x / kXbRows;
-  double v[kW * kXbRows / kXbThreads];
-#pragma unroll
-  for (int i = 0; i < (int)(kW * kXbRows / kXbThreads); ++i) {
-    const uint32_t c = c0 + i * (kXbThreads / kXbRows);
-    v[i] = r0 + r < r1 && c < w ? a[(uint64_t)c * g + r0 + r] : 0.0;
+  for (uint32_t x = threadIdx.x; x < kXbRows * kW; x += kXbThreads) {
+    const uint32_t r = x % kXbRows, c = x / kXbRows;
+    sh.rows[r][c] = r0 + r < r1 && c < w ? a[(uint64_t)c * g + r0 + r] : 0.0;
   }
-#pragma unroll
-  for (int i = 0; i < (int)(kW * kXbRows / kXbThreads); ++i)
-    sh.rows[r][c0 + i * (kXbThreads / kXbRows)] = v[i];
 }
 
 // The orthonormalisation of a Krylov block in one launch: shifted CholeskyQR3 (Fukaya,
@@ -272,14 +220,12 @@ __device__ __forceinline__ void stage_rows(XbShared& sh, const double* a, uint32
 // registers, rows published through shared memory, LDL^T so that a step waits for one
 // reciprocal), and the rows' triangular solve (a thread a row, 8-column blocks). Rank 0
 // runs the Jacobi while the others wait.
-// Latency bounds it (a 2,000 x 60 block is 1 MB, 3 x 7 Mflop): 0.43 ms on 2,000 x 60, of
-// it 0.32 ms in the Jacobi. The same steps as separate launches (three Gram GEMMs, factors
-// and solves of cuBLAS and one-CTA kernels, the SVD, the last GEMM, two norms read by the
-// host) took 2.02 ms a block.
+// Latency bounds it (a 2,000 x 60 block is 1 MB, 3 x 7 Mflop): the same steps as separate
+// launches (three Gram GEMMs, factors and solves of cuBLAS and one-CTA kernels, the SVD,
+// the last GEMM, two norms read by the host) took 2.02 ms a block.
 __global__ void __launch_bounds__(kXbThreads, 1)
 extend_svd_kernel(const double* __restrict__ block, const double* __restrict__ rest, uint32_t g,
-                  uint32_t w, double shift, double* q, double* __restrict__ u, double* ur,
-                  double* out) {
+                  uint32_t w, double shift, double* q, double* __restrict__ u, double* out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   XbShared& sh = *reinterpret_cast<XbShared*>(smem_raw);
   cg::cluster_group cl = cg::this_cluster();
@@ -411,30 +357,49 @@ extend_svd_kernel(const double* __restrict__ block, const double* __restrict__ r
       const uint32_t j = x / kW, c = x % kW;
       sh.r[j][c] = c >= j ? sh.r[j][c] * sh.dinv[j] : 0.0;
     }
-    // Q = A R^-1 on this CTA's rows, a thread a row, 128 rows a pass, the next columns'
-    // loads ahead of the current ones' arithmetic. Rank 0's other 128 threads make
-    // rtot = R rtot meanwhile (R itself in the first round).
-    if (tid < kXbSolve) {
-      for (uint32_t row = row0 + tid; row < row1; row += kXbSolve) {
-        double nb[8];
+    __syncthreads();
+    // rtot = R rtot (rank 0; R itself in the first round).
+    if (rank == 0) {
+      double(*dst)[kW] = sh.rtot[round & 1];
+      const double(*src)[kW] = sh.rtot[(round & 1) ^ 1];
+      if (round == 0) {
+        for (uint32_t x = tid; x < kW * kW; x += kXbThreads) dst[x / kW][x % kW] = sh.r[x / kW][x % kW];
+      } else {
+        double t[4][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) nb[i] = (uint32_t)i < w ? a[(uint64_t)i * g + row] : 0.0;
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) t[i][c] = 0.0;
+        for (uint32_t k = 0; k < w; ++k) {
+          double x[4], y[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) x[i] = sh.r[ty + 16 * i][k];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) y[i] = src[k][tx + 16 * i];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) t[i][c] = fma(x[i], y[c], t[i][c]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) dst[ty + 16 * i][tx + 16 * c] = t[i][c];
+      }
+    }
+    __syncthreads();
+    // Q = A R^-1 on this CTA's rows, a thread a row, 128 rows a pass.
+    for (uint32_t r0 = row0; r0 < row1; r0 += kXbSolve) {
+      if (tid < kXbSolve && r0 + tid < row1) {
+        const uint32_t row = r0 + tid;
         for (uint32_t jb = 0; jb < w; jb += 8) {
           double b[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            b[i] = nb[i];
-            const uint32_t c = jb + 8 + i;
-            nb[i] = c < w ? a[(uint64_t)c * g + row] : 0.0;
-          }
-          for (uint32_t k0 = 0; k0 < jb; k0 += 8) {
-            double xk[8];
+          for (int i = 0; i < 8; ++i) b[i] = jb + i < w ? a[(uint64_t)(jb + i) * g + row] : 0.0;
+          for (uint32_t k = 0; k < jb; ++k) {
+            const double xk = sh.x[k][tid];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) xk[k] = sh.x[k0 + k][tid];
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-#pragma unroll
-              for (int i = 0; i < 8; ++i) b[i] = fma(-xk[k], sh.r[k0 + k][jb + i], b[i]);
+            for (int i = 0; i < 8; ++i) b[i] = fma(-xk, sh.r[k][jb + i], b[i]);
           }
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -445,36 +410,6 @@ extend_svd_kernel(const double* __restrict__ block, const double* __restrict__ r
             if (jb + i < w) q[(uint64_t)(jb + i) * g + row] = b[i];
           }
         }
-      }
-    } else if (rank == 0) {
-      double(*dst)[kW] = sh.rtot[round & 1];
-      const double(*src)[kW] = sh.rtot[(round & 1) ^ 1];
-      const uint32_t t2 = tid - kXbSolve;
-      if (round == 0) {
-        for (uint32_t x = t2; x < kW * kW; x += kXbThreads - kXbSolve)
-          dst[x / kW][x % kW] = sh.r[x / kW][x % kW];
-      } else {
-        const uint32_t ry = t2 >> 4;
-        double t[8][4];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) t[i][c] = 0.0;
-        for (uint32_t k = 0; k < w; ++k) {
-          double x[8], y[4];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) x[i] = sh.r[ry + 8 * i][k];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) y[i] = src[k][tx + 16 * i];
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) t[i][c] = fma(x[i], y[c], t[i][c]);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) dst[ry + 8 * i][tx + 16 * c] = t[i][c];
       }
     }
     __syncthreads();
@@ -497,13 +432,14 @@ extend_svd_kernel(const double* __restrict__ block, const double* __restrict__ r
         const double nv = sh.jac.norms[o];
         v = nv > 0.0 ? sh.jac.a[o][i] / nv : 0.0;
       }
-      ur[x] = v;
+      sh.rtot[1][i][c] = v;
     }
     if (tid == 0) out[w + 1] = failed || sh.bad ? 1.0 : 0.0;
   }
-  // U_R goes through global memory (16 CTAs reading rank 0's shared memory queue there).
   cl.sync();
-  for (uint32_t x = tid; x < kW * kW; x += kXbThreads) sh.r[x / kW][x % kW] = ur[x];
+  for (uint32_t x = tid; x < kW * kW; x += kXbThreads)
+    sh.r[x / kW][x % kW] = *cl.map_shared_rank(&sh.rtot[1][x / kW][x % kW], 0);
+  cl.sync();  // rank 0's shared memory is read until here
   for (uint32_t r0 = row0; r0 < row1; r0 += kXbRows) {
     __syncthreads();
     stage_rows(sh, q, g, w, r0, row1);
@@ -674,10 +610,8 @@ void extend_svd(const double* block, const double* rest, uint32_t g, uint32_t w,
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  // The first round's shift (times the trace): 11 (g w + w (w + 1)) u.
   const double shift = 11.0 * ((double)g * w + (double)w * (w + 1)) * 0x1p-53;
-  KG_CUDA(cudaLaunchKernelEx(&cfg, extend_svd_kernel, block, rest, g, w, shift, q,
-                             u, q + (uint64_t)g * w, out));
+  KG_CUDA(cudaLaunchKernelEx(&cfg, extend_svd_kernel, block, rest, g, w, shift, q, u, out));
   KG_LAUNCH_CHECK();
 }
 

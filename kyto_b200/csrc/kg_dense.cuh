@@ -15,7 +15,7 @@ constexpr uint32_t kQrMaxCols = 64;
 // the left singular vectors, out[0 .. w) the singular values (descending, ties to the lower
 // column), out[w] = |block|_F of the g x w `block`, out[w + 1] = 0, or 1 if a Cholesky pivot
 // was not positive (a numerically rank-deficient block: use qr_svd) or Jacobi did not
-// converge. q: scratch of g w + 64 * 64 values.
+// converge. q: g x w scratch.
 void extend_svd(const double* block, const double* rest, uint32_t g, uint32_t w, double* q,
                 double* u, double* out, cudaStream_t s);
 

@@ -1053,7 +1053,7 @@ struct Dense {
     DeviceBuffer<double> u((uint64_t)g * w, s);
     DeviceBuffer<uint32_t> order;
     if (narrow) {
-      DeviceBuffer<double> q((uint64_t)g * w + kQrMaxCols * kQrMaxCols, s);
+      DeviceBuffer<double> q((uint64_t)g * w, s);
       extend_svd(block, from, g, w, q.ptr, u.ptr, out.ptr, s);
       read_back();
     } else {
