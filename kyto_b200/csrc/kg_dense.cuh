@@ -1,0 +1,36 @@
+// The PCA's dense FP64 steps on blocks of up to 64 columns (kg_dense.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+namespace kg {
+
+constexpr uint32_t kQrMaxCols = 64;
+
+// One step of shifted CholeskyQR3 (Fukaya, Kannan, Nakatsukasa, Yamamoto and Yanagisawa,
+// "Shifted Cholesky QR for computing the QR factorization of ill-conditioned matrices",
+// SIAM J. Sci. Comput. 2020), w <= 64: the upper Cholesky factor R of the Gram matrix G
+// (w x w, column-major) plus shift * trace(G) on the diagonal (trace(G) = |A|_F^2 >=
+// |A|_2^2), into r (w x w column-major, zeros below). *status = 1 (and r left as it is) if
+// a pivot is not positive (the caller then uses Householder QR).
+void cholesky_step(const double* gram, uint32_t w, double shift, double* r, int* status,
+                   cudaStream_t s);
+
+// The SVD of R = R_3 R_2 R_1, the steps' factors one after another in r (w x w upper
+// triangular, column-major, w <= 64): out[0 .. w) the singular values (descending, ties to
+// the lower column), u_r (w x w: column c the unit left singular vector of out[c]; zero for
+// 0), out[w] = the Frobenius norm of `block` (n values), out[w + 1] = 0, or 1 if *status
+// was set or Jacobi did not converge.
+void small_svd(const double* r, uint32_t w, const double* block, uint64_t n, const int* status,
+               double* u_r, double* out, cudaStream_t s);
+
+// The thin SVD of the g x w column-major block `b` (overwritten): u the left singular
+// vectors, out[0 .. w) and out[w + 1] as above (out[w] is left as it is).
+void qr_svd(double* b, uint32_t g, uint32_t w, double* u, double* out, cudaStream_t s);
+
+// *out = the Frobenius norm of m (n values).
+void frobenius(const double* m, uint64_t n, double* out, cudaStream_t s);
+
+}  // namespace kg

@@ -21,6 +21,7 @@
 #include <cmath>
 #include <vector>
 
+#include "kg_dense.cuh"
 #include "kg_internal.cuh"
 #include "kg_knn.cuh"
 #include "kg_maps.cuh"
@@ -391,7 +392,7 @@ constexpr uint32_t kJacobiMaxCols = 256;
 // needs. status: 0, or 1 if 60 sweeps did not converge.
 __global__ void __launch_bounds__(1024)
 jacobi_svd_kernel(double* a, uint32_t g, uint32_t w, double* sigma, uint32_t* order,
-                  int* status) {
+                  double* status) {
   __shared__ int rotated;
   __shared__ double norms[kJacobiMaxCols];
   const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -468,273 +469,8 @@ jacobi_svd_kernel(double* a, uint32_t g, uint32_t w, double* sigma, uint32_t* or
       order[c] = idx[c];
       sigma[c] = norms[idx[c]];
     }
-    *status = sweep >= 60 ? 1 : 0;
+    *status = sweep >= 60 ? 1.0 : 0.0;
   }
-}
-
-constexpr uint32_t kQrMaxCols = 64;
-
-// Hestenes' one-sided Jacobi on the w columns of the w x w matrix in shared memory `rs`
-// (by column; round-robin tournament, one warp per pair, pairs orthogonal to 1e-15 of
-// their norms): rs becomes U_R diag(sigma). Then norms[c] = sigma of column c, order =
-// the columns by descending sigma (ties to the lower column), sigma[] (global) in that
-// order and *status = 0, or 1 if 60 sweeps did not converge. All threads call it.
-__device__ void jacobi_square(double (*rs)[kQrMaxCols + 1], uint32_t w, double* norms,
-                              uint32_t* order, int* rotated_flag, double* sigma, int* status) {
-  const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const unsigned warps = blockDim.x >> 5;
-  int& rotated = *rotated_flag;
-  const uint32_t players = (w + 1) & ~1u;
-  int sweep = 0;
-  for (; sweep < 60; ++sweep) {
-    if (threadIdx.x == 0) rotated = 0;
-    __syncthreads();
-    for (uint32_t r = 0; r + 1 < players; ++r) {
-      for (uint32_t pr = warp; pr < players / 2; pr += warps) {
-        auto at = [&](uint32_t pos) {
-          return pos == 0 ? 0u : ((pos - 1 + r) % (players - 1)) + 1;
-        };
-        uint32_t i = at(pr), j2 = at(players - 1 - pr);
-        if (i > j2) {
-          uint32_t tt = i;
-          i = j2;
-          j2 = tt;
-        }
-        if (j2 >= w) continue;
-        double al = 0.0, be = 0.0, ga = 0.0;
-        for (uint32_t x = lane; x < w; x += 32) {
-          double p = rs[i][x], q = rs[j2][x];
-          al = fma(p, p, al);
-          be = fma(q, q, be);
-          ga = fma(p, q, ga);
-        }
-        for (int o = 16; o; o >>= 1) {
-          al += __shfl_xor_sync(0xFFFFFFFFu, al, o);
-          be += __shfl_xor_sync(0xFFFFFFFFu, be, o);
-          ga += __shfl_xor_sync(0xFFFFFFFFu, ga, o);
-        }
-        if (!(al > 0.0) || !(be > 0.0) || !(fabs(ga) > 1e-15 * sqrt(al) * sqrt(be))) continue;
-        double zeta = (be - al) / (2.0 * ga);
-        double tn = (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + hypot(1.0, zeta));
-        double cs = 1.0 / sqrt(1.0 + tn * tn), sn = cs * tn;
-        for (uint32_t x = lane; x < w; x += 32) {
-          double p = rs[i][x], q = rs[j2][x];
-          rs[i][x] = cs * p - sn * q;
-          rs[j2][x] = sn * p + cs * q;
-        }
-        if (lane == 0) rotated = 1;
-      }
-      __syncthreads();
-    }
-    bool again = rotated != 0;
-    __syncthreads();
-    if (!again) break;
-  }
-  // Column norms = singular values; the order (descending, ties to the lower column).
-  for (uint32_t c = warp; c < w; c += warps) {
-    double ss = 0.0;
-    for (uint32_t x = lane; x < w; x += 32) ss = fma(rs[c][x], rs[c][x], ss);
-    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-    if (lane == 0) norms[c] = sqrt(ss);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (uint32_t c = 0; c < w; ++c) order[c] = c;
-    for (uint32_t c = 1; c < w; ++c) {
-      uint32_t v = order[c], pos = c;
-      while (pos > 0 && norms[order[pos - 1]] < norms[v]) {
-        order[pos] = order[pos - 1];
-        --pos;
-      }
-      order[pos] = v;
-    }
-    for (uint32_t c = 0; c < w; ++c) sigma[c] = norms[order[c]];
-    *status = sweep >= 60 ? 1 : 0;
-  }
-  __syncthreads();
-}
-
-// The thin SVD's left singular vectors of the g x w column-major block `b` (w <= 64,
-// overwritten), one CTA of 32 warps: Householder QR in place (b = Q R, the reflectors
-// below the diagonal, LAPACK's dlarfg convention v_j = 1), then Hestenes' one-sided
-// Jacobi on R in shared memory (R V = U_R diag(sigma); pairs orthogonal to 1e-15 of
-// their norms), then U = Q [U_R; 0] by applying the reflectors backwards. QR is
-// backward stable, so sigma carries an absolute error of about 1e-16 |b|: the drop rule
-// (sigma > 1e-10 |b|_F) sees rank deficiency as an SVD of b would.
-// Outputs: sigma (w, descending; ties to the lower column), u (g x w: column c the
-// unit vector of sigma[c]). status: 0, or 1 if 60 sweeps did not converge.
-__global__ void __launch_bounds__(1024)
-qr_svd_kernel(double* b, uint32_t g, uint32_t w, double* sigma, double* u, int* status) {
-  __shared__ double rs[kQrMaxCols][kQrMaxCols + 1];  // R, then U_R diag(sigma), by column
-  __shared__ double tau[kQrMaxCols];
-  __shared__ double norms[kQrMaxCols];
-  __shared__ uint32_t order[kQrMaxCols];
-  __shared__ int rotated;
-  const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const unsigned warps = blockDim.x >> 5;
-  auto colp = [&](uint32_t c) { return b + (uint64_t)c * g; };
-
-  // Householder QR.
-  for (uint32_t j = 0; j < w; ++j) {
-    if (warp == 0) {
-      const double* bj = colp(j);
-      double ss = 0.0;
-      for (uint32_t i = j + 1 + lane; i < g; i += 32) ss = fma(bj[i], bj[i], ss);
-      for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-      if (lane == 0) {
-        double alpha = bj[j];
-        double normx = sqrt(fma(alpha, alpha, ss));
-        if (ss == 0.0) {
-          tau[j] = 0.0;  // already upper triangular in this column
-        } else {
-          double beta = alpha >= 0.0 ? -normx : normx;
-          tau[j] = (beta - alpha) / beta;
-          norms[j] = 1.0 / (alpha - beta);  // scale of v below the diagonal
-          colp(j)[j] = beta;
-        }
-      }
-    }
-    __syncthreads();
-    const double t = tau[j];
-    if (t != 0.0) {
-      double* bj = colp(j);
-      const double sc = norms[j];
-      for (uint32_t i = j + 1 + threadIdx.x; i < g; i += blockDim.x) bj[i] *= sc;
-      __syncthreads();
-      for (uint32_t c = j + 1 + warp; c < w; c += warps) {
-        double* bc = colp(c);
-        double d = (lane == 0) ? bc[j] : 0.0;
-        for (uint32_t i = j + 1 + lane; i < g; i += 32) d = fma(bj[i], bc[i], d);
-        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xFFFFFFFFu, d, o);
-        const double f = t * d;
-        if (lane == 0) bc[j] -= f;
-        for (uint32_t i = j + 1 + lane; i < g; i += 32) bc[i] = fma(-f, bj[i], bc[i]);
-      }
-    }
-    __syncthreads();
-  }
-  // R into shared memory.
-  for (uint32_t x = threadIdx.x; x < w * w; x += blockDim.x) {
-    uint32_t c = x / w, r = x % w;
-    rs[c][r] = r <= c ? colp(c)[r] : 0.0;
-  }
-  __syncthreads();
-  jacobi_square(rs, w, norms, order, &rotated, sigma, status);
-  // U = Q [U_R; 0]: start from U_R's unit columns, apply H_{w-1}, ..., H_0.
-  for (uint64_t x = threadIdx.x; x < (uint64_t)g * w; x += blockDim.x) {
-    uint32_t c = (uint32_t)(x / g), r = (uint32_t)(x % g);
-    double nv = norms[order[c]];
-    u[x] = (r < w && nv > 0.0) ? rs[order[c]][r] / nv : 0.0;
-  }
-  __syncthreads();
-  for (int j = (int)w - 1; j >= 0; --j) {
-    const double t = tau[j];
-    if (t == 0.0) continue;
-    const double* v = colp(j);
-    for (uint32_t c = warp; c < w; c += warps) {
-      double* uc = u + (uint64_t)c * g;
-      double d = (lane == 0) ? uc[j] : 0.0;
-      for (uint32_t i = j + 1 + lane; i < g; i += 32) d = fma(v[i], uc[i], d);
-      for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xFFFFFFFFu, d, o);
-      const double f = t * d;
-      if (lane == 0) uc[j] -= f;
-      for (uint32_t i = j + 1 + lane; i < g; i += 32) uc[i] = fma(-f, v[i], uc[i]);
-    }
-    __syncthreads();
-  }
-}
-
-// One step of shifted CholeskyQR3 (Fukaya, Kannan, Nakatsukasa, Yamamoto and Yanagisawa,
-// "Shifted Cholesky QR for computing the QR factorization of ill-conditioned
-// matrices", SIAM J. Sci. Comput. 2020), one CTA, w <= 64: the upper Cholesky factor R
-// of the Gram matrix G (w x w, column-major) plus shift * trace(G) on the diagonal
-// (trace(G) = |A|_F^2 >= |A|_2^2), into r (w x w column-major, zeros below), and the
-// running product r_total = R r_total (R itself when first). *status = 1 if a pivot is
-// not positive (the caller then uses Householder QR).
-__global__ void __launch_bounds__(1024)
-cholesky_step_kernel(const double* gram, uint32_t w, double shift, int first, double* r,
-                     double* r_total, int* status) {
-  __shared__ double a[kQrMaxCols][kQrMaxCols + 1];  // a[row][col]
-  __shared__ double trace;
-  __shared__ int bad;
-  for (uint32_t x = threadIdx.x; x < w * w; x += blockDim.x) a[x % w][x / w] = gram[x];
-  if (threadIdx.x == 0) bad = 0;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double tr = 0.0;
-    for (uint32_t j = 0; j < w; ++j) tr += a[j][j];
-    trace = tr;
-  }
-  __syncthreads();
-  if (threadIdx.x < w) a[threadIdx.x][threadIdx.x] += shift * trace;
-  __syncthreads();
-  for (uint32_t j = 0; j < w; ++j) {
-    const double d = a[j][j];
-    if (!(d > 0.0)) {
-      if (threadIdx.x == 0) bad = 1;
-      break;  // every thread reads the same d and leaves together
-    }
-    const double piv = sqrt(d);
-    __syncthreads();
-    // Row j of R: a[j][c] / piv for c > j (the diagonal written after the reads).
-    for (uint32_t c = j + 1 + threadIdx.x; c < w; c += blockDim.x) a[j][c] /= piv;
-    __syncthreads();
-    if (threadIdx.x == 0) a[j][j] = piv;
-    // Trailing update: a[i][c] -= R[j][i] R[j][c] for j < i <= c.
-    const uint32_t m = w - j - 1;
-    for (uint32_t x = threadIdx.x; x < m * m; x += blockDim.x) {
-      uint32_t i = j + 1 + x / m, c = j + 1 + x % m;
-      if (i <= c) a[i][c] -= a[j][i] * a[j][c];
-    }
-    __syncthreads();
-  }
-  __syncthreads();
-  if (bad) {
-    if (threadIdx.x == 0) *status = 1;
-    return;
-  }
-  for (uint32_t x = threadIdx.x; x < w * w; x += blockDim.x) {
-    uint32_t c = x / w, i = x % w;
-    r[x] = i <= c ? a[i][c] : 0.0;
-  }
-  // r_total = R r_total (both upper triangular): every thread computes its (at most 4,
-  // w <= 64 with 1024 threads) entries from the old r_total before any is written.
-  double v[4] = {0.0, 0.0, 0.0, 0.0};
-  for (uint32_t x = threadIdx.x, e = 0; x < w * w; x += blockDim.x, ++e) {
-    uint32_t c = x / w, i = x % w;
-    if (i > c) continue;
-    if (first) {
-      v[e] = a[i][c];
-    } else {
-      double acc = 0.0;
-      for (uint32_t q = i; q <= c; ++q) acc = fma(a[i][q], r_total[(uint64_t)c * w + q], acc);
-      v[e] = acc;
-    }
-  }
-  __syncthreads();
-  for (uint32_t x = threadIdx.x, e = 0; x < w * w; x += blockDim.x, ++e) r_total[x] = v[e];
-}
-
-// The SVD of the w x w upper-triangular r (column-major, w <= 64): sigma (descending,
-// ties to the lower column) and u_r (w x w: column c the unit left singular vector of
-// sigma[c]; zero for sigma 0). *status |= 1 if Jacobi did not converge.
-__global__ void __launch_bounds__(1024)
-small_svd_kernel(const double* r, uint32_t w, double* sigma, double* u_r, int* status) {
-  __shared__ double rs[kQrMaxCols][kQrMaxCols + 1];
-  __shared__ double norms[kQrMaxCols];
-  __shared__ uint32_t order[kQrMaxCols];
-  __shared__ int rotated;
-  __shared__ int jstatus;
-  for (uint32_t x = threadIdx.x; x < w * w; x += blockDim.x) rs[x / w][x % w] = r[x];
-  __syncthreads();
-  jacobi_square(rs, w, norms, order, &rotated, sigma, &jstatus);
-  __syncthreads();
-  for (uint32_t x = threadIdx.x; x < w * w; x += blockDim.x) {
-    uint32_t c = x / w, i = x % w;
-    double nv = norms[order[c]];
-    u_r[x] = nv > 0.0 ? rs[order[c]][i] / nv : 0.0;
-  }
-  if (threadIdx.x == 0 && jstatus) *status = 1;
 }
 
 // out[:, c] = a[:, order[c]] / sigma[c] (the left singular vectors kept).
@@ -1261,24 +997,20 @@ struct Dense {
   cudaStream_t s;
   uint32_t g;
 
-  double fro_norm(const double* m, uint64_t count) {
-    double out = 0.0;
-    KG_CUBLAS(cublasDnrm2(p->cublas, (int)count, m, 1, &out));
-    return out;
-  }
-
   // pca_dense.rs:105-129: the directions `block` (g x w) adds to `basis` (g x m):
-  // CGS twice, thin SVD, keep sigma > 1e-10 |block|_F. Returns the new block.
+  // CGS twice, thin SVD, keep sigma > 1e-10 |block|_F. Returns the new block (its first
+  // *keep_out columns).
   DeviceBuffer<double> extend_basis(const double* basis, uint32_t m, const double* block,
                                     uint32_t w, uint32_t* keep_out) {
     *keep_out = 0;
     DeviceBuffer<double> none;
     if (w == 0) return none;
-    double scale = fro_norm(block, (uint64_t)g * w);
-    if (!(scale > 0.0)) {
-      if (std::isnan(scale)) fail(KG_ERR_INVALID, "pca: the Krylov block is not finite");
-      return none;
-    }
+    if (w > kJacobiMaxCols) fail(KG_ERR_INVALID, "pca: a Krylov block wider than 256 columns");
+    // Blocks of up to 64 columns (and g >= w, always true here): shifted CholeskyQR3
+    // (rest = Q R: three Gram / Cholesky / triangular-solve rounds), the SVD of R in one
+    // CTA, U = Q U_R; Householder QR in one CTA if a Cholesky pivot fails (a numerically
+    // rank-deficient block). One-sided Jacobi on the whole block beyond 64 columns.
+    const bool narrow = w <= kQrMaxCols;
     DeviceBuffer<double> rest((uint64_t)g * w, s);
     KG_CUDA(cudaMemcpyAsync(rest.ptr, block, rest.bytes(), cudaMemcpyDeviceToDevice, s));
     if (m > 0) {
@@ -1291,73 +1023,65 @@ struct Dense {
                               proj.ptr, m, &one, rest.ptr, g));
       }
     }
-    // Thin SVD in one kernel: QR + Jacobi on R for blocks of up to 64 columns (and
-    // g >= w, always true here), one-sided Jacobi on the whole block beyond that.
-    if (w > kJacobiMaxCols) fail(KG_ERR_INVALID, "pca: a Krylov block wider than 256 columns");
-    DeviceBuffer<double> sv(w, s);
-    DeviceBuffer<uint32_t> order(w, s);
-    DeviceBuffer<int> info(1, s);
-    DeviceBuffer<double> u;
-    const bool qr = w <= kQrMaxCols;
-    std::vector<double> h_sv(w);
-    int h_info = 0;
+    // Singular values, |block|_F, status.
+    DeviceBuffer<double> out(w + 2, s);
+    std::vector<double> h(w + 2);
     auto read_back = [&]() {
-      KG_CUDA(cudaMemcpyAsync(h_sv.data(), sv.ptr, w * 8ull, cudaMemcpyDeviceToHost, s));
-      KG_CUDA(cudaMemcpyAsync(&h_info, info.ptr, 4, cudaMemcpyDeviceToHost, s));
+      KG_CUDA(cudaMemcpyAsync(h.data(), out.ptr, out.bytes(), cudaMemcpyDeviceToHost, s));
       KG_CUDA(cudaStreamSynchronize(s));
     };
-    if (qr) {
-      // Shifted CholeskyQR3 (rest = Q R: three Gram/Cholesky/triangular-solve rounds
-      // across the GPU), the SVD of R in one CTA, U = Q U_R; Householder QR in one CTA
-      // if a Cholesky pivot fails (a numerically rank-deficient block).
-      u.alloc((uint64_t)g * w, s);
-      DeviceBuffer<double> saved((uint64_t)g * w, s), gram((uint64_t)w * w, s),
-          rt((uint64_t)w * w, s), rtot((uint64_t)w * w, s), ur((uint64_t)w * w, s);
+    DeviceBuffer<double> u((uint64_t)g * w, s);
+    DeviceBuffer<uint32_t> order;
+    DeviceBuffer<double> saved;
+    if (narrow) {
+      saved.alloc((uint64_t)g * w, s);
       KG_CUDA(cudaMemcpyAsync(saved.ptr, rest.ptr, rest.bytes(), cudaMemcpyDeviceToDevice, s));
+      const uint64_t ww = (uint64_t)w * w;
+      DeviceBuffer<double> gram(ww, s), r3(3 * ww, s), ur(ww, s);
+      DeviceBuffer<int> info(1, s);
       info.zero();
       const double one = 1.0, zero = 0.0;
       const double shift = 11.0 * ((double)g * w + (double)w * (w + 1)) * 0x1p-53;
       for (int round = 0; round < 3; ++round) {
         KG_CUBLAS(cublasDgemm(p->cublas, CUBLAS_OP_T, CUBLAS_OP_N, w, w, g, &one, rest.ptr, g,
                               rest.ptr, g, &zero, gram.ptr, w));
-        cholesky_step_kernel<<<1, 1024, 0, s>>>(gram.ptr, w, round == 0 ? shift : 0.0,
-                                                round == 0, rt.ptr, rtot.ptr, info.ptr);
-        KG_LAUNCH_CHECK();
+        double* r = r3.ptr + round * ww;
+        cholesky_step(gram.ptr, w, round == 0 ? shift : 0.0, r, info.ptr, s);
         KG_CUBLAS(cublasDtrsm(p->cublas, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N,
-                              CUBLAS_DIAG_NON_UNIT, g, w, &one, rt.ptr, w, rest.ptr, g));
+                              CUBLAS_DIAG_NON_UNIT, g, w, &one, r, w, rest.ptr, g));
       }
-      small_svd_kernel<<<1, 1024, 0, s>>>(rtot.ptr, w, sv.ptr, ur.ptr, info.ptr);
-      KG_LAUNCH_CHECK();
+      small_svd(r3.ptr, w, block, (uint64_t)g * w, info.ptr, ur.ptr, out.ptr, s);
       KG_CUBLAS(cublasDgemm(p->cublas, CUBLAS_OP_N, CUBLAS_OP_N, g, w, w, &one, rest.ptr, g,
                             ur.ptr, w, &zero, u.ptr, g));
       read_back();
-      if (h_info != 0) {
-        KG_CUDA(cudaMemcpyAsync(rest.ptr, saved.ptr, rest.bytes(), cudaMemcpyDeviceToDevice, s));
-        info.zero();
-        qr_svd_kernel<<<1, 1024, 0, s>>>(rest.ptr, g, w, sv.ptr, u.ptr, info.ptr);
-        KG_LAUNCH_CHECK();
-        read_back();
-      }
     } else {
-      jacobi_svd_kernel<<<1, 1024, 0, s>>>(rest.ptr, g, w, sv.ptr, order.ptr, info.ptr);
+      order.alloc(w, s);
+      frobenius(block, (uint64_t)g * w, out.ptr + w, s);
+      jacobi_svd_kernel<<<1, 1024, 0, s>>>(rest.ptr, g, w, out.ptr, order.ptr, out.ptr + w + 1);
       KG_LAUNCH_CHECK();
       read_back();
     }
-    if (h_info != 0)
+    const double scale = h[w];
+    if (!(scale > 0.0)) {
+      if (std::isnan(scale)) fail(KG_ERR_INVALID, "pca: the Krylov block is not finite");
+      return none;
+    }
+    if (narrow && h[w + 1] != 0.0) {
+      qr_svd(saved.ptr, g, w, u.ptr, out.ptr, s);
+      read_back();
+    }
+    if (h[w + 1] != 0.0)
       fail(KG_ERR_INVALID, "pca: orthonormalising a Krylov block did not converge");
     uint32_t keep = 0;
-    while (keep < w && h_sv[keep] > kDropTolerance * scale) ++keep;
+    while (keep < w && h[keep] > kDropTolerance * scale) ++keep;
     *keep_out = keep;
     if (keep == 0) return none;
-    DeviceBuffer<double> out((uint64_t)g * keep, s);
-    if (qr) {
-      KG_CUDA(cudaMemcpyAsync(out.ptr, u.ptr, out.bytes(), cudaMemcpyDeviceToDevice, s));
-    } else {
+    if (!narrow) {
       gather_unit_columns_kernel<<<blocks_for((uint64_t)g * keep, 256), 256, 0, s>>>(
-          rest.ptr, g, keep, sv.ptr, order.ptr, out.ptr);
+          rest.ptr, g, keep, out.ptr, order.ptr, u.ptr);
       KG_LAUNCH_CHECK();
     }
-    return out;
+    return u;
   }
 
   void mean_dot(const double* m, const double* means, uint32_t w, double* out) {
