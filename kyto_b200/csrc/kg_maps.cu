@@ -12,16 +12,6 @@
 
 namespace kg {
 
-// Sets *flag when a u32 count is above 2^24 and not a float32 (elementwise.rs:241-257:
-// then every value of the block is rounded to float32 before the row sums).
-__global__ void inexact_counts_kernel(const uint32_t* values, uint64_t nnz, int* flag) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nnz;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t c = values[i];
-    if (c > (1u << 24) && (uint32_t)__uint2float_rn(c) != c) *flag = 1;
-  }
-}
-
 // The largest gene index of a block (a block's indices must be below its genes).
 __global__ void max_index_kernel(const uint32_t* idx, uint64_t nnz, unsigned int* out) {
   unsigned int m = 0;
@@ -30,6 +20,13 @@ __global__ void max_index_kernel(const uint32_t* idx, uint64_t nnz, unsigned int
     m = max(m, idx[i]);
   for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
   if ((threadIdx.x & 31u) == 0) atomicMax(out, m);
+}
+
+// Refuses a block whose largest gene index is `worst`.
+void check_worst_index(uint32_t worst, uint32_t n_genes) {
+  if (worst >= n_genes)
+    fail(KG_ERR_INVALID, "a block holds gene index " + std::to_string(worst) + " but has " +
+                             std::to_string(n_genes) + " genes");
 }
 
 void check_indices(const uint32_t* d_idx, uint64_t nnz, uint32_t n_genes, cudaStream_t s) {
@@ -42,68 +39,52 @@ void check_indices(const uint32_t* d_idx, uint64_t nnz, uint32_t n_genes, cudaSt
   unsigned int h = 0;
   KG_CUDA(cudaMemcpyAsync(&h, m.ptr, 4, cudaMemcpyDeviceToHost, s));
   KG_CUDA(cudaStreamSynchronize(s));
-  if (h >= n_genes)
-    fail(KG_ERR_INVALID, "a block holds gene index " + std::to_string(h) + " but has " +
-                             std::to_string(n_genes) + " genes");
+  check_worst_index(h, n_genes);
 }
 
-// 8 threads per row: the row's divisor (kg_maps.cuh) then its mapped values.
+// A warp per row: the row's divisor, its table (kg_maps.cuh), then its mapped values, four
+// loads in flight a lane. HBM-bound: 8 bytes a value (the second read of a row comes from
+// L2); 8,192 rows of 1,900 counts: 39 us, 3.2 TB/s (eight threads a row with a log1p a value
+// and a rounding pass before: 296 us).
+constexpr int kMapWarps = 8;
 template <class V>
-__global__ void normalize_log1p_kernel(const uint64_t* indptr, const V* values,
-                                       uint64_t n_rows, float target32, int normalize,
-                                       int do_log1p, const int* inexact, float* out) {
-  uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  uint64_t row = t >> 3;
-  unsigned c = threadIdx.x & 7u;
-  uint64_t s = 0, e = 0;
-  if (row < n_rows) {
-    s = indptr[row];
-    e = indptr[row + 1];
+__global__ void __launch_bounds__(kMapWarps * 32)
+normalize_log1p_kernel(const uint64_t* indptr, const V* __restrict__ values, uint64_t n_rows,
+                       float target32, int normalize, int do_log1p, float* __restrict__ out) {
+  __shared__ float tables[kMapWarps][kMapTable];
+  const uint64_t row = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const unsigned lane = threadIdx.x & 31u;
+  if (row >= n_rows) return;  // whole warps leave together
+  const uint64_t s = indptr[row], e = indptr[row + 1];
+  RowMap map{tables[threadIdx.x >> 5], 1.0f, normalize != 0, do_log1p != 0};
+  if (normalize) map.divisor = warp_row_divisor(values, s, e, target32);
+  map.fill();
+  uint64_t i = s + lane;
+  for (; i + 96 < e; i += 128) {
+    const V a = values[i], b = values[i + 32], c = values[i + 64], d = values[i + 96];
+    out[i] = map.at(a);
+    out[i + 32] = map.at(b);
+    out[i + 64] = map.at(c);
+    out[i + 96] = map.at(d);
   }
-  float divisor = 1.0f;
-  if (normalize) divisor = row_divisor(values, s, e, target32, inexact && *inexact);
-  for (uint64_t i = s + c; i < e; i += 8)
-    out[i] = mapped_value(values, i, normalize != 0, divisor, do_log1p != 0);
-}
-
-template <class V>
-void launch_normalize(const uint64_t* indptr, const void* values, uint64_t n_rows,
-                      double target_sum, int do_log1p, const int* inexact, float* out,
-                      cudaStream_t stream) {
-  bool normalize = !std::isnan(target_sum);
-  unsigned threads = 256;
-  normalize_log1p_kernel<V><<<blocks_for(n_rows * 8, threads), threads, 0, stream>>>(
-      indptr, (const V*)values, n_rows, (float)target_sum, normalize ? 1 : 0, do_log1p,
-      inexact, out);
-  KG_LAUNCH_CHECK();
-}
-
-// The device flag of inexact_counts_kernel for a block about to be normalized (left
-// unallocated, NULL, when no u32 count of the block can need rounding).
-void inexact_flag(const void* d_values, kg_dtype dtype, uint64_t nnz, double target_sum,
-                  DeviceBuffer<int>& flag, cudaStream_t stream) {
-  if (dtype != KG_U32 || std::isnan(target_sum) || !nnz) return;
-  flag.alloc(1, stream);
-  flag.zero();
-  unsigned threads = 256;
-  unsigned blocks = std::min<unsigned>(blocks_for(nnz, threads), 4096);
-  inexact_counts_kernel<<<blocks, threads, 0, stream>>>((const uint32_t*)d_values, nnz,
-                                                        flag.ptr);
-  KG_LAUNCH_CHECK();
+  for (; i < e; i += 32) out[i] = map.at(values[i]);
 }
 
 // Device f32 map outputs of a (device) CSR block.
 void map_block(const uint64_t* d_indptr, const void* d_values, kg_dtype dtype,
-               uint64_t n_rows, uint64_t nnz, double target_sum, int do_log1p,
-               float* d_out, cudaStream_t stream) {
-  DeviceBuffer<int> inexact;
-  inexact_flag(d_values, dtype, nnz, target_sum, inexact, stream);
+               uint64_t n_rows, double target_sum, int do_log1p, float* d_out,
+               cudaStream_t stream) {
+  if (!n_rows) return;
+  const int normalize = std::isnan(target_sum) ? 0 : 1;
+  const unsigned blocks = blocks_for(n_rows, kMapWarps);
   if (dtype == KG_U32)
-    launch_normalize<uint32_t>(d_indptr, d_values, n_rows, target_sum, do_log1p, inexact.ptr,
-                               d_out, stream);
+    normalize_log1p_kernel<uint32_t><<<blocks, kMapWarps * 32, 0, stream>>>(
+        d_indptr, (const uint32_t*)d_values, n_rows, (float)target_sum, normalize, do_log1p,
+        d_out);
   else
-    launch_normalize<float>(d_indptr, d_values, n_rows, target_sum, do_log1p, inexact.ptr,
-                            d_out, stream);
+    normalize_log1p_kernel<float><<<blocks, kMapWarps * 32, 0, stream>>>(
+        d_indptr, (const float*)d_values, n_rows, (float)target_sum, normalize, do_log1p, d_out);
+  KG_LAUNCH_CHECK();
 }
 
 // seurat's transformed value and its f32 square (hvg_pass.rs:189-206).
@@ -126,61 +107,362 @@ __global__ void column_starts_kernel(const uint32_t* sorted_genes, uint64_t nnz,
   colptr[g] = lo;
 }
 
-// One warp per gene, its cells in cell order: the bits of kyto's single-leaf fold (two
-// f64 sums in one fixed sequential order, made by lane 0). The other lanes keep the next
-// 128 values on their way while lane 0 folds the current 128 from shared memory, so the
-// fold's dependent adds, not the loads, set the pace; many genes' warps share an SM.
-constexpr int kMomentWarps = 4;
-constexpr int kMomentChunk = 128;
+// ----- The moments without a sort. seurat_rows_kernel maps the rows once (and notes where
+// each crosses from one group of genes to the next); group_moments_kernel then gives every
+// group of genes a CTA that walks all rows in order. A radix sort of (gene, value) pairs and
+// one chain a gene over the sorted values, behind separate map, expm1, range and rounding
+// passes, took 5.4 ms for 95M values of 20,000 genes; placing the values gene by gene with
+// scattered writes instead of the sort, 2.7 ms (23 four-byte writes a clock, all SMs); this,
+// 1.6 ms.
 
-__global__ void __launch_bounds__(kMomentWarps * 32)
-gene_moments_kernel(const uint64_t* colptr, const float* t, uint32_t n_genes, double* sums,
-                    double* squares, uint64_t* positives) {
-  __shared__ float buf[kMomentWarps][2][kMomentChunk];
-  const unsigned lane = threadIdx.x & 31u, wi = threadIdx.x >> 5;
-  const uint32_t g = blockIdx.x * kMomentWarps + wi;
-  if (g >= n_genes) return;
-  const uint64_t a = colptr[g], e = colptr[g + 1];
-  float nxt[kMomentChunk / 32];
-  auto load = [&](uint64_t c0) {
+enum : int { kFlagWorst = 0, kFlagUnsorted = 1, kFlagWide = 2, kFlags = 3 };
+constexpr int kSeuratThreads = 256;       // 32 rows, four a warp
+constexpr uint32_t kGroupsMax = 1024;     // groups of genes (their bounds a shared-memory tile)
+
+__device__ __forceinline__ float seurat_value(float mapped) { return (float)expm1((double)mapped); }
+
+// t[i] = seurat's f32(expm1(f64(mapped value))) of every stored value; bounds[(k - 1) * n_rows
+// + row] = the row's first entry of a gene in group k >= 1 (group_genes genes each) or later;
+// flags: [kFlagWorst] the largest gene index at or past n_genes (0: none), [kFlagUnsorted]
+// set by a row whose genes do not increase strictly, [kFlagWide] set by a seurat value that
+// is not 0 nor of a magnitude in [2^-28, 2^60). HBM-bound: 8 bytes a value in, 4 out.
+template <class V>
+__global__ void __launch_bounds__(kSeuratThreads, 5)
+seurat_rows_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
+                   const V* __restrict__ values, uint64_t n_rows, uint32_t n_genes,
+                   uint32_t magic, uint32_t groups, int normalize,
+                   float target32, int do_log1p, float* __restrict__ t, uint32_t* bounds, unsigned int* flags) {
+  __shared__ float tables[kSeuratThreads / 32][kMapTable];
+  extern __shared__ uint32_t crossing[];  // [groups - 1][33]
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint64_t rb = blockIdx.x * 32ull;
+  for (uint32_t rr = warp; rr < 32 && rb + rr < n_rows; rr += kSeuratThreads / 32) {
+    const uint64_t r = rb + rr;
+    const uint64_t s = indptr[r], e = indptr[r + 1];
+    RowMap map{tables[warp], 1.0f, normalize != 0, do_log1p != 0};
+    if (normalize) map.divisor = warp_row_divisor(values, s, e, target32);
+    __syncwarp();
+    for (uint32_t c = lane; c < kMapTable; c += 32)
+      map.table[c] = seurat_value(mapped_f32((float)c, map.normalize, map.divisor, map.do_log1p));
+    __syncwarp();
+    // gene / group_genes: exact for genes below 2^24 (magic = ceil(2^32 / group_genes), a
+    // divisor of at most 2^8); a gene out of range may land in any group.
+    auto group_of = [&](uint32_t gene) { return min(__umulhi(gene, magic), groups - 1); };
+    const uint32_t* row_idx = idx + s;
+    const V* row_values = values + s;
+    float* row_t = t + s;
+    const uint32_t len = (uint32_t)(e - s), at = (uint32_t)s;
+    bool unsorted = false, wide = false;
+    uint32_t worst = 0, carry = 0;  // carry: the gene before the chunk's first
+    for (uint32_t j0 = 0; j0 < len; j0 += 128) {
+      uint32_t gene[4];
+      V v[4];
 #pragma unroll
-    for (int m = 0; m < kMomentChunk / 32; ++m) {
-      const uint64_t i = c0 + m * 32 + lane;
-      nxt[m] = i < e ? __ldg(t + i) : 0.0f;
-    }
-  };
-  auto stash = [&](int half) {
+      for (int m = 0; m < 4; ++m) {
+        const uint32_t j = j0 + 32 * m + lane;
+        gene[m] = j < len ? row_idx[j] : 0;
+        v[m] = j < len ? row_values[j] : V(0);
+      }
 #pragma unroll
-    for (int m = 0; m < kMomentChunk / 32; ++m) buf[wi][half][m * 32 + lane] = nxt[m];
-  };
-  double s = 0.0, q = 0.0;
-  uint64_t p = 0;
-  load(a);
-  stash(0);
-  __syncwarp();
-  int half = 0;
-  for (uint64_t c0 = a; c0 < e; c0 += kMomentChunk, half ^= 1) {
-    if (c0 + kMomentChunk < e) load(c0 + kMomentChunk);
-    if (lane == 0) {
-      const uint32_t n = e - c0 < (uint64_t)kMomentChunk ? (uint32_t)(e - c0) : (uint32_t)kMomentChunk;
-      const float* v = buf[wi][half];
-#pragma unroll 8
-      for (uint32_t j = 0; j < n; ++j) {
-        const float x = v[j];
-        if (x > 0.0f) ++p;  // t > 0 exactly when the log1p value > 0 (expm1 keeps sign)
-        s = __dadd_rn(s, (double)x);
-        q = __dadd_rn(q, (double)__fmul_rn(x, x));
+      for (int m = 0; m < 4; ++m) {
+        const uint32_t j = j0 + 32 * m + lane;
+        uint32_t before = __shfl_up_sync(0xFFFFFFFFu, gene[m], 1);
+        if (lane == 0) before = carry;
+        carry = __shfl_sync(0xFFFFFFFFu, gene[m], 31);
+        if (j >= len) continue;
+        unsorted |= j > 0 && before >= gene[m];
+        worst = max(worst, gene[m]);
+        // The groups whose first entry this is: those after the previous entry's.
+        const uint32_t to = group_of(gene[m]);
+        for (uint32_t k = j > 0 ? group_of(before) : 0; k < to; ++k) crossing[k * 33 + rr] = at + j;
+        uint32_t c;
+        const float x = map_tabled(v[m], c)
+                            ? map.table[c]
+                            : seurat_value(mapped_f32(to_f32(v[m]), map.normalize, map.divisor,
+                                                      map.do_log1p));
+        wide |= x != 0.0f && !(fabsf(x) >= 0x1p-28f && fabsf(x) < 0x1p60f);
+        row_t[j] = x;
       }
     }
-    __syncwarp();
-    if (c0 + kMomentChunk < e) stash(half ^ 1);
+    for (uint32_t k = (len ? group_of(row_idx[len - 1]) : 0) + lane; k + 1 < groups; k += 32)
+      crossing[k * 33 + rr] = at + len;
+    if (worst >= n_genes) atomicMax(flags + kFlagWorst, worst);
+    if (__any_sync(0xFFFFFFFFu, unsorted) && lane == 0) flags[kFlagUnsorted] = 1;
+    if (__any_sync(0xFFFFFFFFu, wide) && lane == 0) flags[kFlagWide] = 1;
+  }
+  __syncthreads();
+  for (uint32_t k = 1 + warp; k < groups; k += kSeuratThreads / 32)
+    if (rb + lane < n_rows) bounds[(uint64_t)(k - 1) * n_rows + rb + lane] = crossing[(k - 1) * 33 + lane];
+}
+
+// The moments of group blockIdx.x's genes: the bits of kyto's single-leaf fold (per gene two
+// f64 sums, each in cell order). Rows come through a ring of kRing dense tiles of kTileRows
+// rows x the group's genes in shared memory (f32, zeros where a row holds nothing: adding
+// them changes no sum). kRing teams of loading warps fill every kRing-th tile each: zeros,
+// the rows' entries, so their loads' latency spreads over as many tiles' time. The chain warps, a
+// gene a lane, then add a tile's rows in order.
+// The chains' instructions bound it: per row and lane two dependent f64 additions and the
+// conversions before them, one through the conversion unit (16 lanes a clock an SM), the
+// square's by shifting its bits. That shift reads an f32 zero as 2^-127, which any real
+// square added to it swallows while every nonzero value is at least 2^-28 (a gene of no
+// nonzero value is put right at the end); a block with other values converts both.
+constexpr int kTileRows = 32;
+constexpr int kRing = 7;               // two named barriers a slot, 15 in all
+constexpr int kTeamWarps = 2;
+constexpr int kLoadWarps = kRing * kTeamWarps;
+constexpr uint32_t kGroupGenes = 192;  // at most (6 chain warps)
+constexpr int kRowsAWarp = kTileRows / kTeamWarps;
+
+__device__ __forceinline__ double widen_square(float v) {
+  const uint32_t b = __float_as_uint(v);
+  return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+}
+
+__global__ void __launch_bounds__(kLoadWarps * 32 + kGroupGenes, 1)
+group_moments_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
+                     const float* __restrict__ t, uint64_t n_rows, uint32_t n_genes,
+                     uint32_t group_genes, uint32_t groups, const uint32_t* __restrict__ bounds,
+                     const unsigned int* flags, double* sums, double* squares,
+                     uint64_t* positives) {
+  extern __shared__ float tiles[];  // [kRing][kTileRows][group_genes], then two counts a gene
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t k = blockIdx.x, g0 = k * group_genes;
+  const uint32_t genes = min(group_genes, n_genes - g0);
+  const uint64_t n_tiles = (n_rows + kTileRows - 1) / kTileRows;
+  const uint32_t tile_floats = kTileRows * group_genes;
+  uint32_t* n_positive = reinterpret_cast<uint32_t*>(tiles + kRing * tile_floats);
+  uint32_t* n_other = n_positive + group_genes;
+  for (uint32_t x = threadIdx.x; x < 2 * group_genes; x += blockDim.x) n_positive[x] = 0;
+  __syncthreads();
+  // Barrier 1 + slot: a filled tile (its team arrives, the chain warps wait); barrier 1 +
+  // kRing + slot: an emptied one (the other way round).
+  const uint32_t both = kTeamWarps * 32 + group_genes;
+  if (warp < kLoadWarps) {
+    const uint32_t slot = warp / kTeamWarps, member = warp % kTeamWarps;
+    const uint32_t half = lane >> 4, l = lane & 15u;  // two rows at a time
+    float* rows = tiles + slot * tile_floats + member * kRowsAWarp * group_genes;
+    auto put = [&](uint32_t row, uint32_t gene, float v) {
+      if (gene >= genes) return;
+      rows[row * group_genes + gene] = v;
+      // t > 0 exactly when the log1p value > 0.
+      if (v != 0.0f) atomicAdd((v > 0.0f ? n_positive : n_other) + gene, 1u);
+    };
+    // A row's range: lane j the warp's row j of tile b.
+    auto ranges = [&](uint64_t b, uint32_t& from, uint32_t& to) {
+      const uint64_t r = b * kTileRows + member * kRowsAWarp + lane;
+      from = to = 0;
+      if (lane < kRowsAWarp && r < n_rows) {
+        from = k == 0 ? (uint32_t)indptr[r] : bounds[(uint64_t)(k - 1) * n_rows + r];
+        to = k + 1 == groups ? (uint32_t)indptr[r + 1] : bounds[(uint64_t)k * n_rows + r];
+      }
+    };
+    uint32_t next_lo = 0, next_hi = 0;
+    ranges(slot, next_lo, next_hi);
+    for (uint64_t b = slot; b < n_tiles; b += kRing) {
+      // The warp's rows' entries (and the next tile's ranges), before the tile is free.
+      const uint32_t lo = next_lo, hi = next_hi;
+      uint32_t gene[kRowsAWarp / 2][2];
+      float v[kRowsAWarp / 2][2];
+      bool more = false;
+#pragma unroll
+      for (int j = 0; j < kRowsAWarp / 2; ++j) {
+        const uint32_t a = __shfl_sync(0xFFFFFFFFu, lo, 2 * j + half) + l;
+        const uint32_t e = __shfl_sync(0xFFFFFFFFu, hi, 2 * j + half);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const bool in = a < e && e - a > 16u * m;
+          gene[j][m] = in ? idx[a + 16 * m] - g0 : 0xFFFFFFFFu;
+          v[j][m] = in ? t[a + 16 * m] : 0.0f;
+        }
+        more |= a < e && e - a > 32;
+      }
+      ranges(b + kRing, next_lo, next_hi);
+      if (b >= kRing) asm volatile("bar.sync %0, %1;" ::"r"(1 + kRing + slot), "r"(both) : "memory");
+      for (uint32_t x = lane * 4; x < kRowsAWarp * group_genes; x += 128)
+        *reinterpret_cast<float4*>(rows + x) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < kRowsAWarp / 2; ++j)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) put(2 * j + half, gene[j][m], v[j][m]);
+      if (__any_sync(0xFFFFFFFFu, more)) {  // a row of over 32 values in the group
+        for (int j = 0; j < kRowsAWarp / 2; ++j) {
+          const uint32_t a = __shfl_sync(0xFFFFFFFFu, lo, 2 * j + half) + 32 + l;
+          const uint32_t e = __shfl_sync(0xFFFFFFFFu, hi, 2 * j + half);
+          for (uint32_t i = a; i < e; i += 16) put(2 * j + half, idx[i] - g0, t[i]);
+        }
+      }
+      asm volatile("bar.arrive %0, %1;" ::"r"(1 + slot), "r"(both) : "memory");
+    }
+    __syncthreads();
+  } else {
+    const uint32_t c = threadIdx.x - kLoadWarps * 32;  // < group_genes (the block's size)
+    const bool wide = flags[kFlagWide] != 0;
+    double s = 0.0, q = 0.0;
+    for (uint64_t b = 0; b < n_tiles; ++b) {
+      const uint32_t slot = (uint32_t)(b % kRing);
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(both) : "memory");
+      const float* at = tiles + slot * tile_floats + c;
+      for (int r0 = 0; r0 < kTileRows; r0 += 16) {
+        float x[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) x[r] = at[(r0 + r) * group_genes];
+        if (!wide) {
+#pragma unroll
+          for (int r = 0; r < 16; ++r) {
+            s = __dadd_rn(s, (double)x[r]);
+            q = __dadd_rn(q, widen_square(__fmul_rn(x[r], x[r])));
+          }
+        } else {
+#pragma unroll
+          for (int r = 0; r < 16; ++r) {
+            s = __dadd_rn(s, (double)x[r]);
+            q = __dadd_rn(q, (double)__fmul_rn(x[r], x[r]));
+          }
+        }
+      }
+      if (b + kRing < n_tiles)
+        asm volatile("bar.arrive %0, %1;" ::"r"(1 + kRing + slot), "r"(both) : "memory");
+    }
+    __syncthreads();
+    if (c < genes) {
+      sums[g0 + c] = s;
+      squares[g0 + c] = n_positive[c] + n_other[c] ? q : 0.0;
+      positives[g0 + c] = n_positive[c];
+    }
+  }
+}
+
+// ----- The moments of values already sorted by gene.
+
+// A warp per four genes, their cells in cell order: the bits of kyto's single-leaf fold (two
+// f64 sums a gene, each in one fixed sequential order). The lanes bring the next 64 values
+// of each gene and leave them, and their squares, in shared memory as f64 while the eight
+// sums (lane modulo 8) run over the 64 before: a chain of dependent additions each, with the
+// conversions between them. The longest gene's chain bounds it (8.5 cycles an addition; one
+// lane converting, squaring and adding both sums took 94 cycles a value, 2.45 ms for genes of
+// 50,000 cells).
+constexpr int kMomentWarps = 4;
+constexpr int kMomentGenes = 4;
+constexpr int kMomentChunk = 64;
+
+__global__ void __launch_bounds__(kMomentWarps * 32)
+gene_moments_kernel(const uint64_t* colptr, const float* __restrict__ t, uint32_t n_genes,
+                    double* sums, double* squares, uint64_t* positives) {
+  constexpr int kParts = kMomentChunk / 32;
+  // Rows of 16-byte multiples whose starts fall on different banks.
+  __shared__ __align__(16) double buf[kMomentWarps][2][2 * kMomentGenes][kMomentChunk + 2];
+  const unsigned lane = threadIdx.x & 31u, wi = threadIdx.x >> 5;
+  const uint32_t g0 = (blockIdx.x * kMomentWarps + wi) * kMomentGenes;
+  if (g0 >= n_genes) return;
+  uint64_t at[kMomentGenes], end[kMomentGenes], longest = 0;
+  uint32_t p[kMomentGenes];
+#pragma unroll
+  for (int k = 0; k < kMomentGenes; ++k) {
+    const bool in = g0 + k < n_genes;
+    at[k] = in ? colptr[g0 + k] : 0;
+    end[k] = in ? colptr[g0 + k + 1] : 0;
+    longest = max(longest, end[k] - at[k]);
+    p[k] = 0;
+  }
+  float x[kMomentGenes * kParts];
+  auto load = [&]() {
+#pragma unroll
+    for (int k = 0; k < kMomentGenes; ++k) {
+#pragma unroll
+      for (int m = 0; m < kParts; ++m) {
+        const uint64_t i = at[k] + m * 32 + lane;
+        x[k * kParts + m] = i < end[k] ? t[i] : 0.0f;  // past the gene: adds nothing
+      }
+      at[k] += kMomentChunk;
+    }
+  };
+  auto stash = [&](int half, int q) {  // value q of x
+    const int k = q / kParts, m = q % kParts;
+    const float v = x[q];
+    buf[wi][half][2 * k][m * 32 + lane] = (double)v;
+    buf[wi][half][2 * k + 1][m * 32 + lane] = (double)__fmul_rn(v, v);
+    p[k] += v > 0.0f ? 1u : 0u;  // t > 0 exactly when the log1p value > 0
+  };
+  constexpr int kHeld = kMomentGenes * kParts;
+  const unsigned chain = lane % (2 * kMomentGenes);  // gene chain / 2, its sum or its squares
+  double acc = 0.0;
+  load();
+#pragma unroll
+  for (int q = 0; q < kHeld; ++q) stash(0, q);
+  load();
+  __syncwarp();
+  int half = 0;
+  for (uint64_t done = 0; done < longest; done += kMomentChunk, half ^= 1) {
+    const double2* row = reinterpret_cast<const double2*>(buf[wi][half][chain]);
+#pragma unroll
+    for (int q = 0; q < kHeld; ++q) {
+#pragma unroll
+      for (int j = 0; j < kMomentChunk / 2 / kHeld; ++j) {
+        const double2 d = lane < 2 * kMomentGenes ? row[q * (kMomentChunk / 2 / kHeld) + j]
+                                                  : make_double2(0.0, 0.0);
+        acc = __dadd_rn(acc, d.x);
+        acc = __dadd_rn(acc, d.y);
+      }
+      stash(half ^ 1, q);
+    }
+    load();
     __syncwarp();
   }
-  if (lane == 0) {
-    sums[g] = s;
-    squares[g] = q;
-    positives[g] = p;
+#pragma unroll
+  for (int k = 0; k < kMomentGenes; ++k) {
+    uint32_t c = p[k];
+    for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
+    if (lane == 0 && g0 + k < n_genes) positives[g0 + k] = c;
   }
+  const uint32_t g = g0 + chain / 2;
+  if (lane < 2 * kMomentGenes && g < n_genes) ((chain & 1u) ? squares : sums)[g] = acc;
+}
+
+void gene_moments(const uint64_t* colptr, const float* t, uint32_t n_genes, double* sums,
+                  double* squares, uint64_t* positives, cudaStream_t s) {
+  if (!n_genes) return;
+  const uint32_t per = kMomentWarps * kMomentGenes;
+  gene_moments_kernel<<<(n_genes + per - 1) / per, kMomentWarps * 32, 0, s>>>(
+      colptr, t, n_genes, sums, squares, positives);
+  KG_LAUNCH_CHECK();
+}
+
+// The moments of a block whose rows hold their genes in strictly increasing order, without a
+// sort; false (and nothing queued) for a shape outside the kernels' (more groups of genes than
+// their bounds' tile holds). The flags are read by the caller once its work is queued: a
+// block with an index out of range or an unsorted row leaves the moments meaningless (every
+// access stays inside the arrays).
+template <class V>
+bool moments_by_group(const uint64_t* indptr, const uint32_t* idx, const V* values,
+                      uint64_t n_rows, uint64_t nnz, uint32_t n_genes, double target_sum,
+                      int do_log1p, int sm_count, double* sums, double* squares,
+                      uint64_t* positives, unsigned int* flags, cudaStream_t s) {
+  // About a group an SM, in whole warps of genes.
+  const uint32_t gg =
+      std::min(kGroupGenes, ((n_genes + sm_count - 1) / sm_count + 31) / 32 * 32);
+  const uint32_t groups = (n_genes + gg - 1) / gg;
+  if (groups > kGroupsMax) return false;
+  static std::once_flag attr;
+  std::call_once(attr, [] {
+    KG_CUDA(cudaFuncSetAttribute(seurat_rows_kernel<V>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(kGroupsMax * 33 * 4)));
+    KG_CUDA(cudaFuncSetAttribute(group_moments_kernel,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)((kRing * kTileRows + 2) * kGroupGenes * 4)));
+  });
+  DeviceBuffer<float> t(nnz, s);
+  DeviceBuffer<uint32_t> bounds((uint64_t)(groups - 1) * n_rows, s);
+  seurat_rows_kernel<V><<<blocks_for(n_rows, 32), kSeuratThreads, (groups - 1) * 33 * 4, s>>>(
+      indptr, idx, values, n_rows, n_genes, (uint32_t)(((1ull << 32) + gg - 1) / gg), groups,
+      std::isnan(target_sum) ? 0 : 1, (float)target_sum, do_log1p, t.ptr, bounds.ptr, flags);
+  KG_LAUNCH_CHECK();
+  group_moments_kernel<<<groups, kLoadWarps * 32 + gg, (kRing * kTileRows + 2) * gg * 4, s>>>(
+      indptr, idx, t.ptr, n_rows, n_genes, gg, groups, bounds.ptr, flags, sums, squares,
+      positives);
+  KG_LAUNCH_CHECK();
+  return true;
 }
 
 int bits_for(uint32_t n) {
@@ -268,19 +550,22 @@ kg_status kg_normalize_log1p(kg_ctx* ctx, const uint64_t* indptr, const void* va
     cudaStream_t s = ctx->stream;
     DeviceBuffer<uint64_t> hp;
     const uint64_t* d_indptr = device_view(indptr, n_rows + 1, hp, s);
+    // The stored values' count is needed for host arrays only (the kernel reads the offsets).
+    const bool out_dev = is_device_pointer(out);
     uint64_t nnz = 0;
-    KG_CUDA(cudaMemcpyAsync(&nnz, d_indptr + n_rows, 8, cudaMemcpyDefault, s));
-    KG_CUDA(cudaStreamSynchronize(s));
+    if (!out_dev || (values && !is_device_pointer(values))) {
+      KG_CUDA(cudaMemcpyAsync(&nnz, indptr + n_rows, 8, cudaMemcpyDefault, s));
+      KG_CUDA(cudaStreamSynchronize(s));
+    }
     DeviceBuffer<uint32_t> hv;
     const void* d_values = device_view((const uint32_t*)values, nnz, hv, s);
     DeviceBuffer<float> ho;
-    bool out_dev = is_device_pointer(out);
     float* d_out = out;
     if (!out_dev) {
       ho.alloc(nnz, s);
       d_out = ho.ptr;
     }
-    map_block(d_indptr, d_values, dtype, n_rows, nnz, target_sum, log1p, d_out, s);
+    map_block(d_indptr, d_values, dtype, n_rows, target_sum, log1p, d_out, s);
     if (!out_dev && nnz)
       KG_CUDA(cudaMemcpyAsync(out, d_out, nnz * 4, cudaMemcpyDeviceToHost, s));
     wait_stream(ctx, s);
@@ -305,27 +590,47 @@ kg_status kg_hvg_moments(kg_ctx* ctx, const uint64_t* indptr, const uint32_t* in
     DeviceBuffer<uint32_t> hi, hv;
     const uint32_t* d_idx = device_view(indices, nnz, hi, s);
     const void* d_values = device_view((const uint32_t*)values, nnz, hv, s);
-    check_indices(d_idx, nnz, n_genes, s);
-    DeviceBuffer<float> mapped(nnz, s), t(nnz, s);
-    map_block(d_indptr, d_values, dtype, n_rows, nnz, target_sum, log1p, mapped.ptr, s);
-    if (nnz) {
-      unsigned blocks = std::min<unsigned>(blocks_for(nnz, 256), 8192);
-      expm1_kernel<<<blocks, 256, 0, s>>>(mapped.ptr, nnz, t.ptr);
-      KG_LAUNCH_CHECK();
-    }
-    mapped.reset();
-    DeviceBuffer<uint32_t> genes_sorted, t_sorted;
-    sort_by_gene<uint32_t>(d_idx, (const uint32_t*)t.ptr, nnz, n_genes, genes_sorted,
-                           t_sorted, s);
-    t.reset();
-    DeviceBuffer<uint64_t> colptr((uint64_t)n_genes + 1, s);
-    column_starts(genes_sorted.ptr, nnz, n_genes, colptr.ptr, s);
     DeviceBuffer<double> dsum(n_genes, s), dsq(n_genes, s);
     DeviceBuffer<uint64_t> dpos(n_genes, s);
-    gene_moments_kernel<<<(n_genes + kMomentWarps - 1) / kMomentWarps, kMomentWarps * 32, 0,
-                          s>>>(colptr.ptr, (const float*)t_sorted.ptr, n_genes, dsum.ptr,
-                               dsq.ptr, dpos.ptr);
-    KG_LAUNCH_CHECK();
+    // Rows of strictly increasing genes (kyto's) need no sort; a block with any other row,
+    // found on the way, is sorted.
+    bool sorted = nnz > 0 && n_genes > 0 && nnz <= (uint64_t)std::numeric_limits<int>::max();
+    if (sorted) {
+      DeviceBuffer<unsigned int> flags(kFlags, s);
+      flags.zero();
+      if (dtype == KG_U32)
+        sorted = moments_by_group(d_indptr, d_idx, (const uint32_t*)d_values, n_rows, nnz,
+                                  n_genes, target_sum, log1p, ctx->sm_count, dsum.ptr, dsq.ptr,
+                                  dpos.ptr, flags.ptr, s);
+      else
+        sorted = moments_by_group(d_indptr, d_idx, (const float*)d_values, n_rows, nnz, n_genes,
+                                  target_sum, log1p, ctx->sm_count, dsum.ptr, dsq.ptr, dpos.ptr,
+                                  flags.ptr, s);
+      if (sorted) {
+        unsigned int h[kFlags] = {};
+        KG_CUDA(cudaMemcpyAsync(h, flags.ptr, sizeof h, cudaMemcpyDeviceToHost, s));
+        wait_stream(ctx, s);
+        check_worst_index(h[kFlagWorst], n_genes);
+        sorted = h[kFlagUnsorted] == 0;
+      }
+    }
+    if (!sorted) {
+      check_indices(d_idx, nnz, n_genes, s);
+      DeviceBuffer<float> t(nnz, s);
+      map_block(d_indptr, d_values, dtype, n_rows, target_sum, log1p, t.ptr, s);
+      if (nnz) {
+        unsigned blocks = std::min<unsigned>(blocks_for(nnz, 256), 8192);
+        expm1_kernel<<<blocks, 256, 0, s>>>(t.ptr, nnz, t.ptr);
+        KG_LAUNCH_CHECK();
+      }
+      DeviceBuffer<uint32_t> genes_sorted, t_sorted;
+      sort_by_gene<uint32_t>(d_idx, (const uint32_t*)t.ptr, nnz, n_genes, genes_sorted,
+                             t_sorted, s);
+      DeviceBuffer<uint64_t> colptr((uint64_t)n_genes + 1, s);
+      column_starts(genes_sorted.ptr, nnz, n_genes, colptr.ptr, s);
+      gene_moments(colptr.ptr, (const float*)t_sorted.ptr, n_genes, dsum.ptr, dsq.ptr, dpos.ptr,
+                   s);
+    }
     KG_CUDA(cudaMemcpyAsync(sums, dsum.ptr, n_genes * 8ull, cudaMemcpyDefault, s));
     KG_CUDA(cudaMemcpyAsync(sums_of_squares, dsq.ptr, n_genes * 8ull, cudaMemcpyDefault, s));
     KG_CUDA(cudaMemcpyAsync(positives, dpos.ptr, n_genes * 8ull, cudaMemcpyDefault, s));
@@ -445,7 +750,7 @@ namespace kg {
 constexpr size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // The limits of kg_hvg_moments_noalloc and the layout of its scratch (byte offsets):
-// two flags, the sort's key and payload double buffers, the per-gene arrays, the radix
+// the largest index, the sort's key and payload double buffers, the per-gene arrays, the radix
 // sort's temporary storage. 22.1 MB in all.
 constexpr uint64_t kNoAllocMaxValues = 1ull << 20;  // stored values of one block
 constexpr uint32_t kNoAllocMaxGenes = 1u << 16;
@@ -523,8 +828,7 @@ kg_status kg_hvg_moments_noalloc(kg_ctx* ctx, const uint64_t* indptr, const uint
                                std::to_string(kNoAllocMaxValues) + " (use kg_hvg_moments)");
     if (nnz && (!is_device_pointer(indices) || !is_device_pointer(values)))
       fail(KG_ERR_INVALID, "kg_hvg_moments_noalloc: indices and values must be device memory");
-    int* inexact = (int*)base;
-    unsigned int* max_index = (unsigned int*)(base + 4);
+    unsigned int* max_index = (unsigned int*)base;
     uint32_t* keys0 = (uint32_t*)(base + kNoAllocKeys0);
     uint32_t* keys1 = (uint32_t*)(base + kNoAllocKeys1);
     float* vals0 = (float*)(base + kNoAllocVals0);
@@ -533,7 +837,7 @@ kg_status kg_hvg_moments_noalloc(kg_ctx* ctx, const uint64_t* indptr, const uint
     double* dsum = (double*)(base + kNoAllocSums);
     double* dsq = (double*)(base + kNoAllocSquares);
     uint64_t* dpos = (uint64_t*)(base + kNoAllocPositives);
-    KG_CUDA(cudaMemsetAsync(base, 0, 8, s));  // both flags start at zero
+    KG_CUDA(cudaMemsetAsync(base, 0, 8, s));
     cub::DoubleBuffer<uint32_t> keys(keys0, keys1), vals((uint32_t*)vals0, (uint32_t*)vals1);
     if (nnz) {
       unsigned blocks = std::min<unsigned>(blocks_for(nnz, 256), 4096);
@@ -542,19 +846,8 @@ kg_status kg_hvg_moments_noalloc(kg_ctx* ctx, const uint64_t* indptr, const uint
       unsigned int h = 0;
       KG_CUDA(cudaMemcpyAsync(&h, max_index, 4, cudaMemcpyDeviceToHost, s));
       KG_CUDA(cudaStreamSynchronize(s));
-      if (h >= n_genes)
-        fail(KG_ERR_INVALID, "a block holds gene index " + std::to_string(h) + " but has " +
-                                 std::to_string(n_genes) + " genes");
-      const int* flag = nullptr;
-      if (dtype == KG_U32 && !std::isnan(target_sum)) {
-        inexact_counts_kernel<<<blocks, 256, 0, s>>>((const uint32_t*)values, nnz, inexact);
-        KG_LAUNCH_CHECK();
-        flag = inexact;
-      }
-      if (dtype == KG_U32)
-        launch_normalize<uint32_t>(indptr, values, n_rows, target_sum, log1p, flag, vals0, s);
-      else
-        launch_normalize<float>(indptr, values, n_rows, target_sum, log1p, flag, vals0, s);
+      check_worst_index(h, n_genes);
+      map_block(indptr, values, dtype, n_rows, target_sum, log1p, vals0, s);
       expm1_kernel<<<std::min<unsigned>(blocks_for(nnz, 256), 8192), 256, 0, s>>>(vals0, nnz,
                                                                                  vals0);
       KG_LAUNCH_CHECK();
@@ -573,9 +866,7 @@ kg_status kg_hvg_moments_noalloc(kg_ctx* ctx, const uint64_t* indptr, const uint
     }
     if (n_genes) {
       column_starts(keys.Current(), nnz, n_genes, colptr, s);
-      gene_moments_kernel<<<(n_genes + kMomentWarps - 1) / kMomentWarps, kMomentWarps * 32, 0,
-                            s>>>(colptr, (const float*)vals.Current(), n_genes, dsum, dsq, dpos);
-      KG_LAUNCH_CHECK();
+      gene_moments(colptr, (const float*)vals.Current(), n_genes, dsum, dsq, dpos, s);
       KG_CUDA(cudaMemcpyAsync(sums, dsum, n_genes * 8ull, cudaMemcpyDefault, s));
       KG_CUDA(cudaMemcpyAsync(sums_of_squares, dsq, n_genes * 8ull, cudaMemcpyDefault, s));
       KG_CUDA(cudaMemcpyAsync(positives, dpos, n_genes * 8ull, cudaMemcpyDefault, s));

@@ -8,10 +8,6 @@
 namespace kg {
 
 // A stored value as kyto's KernelValue reads it (crates/kyto-exec/src/kernels.rs:48-90).
-__device__ __forceinline__ float value_f32(const uint32_t* v, uint64_t i) {
-  return __uint2float_rn(v[i]);  // Rust `as f32`: round to nearest even
-}
-__device__ __forceinline__ float value_f32(const float* v, uint64_t i) { return v[i]; }
 __device__ __forceinline__ double value_wide(const uint32_t* v, uint64_t i, bool round32) {
   return round32 ? (double)__uint2float_rn(v[i]) : (double)v[i];
 }
@@ -53,13 +49,85 @@ __device__ __forceinline__ float row_divisor(const V* values, uint64_t s, uint64
 __device__ __forceinline__ float log1p_f32(float x) { return (float)log1p((double)x); }
 
 // One stored value after the maps: f32(v) / divisor (IEEE division), then log1p.
-template <class V>
-__device__ __forceinline__ float mapped_value(const V* values, uint64_t i, bool normalize,
-                                              float divisor, bool do_log1p) {
-  float v = value_f32(values, i);
+__device__ __forceinline__ float mapped_f32(float v, bool normalize, float divisor, bool do_log1p) {
   if (normalize) v = __fdiv_rn(v, divisor);
   if (do_log1p) v = log1p_f32(v);
   return v;
 }
+// Rust's `as f32`: round to nearest even.
+__device__ __forceinline__ float to_f32(uint32_t v) { return __uint2float_rn(v); }
+__device__ __forceinline__ float to_f32(float v) { return v; }
+
+// Counts are mostly small whole numbers and a row's values share one divisor, so a row's
+// maps are a table of its first kMapTable counts, one f64 log1p an entry instead of one a
+// stored value (a block of 8,192 x 1,900 counts: 264 us with a log1p a value, bound by the
+// FP64 pipe). Whether v is in the table (f32 -0 is not: its maps keep the sign).
+constexpr uint32_t kMapTable = 64;
+__device__ __forceinline__ bool map_tabled(uint32_t v, uint32_t& c) {
+  c = v;
+  return v < kMapTable;
+}
+__device__ __forceinline__ bool map_tabled(float v, uint32_t& c) {
+  c = (uint32_t)v;
+  return v < (float)kMapTable && (float)c == v && __float_as_uint(v) != 0x80000000u;
+}
+
+// A whole value's place in an exact sum (false for a value that is not a whole number up to
+// 2^24); u32 counts above 2^24 as kyto sums them, rounded to f32 (elementwise.rs:241-257
+// rounds a block's values when one of them is not an f32; the others do not change).
+__device__ __forceinline__ bool whole_value(uint32_t v, unsigned long long& out) {
+  out = v <= (1u << 24) ? v : (unsigned long long)__uint2float_rn(v);
+  return true;
+}
+__device__ __forceinline__ bool whole_value(float v, unsigned long long& out) {
+  out = (uint32_t)v;
+  return v >= 0.0f && v <= 16777216.0f && (float)(uint32_t)v == v;
+}
+
+// The normalize divisor of the row [s, e), by a whole warp (every lane gets it). Whole
+// numbers whose sum stays below 2^53 add up exactly in any order, so the lanes sum integers;
+// any other row takes kyto's order (row_divisor: eight chains of dependent f64 additions).
+template <class V>
+__device__ __forceinline__ float warp_row_divisor(const V* values, uint64_t s, uint64_t e,
+                                                  float target32) {
+  const unsigned lane = threadIdx.x & 31u;
+  unsigned long long sum = 0;
+  bool whole = true;
+  auto add = [&](V v) {
+    unsigned long long w;
+    whole &= whole_value(v, w);
+    sum += w;
+  };
+  uint64_t i = s + lane;
+  for (; i + 96 < e; i += 128) {
+    const V a = values[i], b = values[i + 32], c = values[i + 64], d = values[i + 96];
+    add(a), add(b), add(c), add(d);
+  }
+  for (; i < e; i += 32) add(values[i]);
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+  if (!__all_sync(0xFFFFFFFFu, whole) || sum >= (1ull << 53))
+    return row_divisor(values, s, e, target32, true);
+  const float divisor = __fdiv_rn((float)(double)sum, target32);
+  return divisor == 0.0f ? 1.0f : divisor;
+}
+
+// A row's maps by a warp: fill() makes the table (kMapTable floats of the warp's own), at()
+// maps a value.
+struct RowMap {
+  float* table;
+  float divisor;
+  bool normalize, do_log1p;
+  __device__ __forceinline__ void fill() const {
+    __syncwarp();
+    for (uint32_t c = threadIdx.x & 31u; c < kMapTable; c += 32)
+      table[c] = mapped_f32((float)c, normalize, divisor, do_log1p);
+    __syncwarp();
+  }
+  template <class V>
+  __device__ __forceinline__ float at(V v) const {
+    uint32_t c;
+    return map_tabled(v, c) ? table[c] : mapped_f32(to_f32(v), normalize, divisor, do_log1p);
+  }
+};
 
 }  // namespace kg

@@ -32,16 +32,12 @@
 namespace kg {
 
 // Declared in kg_maps.cu.
-void inexact_flag(const void* d_values, kg_dtype dtype, uint64_t nnz, double target_sum,
-                  DeviceBuffer<int>& flag, cudaStream_t stream);
 template <class P>
 void sort_by_gene(const uint32_t* genes, const P* payload, uint64_t nnz, uint32_t n_genes,
                   DeviceBuffer<uint32_t>& genes_out, DeviceBuffer<P>& payload_out,
                   cudaStream_t stream);
 void column_starts(const uint32_t* sorted_genes, uint64_t nnz, uint32_t n_genes,
                    uint64_t* colptr, cudaStream_t stream);
-void check_indices(const uint32_t* d_idx, uint64_t nnz, uint32_t n_genes, cudaStream_t s);
-
 constexpr uint32_t kNoGene = 0xFFFFFFFFu;
 constexpr int kPasses = 11;            // 2 + PCA_POWER_ITERATIONS (pca.rs:123)
 constexpr uint32_t kOversamples = 10;  // PCA_OVERSAMPLES (estimate.rs:153)
@@ -49,65 +45,115 @@ constexpr double kDropTolerance = 1e-10;  // pca_dense.rs:30
 
 // ----------------------------------------------------------------- pack kernels ----
 
-// Kept entries per row (genes mapped into the PCA's set), one warp per row, and the
-// row's normalize divisor (kg_maps.cuh: every 8-lane group of the warp sums the row in
-// kyto's lane order and gets the same divisor) when divisor is not NULL.
-// A gene index at or past the stream's genes is never kept and sets *bad (an
-// asynchronous push checks the indices only when the run starts).
+constexpr int kPackWarps = 8;
+
+// A gene index at or past the stream's genes: kept out and remembered (the largest).
+__device__ __forceinline__ bool gene_ok(uint32_t gene, uint32_t n_genes, unsigned int* worst) {
+  if (gene < n_genes) return true;
+  atomicMax(worst, gene);
+  return false;
+}
+
+// With a gene set: kept entries per row, one warp per row, four loads in flight a lane, and
+// the row's normalize divisor (kg_maps.cuh) when divisor is not NULL.
 template <class V>
-__global__ void count_kept_kernel(const uint64_t* indptr, const uint32_t* idx, const V* values,
-                                  uint64_t n_rows, const uint32_t* gene_map, uint32_t n_genes,
-                                  float target32, const int* inexact, uint64_t* kept,
-                                  float* divisor, unsigned int* bad) {
-  uint64_t row = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  unsigned lane = threadIdx.x & 31u;
+__global__ void __launch_bounds__(kPackWarps * 32)
+count_kept_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
+                  const V* __restrict__ values, uint64_t n_rows,
+                  const uint32_t* __restrict__ gene_map, uint32_t n_genes, float target32,
+                  uint64_t* kept, float* divisor, unsigned int* worst) {
+  const uint64_t row = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const unsigned lane = threadIdx.x & 31u;
   if (row >= n_rows) return;  // whole warps leave together
-  uint64_t s = indptr[row], e = indptr[row + 1];
-  uint64_t count = 0;
-  for (uint64_t i = s + lane; i < e; i += 32) {
-    const uint32_t gi = idx[i];
-    if (gi >= n_genes) {
-      atomicOr(bad, 1u);
-      continue;
-    }
-    count += (gene_map == nullptr || gene_map[gi] != kNoGene);
+  const uint64_t s = indptr[row], e = indptr[row + 1];
+  uint32_t count = 0;
+  auto one = [&](uint32_t gene) {
+    if (gene_ok(gene, n_genes, worst)) count += gene_map[gene] != kNoGene;
+  };
+  uint64_t i = s + lane;
+  for (; i + 96 < e; i += 128) {
+    const uint32_t a = idx[i], b = idx[i + 32], c = idx[i + 64], d = idx[i + 96];
+    one(a), one(b), one(c), one(d);
   }
+  for (; i < e; i += 32) one(idx[i]);
   for (int o = 16; o; o >>= 1) count += __shfl_down_sync(0xFFFFFFFFu, count, o);
   if (lane == 0) kept[row] = count;
   if (divisor) {
-    float d = row_divisor(values, s, e, target32, inexact && *inexact);
+    const float d = warp_row_divisor(values, s, e, target32);
     if (lane == 0) divisor[row] = d;
   }
 }
 
-// Writes each row's kept entries in order at out_ptr[row] (warp per row, ballot
-// compaction keeps the row's gene order), each value mapped on the way: f32(v) / the
-// row's divisor (when divisor is not NULL), then log1p (kg_maps.cuh).
+// With a gene set: each row's kept entries in order at out_ptr[row] (warp per row, ballot
+// compaction keeps the row's gene order), each value mapped on the way (kg_maps.cuh).
 template <class V>
-__global__ void write_kept_kernel(const uint64_t* indptr, const uint32_t* idx, const V* values,
-                                  const float* divisor, int do_log1p, uint64_t n_rows,
-                                  const uint32_t* gene_map, uint32_t n_genes,
-                                  const uint64_t* out_ptr, uint32_t* col, float* val) {
-  uint64_t row = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  unsigned lane = threadIdx.x & 31u;
+__global__ void __launch_bounds__(kPackWarps * 32)
+write_kept_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
+                  const V* __restrict__ values, const float* divisor, int do_log1p,
+                  uint64_t n_rows, const uint32_t* __restrict__ gene_map, uint32_t n_genes,
+                  const uint64_t* out_ptr, uint32_t* __restrict__ col, float* __restrict__ val) {
+  __shared__ float tables[kPackWarps][kMapTable];
+  const uint64_t row = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const unsigned lane = threadIdx.x & 31u;
   if (row >= n_rows) return;
-  uint64_t s = indptr[row], e = indptr[row + 1];
+  const uint64_t s = indptr[row], e = indptr[row + 1];
   uint64_t base = out_ptr[row];
-  const float d = divisor ? divisor[row] : 1.0f;
-  for (uint64_t i0 = s; i0 < e; i0 += 32) {
-    uint64_t i = i0 + lane;
-    bool in = i < e;
-    uint32_t p = kNoGene;
-    if (in && idx[i] < n_genes) p = gene_map ? gene_map[idx[i]] : idx[i];
-    bool keep = in && p != kNoGene;
-    unsigned ballot = __ballot_sync(0xFFFFFFFFu, keep);
-    if (keep) {
-      uint64_t at = base + __popc(ballot & ((1u << lane) - 1u));
-      col[at] = p;
-      val[at] = mapped_value(values, i, divisor != nullptr, d, do_log1p != 0);
+  const RowMap map{tables[threadIdx.x >> 5], divisor ? divisor[row] : 1.0f, divisor != nullptr,
+                   do_log1p != 0};
+  const bool maps = divisor != nullptr || do_log1p;
+  if (maps) map.fill();
+  for (uint64_t i0 = s; i0 < e; i0 += 128) {
+    uint32_t p[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint64_t i = i0 + 32 * k + lane;
+      p[k] = i < e ? idx[i] : 0xFFFFFFFFu;
     }
-    base += __popc(ballot);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) p[k] = p[k] < n_genes ? gene_map[p[k]] : kNoGene;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const unsigned ballot = __ballot_sync(0xFFFFFFFFu, p[k] != kNoGene);
+      if (p[k] != kNoGene) {
+        const uint64_t at = base + __popc(ballot & ((1u << lane) - 1u));
+        const V v = values[i0 + 32 * k + lane];
+        col[at] = p[k];
+        val[at] = maps ? map.at(v) : to_f32(v);
+      }
+      base += __popc(ballot);
+    }
   }
+}
+
+// Every gene kept: a block's rows in one pass (warp per row), the entries where the block's
+// own offsets put them, each value mapped on the way. HBM-bound: 8 bytes a value in, 8 out.
+template <class V>
+__global__ void __launch_bounds__(kPackWarps * 32)
+pack_rows_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
+                 const V* __restrict__ values, uint64_t n_rows, uint32_t n_genes, int normalize,
+                 float target32, int do_log1p, uint32_t* __restrict__ col,
+                 float* __restrict__ val, unsigned int* worst) {
+  __shared__ float tables[kPackWarps][kMapTable];
+  const uint64_t row = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const unsigned lane = threadIdx.x & 31u;
+  if (row >= n_rows) return;
+  const uint64_t s = indptr[row], e = indptr[row + 1];
+  RowMap map{tables[threadIdx.x >> 5], 1.0f, normalize != 0, do_log1p != 0};
+  const bool maps = normalize || do_log1p;
+  if (normalize) map.divisor = warp_row_divisor(values, s, e, target32);
+  if (maps) map.fill();
+  auto put = [&](uint64_t i, uint32_t gene, V v) {
+    gene_ok(gene, n_genes, worst);
+    col[i] = gene;
+    val[i] = maps ? map.at(v) : to_f32(v);
+  };
+  uint64_t i = s + lane;
+  for (; i + 96 < e; i += 128) {
+    const uint32_t g0 = idx[i], g1 = idx[i + 32], g2 = idx[i + 64], g3 = idx[i + 96];
+    const V v0 = values[i], v1 = values[i + 32], v2 = values[i + 64], v3 = values[i + 96];
+    put(i, g0, v0), put(i + 32, g1, v1), put(i + 64, g2, v2), put(i + 96, g3, v3);
+  }
+  for (; i < e; i += 32) put(i, idx[i], values[i]);
 }
 
 // The row of each held entry (for the gene-major twin).
@@ -135,9 +181,10 @@ __global__ void iota64_kernel(uint64_t* out, uint64_t n, uint64_t first) {
   if (i < n) out[i] = first + i;
 }
 
-__global__ void add_offset_kernel(uint64_t* p, uint64_t n, uint64_t offset) {
+// out[i] = in[i] + offset (in place too).
+__global__ void add_offset_kernel(const uint64_t* in, uint64_t n, uint64_t offset, uint64_t* out) {
   uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i < n) p[i] += offset;
+  if (i < n) out[i] = in[i] + offset;
 }
 
 // --------------------------------------------------------------- small kernels -----
@@ -894,6 +941,7 @@ void kg_pca::push(const uint64_t* in_indptr, const uint32_t* in_idx, const void*
   // The block's first and last offsets: read in place from host memory; from device
   // memory through one copy.
   uint64_t ends[2];
+  unsigned int h_worst = 0;
   DeviceBuffer<uint64_t> hp, hc;
   if (is_device_pointer(in_indptr)) {
     KG_CUDA(cudaMemcpyAsync(&ends[0], in_indptr, 8, cudaMemcpyDeviceToHost, s));
@@ -909,61 +957,88 @@ void kg_pca::push(const uint64_t* in_indptr, const uint32_t* in_idx, const void*
   DeviceBuffer<uint32_t> hi, hv;
   const uint32_t* d_idx = device_view(in_idx, bnnz, hi, s);
   const void* d_values = device_view((const uint32_t*)in_values, bnnz, hv, s);
-  if (!bad_index.ptr) {
+  if (async && !bad_index.ptr) {
     bad_index.alloc(1, s);
     bad_index.zero();
   }
-  if (!async) check_indices(d_idx, bnnz, stream_genes, s);
-  trace.mark("checks");
-  // Kept entries per row and the rows' normalize divisors, then the kept entries'
-  // offsets after the held entries; the maps run inside write_kept.
-  const bool normalize = !std::isnan(target_sum);
-  DeviceBuffer<int> inexact;
-  inexact_flag(d_values, dtype, bnnz, target_sum, inexact, s);
-  DeviceBuffer<uint64_t> kept(n_rows + 1, s);
-  DeviceBuffer<float> divisor;
-  if (normalize) divisor.alloc(n_rows, s);
-  kept.zero();
-  unsigned threads = 256;
-  if (dtype == KG_U32)
-    count_kept_kernel<uint32_t><<<blocks_for(n_rows * 32, threads), threads, 0, s>>>(
-        d_indptr, d_idx, (const uint32_t*)d_values, n_rows, gene_map.ptr, stream_genes,
-        (float)target_sum, inexact.ptr, kept.ptr, divisor.ptr, bad_index.ptr);
-  else
-    count_kept_kernel<float><<<blocks_for(n_rows * 32, threads), threads, 0, s>>>(
-        d_indptr, d_idx, (const float*)d_values, n_rows, gene_map.ptr, stream_genes,
-        (float)target_sum, inexact.ptr, kept.ptr, divisor.ptr, bad_index.ptr);
-  KG_LAUNCH_CHECK();
-  size_t temp = 0;
-  KG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp, kept.ptr, kept.ptr, n_rows + 1, s));
-  DeviceBuffer<unsigned char> scratch(temp, s);
-  KG_CUDA(cub::DeviceScan::ExclusiveSum(scratch.ptr, temp, kept.ptr, kept.ptr, n_rows + 1, s));
-  // Kept entries: every entry when every gene is kept (an out-of-range index makes the
-  // run fail before the held input is used), else counted on the device.
-  uint64_t added = bnnz;
-  if (gene_map.ptr) {
-    KG_CUDA(cudaMemcpyAsync(&added, kept.ptr + n_rows, 8, cudaMemcpyDeviceToHost, s));
-    KG_CUDA(cudaStreamSynchronize(s));
+  // An asynchronous push leaves the index check to the run; a synchronous one reads its own
+  // verdict before the block counts as pushed.
+  DeviceBuffer<unsigned int> own_worst;
+  if (!async) {
+    own_worst.alloc(1, s);
+    own_worst.zero();
   }
-  add_offset_kernel<<<blocks_for(n_rows + 1, 256), 256, 0, s>>>(kept.ptr, n_rows + 1, nnz);
-  KG_LAUNCH_CHECK();
+  unsigned int* worst = async ? bad_index.ptr : own_worst.ptr;
+  auto check_worst = [&] {  // after a synchronisation of h_worst's copy
+    if (h_worst)
+      fail(KG_ERR_INVALID, "a block holds gene index " + std::to_string(h_worst) + " but has " +
+                               std::to_string(stream_genes) + " genes");
+  };
+  const bool normalize = !std::isnan(target_sum);
+  const unsigned blocks = blocks_for(n_rows, kPackWarps);
+  constexpr unsigned threads = kPackWarps * 32;
+  uint64_t added = bnnz;
+  DeviceBuffer<uint64_t> kept;
+  DeviceBuffer<float> divisor;
+  if (gene_map.ptr) {
+    // Kept entries per row and the rows' normalize divisors, then the kept entries' offsets
+    // after the held entries; the maps run as the entries are written.
+    kept.alloc(n_rows + 1, s);
+    KG_CUDA(cudaMemsetAsync(kept.ptr + n_rows, 0, 8, s));
+    if (normalize) divisor.alloc(n_rows, s);
+    if (dtype == KG_U32)
+      count_kept_kernel<uint32_t><<<blocks, threads, 0, s>>>(
+          d_indptr, d_idx, (const uint32_t*)d_values, n_rows, gene_map.ptr, stream_genes,
+          (float)target_sum, kept.ptr, divisor.ptr, worst);
+    else
+      count_kept_kernel<float><<<blocks, threads, 0, s>>>(
+          d_indptr, d_idx, (const float*)d_values, n_rows, gene_map.ptr, stream_genes,
+          (float)target_sum, kept.ptr, divisor.ptr, worst);
+    KG_LAUNCH_CHECK();
+    size_t temp = 0;
+    KG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp, kept.ptr, kept.ptr, n_rows + 1, s));
+    DeviceBuffer<unsigned char> scratch(temp, s);
+    KG_CUDA(cub::DeviceScan::ExclusiveSum(scratch.ptr, temp, kept.ptr, kept.ptr, n_rows + 1, s));
+    KG_CUDA(cudaMemcpyAsync(&added, kept.ptr + n_rows, 8, cudaMemcpyDeviceToHost, s));
+    if (!async) KG_CUDA(cudaMemcpyAsync(&h_worst, worst, 4, cudaMemcpyDeviceToHost, s));
+    KG_CUDA(cudaStreamSynchronize(s));
+    check_worst();
+  }
   trace.mark("kept counts");
   grow(indptr, n_cells + 1, n_cells + n_rows + 1);
   grow(col, nnz, nnz + added);
   grow(val, nnz, nnz + added);
   grow(cells, n_cells, n_cells + n_rows);
   trace.mark("held buffers");
-  KG_CUDA(cudaMemcpyAsync(indptr.ptr + n_cells, kept.ptr, (n_rows + 1) * 8,
-                          cudaMemcpyDeviceToDevice, s));
-  if (dtype == KG_U32)
-    write_kept_kernel<uint32_t><<<blocks_for(n_rows * 32, threads), threads, 0, s>>>(
-        d_indptr, d_idx, (const uint32_t*)d_values, divisor.ptr, log1p, n_rows, gene_map.ptr,
-        stream_genes, kept.ptr, col.ptr, val.ptr);
-  else
-    write_kept_kernel<float><<<blocks_for(n_rows * 32, threads), threads, 0, s>>>(
-        d_indptr, d_idx, (const float*)d_values, divisor.ptr, log1p, n_rows, gene_map.ptr,
-        stream_genes, kept.ptr, col.ptr, val.ptr);
+  uint64_t* held = indptr.ptr + n_cells;
+  add_offset_kernel<<<blocks_for(n_rows + 1, 256), 256, 0, s>>>(
+      gene_map.ptr ? kept.ptr : d_indptr, n_rows + 1, nnz, held);
   KG_LAUNCH_CHECK();
+  if (gene_map.ptr) {
+    if (dtype == KG_U32)
+      write_kept_kernel<uint32_t><<<blocks, threads, 0, s>>>(
+          d_indptr, d_idx, (const uint32_t*)d_values, divisor.ptr, log1p, n_rows, gene_map.ptr,
+          stream_genes, held, col.ptr, val.ptr);
+    else
+      write_kept_kernel<float><<<blocks, threads, 0, s>>>(
+          d_indptr, d_idx, (const float*)d_values, divisor.ptr, log1p, n_rows, gene_map.ptr,
+          stream_genes, held, col.ptr, val.ptr);
+    KG_LAUNCH_CHECK();
+  } else {
+    // Every entry is kept (an out-of-range index fails the push, or the run, before the held
+    // input is used).
+    if (dtype == KG_U32)
+      pack_rows_kernel<uint32_t><<<blocks, threads, 0, s>>>(
+          d_indptr, d_idx, (const uint32_t*)d_values, n_rows, stream_genes, normalize ? 1 : 0,
+          (float)target_sum, log1p, col.ptr + nnz, val.ptr + nnz, worst);
+    else
+      pack_rows_kernel<float><<<blocks, threads, 0, s>>>(
+          d_indptr, d_idx, (const float*)d_values, n_rows, stream_genes, normalize ? 1 : 0,
+          (float)target_sum, log1p, col.ptr + nnz, val.ptr + nnz, worst);
+    KG_LAUNCH_CHECK();
+    if (!async) KG_CUDA(cudaMemcpyAsync(&h_worst, worst, 4, cudaMemcpyDeviceToHost, s));
+  }
+  uint64_t next = next_cell + n_rows;
   if (in_cells) {
     const uint64_t* d_cells = device_view(in_cells, n_rows, hc, s);
     KG_CUDA(cudaMemcpyAsync(cells.ptr + n_cells, d_cells, n_rows * 8, cudaMemcpyDeviceToDevice, s));
@@ -974,18 +1049,21 @@ void kg_pca::push(const uint64_t* in_indptr, const uint32_t* in_idx, const void*
     } else {
       last = in_cells[n_rows - 1];
     }
-    next_cell = last + 1;
+    next = last + 1;
   } else {
     iota64_kernel<<<blocks_for(n_rows, 256), 256, 0, s>>>(cells.ptr + n_cells, n_rows, next_cell);
     KG_LAUNCH_CHECK();
-    next_cell += n_rows;
   }
-  n_cells += n_rows;
-  nnz += added;
   // A synchronous push returns once the block is on the device (the caller may then
   // reuse its host arrays); an asynchronous one leaves the copies and kernels queued on
   // the session's stream (its host arrays stay in use until kg_pca_run returns).
-  if (!async) KG_CUDA(cudaStreamSynchronize(s));
+  if (!async) {
+    KG_CUDA(cudaStreamSynchronize(s));
+    check_worst();
+  }
+  n_cells += n_rows;
+  nnz += added;
+  next_cell = next;
   trace.mark("held block");
 }
 
