@@ -3,24 +3,25 @@
 // (crates/kyto-store/src/tile_decode.rs:74-196), which kyto runs on the host before
 // kyto-exec rebuilds the rows once more for its GPU path (pca/gpu.rs:73-115).
 //
-// Three kernels, every one a pass over bytes (HBM-bound, no arithmetic to speak of):
-//   1. tile_indptr_check_kernel: a thread per value of the block's indptr shard checks
-//      kyto's four indptr rules (starts at 0, ends at the tile's nnz, never decreases,
-//      flat over padding rows) and marks the tiles that break one;
-//   2. tile_rows_kernel: a warp per row walks the row's segment in every tile whose
-//      indptr passed (so every entry it reads lies inside that tile), checks that the
-//      local indices strictly increase below the block width, and sums the row's length;
-//   3. after a scan of the lengths, tile_join_kernel: a warp per row copies its segments
-//      in gene-block order, adding each block's first gene to the local indices, unless
-//      the checks found a problem (then it writes nothing).
+// Two kernels, each a pass over bytes (no arithmetic to speak of; latency and launches bound
+// a block's few MB):
+//   1. tile_check_kernel: a thread per value of the block's indptr shard checks kyto's four
+//      indptr rules (starts at 0, ends at the tile's nnz, never decreases, flat over padding
+//      rows); a warp per row and tile checks that the row's local indices strictly increase
+//      below the block width, its range cut to the tile (a tile whose indptr breaks a rule is
+//      reported for that rule first, whatever its rows hold);
+//   2. tile_join_kernel: a warp per row and tile copies its segment, adding the block's first
+//      gene to the local indices, unless the checks found a problem (then it writes nothing).
+//      A tile's indptr counts its entries in the rows before, so a segment's place is a sum
+//      over the tiles' indptrs (row r, and row r + 1 of the tiles before it): no scan.
 // Every problem found becomes one 64-bit key ordered as kyto reports problems (gene
 // block, then the check in kyto's order, then the row, then which of a row's two checks
-// fails), and the smallest key wins (atomicMin). All three kernels are queued at once;
-// the host reads the key once, after the join, and words a problem as kyto does
-// (KG_ERR_CORRUPT, kyto's KY-E107). A call waits once (twice with host outputs, three
-// times with device-resident tile_offsets).
-
-#include <cub/cub.cuh>
+// fails), and the smallest key wins (atomicMin). Both kernels are queued at once; the host
+// reads the key once, after the join, and words a problem as kyto does (KG_ERR_CORRUPT,
+// kyto's KY-E107). A call waits once (twice with host outputs, three times with
+// device-resident tile_offsets).
+// A block of 4,096 x 627 entries in two tiles: 48 us a call, 20 us in the kernels; checking and summing the rows,
+// scanning their lengths and joining a row a warp took 81 us (the join alone 33 us).
 
 #include <algorithm>
 #include <cstring>
@@ -42,84 +43,123 @@ __host__ __device__ __forceinline__ unsigned long long problem_key(uint64_t g, u
   return (g << 38) | (check << 35) | (row << 1) | sub;
 }
 
-// A thread per value i of the shard (tile g = i / (C + 1), row r = i % (C + 1)).
-__global__ void tile_indptr_check_kernel(const uint32_t* shard, uint32_t n_gb, uint64_t row_len,
-                                         uint32_t rows, const uint64_t* start,
-                                         unsigned long long* problem, uint32_t* tile_bad) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= (uint64_t)n_gb * row_len) return;
-  const uint64_t g = i / row_len, r = i % row_len;
-  const uint32_t v = shard[i];
-  unsigned long long key = kNoProblem;
-  if (r == 0 && v != 0) key = problem_key(g, kStart, 0, 0);
-  if (r + 1 == row_len && (uint64_t)v != start[g + 1] - start[g])
-    key = min(key, problem_key(g, kEnd, 0, 0));
-  if (r + 1 < row_len && shard[i + 1] < v) key = min(key, problem_key(g, kDecrease, r, 0));
-  if (r > rows && v != shard[g * row_len + rows]) key = min(key, problem_key(g, kFlat, 0, 0));
-  if (key != kNoProblem) {
-    atomicMin(problem, key);
-    tile_bad[g] = 1;
-  }
-}
+// Where each tile starts among the block's entries, and their end: as a kernel argument for
+// up to kStartsInline tiles, else in device memory.
+constexpr uint32_t kStartsInline = 64;
+struct TileStarts {
+  uint64_t v[kStartsInline + 1];
+  const uint64_t* more;
+  __device__ __forceinline__ uint64_t operator[](uint32_t g) const { return more ? more[g] : v[g]; }
+};
 
-// A warp per row r < rows: the row's segments in the tiles whose indptr passed (their
-// values run from 0 to the tile's nnz without decreasing, so [a, e) lies in the tile).
-__global__ void tile_rows_kernel(const uint32_t* shard, uint32_t n_gb, uint64_t row_len,
-                                 uint32_t rows, const uint64_t* start, const uint32_t* idx,
-                                 uint64_t gene_block, uint64_t n_genes, const uint32_t* tile_bad,
-                                 unsigned long long* problem, uint64_t* lengths) {
-  const uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+constexpr unsigned kTileThreads = 256;
+
+// Blocks [0, shard_blocks): a thread per value i of the shard (tile g = i / (C + 1), row r =
+// i % (C + 1)). The others: a warp per (tile, row).
+__global__ void __launch_bounds__(kTileThreads)
+tile_check_kernel(const uint32_t* __restrict__ shard, uint32_t n_gb, uint64_t row_len,
+                  uint32_t rows, const __grid_constant__ TileStarts start,
+                  const uint32_t* __restrict__ idx, uint64_t gene_block, uint64_t n_genes,
+                  uint64_t shard_blocks, unsigned long long* problem) {
+  if (blockIdx.x < shard_blocks) {
+    const uint64_t i = blockIdx.x * (uint64_t)kTileThreads + threadIdx.x;
+    if (i >= (uint64_t)n_gb * row_len) return;
+    const uint64_t g = i / row_len, r = i % row_len;
+    const uint32_t v = shard[i];
+    unsigned long long key = kNoProblem;
+    if (r == 0 && v != 0) key = problem_key(g, kStart, 0, 0);
+    if (r + 1 == row_len && (uint64_t)v != start[g + 1] - start[g])
+      key = min(key, problem_key(g, kEnd, 0, 0));
+    if (r + 1 < row_len && shard[i + 1] < v) key = min(key, problem_key(g, kDecrease, r, 0));
+    if (r > rows && v != shard[g * row_len + rows]) key = min(key, problem_key(g, kFlat, 0, 0));
+    if (key != kNoProblem) atomicMin(problem, key);
+    return;
+  }
   const unsigned lane = threadIdx.x & 31u;
-  if (r >= rows) return;
-  uint64_t total = 0;
-  for (uint32_t g = 0; g < n_gb; ++g) {
-    if (tile_bad[g]) continue;
-    const uint64_t a = shard[g * row_len + r], e = shard[g * row_len + r + 1];
-    total += e - a;
+  const uint64_t warps = (gridDim.x - shard_blocks) * (kTileThreads / 32);
+  uint64_t wq = ((blockIdx.x - shard_blocks) * (uint64_t)kTileThreads + threadIdx.x) >> 5;
+  for (; wq < (uint64_t)n_gb * rows; wq += warps) {
+    const uint32_t g = (uint32_t)(wq / rows), r = (uint32_t)(wq % rows);
+    const uint64_t nnz = start[g + 1] - start[g];
+    const uint64_t a = min((uint64_t)shard[g * row_len + r], nnz);
+    const uint64_t e = min((uint64_t)shard[g * row_len + r + 1], nnz);
     const uint32_t* t = idx + start[g];
     const uint64_t width = min(gene_block, n_genes - g * gene_block);
     bool wide = false, unsorted = false;
-    for (uint64_t x = a + lane; x < e; x += 32) {
-      const uint32_t v = t[x];
-      wide |= v >= width;
-      if (x > a) unsorted |= v <= t[x - 1];
+    uint32_t carry = 0;  // the index before the chunk's first
+    for (uint64_t x0 = a; x0 < e; x0 += 128) {
+      uint32_t v[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) v[m] = x0 + 32 * m + lane < e ? t[x0 + 32 * m + lane] : 0;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const uint64_t x = x0 + 32 * m + lane;
+        uint32_t before = __shfl_up_sync(0xFFFFFFFFu, v[m], 1);
+        if (lane == 0) before = carry;
+        carry = __shfl_sync(0xFFFFFFFFu, v[m], 31);
+        if (x >= e) continue;
+        wide |= v[m] >= width;
+        unsorted |= x > a && v[m] <= before;
+      }
     }
     const unsigned w = __ballot_sync(0xFFFFFFFFu, wide);
     const unsigned u = __ballot_sync(0xFFFFFFFFu, unsorted);
     if (lane == 0 && (w | u)) atomicMin(problem, problem_key(g, kRow, r, w ? 0 : 1));
   }
-  if (lane == 0) lengths[r] = total;
 }
 
-// A warp per row r < rows: its segments in gene-block order, global gene indices, and
-// its end offset. Writes nothing when the checks found a problem (the caller's outputs
-// stay as they were): every thread reads the verdict, final once the checks ran before
-// it on the stream.
-__global__ void tile_join_kernel(const uint32_t* shard, uint32_t n_gb, uint64_t row_len,
-                                 uint32_t rows, const uint64_t* start, const uint32_t* idx,
-                                 const uint32_t* val, uint64_t gene_block,
-                                 const unsigned long long* problem, const uint64_t* ends,
-                                 uint64_t* out_ptr, uint32_t* out_idx, uint32_t* out_val) {
-  const uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+// A warp per (row, tile). Writes nothing when the checks found a problem (the caller's
+// outputs stay as they were): every thread reads the verdict, final once the checks ran
+// before it on the stream.
+__global__ void __launch_bounds__(kTileThreads)
+tile_join_kernel(const uint32_t* __restrict__ shard, uint32_t n_gb, uint64_t row_len,
+                 uint32_t rows, const __grid_constant__ TileStarts start,
+                 const uint32_t* __restrict__ idx, const uint32_t* __restrict__ val,
+                 uint64_t gene_block, const unsigned long long* problem, uint64_t* out_ptr,
+                 uint32_t* __restrict__ out_idx, uint32_t* __restrict__ out_val) {
   const unsigned lane = threadIdx.x & 31u;
-  if (r >= rows || *problem != kNoProblem) return;
-  // ends[r] = the entries of rows 0..r (an inclusive scan of the row lengths).
-  uint64_t dst = r ? ends[r - 1] : 0;
-  if (lane == 0) {
-    out_ptr[r + 1] = ends[r];
-    if (r == 0) out_ptr[0] = 0;
+  const uint64_t warps = gridDim.x * (uint64_t)(kTileThreads / 32);
+  uint64_t wq = (blockIdx.x * (uint64_t)kTileThreads + threadIdx.x) >> 5;
+  if (*problem != kNoProblem) return;
+  if (n_gb == 0) {  // a layer without genes: empty rows
+    for (; wq <= rows; wq += warps)
+      if (lane == 0) out_ptr[wq] = 0;
+    return;
   }
-  for (uint32_t g = 0; g < n_gb; ++g) {
-    const uint64_t a = shard[g * row_len + r], e = shard[g * row_len + r + 1];
-    const uint64_t base = start[g];
+  for (; wq < (uint64_t)n_gb * rows; wq += warps) {
+    const uint32_t r = (uint32_t)(wq / n_gb), g = (uint32_t)(wq % n_gb);
+    uint64_t dst = 0;
+    for (uint32_t h = lane; h < n_gb; h += 32) dst += shard[h * row_len + r + (h < g ? 1 : 0)];
+    for (int o = 16; o; o >>= 1) dst += __shfl_xor_sync(0xFFFFFFFFu, dst, o);
+    const uint64_t a = shard[g * row_len + r], len = shard[g * row_len + r + 1] - a;
+    if (lane == 0) {
+      if (g + 1 == n_gb) out_ptr[r + 1] = dst + len;
+      if (r == 0 && g == 0) out_ptr[0] = 0;
+    }
     // g G + local < n_genes <= 2^32 - 1 (the checks passed).
     const uint32_t first_gene = (uint32_t)(g * gene_block);
-    for (uint64_t x = a + lane; x < e; x += 32) {
-      out_idx[dst + (x - a)] = first_gene + idx[base + x];
-      out_val[dst + (x - a)] = val[base + x];
+    const uint32_t* ti = idx + start[g] + a;
+    const uint32_t* tv = val + start[g] + a;
+    uint32_t* oi = out_idx + dst;
+    uint32_t* ov = out_val + dst;
+    uint64_t x = lane;
+    for (; x + 96 < len; x += 128) {
+      const uint32_t i0 = ti[x], i1 = ti[x + 32], i2 = ti[x + 64], i3 = ti[x + 96];
+      const uint32_t v0 = tv[x], v1 = tv[x + 32], v2 = tv[x + 64], v3 = tv[x + 96];
+      oi[x] = first_gene + i0, oi[x + 32] = first_gene + i1;
+      oi[x + 64] = first_gene + i2, oi[x + 96] = first_gene + i3;
+      ov[x] = v0, ov[x + 32] = v1, ov[x + 64] = v2, ov[x + 96] = v3;
     }
-    dst += e - a;
+    for (; x < len; x += 32) {
+      oi[x] = first_gene + ti[x];
+      ov[x] = tv[x];
+    }
   }
+}
+
+// Blocks of a warp per (tile, row), the warps going on from the grid's end past 2^25 of them.
+unsigned row_blocks_for(uint64_t pairs) {
+  return (unsigned)std::min<uint64_t>((pairs + kTileThreads / 32 - 1) / (kTileThreads / 32), 1u << 22);
 }
 
 template <class T>
@@ -175,30 +215,30 @@ void join_tiles(kg_ctx* ctx, cudaStream_t s, const kg_tile_block* tb, const Tile
   const uint32_t* shard = device_view(tb->indptr, (size_t)n_gb * row_len, hs, s);
   const uint32_t* idx = device_view(tb->indices, sh.nnz, hi, s);
   const uint32_t* val = device_view(static_cast<const uint32_t*>(tb->data), sh.nnz, hv, s);
-  DeviceBuffer<uint64_t> start(n_gb + 1, s), lengths(rows, s);
-  KG_CUDA(cudaMemcpyAsync(start.ptr, sh.start.data(), (n_gb + 1) * 8ull, cudaMemcpyHostToDevice, s));
+  TileStarts start{};
+  DeviceBuffer<uint64_t> more;
+  if (n_gb <= kStartsInline) {
+    std::copy(sh.start.begin(), sh.start.end(), start.v);
+  } else {
+    more.alloc(n_gb + 1, s);
+    KG_CUDA(cudaMemcpyAsync(more.ptr, sh.start.data(), (n_gb + 1) * 8ull, cudaMemcpyHostToDevice, s));
+    start.more = more.ptr;
+  }
   DeviceBuffer<unsigned long long> problem(1, s);
   KG_CUDA(cudaMemsetAsync(problem.ptr, 0xFF, 8, s));
-  DeviceBuffer<uint32_t> tile_bad(n_gb, s);
-  tile_bad.zero();
   if (n_gb) {
-    tile_indptr_check_kernel<<<blocks_for((uint64_t)n_gb * row_len, 256), 256, 0, s>>>(
-        shard, n_gb, row_len, rows, start.ptr, problem.ptr, tile_bad.ptr);
+    const uint64_t shard_blocks = blocks_for((uint64_t)n_gb * row_len, kTileThreads);
+    const uint64_t row_blocks = row_blocks_for((uint64_t)n_gb * rows);
+    tile_check_kernel<<<(unsigned)(shard_blocks + row_blocks), kTileThreads, 0, s>>>(
+        shard, n_gb, row_len, rows, start, idx, tb->gene_block_size, tb->n_genes, shard_blocks,
+        problem.ptr);
     KG_LAUNCH_CHECK();
   }
-  tile_rows_kernel<<<blocks_for((uint64_t)rows * 32, 256), 256, 0, s>>>(
-      shard, n_gb, row_len, rows, start.ptr, idx, tb->gene_block_size, tb->n_genes, tile_bad.ptr,
-      problem.ptr, lengths.ptr);
-  KG_LAUNCH_CHECK();
-  // The rows' ends and the join are queued before the verdict is read (one wait a call);
-  // the join writes only when the checks passed.
-  size_t temp = 0;
-  KG_CUDA(cub::DeviceScan::InclusiveSum(nullptr, temp, lengths.ptr, lengths.ptr, rows, s));
-  DeviceBuffer<unsigned char> scratch(temp, s);
-  KG_CUDA(cub::DeviceScan::InclusiveSum(scratch.ptr, temp, lengths.ptr, lengths.ptr, rows, s));
-  tile_join_kernel<<<blocks_for((uint64_t)rows * 32, 256), 256, 0, s>>>(
-      shard, n_gb, row_len, rows, start.ptr, idx, val, tb->gene_block_size, problem.ptr,
-      lengths.ptr, d_indptr, d_indices, d_values);
+  // The join is queued before the verdict is read (one wait a call); it writes only when the
+  // checks passed.
+  tile_join_kernel<<<row_blocks_for(std::max<uint64_t>(n_gb, 1) * rows), kTileThreads, 0, s>>>(
+      shard, n_gb, row_len, rows, start, idx, val, tb->gene_block_size, problem.ptr, d_indptr,
+      d_indices, d_values);
   KG_LAUNCH_CHECK();
   unsigned long long key = kNoProblem;
   KG_CUDA(cudaMemcpyAsync(&key, problem.ptr, 8, cudaMemcpyDeviceToHost, s));
@@ -268,6 +308,7 @@ kg_status kg_tiles_to_csr(kg_ctx* ctx, const kg_tile_block* block, uint64_t* ind
     uint32_t* d_idx = di ? indices : oi.ptr;
     uint32_t* d_val = dv ? static_cast<uint32_t*>(values) : ov.ptr;
     join_tiles(ctx, s, block, sh, d_ptr, d_idx, d_val);
+    if (dp && di && dv) return;  // join_tiles waited for the join
     if (!dp) KG_CUDA(cudaMemcpyAsync(indptr, d_ptr, (rows + 1) * 8, cudaMemcpyDeviceToHost, s));
     if (!di && sh.nnz)
       KG_CUDA(cudaMemcpyAsync(indices, d_idx, sh.nnz * 4, cudaMemcpyDeviceToHost, s));
