@@ -50,8 +50,9 @@ __global__ void finite_check_kernel(const float* x, uint64_t n, uint32_t width, 
 
 // Column sums, minima and maxima of the leading d components, per chunk of kMeanRows
 // rows (4 row classes of 64 column threads, combined in a fixed order), then over the
-// chunks in order (column_finish_kernel): the same bits on every run.
-constexpr uint32_t kMeanRows = 2048;
+// chunks in 16 classes, in a fixed order (column_finish_kernel): the same bits on every run.
+// (Chunks of 2,048 rows left 60,000 rows to 30 CTAs: 91 us.)
+constexpr uint32_t kMeanRows = 256;
 
 __global__ void __launch_bounds__(256)
 column_partial_kernel(const float* x, uint64_t n, uint32_t width, uint32_t d, double* part_sum,
@@ -84,17 +85,29 @@ column_partial_kernel(const float* x, uint64_t n, uint32_t width, uint32_t d, do
 
 // mean[j] (f64) and, for the first three components, the range of the centred values
 // f32(x - mean) (that map is monotonic, so the range is the centred raw range).
-__global__ void column_finish_kernel(const double* part_sum, const float* part_lo,
-                                     const float* part_hi, uint32_t n_parts, uint64_t n,
-                                     uint32_t d, double* mean, float* lo_hi) {
-  const uint32_t j = threadIdx.x;
-  if (j >= d) return;
+__global__ void __launch_bounds__(1024)
+column_finish_kernel(const double* part_sum, const float* part_lo, const float* part_hi,
+                     uint32_t n_parts, uint64_t n, uint32_t d, double* mean, float* lo_hi) {
+  __shared__ double ss[16][64];
+  __shared__ float sl[16][64], sh[16][64];
+  const uint32_t j = threadIdx.x & 63u, cls = threadIdx.x >> 6;
   double sum = 0.0;
   float lo = INFINITY, hi = -INFINITY;
-  for (uint32_t b = 0; b < n_parts; ++b) {
-    sum = __dadd_rn(sum, part_sum[b * 64ull + j]);
-    lo = fminf(lo, part_lo[b * 64ull + j]);
-    hi = fmaxf(hi, part_hi[b * 64ull + j]);
+  if (j < d)
+    for (uint32_t b = cls; b < n_parts; b += 16) {
+      sum = __dadd_rn(sum, part_sum[b * 64ull + j]);
+      lo = fminf(lo, part_lo[b * 64ull + j]);
+      hi = fmaxf(hi, part_hi[b * 64ull + j]);
+    }
+  ss[cls][j] = sum;
+  sl[cls][j] = lo;
+  sh[cls][j] = hi;
+  __syncthreads();
+  if (cls != 0 || j >= d) return;
+  for (int c = 1; c < 16; ++c) {
+    sum = __dadd_rn(sum, ss[c][j]);
+    lo = fminf(lo, sl[c][j]);
+    hi = fmaxf(hi, sh[c][j]);
   }
   const double m = sum / (double)n;
   mean[j] = m;
@@ -111,7 +124,7 @@ void column_stats(const float* x, uint64_t n, uint32_t width, uint32_t d, double
   DeviceBuffer<float> lo(parts * 64ull, s), hi(parts * 64ull, s);
   column_partial_kernel<<<parts, 256, 0, s>>>(x, n, width, d, sum.ptr, lo.ptr, hi.ptr);
   KG_LAUNCH_CHECK();
-  column_finish_kernel<<<1, 64, 0, s>>>(sum.ptr, lo.ptr, hi.ptr, parts, n, d, mean, lo_hi);
+  column_finish_kernel<<<1, 1024, 0, s>>>(sum.ptr, lo.ptr, hi.ptr, parts, n, d, mean, lo_hi);
   KG_LAUNCH_CHECK();
 }
 
@@ -746,6 +759,34 @@ __device__ void warp_merge(const double* keys, const uint32_t* idx, uint32_t len
   if (lane == 0) *out_len = produced;
 }
 
+constexpr uint32_t kRankKept = 256;  // candidates ranked in shared memory, at most
+
+struct __align__(16) RankCandidate {
+  double key;
+  uint32_t row;
+  float approx;
+};
+
+// count + 1 if (key a, row a) comes before (key b, row b): squared distances are >= 0, so
+// their bits order as they do, and the comparison is one borrow over 96 bits.
+__device__ __forceinline__ uint32_t count_before(uint32_t count, const RankCandidate& a,
+                                                 const RankCandidate& b) {
+  const uint64_t ka = (uint64_t)__double_as_longlong(a.key), kb = (uint64_t)__double_as_longlong(b.key);
+  uint32_t t;
+  asm("{\n\t"
+      ".reg .u32 d;\n\t"
+      "sub.cc.u32 d, %2, %3;\n\t"
+      "subc.cc.u32 d, %4, %5;\n\t"
+      "subc.cc.u32 d, %6, %7;\n\t"
+      "subc.u32 d, 0, 0;\n\t"
+      "sub.u32 %0, %1, d;\n\t"
+      "}"
+      : "=r"(t)
+      : "r"(count), "r"(a.row), "r"(b.row), "r"((uint32_t)ka), "r"((uint32_t)kb),
+        "r"((uint32_t)(ka >> 32)), "r"((uint32_t)(kb >> 32)));
+  return t;
+}
+
 // One warp per query: exact keys of its candidates, the k best by (key, row). A row
 // that overflowed, holds fewer than k candidates or has a candidate outside its slack
 // is flagged for a full search (kyto's rank, neighbors_exact.rs:318-340).
@@ -754,14 +795,26 @@ __device__ void warp_merge(const double* keys, const uint32_t* idx, uint32_t len
 // filter's are distances already: inv_s2 = 1, qn2 = NULL).
 // With `perm`, the filter ran on the rows in scan order: its query position qp and its
 // candidates' rows are positions there, row perm[.] of x (ranks and outputs use x's).
-__global__ void rank_kernel(const float* __restrict__ x, uint32_t width, uint32_t d,
+//
+// Up to kRankKept candidates within the threshold (nearly every query): eight lanes a
+// candidate, lane j with the components j, j + 8, ..., which is the partial sum j of
+// exact_key; sixteen candidates' reads are in flight a warp, and a read is one sector a
+// candidate. Latency bounds it: a lane that read a candidate's row by itself touched a sector
+// a component, waited for each and then merged its ranked list (0.69 ms for 60,000 rows of 50
+// components and 70 candidates each, 10 ms for 1M rows with 63; now 0.43 and 6.4 ms). Past 64 candidates those beyond the k-th smallest of the 32 lanes' smallest keys are
+// dropped (at least k lie at or before it; k <= 32). A candidate's rank is the number of
+// candidates before it. More candidates: ranked lists a lane, merged (warp_merge).
+__global__ void __launch_bounds__(kRankWarps * 32)
+rank_kernel(const float* __restrict__ x, uint32_t width, uint32_t d,
                             uint64_t q_begin, uint64_t q_end, uint32_t k, uint32_t cap,
-                            const float* cand_key, const uint32_t* cand_row,
+                            const float* __restrict__ cand_key,
+                            const uint32_t* __restrict__ cand_row,
                             const uint32_t* cand_count, const float* threshold,
                             const double* slack, double inv_s2, const double* qn2,
                             const uint32_t* qperm, const uint32_t* pperm, double* out_key,
                             uint32_t* out_row, uint32_t* full_flag,
                             unsigned long long* n_candidates) {
+  __shared__ RankCandidate shared[kRankWarps][kRankKept];
   uint64_t qi = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   unsigned lane = threadIdx.x & 31u;
   uint64_t qp = q_begin + qi;
@@ -776,6 +829,122 @@ __global__ void rank_kernel(const float* __restrict__ x, uint32_t width, uint32_
   double sl = slack[qp];
   double shift = qn2 ? qn2[qp] : 0.0;
   const float* qrow = x + q * width;
+  RankCandidate* const cand = shared[threadIdx.x >> 5];
+  uint32_t kept = 0;
+  for (uint32_t c0 = 0; c0 < count; c0 += 32) {
+    const uint32_t c = c0 + lane;
+    const float ak = c < count ? cand_key[qi * (uint64_t)cap + c] : INFINITY;
+    const bool pass = c < count && ak <= th;
+    const unsigned ballot = __ballot_sync(0xFFFFFFFFu, pass);
+    const uint32_t at = kept + __popc(ballot & ((1u << lane) - 1u));
+    if (pass && at < kRankKept) {
+      const uint32_t p = cand_row[qi * (uint64_t)cap + c];
+      cand[at].approx = ak;
+      cand[at].row = pperm ? pperm[p] : p;
+    }
+    kept += __popc(ballot);
+    if (kept > kRankKept) break;
+  }
+  if (kept <= kRankKept) {
+    const uint32_t part = lane & 7u, group = lane >> 3;
+    double query[kDim / 8];
+#pragma unroll
+    for (uint32_t i = 0; i < kDim / 8; ++i)
+      query[i] = 8 * i + part < d ? (double)qrow[8 * i + part] : 0.0;
+    bool bad = false;
+    __syncwarp();
+    for (uint32_t c0 = 0; c0 < kept; c0 += 16) {
+      float b[4][kDim / 8];
+#pragma unroll
+      for (uint32_t g = 0; g < 4; ++g) {
+        const float* pr = x + (uint64_t)cand[min(c0 + 4 * g + group, kept - 1)].row * width + part;
+#pragma unroll
+        for (uint32_t i = 0; i < kDim / 8; ++i) b[g][i] = 8 * i + part < d ? pr[8 * i] : 0.0f;
+      }
+#pragma unroll
+      for (uint32_t g = 0; g < 4; ++g) {
+        // exact_key's operations in its order (a component past d adds +0 to a sum >= 0).
+        double e = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < kDim / 8; ++i) {
+          const double diff = __dsub_rn(query[i], (double)b[g][i]);
+          e = __dadd_rn(e, __dmul_rn(diff, diff));
+        }
+#pragma unroll
+        for (int o = 4; o; o >>= 1) e = __dadd_rn(e, __shfl_xor_sync(0xFFFFFFFFu, e, o));
+        const uint32_t c = c0 + 4 * g + group;
+        if (part == 0 && c < kept) {
+          if (fabs(e - ((double)cand[c].approx * inv_s2 + shift)) > sl) bad = true;
+          cand[c].key = e;
+        }
+      }
+    }
+    __syncwarp();
+    uint32_t m = kept;  // candidates still to rank
+    if (m > 64 && k <= 32) {
+      RankCandidate least = cand[lane];
+      for (uint32_t c = lane + 32; c < m; c += 32) {
+        const RankCandidate o = cand[c];
+        if (count_before(0, o, least)) least = o;
+      }
+      uint32_t at = 0;
+      for (int o = 0; o < 32; ++o) {
+        RankCandidate other;
+        other.key = __shfl_sync(0xFFFFFFFFu, least.key, o);
+        other.row = __shfl_sync(0xFFFFFFFFu, least.row, o);
+        at = count_before(at, other, least);
+      }
+      const int kth = __ffs(__ballot_sync(0xFFFFFFFFu, at == k - 1)) - 1;
+      RankCandidate line;
+      line.key = __shfl_sync(0xFFFFFFFFu, least.key, kth);
+      line.row = __shfl_sync(0xFFFFFFFFu, least.row, kth);
+      uint32_t left = 0;
+      for (uint32_t c0 = 0; c0 < m; c0 += 32) {
+        RankCandidate o;
+        const bool in = c0 + lane < m;
+        if (in) o = cand[c0 + lane];
+        const bool keep = in && count_before(0, line, o) == 0;
+        const unsigned ballot = __ballot_sync(0xFFFFFFFFu, keep);
+        __syncwarp();
+        if (keep) cand[left + __popc(ballot & ((1u << lane) - 1u))] = o;
+        left += __popc(ballot);
+        __syncwarp();
+      }
+      m = left;
+    }
+    for (uint32_t c0 = lane; c0 < m; c0 += 128) {
+      // Four candidates a lane at a time (past the end: the last, its rank unused).
+      RankCandidate own[4];
+      uint32_t rank[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        own[i] = cand[min(c0 + 32 * i, m - 1)];
+        rank[i] = 0;
+      }
+      const uint32_t in_use = (m - c0 + 31) / 32;
+      for (uint32_t o = 0; o < m; ++o) {
+        const RankCandidate other = cand[o];
+        rank[0] = count_before(rank[0], other, own[0]);
+        rank[1] = count_before(rank[1], other, own[1]);
+        if (in_use > 2) {
+          rank[2] = count_before(rank[2], other, own[2]);
+          rank[3] = count_before(rank[3], other, own[3]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (c0 + 32 * i < m && rank[i] < k) {
+          out_key[q * (uint64_t)k + rank[i]] = own[i].key;
+          out_row[q * (uint64_t)k + rank[i]] = own[i].row;
+        }
+    }
+    const bool any_bad = __any_sync(0xFFFFFFFFu, bad);
+    if (lane == 0) {
+      atomicAdd(n_candidates, (unsigned long long)kept);
+      full_flag[q] = (any_bad || kept < k) ? 1u : 0u;
+    }
+    return;
+  }
   double keys[kMaxK];
   uint32_t idx[kMaxK];
   uint32_t len = 0;
@@ -847,23 +1016,29 @@ __global__ void full_rows_kernel(const float* __restrict__ x, uint64_t n, uint32
   }
 }
 
-// Each row's ranked entries sorted by row index, distances f32(sqrt(key))
-// (neighbors.rs:412-435).
-__global__ void graph_kernel(const double* keys, const uint32_t* rows, uint64_t n,
-                             uint32_t k, uint64_t* indptr, uint32_t* indices,
-                             float* distances) {
-  uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (r == 0) indptr[0] = 0;
-  if (r >= n) return;
-  indptr[r + 1] = (r + 1) * (uint64_t)k;
-  const double* kr = keys + r * k;
-  const uint32_t* rr = rows + r * k;
-  uint32_t* oi = indices + r * k;
-  float* od = distances + r * k;
-  // Insertion by row index (k is small; rows are distinct).
+// A row's ranked entries sorted by row index, distances f32(sqrt(key)) (neighbors.rs:412-435),
+// at oi / od, rows counted from `first`; a warp, k <= 32: an entry's place is the number of
+// smaller rows. (A thread a row, inserting in global memory: 0.8 ms for 1M rows of 14.)
+__device__ __forceinline__ void graph_row(const double* kr, const uint32_t* rr, uint32_t k,
+                                          uint32_t first, uint32_t* oi, float* od) {
+  const unsigned lane = threadIdx.x & 31u;
+  const bool in = lane < k;
+  const uint32_t row = in ? rr[lane] - first : 0xFFFFFFFFu;
+  uint32_t at = 0;
+  for (uint32_t j = 0; j < k; ++j) at += __shfl_sync(0xFFFFFFFFu, row, j) < row ? 1u : 0u;
+  if (in) {
+    oi[at] = row;
+    od[at] = (float)sqrt(kr[lane]);
+  }
+}
+
+// The same by one thread, any k.
+__device__ __forceinline__ void graph_row_serial(const double* kr, const uint32_t* rr, uint32_t k,
+                                                 uint32_t first, uint32_t* oi, float* od) {
+  // Insertion by row index (rows are distinct).
   for (uint32_t i = 0; i < k; ++i) {
-    uint32_t row = rr[i];
-    float dist = (float)sqrt(kr[i]);
+    const uint32_t row = rr[i] - first;
+    const float dist = (float)sqrt(kr[i]);
     uint32_t at = i;
     while (at > 0 && oi[at - 1] > row) {
       oi[at] = oi[at - 1];
@@ -873,6 +1048,42 @@ __global__ void graph_kernel(const double* keys, const uint32_t* rows, uint64_t 
     oi[at] = row;
     od[at] = dist;
   }
+}
+
+// The graph's rows: a warp a row (Warp) or a thread a row. With a batch, sample s's CSR:
+// indptr of n_s + 1 entries at indptr + first[s] + s, columns relative to its first row.
+template <bool Warp>
+__global__ void __launch_bounds__(256)
+graph_kernel(const double* keys, const uint32_t* rows, uint64_t n, uint32_t k,
+             const uint32_t* row_sample, const uint64_t* first, uint64_t* indptr,
+             uint32_t* indices, float* distances) {
+  const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const uint64_t r = Warp ? t >> 5 : t;
+  if (r >= n) return;
+  const uint32_t smp = row_sample ? row_sample[r] : 0;
+  const uint64_t f = row_sample ? first[smp] : 0;
+  if (!Warp || (threadIdx.x & 31u) == 0) {
+    uint64_t* ip = indptr + f + smp;
+    if (r == f) ip[0] = 0;
+    ip[r - f + 1] = (r - f + 1) * (uint64_t)k;
+  }
+  if (Warp)
+    graph_row(keys + r * k, rows + r * k, k, (uint32_t)f, indices + r * k, distances + r * k);
+  else
+    graph_row_serial(keys + r * k, rows + r * k, k, (uint32_t)f, indices + r * k,
+                     distances + r * k);
+}
+
+void launch_graph(const double* keys, const uint32_t* rows, uint64_t n, uint32_t k,
+                  const uint32_t* row_sample, const uint64_t* first, uint64_t* indptr,
+                  uint32_t* indices, float* distances, cudaStream_t s) {
+  if (k <= 32)
+    graph_kernel<true><<<blocks_for(n * 32, 256), 256, 0, s>>>(keys, rows, n, k, row_sample,
+                                                               first, indptr, indices, distances);
+  else
+    graph_kernel<false><<<blocks_for(n, 256), 256, 0, s>>>(keys, rows, n, k, row_sample, first,
+                                                           indptr, indices, distances);
+  KG_LAUNCH_CHECK();
 }
 
 __global__ void compact_flags_kernel(const uint32_t* flag, uint64_t n, uint32_t* list,
@@ -1183,14 +1394,10 @@ FilterChoice tune_filter_kind(kg_ctx* ctx, cudaStream_t s, const float* x, uint6
 void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t d, uint32_t k,
               const PlanBuilder* plan, KnnResult& out, Trace& trace, const KnnBatch* batch) {
   cudaStream_t s = ctx->stream;
-  DeviceBuffer<double> mean(d, s), squares(n, s), slack(n, s), largest(1, s);
-  DeviceBuffer<float> rows(n * kDim, s), offsets(n, s), lo_hi(6, s);
+  DeviceBuffer<double> mean(d, s), largest(1, s);
+  DeviceBuffer<float> lo_hi(6, s);
   column_stats(x, n, width, d, mean.ptr, lo_hi.ptr, s);
-  centre_kernel<<<blocks_for(n, 128), 128, 0, s>>>(x, n, width, d, mean.ptr, rows.ptr,
-                                                   offsets.ptr, squares.ptr);
-  max_kernel_launch(squares.ptr, n, largest.ptr, s);
-  slack_kernel<<<blocks_for(n, 256), 256, 0, s>>>(squares.ptr, n, d, largest.ptr, slack.ptr);
-  KG_LAUNCH_CHECK();
+  centred_max(x, n, width, d, mean.ptr, largest.ptr, s);
   double h_largest = 0;
   KG_CUDA(cudaMemcpyAsync(&h_largest, largest.ptr, 8, cudaMemcpyDeviceToHost, s));
   KG_CUDA(cudaStreamSynchronize(s));
@@ -1231,9 +1438,9 @@ void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t 
     uint32_t* cand_row = reinterpret_cast<uint32_t*>(ctx->knn_ws.ptr + slice);
     DeviceBuffer<float> thr(n, s);
     DeviceBuffer<uint32_t> cand_count(n, s);
-    DeviceBuffer<double> qn2(n, s), slack_d(n, s), max_sq(1, s);
+    DeviceBuffer<double> qn2(n, s), slack_d(n, s);
     Timer tf(s);
-    const double scale = tc_scale(x, n, width, d, mean.ptr, max_sq.ptr, s);
+    const double scale = tc_scale(h_largest);
     ScanPlan sp;
     DeviceBuffer<uint32_t> slot_sample;
     if (plan) {
@@ -1310,7 +1517,7 @@ void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t 
     const uint32_t* prows = sp.prows.ptr ? sp.prows.ptr : sp.qrows.ptr;
     if (filter == "auto") {
       const FilterChoice fc = tune_filter_kind(ctx, s, x, n, width, d, k, sp, scan, prows,
-                                               mean.ptr, scale, max_sq.ptr);
+                                               mean.ptr, scale, largest.ptr);
       kind = fc.kind;
       scan.a_mode = fc.a_mode;
       trace.mark("filter tuning");
@@ -1319,7 +1526,7 @@ void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t 
     DeviceBuffer<unsigned long long> tiles(1, s);
     tiles.zero();
     scan.tiles_scanned = tiles.ptr;
-    tc_filter(ctx, s, x, width, d, sp.qrows.ptr, prows, scan, mean.ptr, scale, max_sq.ptr,
+    tc_filter(ctx, s, x, width, d, sp.qrows.ptr, prows, scan, mean.ptr, scale, largest.ptr,
               kind, k, cap, cand_key, cand_row, cand_count.ptr, thr.ptr,
               qn2.ptr, slack_d.ptr, &trace, &point_ops);
     if (sp.q_full.ptr) {
@@ -1415,7 +1622,7 @@ void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t 
       DeviceBuffer<uint32_t> r_row(mv * copy_cap, s), r_count(mv, s);
       DeviceBuffer<double> r_qn2(mv, s), r_slack(mv, s);
       Timer trf(s);
-      tc_filter(ctx, s, x, width, d, r_qrows.ptr, prows, rs, mean.ptr, scale, max_sq.ptr, kind,
+      tc_filter(ctx, s, x, width, d, r_qrows.ptr, prows, rs, mean.ptr, scale, largest.ptr, kind,
                 k, copy_cap, r_key.ptr, r_row.ptr, r_count.ptr, r_thr.ptr, r_qn2.ptr,
                 r_slack.ptr, nullptr, &point_ops);
       filter_ms += trf.stop_ms();
@@ -1453,6 +1660,15 @@ void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t 
     trace.mark("overflow retry");
     ctx->done = n;
   } else {
+    // The SIMT filter's operands: centred f32 rows, their norms, kyto's slacks.
+    DeviceBuffer<double> squares(n, s), slack(n, s);
+    DeviceBuffer<float> rows(n * kDim, s), offsets(n, s);
+    centre_kernel<<<blocks_for(n, 128), 128, 0, s>>>(x, n, width, d, mean.ptr, rows.ptr,
+                                                     offsets.ptr, squares.ptr);
+    KG_LAUNCH_CHECK();
+    max_kernel_launch(squares.ptr, n, largest.ptr, s);
+    slack_kernel<<<blocks_for(n, 256), 256, 0, s>>>(squares.ptr, n, d, largest.ptr, slack.ptr);
+    KG_LAUNCH_CHECK();
     const uint32_t cap = kCandidateCap;
     uint64_t chunk = std::min<uint64_t>(n, kQueryChunk);
     DeviceBuffer<float> cand_key(chunk * cap, s), thr(chunk, s);
@@ -1547,37 +1763,6 @@ void check_finite(const float* x, uint64_t n, uint32_t width, uint32_t d, cudaSt
                              std::to_string(first % width) + " is not finite");
 }
 
-// A batch's graphs: sample s's CSR (indptr of n_s + 1 entries at indptr + first[s] + s,
-// columns relative to its first row) and entries at first[s] * k, rows sorted by column.
-__global__ void batch_graph_kernel(const double* keys, const uint32_t* rows, uint64_t n,
-                                   uint32_t k, const uint32_t* row_sample,
-                                   const uint64_t* first, uint64_t* indptr, uint32_t* indices,
-                                   float* distances) {
-  uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  const uint32_t smp = row_sample[r];
-  const uint64_t f = first[smp];
-  uint64_t* ip = indptr + f + smp;
-  if (r == f) ip[0] = 0;
-  ip[r - f + 1] = (r - f + 1) * (uint64_t)k;
-  const double* kr = keys + r * k;
-  const uint32_t* rr = rows + r * k;
-  uint32_t* oi = indices + r * k;
-  float* od = distances + r * k;
-  for (uint32_t i = 0; i < k; ++i) {
-    const uint32_t row = rr[i] - (uint32_t)f;
-    const float dist = (float)sqrt(kr[i]);
-    uint32_t at = i;
-    while (at > 0 && oi[at - 1] > row) {
-      oi[at] = oi[at - 1];
-      od[at] = od[at - 1];
-      --at;
-    }
-    oi[at] = row;
-    od[at] = dist;
-  }
-}
-
 // The CSR graph (rows sorted by column, f32 sqrt of the key) into host or device memory.
 void write_graph(const KnnResult& r, uint64_t n, uint32_t k, uint64_t* indptr, uint32_t* indices,
                  float* distances, cudaStream_t s) {
@@ -1596,8 +1781,7 @@ void write_graph(const KnnResult& r, uint64_t n, uint32_t k, uint64_t* indptr, u
     gx = g_idx.ptr;
     gd = g_dist.ptr;
   }
-  graph_kernel<<<blocks_for(n, 128), 128, 0, s>>>(r.key.ptr, r.row.ptr, n, k, gi, gx, gd);
-  KG_LAUNCH_CHECK();
+  launch_graph(r.key.ptr, r.row.ptr, n, k, nullptr, nullptr, gi, gx, gd, s);
   if (!dev_out) {
     KG_CUDA(cudaMemcpyAsync(indptr, gi, (n + 1) * 8, cudaMemcpyDeviceToHost, s));
     KG_CUDA(cudaMemcpyAsync(indices, gx, n * k * 4, cudaMemcpyDeviceToHost, s));
@@ -1643,10 +1827,7 @@ void knn_batch_run(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint
     gx = g_idx.ptr;
     gd = g_dist.ptr;
   }
-  batch_graph_kernel<<<blocks_for(n, 128), 128, 0, s>>>(r.key.ptr, r.row.ptr, n, k,
-                                                        batch.row_sample.ptr, batch.d_first.ptr,
-                                                        gi, gx, gd);
-  KG_LAUNCH_CHECK();
+  launch_graph(r.key.ptr, r.row.ptr, n, k, batch.row_sample.ptr, batch.d_first.ptr, gi, gx, gd, s);
   if (!dev_out) {
     KG_CUDA(cudaMemcpyAsync(indptr, gi, (n + n_samples) * 8, cudaMemcpyDeviceToHost, s));
     KG_CUDA(cudaMemcpyAsync(indices, gx, n * k * 4, cudaMemcpyDeviceToHost, s));

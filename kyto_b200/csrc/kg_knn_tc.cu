@@ -1013,17 +1013,23 @@ __global__ void tc_split_operands_kernel(const float* x, uint64_t n, uint32_t wi
   slack2[r] = round_up_f32d(2.0 * e);
 }
 
-// The largest centred squared norm, f64.
-__global__ void centred_norm_kernel(const float* x, uint64_t n, uint32_t width, uint32_t d,
-                                    const double* mean, double* sq) {
+// *out = max(*out, the rows' centred squared norms), f64: norms >= 0, so their bit patterns
+// order as the values do (*out starts at 0; a NaN's are above infinity's).
+__global__ void centred_max_kernel(const float* x, uint64_t n, uint32_t width, uint32_t d,
+                                   const double* mean, unsigned long long* out) {
   uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (r >= n) return;
   double s = 0.0;
-  for (uint32_t j = 0; j < d; ++j) {
-    double c = (double)x[r * width + j] - mean[j];
-    s += c * c;
+  if (r < n)
+    for (uint32_t j = 0; j < d; ++j) {
+      double c = (double)x[r * width + j] - mean[j];
+      s += c * c;
+    }
+  unsigned long long m = (unsigned long long)__double_as_longlong(s) & 0x7FFFFFFFFFFFFFFFull;
+  for (int o = 16; o; o >>= 1) {
+    const unsigned long long t = __shfl_xor_sync(0xFFFFFFFFu, m, o);
+    m = t > m ? t : m;
   }
-  sq[r] = s;
+  if ((threadIdx.x & 31u) == 0) atomicMax(out, m);
 }
 
 // ------------------------------------------------------------------ host -----------
@@ -1065,16 +1071,15 @@ CUtensorMap tile_map(const void* base, uint64_t rows, bool bf16, uint32_t cols =
 
 }  // namespace
 
-double tc_scale(const float* x, uint64_t n, uint32_t width, uint32_t d, const double* mean,
-                double* max_sq, cudaStream_t s) {
-  if (d + 3 > (uint32_t)kTcK) fail(KG_ERR_INVALID, "tensor-core filter: more than 61 components");
-  DeviceBuffer<double> sq(n, s);
-  centred_norm_kernel<<<blocks_for(n, 256), 256, 0, s>>>(x, n, width, d, mean, sq.ptr);
+void centred_max(const float* x, uint64_t n, uint32_t width, uint32_t d, const double* mean,
+                 double* max_sq, cudaStream_t s) {
+  KG_CUDA(cudaMemsetAsync(max_sq, 0, sizeof(double), s));
+  centred_max_kernel<<<blocks_for(n, 256), 256, 0, s>>>(
+      x, n, width, d, mean, reinterpret_cast<unsigned long long*>(max_sq));
   KG_LAUNCH_CHECK();
-  max_kernel_launch(sq.ptr, n, max_sq, s);
-  double h_max = 0.0;
-  KG_CUDA(cudaMemcpyAsync(&h_max, max_sq, 8, cudaMemcpyDeviceToHost, s));
-  KG_CUDA(cudaStreamSynchronize(s));
+}
+
+double tc_scale(double h_max) {
   // Scale so that the largest centred row norm is at most 2^7: squared norms stay below
   // 2^14 (fp16's range) and -2q below 2^8.
   double scale = 1.0;

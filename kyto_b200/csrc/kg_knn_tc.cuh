@@ -60,10 +60,13 @@ struct FilterScan {
   double s2 = 1.0;                       // scale^2 (set by tc_filter)
 };
 
-// The power-of-two scale of the filter's operands (the largest centred row norm of x's
-// n rows scaled to at most 2^7), and that largest squared norm on the device (max_sq).
-double tc_scale(const float* x, uint64_t n, uint32_t width, uint32_t d, const double* mean,
-                double* max_sq, cudaStream_t s);
+// The largest squared norm of x's n centred rows, on the device (max_sq).
+void centred_max(const float* x, uint64_t n, uint32_t width, uint32_t d, const double* mean,
+                 double* max_sq, cudaStream_t s);
+
+// The power-of-two scale of the filter's operands: the largest centred row norm (its square
+// h_max) scaled to at most 2^7.
+double tc_scale(double h_max);
 
 // Fills cand_key/cand_row (n_q x cap), cand_count and threshold (n_q) for every query
 // slot, and per query slot qn2 (the centred squared norm) and slack_d (the bound of
@@ -75,7 +78,5 @@ void tc_filter(kg_ctx* ctx, cudaStream_t s, const float* x, uint32_t width, uint
                uint32_t k, uint32_t cap, float* cand_key, uint32_t* cand_row,
                uint32_t* cand_count, float* threshold, double* qn2, double* slack_d,
                Trace* trace = nullptr, DeviceBuffer<uint16_t>* point_ops = nullptr);
-
-void max_kernel_launch(const double* v, uint64_t n, double* out, cudaStream_t s);
 
 }  // namespace kg
