@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 
 #include "kg_sm100.cuh"
 #include "kg_tma.cuh"
@@ -16,13 +17,108 @@ using namespace sm100;
 
 namespace {
 
-constexpr int kBM = 64, kBN = 64, kBK = 16;  // GEMM block tile
-constexpr int kGemmThreads = 256;            // 16 x 16 threads, 4 x 4 outputs each
+constexpr int kBM = 64, kBN = 64, kBK = 32;  // GEMM block tile
+constexpr int kSliceStep = 16;               // slices of a long K: multiples of this
+constexpr int kGemmThreads = 128;            // 8 x 16 threads, 8 x 4 outputs each
 
 enum : int { kEpiStore = 0, kEpiBiasReluBf16 = 1, kEpiMaskRelu = 2, kEpiBias = 3 };
 
 __device__ __forceinline__ float as_f32(float v) { return v; }
 __device__ __forceinline__ float as_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+// Four elements of an operand as they were read (a widening of bf16 waits for the read, so it
+// happens when the tile is stored).
+template <class T>
+struct Four;
+template <>
+struct Four<float> {
+  float4 raw;
+};
+template <>
+struct Four<__nv_bfloat16> {
+  uint2 raw;
+};
+
+// The first `count` of four elements from p on, one by one (zeros past those).
+__device__ __forceinline__ Four<float> some_of_four(const float* p, int count) {
+  return {make_float4(count > 0 ? p[0] : 0.0f, count > 1 ? p[1] : 0.0f, count > 2 ? p[2] : 0.0f,
+                      count > 3 ? p[3] : 0.0f)};
+}
+__device__ __forceinline__ Four<__nv_bfloat16> some_of_four(const __nv_bfloat16* p, int count) {
+  uint32_t b[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) b[i] = i < count ? (uint32_t)__bfloat16_as_ushort(p[i]) : 0u;
+  return {make_uint2(b[0] | b[1] << 16, b[2] | b[3] << 16)};
+}
+
+__device__ __forceinline__ float low_bf16(uint32_t u) { return __uint_as_float(u << 16); }
+__device__ __forceinline__ float high_bf16(uint32_t u) { return __uint_as_float(u & 0xFFFF0000u); }
+
+// The tiles in shared memory: A's as f32, B's as bf16.
+__device__ __forceinline__ void put_four(float* t, const Four<float>& v) {
+  *reinterpret_cast<float4*>(t) = v.raw;
+}
+__device__ __forceinline__ void put_four(float* t, const Four<__nv_bfloat16>& v) {
+  *reinterpret_cast<float4*>(t) = make_float4(low_bf16(v.raw.x), high_bf16(v.raw.x),
+                                              low_bf16(v.raw.y), high_bf16(v.raw.y));
+}
+__device__ __forceinline__ void put_four(uint16_t* t, const Four<__nv_bfloat16>& v) {
+  *reinterpret_cast<uint2*>(t) = v.raw;
+}
+__device__ __forceinline__ void put_one(float* t, const Four<float>& v, int i) {
+  *t = i == 0 ? v.raw.x : i == 1 ? v.raw.y : i == 2 ? v.raw.z : v.raw.w;
+}
+__device__ __forceinline__ void put_one(float* t, const Four<__nv_bfloat16>& v, int i) {
+  const uint32_t u = i < 2 ? v.raw.x : v.raw.y;
+  *t = i & 1 ? high_bf16(u) : low_bf16(u);
+}
+__device__ __forceinline__ void put_one(uint16_t* t, const Four<__nv_bfloat16>& v, int i) {
+  const uint32_t u = i < 2 ? v.raw.x : v.raw.y;
+  *t = (uint16_t)(i & 1 ? u >> 16 : u);
+}
+
+// A kBK x 64 tile of an operand: kFours fours a thread, along k (KC: k is the contiguous
+// direction; two lanes a sector, and a warp's stores meet no bank twice) or along the other.
+// `Full`: the tile lies inside the matrix and its fours are
+// aligned (one read each).
+constexpr int kFours = kBK * 64 / 4 / kGemmThreads;
+
+template <bool KC, bool Full, class T>
+__device__ __forceinline__ void load_tile(const T* src, size_t ld, int x0, int X, int k0, int k_end,
+                                          Four<T> (&v)[kFours]) {
+#pragma unroll
+  for (int e = 0; e < kFours; ++e) {
+    const int idx = threadIdx.x + e * kGemmThreads;  // 0..511
+    const int x = x0 + (KC ? (idx >> 1) & 63 : (idx & 15) * 4);
+    const int k = k0 + (KC ? (idx & 1) * 4 + (idx >> 7) * 8 : idx >> 4);
+    const T* p = src + (KC ? x * ld + k : k * ld + x);
+    if (Full) {
+      v[e].raw = *reinterpret_cast<const decltype(v[e].raw)*>(p);
+    } else {
+      const int count = KC ? (x < X ? k_end - k : 0) : (k < k_end ? X - x : 0);
+      v[e] = some_of_four(p, count);
+    }
+  }
+}
+
+template <bool KC, int kLd, class S, class T>
+__device__ __forceinline__ void store_tile(S (*t)[kLd], const Four<T> (&v)[kFours]) {
+#pragma unroll
+  for (int e = 0; e < kFours; ++e) {
+    const int idx = threadIdx.x + e * kGemmThreads;
+    if (KC) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) put_one(&t[(idx & 1) * 4 + (idx >> 7) * 8 + i][(idx >> 1) & 63], v[e], i);
+    } else {
+      put_four(&t[idx >> 4][(idx & 15) * 4], v[e]);
+    }
+  }
+}
+
+template <class T>
+__device__ __forceinline__ bool wide_rows(const T* p, int ld) {
+  return ld % 4 == 0 && reinterpret_cast<uintptr_t>(p) % (4 * sizeof(T)) == 0;
+}
 
 // C (M x N, row stride ldc) = op(A) (M x K) . op(B) (K x N), f32 sums of bf16 or f32
 // operands in k order per output (each output is one thread's running sum over the k
@@ -32,80 +128,89 @@ __device__ __forceinline__ float as_f32(__nv_bfloat16 v) { return __bfloat162flo
 // Split over K (gridDim.z > 1, the store epilogue only): slice z sums k in
 // [z * kslice, (z + 1) * kslice) and writes its M x N partial at C + z * M * N (row
 // stride N); split_sum_kernel then adds the slices in order.
+//
+// The gradients' f32 operand and their order of summation keep this off the tensor cores. The
+// weight gradients' slices over k leave 14 warps' worth of 8 x 4 outputs to an SM's two CTAs
+// (8 x 8 a thread: half the warps, and the waits for reads show: 149 us), so latency bounds
+// it before the multiply-adds (two columns an instruction) do: the next 32 k's reads are on
+// their way while these are multiplied (16 k: 157 us), B's tile stays bf16 in shared memory.
+// P x h x rows = 1,024 x 256 x 8,192: 264 us with 4 x 4 outputs a thread, a read and a
+// barrier behind each 16 k; now 122 (82 at the multiply-adds' measured rate); rows x h x P
+// with the mask: 172 us, now 125.
 template <class TA, class TB, bool TRA, bool TRB, int EPI>
 __global__ void __launch_bounds__(kGemmThreads)
 gemm_kernel(int M, int N, int K, const TA* __restrict__ A, int lda, const TB* __restrict__ B,
             int ldb, float* __restrict__ C, int ldc, const float* __restrict__ bias,
             __nv_bfloat16* __restrict__ h, int ldh, const float* __restrict__ z, int ldz,
             int kslice) {
-  __shared__ float as[kBK][kBM + 4];
-  __shared__ float bs[kBK][kBN + 4];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  __shared__ __align__(16) float as[2][kBK][kBM + 4];
+  __shared__ __align__(16) uint16_t bs[2][kBK][kBN + 8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int ty = (lane >> 3) + 4 * (w & 1), tx = (lane & 7) + 8 * (w >> 1);
   const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
   const int k_begin = (int)blockIdx.z * kslice, k_end = min(K, k_begin + kslice);
   if (gridDim.z > 1) {
     C += (size_t)blockIdx.z * M * N;
     ldc = N;
   }
-  float acc[4][4];
+  float2 acc[8][2];  // columns 2 j and 2 j + 1
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-  for (int k0 = k_begin; k0 < k_end; k0 += kBK) {
-    // 64 x 16 of A and 16 x 64 of B, 4 elements a thread each.
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int idx = threadIdx.x + e * kGemmThreads;  // 0..1023
-      int mm, kk;
-      if (TRA) {  // consecutive threads along m
-        mm = idx & 63;
-        kk = idx >> 6;
-      } else {    // consecutive threads along k
-        kk = idx & 15;
-        mm = idx >> 4;
+    for (int j = 0; j < 2; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+  auto run = [&](auto full_a, auto full_b) {
+    constexpr bool FA = decltype(full_a)::value, FB = decltype(full_b)::value;
+    Four<TA> va[kFours];
+    Four<TB> vb[kFours];
+    load_tile<!TRA, FA>(A, (size_t)lda, m0, M, k_begin, k_end, va);
+    load_tile<TRB, FB>(B, (size_t)ldb, n0, N, k_begin, k_end, vb);
+    int half = 0;
+    for (int k0 = k_begin; k0 < k_end; k0 += kBK, half ^= 1) {
+      // (A tile's buffer was last read two tiles ago, before the barrier in between.)
+      store_tile<!TRA>(as[half], va);
+      store_tile<TRB>(bs[half], vb);
+      __syncthreads();
+      if (k0 + kBK < k_end) {
+        load_tile<!TRA, FA>(A, (size_t)lda, m0, M, k0 + kBK, k_end, va);
+        load_tile<TRB, FB>(B, (size_t)ldb, n0, N, k0 + kBK, k_end, vb);
       }
-      const int gm = m0 + mm, gk = k0 + kk;
-      float v = 0.0f;
-      if (gm < M && gk < k_end) v = as_f32(TRA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk]);
-      as[kk][mm] = v;
-      int nn, kb;
-      if (TRB) {
-        kb = idx & 15;
-        nn = idx >> 4;
-      } else {
-        nn = idx & 63;
-        kb = idx >> 6;
+#pragma unroll
+      for (int kk = 0; kk < kBK; ++kk) {
+        const float4 a0 = *reinterpret_cast<const float4*>(&as[half][kk][ty * 8]);
+        const float4 a1 = *reinterpret_cast<const float4*>(&as[half][kk][ty * 8 + 4]);
+        const uint2 u = *reinterpret_cast<const uint2*>(&bs[half][kk][tx * 4]);
+        const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        const uint32_t raw[2] = {u.x, u.y};
+        float2 b[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) b[j] = make_float2(low_bf16(raw[j]), high_bf16(raw[j]));
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            acc[i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[i][j]);
       }
-      const int gn = n0 + nn, gkb = k0 + kb;
-      float w = 0.0f;
-      if (gn < N && gkb < k_end) w = as_f32(TRB ? B[(size_t)gn * ldb + gkb] : B[(size_t)gkb * ldb + gn]);
-      bs[kb][nn] = w;
     }
-    __syncthreads();
+  };
+  // Whole, aligned tiles read four elements at a time; the rest one by one.
+  const bool whole_k = k_end > k_begin && (k_end - k_begin) % kBK == 0;
+  const bool full_a = whole_k && m0 + kBM <= M && wide_rows(A, lda);
+  const bool full_b = whole_k && n0 + kBN <= N && wide_rows(B, ldb);
+  if (full_a && full_b)
+    run(std::true_type{}, std::true_type{});
+  else if (full_a)
+    run(std::true_type{}, std::false_type{});
+  else
+    run(std::false_type{}, std::false_type{});
 #pragma unroll
-    for (int kk = 0; kk < kBK; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = as[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + ty * 4 + i;
+  for (int i = 0; i < 8; ++i) {
+    const int gm = m0 + ty * 8 + i;
     if (gm >= M) continue;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int gn = n0 + tx * 4 + j;
       if (gn >= N) continue;
-      float v = acc[i][j];
+      float v = j & 1 ? acc[i][j / 2].y : acc[i][j / 2].x;
       if (EPI == kEpiBiasReluBf16 || EPI == kEpiBias) v += bias[gn];
       if (EPI == kEpiMaskRelu) v = z[(size_t)gm * ldz + gn] > 0.0f ? v : 0.0f;
       C[(size_t)gm * ldc + gn] = v;
@@ -135,9 +240,9 @@ void gemm(int M, int N, int K, const TA* A, int lda, const TB* B, int ldb, float
   int splits = 1;
   if (EPI == kEpiStore) {
     const int tiles = (int)(grid.x * grid.y);
-    while (tiles * splits < 256 && K / (splits * 2) >= 4 * kBK) splits *= 2;
+    while (tiles * splits < 256 && K / (splits * 2) >= 4 * kSliceStep) splits *= 2;
   }
-  const int kslice = ((K + splits - 1) / splits + kBK - 1) / kBK * kBK;
+  const int kslice = ((K + splits - 1) / splits + kSliceStep - 1) / kSliceStep * kSliceStep;
   grid.z = splits;
   if (splits == 1) {
     gemm_kernel<TA, TB, TRA, TRB, EPI><<<grid, kGemmThreads, 0, s>>>(
@@ -336,21 +441,49 @@ __global__ void softmax_xent_kernel(const float* z, uint32_t rows, uint32_t part
 }
 
 // out[c] = sum over rows of a[r * ld + c], 16 row classes per column summed in order,
-// then the classes in order.
-__global__ void __launch_bounds__(1024)
-column_sums_kernel(const float* a, uint32_t rows, uint32_t cols, uint32_t ld, float* out) {
-  __shared__ float part[16][64];
-  const uint32_t c = blockIdx.x * 64 + (threadIdx.x & 63u), cls = threadIdx.x >> 6;
+// then the classes in order. Eight columns a block (a sector a row) and a class of one column
+// a thread: the sum is one chain, so the next kSumAhead rows' reads are on their way while
+// it adds, and the columns spread over the chip. (64 columns a block, a read at a time: 67 us
+// for 8,192 x 1,024.)
+constexpr int kSumColumns = 8, kSumAhead = 64;
+
+__global__ void __launch_bounds__(16 * kSumColumns)
+column_sums_kernel(const float* __restrict__ a, uint32_t rows, uint32_t cols, uint32_t ld,
+                   float* out) {
+  __shared__ float part[16][kSumColumns];
+  const uint32_t j = threadIdx.x % kSumColumns, cls = threadIdx.x / kSumColumns;
+  const uint32_t c = blockIdx.x * kSumColumns + j;
   float t = 0.0f;
-  if (c < cols)
-    for (uint32_t r = cls; r < rows; r += 16) t += a[(uint64_t)r * ld + c];
-  part[cls][threadIdx.x & 63u] = t;
+  if (c < cols && cls < rows) {
+    const uint32_t n = (rows - cls + 15) / 16;  // the class's rows
+    const float* p = a + (uint64_t)cls * ld + c;
+    const uint64_t step = 16 * (uint64_t)ld;
+    float v[kSumAhead];
+#pragma unroll
+    for (uint32_t i = 0; i < kSumAhead; ++i) v[i] = i < n ? p[i * step] : 0.0f;
+    p += kSumAhead * step;
+    for (uint32_t r = 0; r < n; r += kSumAhead, p += kSumAhead * step) {
+#pragma unroll
+      for (uint32_t i = 0; i < kSumAhead; ++i) {
+        if (r + i < n) t += v[i];
+        v[i] = r + kSumAhead + i < n ? p[i * step] : 0.0f;
+      }
+    }
+  }
+  part[cls][j] = t;
   __syncthreads();
   if (cls == 0 && c < cols) {
     float u = 0.0f;
-    for (int k = 0; k < 16; ++k) u += part[k][threadIdx.x & 63u];
+    for (int k = 0; k < 16; ++k) u += part[k][j];
     out[c] = u;
   }
+}
+
+void column_sums(const float* a, uint32_t rows, uint32_t cols, uint32_t ld, float* out,
+                 cudaStream_t s) {
+  column_sums_kernel<<<(cols + kSumColumns - 1) / kSumColumns, 16 * kSumColumns, 0, s>>>(
+      a, rows, cols, ld, out);
+  KG_LAUNCH_CHECK();
 }
 
 __global__ void adam_kernel(float* p, const float* g, float* m, float* v, uint64_t n, float lr,
@@ -613,24 +746,21 @@ void Mlp::backward(const uint32_t* labels, uint32_t L, MlpBatch& b, cudaStream_t
   // Layer 3: dW3 = dz3^T h2 (P x h), db3 = column sums of dz3, dz2 = (dz3 W3) * (z2 > 0).
   gemm<float, __nv_bfloat16, true, false, kEpiStore>(P, h, n, b.dz3.ptr, P, b.h2.ptr, h,
                                                      G + sh.w_off[2], h, s);
-  column_sums_kernel<<<(P + 63) / 64, 1024, 0, s>>>(b.dz3.ptr, n, P, P, G + sh.b_off[2]);
-  KG_LAUNCH_CHECK();
+  column_sums(b.dz3.ptr, n, P, P, G + sh.b_off[2], s);
   gemm<float, __nv_bfloat16, false, false, kEpiMaskRelu>(n, h, P, b.dz3.ptr, P, W + sh.w_off[2],
                                                          h, b.dz2.ptr, h, s, nullptr, nullptr, 0,
                                                          b.z2.ptr, h);
   // Layer 2.
   gemm<float, __nv_bfloat16, true, false, kEpiStore>(h, h, n, b.dz2.ptr, h, b.h1.ptr, h,
                                                      G + sh.w_off[1], h, s);
-  column_sums_kernel<<<(h + 63) / 64, 1024, 0, s>>>(b.dz2.ptr, n, h, h, G + sh.b_off[1]);
-  KG_LAUNCH_CHECK();
+  column_sums(b.dz2.ptr, n, h, h, G + sh.b_off[1], s);
   gemm<float, __nv_bfloat16, false, false, kEpiMaskRelu>(n, h, h, b.dz2.ptr, h, W + sh.w_off[1],
                                                          h, b.dz1.ptr, h, s, nullptr, nullptr, 0,
                                                          b.z1.ptr, h);
   // Layer 1.
   gemm<float, __nv_bfloat16, true, false, kEpiStore>(h, din, n, b.dz1.ptr, h, b.h0.ptr,
                                                      (int)sh.h0_ld(), G + sh.w_off[0], din, s);
-  column_sums_kernel<<<(h + 63) / 64, 1024, 0, s>>>(b.dz1.ptr, n, h, h, G + sh.b_off[0]);
-  KG_LAUNCH_CHECK();
+  column_sums(b.dz1.ptr, n, h, h, G + sh.b_off[0], s);
 }
 
 void Mlp::adam(float lr, cudaStream_t s) {
