@@ -748,10 +748,8 @@ struct TcHeld {
     g = n_genes;
     this->nnz = nnz;
     sm = sm_count;
-    build_blocked(indptr, col, val, n, g, nnz, bx, s);
-    trace.mark("blocked X");
-    transpose_blocked(indptr, col, val, n, g, nnz, bx, bxt, s);
-    trace.mark("blocked X^T");
+    build_blocked(indptr, col, val, n, g, nnz, bx, &bxt, s);
+    trace.mark("blocked X, X^T");
     dt.alloc(64 * dense_ld(n), s);
     dt.zero();
     qt.alloc(64 * dense_ld(g), s);
@@ -1737,12 +1735,8 @@ kg_status kg_diag_spmm(kg_ctx* ctx, const uint64_t* indptr, const uint32_t* indi
     const uint32_t* d_idx = device_view(indices, nnz, hi_idx, s);
     const float* d_val = device_view(values, nnz, hv, s);
     Blocked bx, bxt;
-    build_blocked(d_ptr, d_idx, d_val, n_rows, n_cols, nnz, bx, s);
-    const Blocked* sp = &bx;
-    if (transposed) {
-      transpose_blocked(d_ptr, d_idx, d_val, n_rows, n_cols, nnz, bx, bxt, s);
-      sp = &bxt;
-    }
+    build_blocked(d_ptr, d_idx, d_val, n_rows, n_cols, nnz, bx, transposed ? &bxt : nullptr, s);
+    const Blocked* sp = transposed ? &bxt : &bx;
     const uint64_t rows = sp->rows, K = sp->K, ld = dense_ld(K);
     DeviceBuffer<double> hd;
     int dscale = 0;

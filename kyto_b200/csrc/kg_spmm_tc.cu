@@ -479,31 +479,51 @@ spmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_dt, const uint64_t* __re
 // ------------------------------------------------------------------ builders -------
 
 // Per row: the sum of squared values (f64) into the largest so far, and the largest and
-// smallest nonzero |value| (non-negative doubles compare as their bit patterns).
-__global__ void csr_stats_kernel(const uint64_t* ptr, const float* val, uint64_t n_rows,
-                                 unsigned long long* max_sq, unsigned long long* max_abs,
-                                 unsigned long long* min_abs) {
-  uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  unsigned lane = threadIdx.x & 31u;
-  if (r >= n_rows) return;
-  double sq = 0.0, hi = 0.0, lo = INFINITY;
-  for (uint64_t i = ptr[r] + lane; i < ptr[r + 1]; i += 32) {
-    const double v = fabs((double)val[i]);
-    sq += v * v;
-    hi = fmax(hi, v);
-    if (v > 0.0) lo = fmin(lo, v);
-    if (v != v) hi = v;  // a NaN dominates
+// smallest nonzero |value| (non-negative doubles compare as their bit patterns). Reading the
+// values once bounds it: a warp takes row after row, four reads a lane on their way, and only
+// its own largest and smallest reach the three totals (three atomics a row: 2.9 ms for 1M rows
+// of 570 values, now 0.64).
+constexpr int kStatsAhead = 4;
+
+__global__ void __launch_bounds__(256)
+csr_stats_kernel(const uint64_t* __restrict__ ptr, const float* __restrict__ val, uint64_t n_rows,
+                 unsigned long long* max_sq, unsigned long long* max_abs,
+                 unsigned long long* min_abs) {
+  const unsigned lane = threadIdx.x & 31u;
+  const uint64_t warps = gridDim.x * (uint64_t)(blockDim.x / 32);
+  double best_sq = 0.0;
+  float hi = 0.0f, lo = INFINITY;
+  bool nan = false;
+  for (uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; r < n_rows; r += warps) {
+    const uint64_t end = ptr[r + 1];
+    double sq = 0.0;
+    for (uint64_t i = ptr[r] + lane; i < end; i += 32 * kStatsAhead) {
+      float v[kStatsAhead];
+#pragma unroll
+      for (int k = 0; k < kStatsAhead; ++k) v[k] = i + 32 * k < end ? fabsf(val[i + 32 * k]) : 0.0f;
+#pragma unroll
+      for (int k = 0; k < kStatsAhead; ++k) {
+        const double w = (double)v[k];
+        sq += w * w;  // (zeros past the row's end change nothing)
+        hi = fmaxf(hi, v[k]);
+        if (v[k] > 0.0f) lo = fminf(lo, v[k]);
+        nan = nan || v[k] != v[k];
+      }
+    }
+    for (int o = 16; o; o >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFu, sq, o);
+    // As the totals compare: by bit pattern (a NaN above everything).
+    if (__double_as_longlong(sq) > __double_as_longlong(best_sq)) best_sq = sq;
   }
   for (int o = 16; o; o >>= 1) {
-    sq += __shfl_xor_sync(0xFFFFFFFFu, sq, o);
-    const double h2 = __shfl_xor_sync(0xFFFFFFFFu, hi, o);
-    hi = (hi != hi) ? hi : ((h2 != h2) ? h2 : fmax(hi, h2));
-    lo = fmin(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
+    lo = fminf(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
   }
+  nan = __any_sync(0xFFFFFFFFu, nan);
   if (lane == 0) {
-    atomicMax(max_sq, (unsigned long long)__double_as_longlong(sq));
-    atomicMax(max_abs, (unsigned long long)__double_as_longlong(hi));
-    atomicMin(min_abs, (unsigned long long)__double_as_longlong(lo));
+    atomicMax(max_sq, (unsigned long long)__double_as_longlong(best_sq));
+    atomicMax(max_abs, nan ? 0x7FF8000000000000ull
+                           : (unsigned long long)__double_as_longlong((double)hi));
+    atomicMin(min_abs, (unsigned long long)__double_as_longlong((double)lo));
   }
 }
 
@@ -519,151 +539,169 @@ __device__ __forceinline__ uint2 make_entry(uint32_t w0, uint32_t w1) {
   return make_uint2((w0 & 0xFFFFu) | (w1 << 16), (w0 >> 16) | (w1 & 0xFFFF0000u));
 }
 
-__device__ __forceinline__ uint64_t lower_bound_u32(const uint32_t* a, uint64_t lo, uint64_t hi,
-                                                    uint32_t v) {
-  while (lo < hi) {
-    const uint64_t mid = (lo + hi) >> 1;
-    if (a[mid] < v) lo = mid + 1; else hi = mid;
+// The layouts of a CSR matrix (X: rows = CSR rows) and of its transpose (rows = CSR columns) are
+// filled from one reading: a CTA takes 32 CSR rows, which are a row quarter of X's tile and one
+// chunk of X^T's columns, through a window of columns at a time in shared memory, a warp four
+// rows, the lanes over each row's entries. Reading the entries and writing both layouts bounds
+// it. (Each layout by itself, a lane writing where its entry goes, every entry a sector:
+// masks 3.8 and values 11.0 ms for 1M rows of 570 entries, now 1.4 and 3.8, 3.3 TB/s.)
+constexpr int kLayWarps = 8;                // a CTA
+constexpr int kLayRows = 32 / kLayWarps;    // CSR rows a warp
+constexpr uint32_t kMaskCols = 512;         // columns a window of masks_kernel
+constexpr uint32_t kValueCols = 256;        // and of values_kernel
+
+// Calls f(row, column - c0, value) for the entries of this warp's rows in columns [c0, c_end)
+// that it has not passed yet (`at` to `end`: each row's entries still to come). The value is 0
+// without `Values`.
+template <bool Values, class F>
+__device__ __forceinline__ void walk_window(const uint32_t* __restrict__ col,
+                                            const float* __restrict__ val, uint64_t (&at)[kLayRows],
+                                            const uint64_t (&end)[kLayRows], uint32_t c0,
+                                            uint32_t c_end, F&& f) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  for (;;) {
+    uint32_t c[kLayRows];
+    float v[kLayRows];
+#pragma unroll
+    for (int k = 0; k < kLayRows; ++k) {
+      const uint64_t i = at[k] + lane;
+      c[k] = i < end[k] ? col[i] : 0xFFFFFFFFu;
+      v[k] = Values && i < end[k] ? val[i] : 0.0f;
+    }
+    bool more = false;
+#pragma unroll
+    for (int k = 0; k < kLayRows; ++k) {
+      const bool in = c[k] < c_end;
+      if (in) f(warp * kLayRows + k, c[k] - c0, v[k]);
+      const uint32_t n = __popc(__ballot_sync(0xFFFFFFFFu, in));  // increasing: the first n
+      at[k] += n;
+      more = more || n == 32;
+    }
+    if (!more) break;
   }
-  return lo;
 }
 
-// ----- X: layout rows = CSR rows.
-
-// Header masks: a warp per (tile, row quarter) walks its 32 rows one after another, the
-// lanes over each row's values (coalesced), setting the row's bit in the quarter's words
-// held in shared memory (a window of kMaskWindow chunks at a time); then the words go out
-// 16 per chunk. Within one row every write sets the same bit, so no atomics are needed.
-constexpr uint32_t kMaskWindow = 128;  // K-chunks a pass (8 KB of words a warp)
-constexpr int kMaskWarps = 4;
-
-__global__ void __launch_bounds__(kMaskWarps * 32)
-rows_mask_kernel(const uint64_t* ptr, const uint32_t* col, uint64_t n_rows, uint32_t n_tiles,
-                 uint32_t n_chunks, uint32_t* masks) {
-  __shared__ uint32_t words[kMaskWarps][kMaskWindow * 16];
-  const unsigned lane = threadIdx.x & 31u, wi = threadIdx.x >> 5;
-  const uint64_t wq = (uint64_t)blockIdx.x * kMaskWarps + wi;
-  if (wq >= (uint64_t)n_tiles * 4) return;
-  const uint64_t tile = wq / 4, q = wq % 4;
-  uint32_t* w = words[wi];
-  for (uint32_t c0 = 0; c0 < n_chunks; c0 += kMaskWindow) {
-    const uint32_t nch = min(kMaskWindow, n_chunks - c0);
-    for (uint32_t x = lane; x < nch * 16; x += 32) w[x] = 0;
-    __syncwarp();
-    const uint32_t g_lo = c0 * kChunk, g_hi = (c0 + nch) * kChunk;
-    for (uint32_t j = 0; j < 32; ++j) {
-      const uint64_t r = tile * kRows + q * 32 + j;
-      if (r >= n_rows) break;
-      uint64_t a = ptr[r], e = ptr[r + 1];
-      if (c0 > 0) a = lower_bound_u32(col, a, e, g_lo);
-      for (uint64_t i = a + lane; i < e; i += 32) {
-        const uint32_t c = col[i];
-        if (c >= g_hi) break;
-        const uint32_t x = (c / kChunk - c0) * 16 + (c % kChunk) / 2;
-        w[x] |= 1u << j;
+// Header masks of X (masks, words of 64 a block) and, if masks_t, of X^T: a byte an entry in
+// shared memory, gathered into words by ballots. Every word of both layouts is written. `groups`:
+// groups of 32 columns to pass, at least X's chunks and four times X^T's tiles.
+__global__ void __launch_bounds__(kLayWarps * 32)
+masks_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint64_t n_rows,
+             uint32_t n_chunks, uint32_t n_tiles_t, uint32_t n_chunks_t, uint32_t groups,
+             uint32_t* masks, uint32_t* masks_t) {
+  constexpr uint32_t kLd = kMaskCols / 4 + 1;  // words a row: an odd stride
+  __shared__ uint32_t flags[32][kLd];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint64_t rb = blockIdx.x, tile = rb / 4, q = rb % 4;
+  uint64_t at[kLayRows], end[kLayRows];
+#pragma unroll
+  for (int k = 0; k < kLayRows; ++k) {
+    const uint64_t r = rb * 32 + warp * kLayRows + k;
+    at[k] = r < n_rows ? ptr[r] : 0;
+    end[k] = r < n_rows ? ptr[r + 1] : 0;
+  }
+  for (uint32_t g0 = 0; g0 < groups; g0 += kMaskCols / 32) {
+    for (uint32_t i = threadIdx.x; i < 32 * kLd; i += kLayWarps * 32) (&flags[0][0])[i] = 0;
+    __syncthreads();
+    const uint32_t c0 = g0 * 32;
+    walk_window<false>(col, nullptr, at, end, c0, c0 + kMaskCols, [&](uint32_t row, uint32_t c, float) {
+      reinterpret_cast<unsigned char*>(flags[row])[c] = 1;
+    });
+    __syncthreads();
+    for (uint32_t g = warp; g < kMaskCols / 32 && g0 + g < groups; g += kLayWarps) {
+      if (g0 + g < n_chunks) {  // lane = row
+        uint32_t mine = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+          const uint32_t w = flags[lane][g * 8 + k];
+          const uint32_t even = __ballot_sync(0xFFFFFFFFu, w & 0xFFFFu);
+          const uint32_t odd = __ballot_sync(0xFFFFFFFFu, w >> 16);
+          if (lane == 2 * k) mine = even;
+          if (lane == 2 * k + 1) mine = odd;
+        }
+        if (lane < 16) masks[(tile * n_chunks + g0 + g) * 64 + q * 16 + lane] = mine;
       }
-      __syncwarp();
+      if (masks_t && g0 + g < 4 * n_tiles_t && rb < n_chunks_t) {  // lane = column
+        uint32_t mine = 0;
+#pragma unroll
+        for (uint32_t p = 0; p < 16; ++p) {
+          const uint32_t w =
+              (uint32_t)reinterpret_cast<const unsigned char*>(flags[2 * p])[g * 32 + lane] |
+              reinterpret_cast<const unsigned char*>(flags[2 * p + 1])[g * 32 + lane];
+          const uint32_t any = __ballot_sync(0xFFFFFFFFu, w);
+          if (lane == p) mine = any;
+        }
+        if (lane < 16)
+          masks_t[((uint64_t)((g0 + g) / 4) * n_chunks_t + rb) * 64 + (g0 + g) % 4 * 16 + lane] = mine;
+      }
     }
-    for (uint32_t x = lane; x < nch * 16; x += 32)
-      masks[(tile * n_chunks + c0 + x / 16) * 64 + q * 16 + x % 16] = w[x];
-    __syncwarp();
+    __syncthreads();
   }
 }
 
-// Entries: a warp per CSR row, the lanes over its values; the lane holding a pair's first
-// value writes the whole entry.
-__global__ void rows_values_kernel(const uint64_t* ptr, const uint32_t* col, const float* val,
-                                   uint64_t n_rows, uint32_t n_chunks, const uint32_t* masks,
-                                   const uint16_t* bases, const uint64_t* off, int scale,
-                                   uint8_t* data) {
-  const uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const unsigned lane = threadIdx.x & 31u;
-  if (r >= n_rows) return;
-  const uint64_t tile = r / kRows;
-  const uint32_t q = (uint32_t)((r % kRows) / 32), bit = (uint32_t)(r % 32);
-  const uint32_t below = (1u << bit) - 1u;
-  const uint64_t a = ptr[r], end = ptr[r + 1];
-  for (uint64_t i = a + lane; i < end; i += 32) {
-    const uint32_t c = col[i];
-    // The pair's odd column after its even one: written with it.
-    if (c % 2 == 1 && i > a && col[i - 1] == c - 1) continue;
-    uint32_t w0 = kAbsentHi, w1 = kAbsentHi;
-    if (c % 2 == 0) {
-      w0 = stored_parts(val[i], scale);
-      if (i + 1 < end && col[i + 1] == c + 1) w1 = stored_parts(val[i + 1], scale);
-    } else {
-      w1 = stored_parts(val[i], scale);
-    }
-    const uint64_t b = tile * n_chunks + c / kChunk;
-    const uint64_t h = b * 64 + q * 16 + (c % kChunk) / 2;
-    const uint32_t e = bases[h] + __popc(masks[h] & below);
-    reinterpret_cast<uint2*>(data + off[b] * 16 + kHeaderBytes)[e] = make_entry(w0, w1);
+// A layout as values_kernel writes it.
+struct LayoutOut {
+  const uint32_t* masks;  // null: not wanted
+  const uint16_t* bases;
+  const uint64_t* off;
+  uint8_t* data;
+  uint32_t n_chunks;
+};
+
+// Quarter q of block b: its header words and entries, pair p's parts words as parts(p, 0) and
+// parts(p, 1) in lane = row.
+template <class P>
+__device__ __forceinline__ void write_quarter(const LayoutOut& o, uint64_t b, uint32_t q, P&& parts) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t start = o.off[b];
+  if (o.off[b + 1] == start) return;
+  uint8_t* block = o.data + start * 16;
+  uint32_t mask = 0, base = 0;
+  if (lane < 16) {
+    mask = o.masks[b * 64 + q * 16 + lane];
+    base = o.bases[b * 64 + q * 16 + lane];
+    reinterpret_cast<uint2*>(block)[q * 16 + lane] = make_uint2(mask, base);
+  }
+  uint2* entries = reinterpret_cast<uint2*>(block + kHeaderBytes);
+#pragma unroll 4
+  for (uint32_t p = 0; p < 16; ++p) {
+    const uint32_t m = __shfl_sync(0xFFFFFFFFu, mask, p), first = __shfl_sync(0xFFFFFFFFu, base, p);
+    const uint2 e = make_entry(parts(p, 0), parts(p, 1));
+    if ((m >> lane) & 1u) entries[first + __popc(m & ((1u << lane) - 1u))] = e;
   }
 }
 
-// ----- X^T: layout rows = CSR columns (genes), layout columns = CSR rows (cells). A warp
-// per pair of CSR rows (one column pair of the layout), lane = a group of 32 genes (one
-// header word of one block), found in each row by binary search.
-
-// Header masks: the word of (gene group, cell pair) = the genes of the group either cell
-// holds; each word written once, no atomics.
-__global__ void cols_mask_kernel(const uint64_t* ptr, const uint32_t* col, uint64_t n_rows,
-                                 uint32_t n_cols, uint32_t n_chunks, uint32_t* masks) {
-  const uint64_t pr = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const unsigned lane = threadIdx.x & 31u;
-  const uint64_t r0 = 2 * pr;
-  if (r0 >= n_rows) return;
-  const bool has1 = r0 + 1 < n_rows;
-  const uint64_t a0 = ptr[r0], e0 = ptr[r0 + 1];
-  const uint64_t a1 = has1 ? ptr[r0 + 1] : 0, e1 = has1 ? ptr[r0 + 2] : 0;
-  const uint32_t groups = (n_cols + 31) / 32;
-  const uint64_t kch = r0 / kChunk;
-  const uint32_t p = (uint32_t)((r0 % kChunk) / 2);
-  for (uint32_t gg = lane; gg < groups; gg += 32) {
-    const uint32_t g0 = gg * 32;
-    uint32_t bits = 0;
-    for (uint64_t i = lower_bound_u32(col, a0, e0, g0); i < e0 && col[i] < g0 + 32; ++i)
-      bits |= 1u << (col[i] - g0);
-    for (uint64_t i = lower_bound_u32(col, a1, e1, g0); i < e1 && col[i] < g0 + 32; ++i)
-      bits |= 1u << (col[i] - g0);
-    if (bits) masks[((uint64_t)(gg / 4) * n_chunks + kch) * 64 + (gg % 4) * 16 + p] = bits;
+// Headers and entries of X and, if wanted, of X^T. `groups` as in masks_kernel.
+__global__ void __launch_bounds__(kLayWarps * 32)
+values_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col,
+              const float* __restrict__ val, uint64_t n_rows, uint32_t n_tiles_t, uint32_t groups,
+              int scale, LayoutOut x, LayoutOut t) {
+  __shared__ uint32_t tile[32][kValueCols + 1];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint64_t rb = blockIdx.x;
+  uint64_t at[kLayRows], end[kLayRows];
+#pragma unroll
+  for (int k = 0; k < kLayRows; ++k) {
+    const uint64_t r = rb * 32 + warp * kLayRows + k;
+    at[k] = r < n_rows ? ptr[r] : 0;
+    end[k] = r < n_rows ? ptr[r + 1] : 0;
   }
-}
-
-// Entries: per gene either cell holds, one whole entry (the two cells' parts), merged in
-// gene order.
-__global__ void cols_values_kernel(const uint64_t* ptr, const uint32_t* col, const float* val,
-                                   uint64_t n_rows, uint32_t n_cols, uint32_t n_chunks,
-                                   const uint32_t* masks, const uint16_t* bases,
-                                   const uint64_t* off, int scale, uint8_t* data) {
-  const uint64_t pr = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const unsigned lane = threadIdx.x & 31u;
-  const uint64_t r0 = 2 * pr;
-  if (r0 >= n_rows) return;
-  const bool has1 = r0 + 1 < n_rows;
-  const uint64_t a0 = ptr[r0], e0 = ptr[r0 + 1];
-  const uint64_t a1 = has1 ? ptr[r0 + 1] : 0, e1 = has1 ? ptr[r0 + 2] : 0;
-  const uint32_t groups = (n_cols + 31) / 32;
-  const uint64_t kch = r0 / kChunk;
-  const uint32_t p = (uint32_t)((r0 % kChunk) / 2);
-  for (uint32_t gg = lane; gg < groups; gg += 32) {
-    const uint32_t g0 = gg * 32;
-    uint64_t i = lower_bound_u32(col, a0, e0, g0), j = lower_bound_u32(col, a1, e1, g0);
-    const uint32_t gi = i < e0 ? col[i] : 0xFFFFFFFFu, gj = j < e1 ? col[j] : 0xFFFFFFFFu;
-    if (min(gi, gj) >= g0 + 32) continue;
-    const uint64_t b = (uint64_t)(gg / 4) * n_chunks + kch;
-    const uint64_t h = b * 64 + (gg % 4) * 16 + p;
-    const uint32_t m = masks[h], base = bases[h];
-    uint2* ent = reinterpret_cast<uint2*>(data + off[b] * 16 + kHeaderBytes);
-    for (;;) {
-      const uint32_t ci = i < e0 ? col[i] : 0xFFFFFFFFu, cj = j < e1 ? col[j] : 0xFFFFFFFFu;
-      const uint32_t g = min(ci, cj);
-      if (g >= g0 + 32) break;
-      uint32_t w0 = kAbsentHi, w1 = kAbsentHi;
-      if (ci == g) w0 = stored_parts(val[i++], scale);
-      if (cj == g) w1 = stored_parts(val[j++], scale);
-      ent[base + __popc(m & ((1u << (g - g0)) - 1u))] = make_entry(w0, w1);
+  for (uint32_t g0 = 0; g0 < groups; g0 += kValueCols / 32) {
+    for (uint32_t i = threadIdx.x; i < 32 * (kValueCols + 1); i += kLayWarps * 32)
+      (&tile[0][0])[i] = kAbsentHi;
+    __syncthreads();
+    walk_window<true>(col, val, at, end, g0 * 32, g0 * 32 + kValueCols,
+                      [&](uint32_t row, uint32_t c, float v) { tile[row][c] = stored_parts(v, scale); });
+    __syncthreads();
+    for (uint32_t g = warp; g < kValueCols / 32 && g0 + g < groups; g += kLayWarps) {
+      if (g0 + g < x.n_chunks)
+        write_quarter(x, rb / 4 * x.n_chunks + g0 + g, rb % 4, [&](uint32_t p, uint32_t odd) {
+          return tile[lane][g * 32 + 2 * p + odd];
+        });
+      if (t.masks && g0 + g < 4 * n_tiles_t && rb < t.n_chunks)
+        write_quarter(t, (uint64_t)((g0 + g) / 4) * t.n_chunks + rb, (g0 + g) % 4,
+                      [&](uint32_t p, uint32_t odd) { return tile[2 * p + odd][g * 32 + lane]; });
     }
+    __syncthreads();
   }
 }
 
@@ -691,82 +729,71 @@ __global__ void pair_base_kernel(const uint32_t* masks, uint64_t n_blocks, uint1
   if (lane == 0) units[b] = total ? (kHeaderBytes + 8ull * total + 15) / 16 : 0;
 }
 
-// Per block (warp): the header (every entry is then written whole by the values kernel).
-__global__ void pair_header_kernel(const uint32_t* masks, const uint16_t* bases,
-                                   const uint64_t* off, uint64_t n_blocks, uint8_t* data) {
-  const uint64_t b = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const unsigned lane = threadIdx.x & 31u;
-  if (b >= n_blocks || off[b + 1] == off[b]) return;
-  uint2* blk = reinterpret_cast<uint2*>(data + off[b] * 16);
-  for (uint32_t h = lane; h < 64; h += 32) blk[h] = make_uint2(masks[b * 64 + h], bases[b * 64 + h]);
-}
-
-// The layout (rows x K) of the CSR (n_rows x n_cols) or of its transpose.
-void build_pairs(const uint64_t* ptr, const uint32_t* col, const float* val, uint64_t n_rows,
-                 uint64_t nnz, bool transposed, Blocked& out, cudaStream_t s) {
-  out.n_tiles = (uint32_t)((out.rows + kRows - 1) / kRows);
-  out.n_chunks = (uint32_t)((out.K + kChunk - 1) / kChunk);
-  const uint64_t nb = (uint64_t)out.n_tiles * out.n_chunks;
-  DeviceBuffer<uint32_t> masks(nb * 64, s);
-  masks.zero();
-  // Warps: one per (tile, row quarter) of X, or one per pair of CSR rows for X^T.
-  const uint64_t warps = transposed ? (n_rows + 1) / 2 : (uint64_t)out.n_tiles * 4;
-  if (nnz) {
-    if (transposed)
-      cols_mask_kernel<<<blocks_for(warps * 32, 256), 256, 0, s>>>(ptr, col, n_rows,
-                                                                   (uint32_t)out.rows,
-                                                                   out.n_chunks, masks.ptr);
-    else
-      rows_mask_kernel<<<(unsigned)((warps + kMaskWarps - 1) / kMaskWarps), kMaskWarps * 32, 0,
-                         s>>>(ptr, col, n_rows, out.n_tiles, out.n_chunks, masks.ptr);
-    KG_LAUNCH_CHECK();
-  }
-  DeviceBuffer<uint16_t> bases(nb * 64, s);
-  out.off.alloc(nb + 1, s);
-  pair_base_kernel<<<blocks_for((nb + 1) * 32, 256), 256, 0, s>>>(masks.ptr, nb, bases.ptr,
-                                                                  out.off.ptr);
-  KG_LAUNCH_CHECK();
-  size_t temp = 0;
-  KG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp, out.off.ptr, out.off.ptr, nb + 1, s));
-  DeviceBuffer<unsigned char> scratch(temp, s);
-  KG_CUDA(cub::DeviceScan::ExclusiveSum(scratch.ptr, temp, out.off.ptr, out.off.ptr, nb + 1, s));
+// A layout on its way: its masks, then its bases and offsets.
+struct Building {
+  Blocked* out = nullptr;
+  DeviceBuffer<uint32_t> masks;
+  DeviceBuffer<uint16_t> bases;
+  DeviceBuffer<unsigned char> scratch;
   uint64_t units = 0;
-  KG_CUDA(cudaMemcpyAsync(&units, out.off.ptr + nb, 8, cudaMemcpyDeviceToHost, s));
-  KG_CUDA(cudaStreamSynchronize(s));
-  out.bytes = units * 16;
-  out.data.alloc(std::max<uint64_t>(out.bytes, 16), s);
-  if (!units) return;
-  pair_header_kernel<<<blocks_for(nb * 32, 256), 256, 0, s>>>(masks.ptr, bases.ptr, out.off.ptr,
-                                                              nb, out.data.ptr);
-  KG_LAUNCH_CHECK();
-  if (transposed)
-    cols_values_kernel<<<blocks_for(warps * 32, 256), 256, 0, s>>>(
-        ptr, col, val, n_rows, (uint32_t)out.rows, out.n_chunks, masks.ptr, bases.ptr,
-        out.off.ptr, out.scale, out.data.ptr);
-  else
-    rows_values_kernel<<<blocks_for(n_rows * 32, 256), 256, 0, s>>>(
-        ptr, col, val, n_rows, out.n_chunks, masks.ptr, bases.ptr, out.off.ptr, out.scale,
-        out.data.ptr);
-  KG_LAUNCH_CHECK();
-}
+  uint64_t blocks() const { return (uint64_t)out->n_tiles * out->n_chunks; }
+  void start(Blocked& b, uint64_t rows, uint64_t K, cudaStream_t s) {
+    out = &b;
+    b.rows = rows;
+    b.K = K;
+    b.n_tiles = (uint32_t)((rows + kRows - 1) / kRows);
+    b.n_chunks = (uint32_t)((K + kChunk - 1) / kChunk);
+    masks.alloc(blocks() * 64, s);
+  }
+  // (`units` is read back on the stream.)
+  void offsets(cudaStream_t s) {
+    const uint64_t nb = blocks();
+    bases.alloc(nb * 64, s);
+    out->off.alloc(nb + 1, s);
+    pair_base_kernel<<<blocks_for((nb + 1) * 32, 256), 256, 0, s>>>(masks.ptr, nb, bases.ptr,
+                                                                    out->off.ptr);
+    KG_LAUNCH_CHECK();
+    size_t temp = 0;
+    KG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp, out->off.ptr, out->off.ptr, nb + 1, s));
+    scratch.alloc(temp, s);
+    KG_CUDA(cub::DeviceScan::ExclusiveSum(scratch.ptr, temp, out->off.ptr, out->off.ptr, nb + 1, s));
+    KG_CUDA(cudaMemcpyAsync(&units, out->off.ptr + nb, 8, cudaMemcpyDeviceToHost, s));
+  }
+  LayoutOut layout(cudaStream_t s) {
+    out->bytes = units * 16;
+    out->data.alloc(std::max<uint64_t>(out->bytes, 16), s);
+    return {masks.ptr, bases.ptr, out->off.ptr, out->data.ptr, out->n_chunks};
+  }
+};
 
 }  // namespace
 
 void build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val, uint64_t n_rows,
-                   uint64_t n_cols, uint64_t nnz, Blocked& out, cudaStream_t s) {
-  out.rows = n_rows;
-  out.K = n_cols;
+                   uint64_t n_cols, uint64_t nnz, Blocked& out, Blocked* twin, cudaStream_t s) {
   // The values' range (the scale of their fp16 parts) and the largest row norm.
   DeviceBuffer<unsigned long long> st(3, s);
   const unsigned long long init[3] = {0ull, 0ull, 0x7FF0000000000000ull};  // 0, 0, +inf
   KG_CUDA(cudaMemcpyAsync(st.ptr, init, sizeof init, cudaMemcpyHostToDevice, s));
   if (nnz) {
-    csr_stats_kernel<<<blocks_for(n_rows * 32, 256), 256, 0, s>>>(ptr, val, n_rows, st.ptr,
-                                                                  st.ptr + 1, st.ptr + 2);
+    csr_stats_kernel<<<std::min<unsigned>(blocks_for(n_rows * 32, 256), 2048), 256, 0, s>>>(
+        ptr, val, n_rows, st.ptr, st.ptr + 1, st.ptr + 2);
     KG_LAUNCH_CHECK();
   }
   unsigned long long h_st[3];
   KG_CUDA(cudaMemcpyAsync(h_st, st.ptr, sizeof h_st, cudaMemcpyDeviceToHost, s));
+  Building x, t;
+  x.start(out, n_rows, n_cols, s);
+  if (twin) t.start(*twin, n_cols, n_rows, s);
+  const uint32_t tiles_t = twin ? twin->n_tiles : 0, chunks_t = twin ? twin->n_chunks : 0;
+  const uint32_t groups = std::max(out.n_chunks, 4 * tiles_t);
+  const unsigned grid = out.n_tiles * 4;
+  if (grid) {
+    masks_kernel<<<grid, kLayWarps * 32, 0, s>>>(ptr, col, n_rows, out.n_chunks, tiles_t, chunks_t,
+                                                 groups, x.masks.ptr, t.masks.ptr);
+    KG_LAUNCH_CHECK();
+  }
+  x.offsets(s);
+  if (twin) t.offsets(s);
   KG_CUDA(cudaStreamSynchronize(s));
   double d[3];
   std::memcpy(d, h_st, sizeof d);
@@ -774,19 +801,18 @@ void build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val, u
   out.max_abs = d[1];
   out.min_abs = std::isinf(d[2]) ? 0.0 : d[2];
   out.scale = part_scale(out.max_abs);
-  build_pairs(ptr, col, val, n_rows, nnz, false, out, s);
-}
-
-void transpose_blocked(const uint64_t* ptr, const uint32_t* col, const float* val,
-                       uint64_t n_rows, uint64_t n_cols, uint64_t nnz, const Blocked& x,
-                       Blocked& out, cudaStream_t s) {
-  out.rows = n_cols;
-  out.K = n_rows;
-  out.scale = x.scale;
-  out.max_abs = x.max_abs;
-  out.min_abs = x.min_abs;
-  out.max_row_norm = 0.0;  // not tracked for the transpose
-  build_pairs(ptr, col, val, n_rows, nnz, true, out, s);
+  if (twin) {
+    twin->scale = out.scale;
+    twin->max_abs = out.max_abs;
+    twin->min_abs = out.min_abs;
+    twin->max_row_norm = 0.0;  // not tracked for the transpose
+  }
+  const LayoutOut xo = x.layout(s);
+  const LayoutOut to = twin ? t.layout(s) : LayoutOut{nullptr, nullptr, nullptr, nullptr, 0};
+  if (!x.units) return;
+  values_kernel<<<grid, kLayWarps * 32, 0, s>>>(ptr, col, val, n_rows, tiles_t, groups, out.scale, xo,
+                                                to);
+  KG_LAUNCH_CHECK();
 }
 
 void spmm_tc(const SpmmArgs& a, cudaStream_t s) {

@@ -37,16 +37,11 @@ struct Blocked {
   DeviceBuffer<uint8_t> data;
 };
 
-// The blocked layout of a CSR matrix (n_rows x n_cols, u32 column indices, each row's
-// columns strictly increasing).
+// The blocked layout of a CSR matrix (n_rows x n_cols, u32 column indices, each row's columns
+// strictly increasing) and, if `twin`, of its transpose with the same scale and value range.
+// Waits for the stream once.
 void build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val, uint64_t n_rows,
-                   uint64_t n_cols, uint64_t nnz, Blocked& out, cudaStream_t s);
-
-// The blocked layout of the same CSR's transpose (n_cols x n_rows), with x's scale and
-// value range (x = build_blocked of that CSR).
-void transpose_blocked(const uint64_t* ptr, const uint32_t* col, const float* val,
-                       uint64_t n_rows, uint64_t n_cols, uint64_t nnz, const Blocked& x,
-                       Blocked& out, cudaStream_t s);
+                   uint64_t n_cols, uint64_t nnz, Blocked& out, Blocked* twin, cudaStream_t s);
 
 // The dense operand D (K x 64) as the products read it: D^T, 64 rows of fp16 parts of
 // each value times 2^scale, interleaved by chunk: for chunk c, row j holds the 32 high

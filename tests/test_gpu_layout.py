@@ -1,0 +1,32 @@
+"""The blocked layouts at the sizes where their builders' windows end: rows around a quarter and a
+tile, columns around the windows of 256 and 512, rows empty, sparse and full.
+
+A product through the layout stays within the product's own bar, 2^-15 sum |s| |d|; an entry lost,
+doubled or misplaced is off by the entry."""
+
+import numpy as np
+import pytest
+
+import kyto_b200 as K
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 129])
+@pytest.mark.parametrize("g", [1, 33, 255, 256, 257, 513, 1030])
+@pytest.mark.parametrize("density", [0.02, 1.0])
+def test_window_edges(n, g, density):
+    rng = np.random.default_rng(n * 2000 + g)
+    s = rng.uniform(0.5, 2.0, (n, g)) * (rng.random((n, g)) < density)
+    s[n // 2] = 0.0  # an empty row
+    s[:, g - 1] = 1.0  # and a full last column
+    s = s.astype(np.float32).astype(np.float64)
+    rows, idx = np.nonzero(s)
+    indptr = np.zeros(n + 1, dtype=np.uint64)
+    indptr[1:] = np.cumsum(np.bincount(rows, minlength=n))
+    args = indptr, idx.astype(np.uint32), s[rows, idx].astype(np.float32), g
+    for transposed in (False, True):
+        m = s.T if transposed else s
+        d = rng.uniform(-1.0, 1.0, (m.shape[1], 5))
+        got = K.product(*args, d, transposed)
+        assert np.all(np.abs(got - m @ d) <= (np.abs(m) @ np.abs(d)) * 2.0**-15 + 1e-300)
