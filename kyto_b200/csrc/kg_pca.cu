@@ -216,13 +216,13 @@ __global__ void omega_kernel(const uint64_t* cells, uint64_t n, uint32_t width,
   for (uint32_t j = 0; j < width; ++j) row[j] = omega_next(state);
 }
 
-// D^T = [1 ... 1; 0 ...] in the dense layout (row 0: ones over the n cells, scale 0; all
-// else zero).
-__global__ void fill_rows_kernel(uint16_t* t, uint64_t n, uint64_t ld) {
+// D^T = [1 ... 1; 0 ...] in the dense layout (row 0: `one`, the fp16 of a scaled 1, over the n
+// cells; all else zero).
+__global__ void fill_rows_kernel(uint16_t* t, uint64_t n, uint64_t ld, uint16_t one) {
   uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= 64 * ld) return;
   const uint64_t k = i % 64, r = (i / 64) * 32 + k;  // row 0's column r (hi parts)
-  t[i] = (i < ld && k < 32 && r < n) ? (uint16_t)0x3C00u : (uint16_t)0;
+  t[i] = (i < ld && k < 32 && r < n) ? one : (uint16_t)0;
 }
 
 __global__ void fill_kernel(double* p, uint64_t n, double v) {
@@ -565,12 +565,13 @@ __global__ void split_t_kernel(const double* cm, uint32_t g, uint32_t w, uint64_
   at[32] = lo;
 }
 
-// Omega^T in the dense layout (values times 2^scale; rows past width zero), and each
+// Omega^T in the dense layout (values times 2^scale; row `width` holds `one`, the fp16 of a
+// scaled 1, for the n cells, rows past it zero), and each
 // block's Omega column sums of the split values (as the products see them; f64, a fixed
 // tree) for the centring.
 __global__ void omega_t_kernel(const uint64_t* cells, uint64_t n, uint32_t width,
-                               uint64_t seed, uint64_t ld, int scale, uint16_t* t,
-                               double* block_sums) {
+                               uint64_t seed, uint64_t ld, int scale, uint16_t one,
+                               uint16_t* t, double* block_sums) {
   __shared__ double red[8][64];
   uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   bool live = r < n;
@@ -580,6 +581,7 @@ __global__ void omega_t_kernel(const uint64_t* cells, uint64_t n, uint32_t width
   for (uint32_t j = 0; j < 64; ++j) {
     uint16_t hi = 0, lo = 0;
     if (live && j < width) split_half(omega_next(state), mul, hi, lo);
+    if (live && j == width) hi = one;
     if (r < ld / 2) {
       uint16_t* at = t + (uint64_t)j * ld + (r / 32) * 64 + (r % 32);
       at[0] = hi;
@@ -618,15 +620,17 @@ sum_blocks_kernel(const double* partial, uint64_t nb, uint32_t w, double* out) {
   }
 }
 
-// out (g x w column-major) = sum over segments (in order) of partial[seg][gene][j].
+// The sums over segments (in order) of partial[seg][gene][first + j], j < w: column-major into
+// out for j < own, into rest from there on.
 __global__ void reduce_segments_kernel(const double* partial, uint32_t segs, uint32_t g,
-                                       uint32_t w, double* out) {
+                                       uint32_t first, uint32_t w, uint32_t own, double* out,
+                                       double* rest) {
   uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= (uint64_t)g * w) return;
   uint32_t gene = (uint32_t)(i / w), j = (uint32_t)(i % w);
   double t = 0.0;
-  for (uint32_t sg = 0; sg < segs; ++sg) t += partial[((uint64_t)sg * g + gene) * 64 + j];
-  out[(uint64_t)j * g + gene] = t;
+  for (uint32_t sg = 0; sg < segs; ++sg) t += partial[((uint64_t)sg * g + gene) * 64 + first + j];
+  (j < own ? out + (uint64_t)j * g : rest + (uint64_t)(j - own) * g)[gene] = t;
 }
 
 // Each gene's sum of (x - mean)^2 over its stored values: a warp per gene, lanes over
@@ -726,6 +730,7 @@ struct ProductClock {
 struct TcHeld {
   static constexpr uint64_t kSegChunks = 512;  // K-chunks (16,384 cells) per X^T work item
   static constexpr int kUnitScale = 14;        // |Omega|, |Q|, |V| <= 1: parts times 2^14
+  static constexpr uint16_t kUnitOne = (15 + kUnitScale) << 10;  // fp16 2^14: a scaled one
   uint64_t n = 0, g = 0, nnz = 0;
   ProductClock clock;
   // A product's algorithmic bytes, S (rows x K, nnz values) . D (K x l) read once and
@@ -735,9 +740,11 @@ struct TcHeld {
     return 8.0 * (double)nnz + 4.0 * (double)(n + 1) + 4.0 * (double)g * l + 4.0 * (double)n * l;
   }
   Blocked bx, bxt;
+  DeviceBuffer<unsigned long long> counts;  // each gene's stored values
   DeviceBuffer<uint16_t> dt;   // 64 x dense_ld(n): Omega^T, the ones row or W^T
   DeviceBuffer<uint16_t> qt;   // 64 x dense_ld(g): Q^T or V^T
   int dt_scale = 0;
+  uint32_t ones = 0;           // the column of ones in dt, after sketch
   double mean_norm = 0.0;      // |mu| (the gene means), for the bound on W's entries
   DeviceBuffer<int> error;     // set by a product whose bounded wait ran out
   int sm = 148;
@@ -748,7 +755,8 @@ struct TcHeld {
     g = n_genes;
     this->nnz = nnz;
     sm = sm_count;
-    build_blocked(indptr, col, val, n, g, nnz, bx, &bxt, s);
+    counts.alloc(g, s);
+    build_blocked(indptr, col, val, n, g, nnz, bx, &bxt, counts.ptr, s);
     trace.mark("blocked X, X^T");
     dt.alloc(64 * dense_ld(n), s);
     dt.zero();
@@ -767,32 +775,43 @@ struct TcHeld {
     if (h) fail(KG_ERR_TIMEOUT, "a tensor-core product gave up waiting on its pipeline");
   }
 
-  // out (g x width column-major) = X^T Omega; omega_sums (width).
+  // out (g x width column-major) = X^T Omega; omega_sums (width). Omega leaves a column of the
+  // products' 64 free (width < 64): it holds ones, so that sums (g) comes with the sketch; the
+  // ones' scale is a power of two, which moves no bit of a sum.
   void sketch(const uint64_t* cells, uint32_t width, uint64_t seed, double* out,
-              double* omega_sums, cudaStream_t s) {
+              double* omega_sums, double* sums, cudaStream_t s) {
     const uint64_t ld = dense_ld(n);
     unsigned nb = blocks_for(ld / 2, 256);
     DeviceBuffer<double> bsum((uint64_t)nb * 64, s);
-    omega_t_kernel<<<nb, 256, 0, s>>>(cells, n, width, seed, ld, kUnitScale, dt.ptr, bsum.ptr);
+    omega_t_kernel<<<nb, 256, 0, s>>>(cells, n, width, seed, ld, kUnitScale, kUnitOne, dt.ptr,
+                                      bsum.ptr);
     KG_LAUNCH_CHECK();
     dt_scale = kUnitScale;
     sum_blocks_kernel<<<1, 1024, 0, s>>>(bsum.ptr, nb, width, omega_sums);
     KG_LAUNCH_CHECK();
-    transposed(width, out, s);
+    if (width < 64) {
+      transposed(0, width, out, s, kValuePlain, nullptr, sums);
+      ones = width;
+    } else {
+      transposed(0, width, out, s);
+      fill_rows_kernel<<<blocks_for(64 * ld, 256), 256, 0, s>>>(dt.ptr, n, ld, kUnitOne);
+      KG_LAUNCH_CHECK();
+      ones = 0;
+      transposed(ones, 1, sums, s);
+    }
   }
 
-  // D^T = a row of ones (the stored values' gene sums, counts, squares).
-  void ones_column() {
-    const uint64_t ld = dense_ld(n);
-    fill_rows_kernel<<<blocks_for(64 * ld, 256), 256, 0, dt.stream>>>(dt.ptr, n, ld);
-    KG_LAUNCH_CHECK();
-    dt_scale = 0;
+  // out (g) = each gene's sum of (x - mean)^2 over its stored values (after sketch).
+  void centred_squares(const double* means, double* out, cudaStream_t s) {
+    transposed(ones, 1, out, s, kValueCentredSquare, means);
   }
 
-  // out (g x w column-major) = X^T W with W^T in dt (the stored values mapped by
-  // value_mode first).
-  void transposed(uint32_t w, double* out, cudaStream_t s, int value_mode = kValuePlain,
-                  const double* row_means = nullptr) {
+  // out (g x w column-major) = X^T W for the columns first .. first + w - 1 of the W whose W^T
+  // is in dt (the stored values mapped by value_mode first), and column w of those into `last`
+  // if given.
+  void transposed(uint32_t first, uint32_t w, double* out, cudaStream_t s,
+                  int value_mode = kValuePlain, const double* row_means = nullptr,
+                  double* last = nullptr) {
     uint64_t segs = (bxt.n_chunks + kSegChunks - 1) / kSegChunks;
     DeviceBuffer<double> partial(segs * g * 64, s);
     SpmmArgs a;
@@ -810,8 +829,9 @@ struct TcHeld {
     clock.begin(s, product_bytes(w));
     spmm_tc(a, s);
     clock.end();
-    reduce_segments_kernel<<<blocks_for(g * w, 256), 256, 0, s>>>(partial.ptr, (uint32_t)segs,
-                                                                  (uint32_t)g, w, out);
+    const uint32_t columns = w + (last ? 1 : 0);
+    reduce_segments_kernel<<<blocks_for(g * columns, 256), 256, 0, s>>>(
+        partial.ptr, (uint32_t)segs, (uint32_t)g, first, columns, w, out, last);
     KG_LAUNCH_CHECK();
   }
 
@@ -1216,23 +1236,23 @@ void kg_pca::run() {
         fail(KG_ERR_INVALID, "pca: gene " + std::to_string(i) +
                                  " holds a value that is not finite (NaN or infinity)");
   };
+  DeviceBuffer<double> omega_sums(l, s), sketch1((uint64_t)g * l, s);
   if (tc) {
-    // Gene means (pass 0's sums, pca.rs:707-717), stored counts and centred sums of
-    // squares over the stored values (the last pass's, pca.rs:664-676), as products
-    // with a column of ones.
+    // Pass 0's sketch X^T Omega (pca.rs:588-622) and gene means (its sums, pca.rs:707-717, with
+    // the sketch), and the centred sums of squares over the stored values (the last pass's,
+    // pca.rs:664-676), as products with a column of ones; the stored counts from the layout.
     th.build(indptr.ptr, col.ptr, val.ptr, n, g, nnz, c->sm_count, s, trace);
     trace.mark("operand buffers");
-    DeviceBuffer<double> sums(g, s), cnt(g, s), sq(g, s);
-    th.ones_column();
-    th.transposed(1, sums.ptr, s, kValuePlain, nullptr);
+    DeviceBuffer<double> sums(g, s), sq(g, s);
+    th.sketch(cells.ptr, l, seed, sketch1.ptr, omega_sums.ptr, sums.ptr, s);
+    trace.mark("sketch pass");
     divide_kernel<<<blocks_for(g, 256), 256, 0, s>>>(sums.ptr, g, (double)n, means.ptr);
     KG_LAUNCH_CHECK();
-    th.transposed(1, cnt.ptr, s, kValueOne, nullptr);
-    th.transposed(1, sq.ptr, s, kValueCentredSquare, means.ptr);
-    std::vector<double> h_cnt(g);
+    th.centred_squares(means.ptr, sq.ptr, s);
+    std::vector<unsigned long long> h_cnt(g);
     KG_CUDA(cudaMemcpyAsync(h_means.data(), means.ptr, g * 8ull, cudaMemcpyDeviceToHost, s));
     KG_CUDA(cudaMemcpyAsync(squares.data(), sq.ptr, g * 8ull, cudaMemcpyDeviceToHost, s));
-    KG_CUDA(cudaMemcpyAsync(h_cnt.data(), cnt.ptr, g * 8ull, cudaMemcpyDeviceToHost, s));
+    KG_CUDA(cudaMemcpyAsync(h_cnt.data(), th.counts.ptr, g * 8ull, cudaMemcpyDeviceToHost, s));
     KG_CUDA(cudaStreamSynchronize(s));
     check_means();
     th.check(s);
@@ -1240,7 +1260,7 @@ void kg_pca::run() {
     for (uint32_t i = 0; i < g; ++i) mn += h_means[i] * h_means[i];
     th.mean_norm = std::sqrt(mn);
     colptr[0] = 0;
-    for (uint32_t i = 0; i < g; ++i) colptr[i + 1] = colptr[i] + (uint64_t)std::llround(h_cnt[i]);
+    for (uint32_t i = 0; i < g; ++i) colptr[i + 1] = colptr[i] + (uint64_t)h_cnt[i];
     double worst_ratio = 0.0;
     for (uint32_t i = 0; i < g; ++i) {
       uint64_t stored = colptr[i + 1] - colptr[i];
@@ -1308,11 +1328,8 @@ void kg_pca::run() {
     KG_LAUNCH_CHECK();
   };
 
-  // ---- pass 0: sketch X^T Omega (pca.rs:588-622, end_pass pca.rs:707-749) ----
-  DeviceBuffer<double> omega_sums(l, s), sketch1((uint64_t)g * l, s);
-  if (tc) {
-    th.sketch(cells.ptr, l, seed, sketch1.ptr, omega_sums.ptr, s);
-  } else {
+  // ---- pass 0: the centred sketch (end_pass pca.rs:707-749) ----
+  if (!tc) {
     DeviceBuffer<double> omega(n * l, s);
     omega_kernel<<<blocks_for(n, 128), 128, 0, s>>>(cells.ptr, n, l, seed, omega.ptr);
     KG_LAUNCH_CHECK();
@@ -1403,7 +1420,7 @@ void kg_pca::run() {
     double* product = products.ptr + (uint64_t)m * g;
     if (tc) {
       th.rows(block.ptr, w, block_means.ptr, wsums.ptr, nullptr, s);
-      th.transposed(w, product, s);
+      th.transposed(0, w, product, s);
     } else {
       DeviceBuffer<double> block_rm((uint64_t)g * w, s), wrows(n * w, s);
       to_row_major_kernel<<<blocks_for((uint64_t)g * w, 256), 256, 0, s>>>(block.ptr, g, w,
@@ -1735,7 +1752,7 @@ kg_status kg_diag_spmm(kg_ctx* ctx, const uint64_t* indptr, const uint32_t* indi
     const uint32_t* d_idx = device_view(indices, nnz, hi_idx, s);
     const float* d_val = device_view(values, nnz, hv, s);
     Blocked bx, bxt;
-    build_blocked(d_ptr, d_idx, d_val, n_rows, n_cols, nnz, bx, transposed ? &bxt : nullptr, s);
+    build_blocked(d_ptr, d_idx, d_val, n_rows, n_cols, nnz, bx, transposed ? &bxt : nullptr, nullptr, s);
     const Blocked* sp = transposed ? &bxt : &bx;
     const uint64_t rows = sp->rows, K = sp->K, ld = dense_ld(K);
     DeviceBuffer<double> hd;
@@ -1754,7 +1771,7 @@ kg_status kg_diag_spmm(kg_ctx* ctx, const uint64_t* indptr, const uint32_t* indi
                                                                   dscale, dt.ptr);
       KG_LAUNCH_CHECK();
     } else {
-      fill_rows_kernel<<<blocks_for(64 * ld, 256), 256, 0, s>>>(dt.ptr, K, ld);
+      fill_rows_kernel<<<blocks_for(64 * ld, 256), 256, 0, s>>>(dt.ptr, K, ld, (uint16_t)0x3C00u);
       KG_LAUNCH_CHECK();
     }
     DeviceBuffer<double> hm;
@@ -1782,7 +1799,7 @@ kg_status kg_diag_spmm(kg_ctx* ctx, const uint64_t* indptr, const uint32_t* indi
     a.error = err.ptr;
     spmm_tc(a, s);
     reduce_segments_kernel<<<blocks_for(rows * width, 256), 256, 0, s>>>(
-        partial.ptr, (uint32_t)segs, (uint32_t)rows, width, res.ptr);
+        partial.ptr, (uint32_t)segs, (uint32_t)rows, 0, width, width, res.ptr, nullptr);
     KG_LAUNCH_CHECK();
     KG_CUDA(cudaMemcpyAsync(out, res.ptr, rows * width * 8, cudaMemcpyDefault, s));
     wait_stream(ctx, s);

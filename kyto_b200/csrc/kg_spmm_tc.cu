@@ -583,11 +583,12 @@ __device__ __forceinline__ void walk_window(const uint32_t* __restrict__ col,
 
 // Header masks of X (masks, words of 64 a block) and, if masks_t, of X^T: a byte an entry in
 // shared memory, gathered into words by ballots. Every word of both layouts is written. `groups`:
-// groups of 32 columns to pass, at least X's chunks and four times X^T's tiles.
+// groups of 32 columns to pass, at least X's chunks and four times X^T's tiles. With X^T each
+// column's entries are counted too (counts, if given: whole numbers, so any order).
 __global__ void __launch_bounds__(kLayWarps * 32)
 masks_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint64_t n_rows,
              uint32_t n_chunks, uint32_t n_tiles_t, uint32_t n_chunks_t, uint32_t groups,
-             uint32_t* masks, uint32_t* masks_t) {
+             uint32_t* masks, uint32_t* masks_t, unsigned long long* counts) {
   constexpr uint32_t kLd = kMaskCols / 4 + 1;  // words a row: an odd stride
   __shared__ uint32_t flags[32][kLd];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -621,15 +622,17 @@ masks_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col,
         if (lane < 16) masks[(tile * n_chunks + g0 + g) * 64 + q * 16 + lane] = mine;
       }
       if (masks_t && g0 + g < 4 * n_tiles_t && rb < n_chunks_t) {  // lane = column
-        uint32_t mine = 0;
+        uint32_t mine = 0, held = 0;
 #pragma unroll
         for (uint32_t p = 0; p < 16; ++p) {
           const uint32_t w =
-              (uint32_t)reinterpret_cast<const unsigned char*>(flags[2 * p])[g * 32 + lane] |
+              (uint32_t)reinterpret_cast<const unsigned char*>(flags[2 * p])[g * 32 + lane] +
               reinterpret_cast<const unsigned char*>(flags[2 * p + 1])[g * 32 + lane];
           const uint32_t any = __ballot_sync(0xFFFFFFFFu, w);
           if (lane == p) mine = any;
+          held += w;
         }
+        if (counts && held) atomicAdd(&counts[(g0 + g) * 32 + lane], (unsigned long long)held);
         if (lane < 16)
           masks_t[((uint64_t)((g0 + g) / 4) * n_chunks_t + rb) * 64 + (g0 + g) % 4 * 16 + lane] = mine;
       }
@@ -769,7 +772,9 @@ struct Building {
 }  // namespace
 
 void build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val, uint64_t n_rows,
-                   uint64_t n_cols, uint64_t nnz, Blocked& out, Blocked* twin, cudaStream_t s) {
+                   uint64_t n_cols, uint64_t nnz, Blocked& out, Blocked* twin,
+                   unsigned long long* col_counts, cudaStream_t s) {
+  if (col_counts) KG_CUDA(cudaMemsetAsync(col_counts, 0, n_cols * sizeof *col_counts, s));
   // The values' range (the scale of their fp16 parts) and the largest row norm.
   DeviceBuffer<unsigned long long> st(3, s);
   const unsigned long long init[3] = {0ull, 0ull, 0x7FF0000000000000ull};  // 0, 0, +inf
@@ -789,7 +794,7 @@ void build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val, u
   const unsigned grid = out.n_tiles * 4;
   if (grid) {
     masks_kernel<<<grid, kLayWarps * 32, 0, s>>>(ptr, col, n_rows, out.n_chunks, tiles_t, chunks_t,
-                                                 groups, x.masks.ptr, t.masks.ptr);
+                                                 groups, x.masks.ptr, t.masks.ptr, col_counts);
     KG_LAUNCH_CHECK();
   }
   x.offsets(s);
