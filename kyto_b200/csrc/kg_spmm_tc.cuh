@@ -53,7 +53,7 @@ inline uint64_t dense_ld(uint64_t K) { return (K + 31) / 32 * 64; }
 // The exponent that puts the largest magnitude `bound` in [2^14, 2^15) (0 for 0).
 int part_scale(double bound);
 
-enum : int { kOutRows = 0, kOutPartial = 1 };
+enum : int { kOutRows = 0, kOutPartial = 1, kOutGroups = 2 };
 enum : int { kValuePlain = 0, kValueCentredSquare = 1, kValueOne = 2 };
 
 // Where C = S D goes.
@@ -71,6 +71,9 @@ struct SpmmOut {
                                      // (n_tiles x 64 f64).
   // kOutPartial: each K segment's C as f64 (segments x rows x 64).
   double* partial = nullptr;
+  // kOutGroups (spmm_tc's own way to kOutPartial): each flush group's f32 sums (groups x rows x
+  // 64).
+  float* groups = nullptr;
 };
 
 struct SpmmArgs {

@@ -30,3 +30,30 @@ def test_window_edges(n, g, density):
         d = rng.uniform(-1.0, 1.0, (m.shape[1], 5))
         got = K.product(*args, d, transposed)
         assert np.all(np.abs(got - m @ d) <= (np.abs(m) @ np.abs(d)) * 2.0**-15 + 1e-300)
+
+
+@pytest.mark.parametrize("n", [40, 600, 16_400, 33_000])
+def test_split_work_items_keep_the_bits(n):
+    # 16,000 columns are work items enough for the chip, 300 are not and are split: a column's
+    # f64 sums come out in the same order either way.
+    g, few = 16_000, 300
+    rng = np.random.default_rng(n)
+    rows = np.repeat(np.arange(n), 6)
+    idx = (rng.integers(0, few // 6, (n, 6)) * 6 + np.arange(6)) % few
+    idx[:, 5] = rng.integers(few, g, n)  # one entry a row past the few
+    idx.sort(axis=1)
+    assert np.all(np.diff(idx, axis=1) > 0)
+    val = rng.uniform(0.5, 2.0, (n, 6)).astype(np.float32)
+    val[0, 0] = 2.0  # the same largest value in both
+    d = rng.uniform(-1.0, 1.0, (n, 7))
+    d[0] = 1.0
+    whole = K.product(np.arange(n + 1, dtype=np.uint64) * 6, idx.ravel().astype(np.uint32),
+                      val.ravel(), g, d, True)
+    keep = idx < few
+    indptr = np.zeros(n + 1, dtype=np.uint64)
+    indptr[1:] = np.cumsum(keep.sum(1))
+    part = K.product(indptr, idx[keep].astype(np.uint32), val[keep], few, d, True)
+    assert np.array_equal(whole[:few].view(np.uint64), part.view(np.uint64))
+    m = np.zeros((n, few))
+    m[rows[keep.ravel()], idx[keep]] = val[keep]
+    assert np.all(np.abs(part - m.T @ d) <= (m.T @ np.abs(d)) * 2.0**-15 + 1e-300)
