@@ -35,16 +35,55 @@ __device__ __forceinline__ uint32_t gathered(uint32_t c) {
   return (c % kTriCtas) * kGatherLd + c / kTriCtas;
 }
 
-// Slot `lane` (low) and 32 + lane (high) of this CTA into every CTA's `to`, two CTAs a warp.
-__device__ __forceinline__ void gather(cg::cluster_group& cluster, double* to, uint32_t rank,
-                                       double low, double high) {
+// A gathered vector's barrier: a phase completes when every CTA's slots have arrived.
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t cta) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(cta));
+  return a;
+}
+__device__ __forceinline__ void store_async(uint32_t to, double v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(to),
+               "l"(__double_as_longlong(v)), "r"(bar)
+               : "memory");
+}
+
+// Slot `lane` (low) and 32 + lane (high) of this CTA into every CTA's `to`, two CTAs a warp,
+// counted on that CTA's `bar`.
+__device__ __forceinline__ void gather(double* to, uint64_t* bar, uint32_t rank, double low,
+                                       double high) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 #pragma unroll
   for (uint32_t k = 0; k < kTriCtas / kTriWarps; ++k) {
-    double* peer = cluster.map_shared_rank(to, warp * (kTriCtas / kTriWarps) + k) + rank * kGatherLd;
-    peer[lane] = low;
-    if (lane < kTriSlots - 32) peer[32 + lane] = high;
+    const uint32_t peer = warp * (kTriCtas / kTriWarps) + k;
+    const uint32_t at = cluster_addr(to + rank * kGatherLd, peer), b = cluster_addr(bar, peer);
+    store_async(at + lane * 8, low, b);
+    if (lane < kTriSlots - 32) store_async(at + (32 + lane) * 8, high, b);
   }
+}
+
+// Waits for phase `phase` of a gathered vector (thread 0 says how many bytes make it up). A wait
+// that runs out sets *stuck, after which no wait waits: the kernel ends with d[0] a NaN.
+constexpr uint32_t kGatherPolls = 1u << 22;
+__device__ __forceinline__ void await(uint64_t* bar, uint32_t phase, volatile int* stuck) {
+  const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
+  if (threadIdx.x == 0)
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b),
+                 "r"(kTriCtas * kTriSlots * 8u)
+                 : "memory");
+  for (uint32_t n = 0; n < kGatherPolls && !*stuck; ++n) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}"
+        : "=r"(done)
+        : "r"(b), "r"(phase)
+        : "memory");
+    if (done) return;
+  }
+  *stuck = 1;
 }
 
 // The sum of one value a thread, the same bits in every thread and in every CTA that adds the
@@ -92,11 +131,27 @@ __device__ __forceinline__ void pass_over(double (&h)[kTriCols][kTriRows], const
       if (r < 4 * Q + 5 && i == j + 1) next[q * kTriWarps + warp] = h[q][r];
     }
   }
+  // The columns' sums over the lanes, four columns together: the first two steps halve how many
+  // columns a lane adds up, so that lane 8 i ends with column Q + i's.
+  constexpr uint32_t kFour = kTriCols - Q < 4 ? kTriCols - Q : 4;
+  double v[4];
 #pragma unroll
-  for (uint32_t q = Q; q < kTriCols; ++q) {
+  for (uint32_t i = 0; i < 4; ++i) v[i] = i < kFour ? acc[(Q + i) % kTriCols] : 0.0;
+  const bool up = lane & 16u, upper = lane & 8u;
+  double a = up ? v[2] : v[0], b = up ? v[3] : v[1];
+  a += __shfl_xor_sync(0xFFFFFFFFu, up ? v[0] : v[2], 16);
+  b += __shfl_xor_sync(0xFFFFFFFFu, up ? v[1] : v[3], 16);
+  double t = upper ? b : a;
+  t += __shfl_xor_sync(0xFFFFFFFFu, upper ? a : b, 8);
 #pragma unroll
-    for (int o = 16; o; o >>= 1) acc[q] += __shfl_xor_sync(0xFFFFFFFFu, acc[q], o);
-    if (lane == 0) dots[q * kTriWarps + warp] = acc[q];
+  for (int o = 4; o; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+  const uint32_t mine = (up ? 2u : 0u) + (upper ? 1u : 0u);
+  if (lane % 8 == 0 && mine < kFour) dots[(Q + mine) * kTriWarps + warp] = t;
+  if (Q + 4 < kTriCols) {
+    double last = acc[kTriCols - 1];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) last += __shfl_xor_sync(0xFFFFFFFFu, last, o);
+    if (lane == 0) dots[(kTriCols - 1) * kTriWarps + warp] = last;
   }
 }
 
@@ -109,10 +164,12 @@ __device__ __forceinline__ void pass_over(double (&h)[kTriCols][kTriRows], const
 // One cluster of 16 CTAs holds the matrix in registers: column c in CTA c % 16, warp and slot
 // (c / 16) % 8 and c / 128, a lane every 32nd row. A step's two vectors, the column (which is
 // the row by symmetry: every CTA holds the entries of its own columns) and A v, are gathered
-// into every CTA's shared memory by distributed stores, a cluster barrier behind each; the
-// reflector is then computed in every CTA alike. Latency bounds it: two cluster barriers, two
-// block sums and the pass over the held columns a step, 7,600 cycles in all (a third of it the
-// barriers' wait for the stores): 2.1 ms for 540 columns (cuSOLVER's reduction 4.4).
+// into every CTA's shared memory by asynchronous stores counted on its barrier; the reflector is
+// then computed in every CTA alike. A CTA sends its part of a step's vector only when it has read
+// the vector before, and none can be a step ahead without every other's part, so one buffer a
+// vector does. Latency bounds it: two exchanges, two block sums and the pass over the held columns
+// a step, 5,900 cycles in all, 1.65 ms for 540 columns (with plain distributed stores, a cluster
+// barrier behind each, 2.1 ms; cuSOLVER's reduction takes 4.4).
 __global__ void __cluster_dims__(kTriCtas, 1, 1) __launch_bounds__(kTriThreads, 1)
 tridiagonalise_kernel(const double* __restrict__ a, uint32_t m, double* d, double* e, double* tau,
                       double* reflect) {
@@ -126,6 +183,8 @@ tridiagonalise_kernel(const double* __restrict__ a, uint32_t m, double* d, doubl
   __shared__ double next[kTriSlots];  // this CTA's entries of the next row
   __shared__ double dots[kTriSlots];  // and of A v
   __shared__ double red[2][kTriWarps];
+  __shared__ uint64_t row_bar, prod_bar;
+  __shared__ int stuck;
   // Step j's reflector in CTA j % 16, and d, e and tau in CTA 0: written out at the end (a store
   // to global memory inside a step is one more trip that its barriers wait for).
   extern __shared__ double kept[];
@@ -147,6 +206,13 @@ tridiagonalise_kernel(const double* __restrict__ a, uint32_t m, double* d, doubl
     wv[i] = 0.0;  // (rows past m stay zero in all three)
   }
   if (tid < kTriSlots) dots[tid] = 0.0;
+  if (tid == 0) {
+    stuck = 0;
+    for (uint64_t* bar : {&row_bar, &prod_bar})
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(bar))
+                   : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   cluster.sync();
   for (uint32_t j = 0; j < m; ++j) {
     const double* old_v = vec[(j + 1) & 1u];
@@ -158,9 +224,9 @@ tridiagonalise_kernel(const double* __restrict__ a, uint32_t m, double* d, doubl
       double low = 0.0, high = 0.0;
       if (c0 < m) low = next[lane] - vj * wv[c0] - wj * old_v[c0];
       if (c1 < m && lane < kTriSlots - 32) high = next[32 + lane] - vj * wv[c1] - wj * old_v[c1];
-      gather(cluster, row, rank, low, high);
+      gather(row, &row_bar, rank, low, high);
     }
-    cluster.sync();
+    await(&row_bar, j & 1u, &stuck);
     if (tid == 0) out_d[j] = row[gathered(j)];
     if (j + 1 == m) break;
     // The reflector of row[j + 1 ..): every CTA computes it, CTA 0 writes it.
@@ -197,8 +263,8 @@ tridiagonalise_kernel(const double* __restrict__ a, uint32_t m, double* d, doubl
       default: pass_over<4>(h, old_v, wv, new_v, next, dots, m, j, rank); break;
     }
     __syncthreads();
-    gather(cluster, prod, rank, dots[lane], lane < kTriSlots - 32 ? dots[32 + lane] : 0.0);
-    cluster.sync();
+    gather(prod, &prod_bar, rank, dots[lane], lane < kTriSlots - 32 ? dots[32 + lane] : 0.0);
+    await(&prod_bar, j & 1u, &stuck);
     part = 0.0;
     for (uint32_t i = tid; i < m; i += kTriThreads)
       if (i > j) part += prod[gathered(i)] * new_v[i];
@@ -207,6 +273,11 @@ tridiagonalise_kernel(const double* __restrict__ a, uint32_t m, double* d, doubl
     for (uint32_t i = tid; i < m; i += kTriThreads)
       wv[i] = i > j ? t * prod[gathered(i)] - half * new_v[i] : 0.0;
     __syncthreads();
+  }
+  __syncthreads();
+  if (stuck) {
+    if (tid == 0) out_d[0] = NAN;
+    for (int n = 0; n < 1000; ++n) __nanosleep(1000);  // for what is still on its way
   }
   cluster.sync();  // no CTA leaves while another may still write to it
   for (uint32_t j = rank; j + 1 < m; j += kTriCtas)
