@@ -122,16 +122,25 @@ __global__ void seed_centres_kernel(const float* sample, uint64_t m, uint32_t d,
   centre[i] = j < d ? (double)sample[(c * m / K) * d + j] : 0.0;
 }
 
-__global__ void centres_f32_kernel(const double* centre, uint32_t K, float* cf, float* cn) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= K) return;
-  float s = 0.0f;
-  for (uint32_t j = 0; j < kClusterDim; ++j) {
-    const float v = (float)centre[(uint64_t)c * kClusterDim + j];
-    cf[(uint64_t)c * kClusterDim + j] = v;
-    s = fmaf(v, v, s);
+// A centre's f32 components and their squared norm (summed in order by one lane; the components
+// are read by kClusterDim lanes, since a lane reading them all waits 13 us).
+constexpr uint32_t kCentresABlock = 4;
+
+__global__ void __launch_bounds__(kCentresABlock * kClusterDim)
+centres_f32_kernel(const double* centre, uint32_t K, float* cf, float* cn) {
+  __shared__ float v[kCentresABlock][kClusterDim];
+  const uint32_t i = threadIdx.x / kClusterDim, j = threadIdx.x % kClusterDim;
+  const uint32_t c = blockIdx.x * kCentresABlock + i;
+  if (c < K) {
+    v[i][j] = (float)centre[(uint64_t)c * kClusterDim + j];
+    cf[(uint64_t)c * kClusterDim + j] = v[i][j];
   }
-  cn[c] = s;
+  __syncthreads();
+  if (c < K && j == 0) {
+    float s = 0.0f;
+    for (uint32_t k = 0; k < kClusterDim; ++k) s = fmaf(v[i][k], v[i][k], s);
+    cn[c] = s;
+  }
 }
 
 // key = (label << 32) | the first component's f32 bits mapped to an unsigned order.
@@ -145,15 +154,36 @@ __global__ void order_key_kernel(const float* x, uint64_t n, uint32_t width, con
   iota[r] = (uint32_t)r;
 }
 
+// key = the first component's f32 bits mapped to an unsigned order.
+__global__ void component_key_kernel(const float* x, uint64_t n, uint32_t width, uint32_t* key,
+                                     uint32_t* iota) {
+  uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  uint32_t b = __float_as_uint(x[r * width]);
+  key[r] = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+  iota[r] = (uint32_t)r;
+}
+
+// out row i = row order[i] of x (d components each).
+__global__ void permute_rows_kernel(const float* x, uint64_t n, uint32_t d, const uint32_t* order,
+                                    float* out) {
+  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (i >= n * d) return;
+  out[i] = x[(uint64_t)order[i / d] * d + i % d];
+}
+
+__device__ __forceinline__ uint32_t label_of(unsigned long long key) { return (uint32_t)(key >> 32); }
+__device__ __forceinline__ uint32_t label_of(uint32_t label) { return label; }
+
 // starts[c] = the first position whose key's label is >= c (c = 0..K).
-__global__ void key_starts_kernel(const unsigned long long* sorted, uint64_t n, uint32_t K,
-                                  uint32_t* starts) {
+template <class Key>
+__global__ void key_starts_kernel(const Key* sorted, uint64_t n, uint32_t K, uint32_t* starts) {
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c > K) return;
   uint64_t lo = 0, hi = n;
   while (lo < hi) {
     const uint64_t mid = (lo + hi) >> 1;
-    if ((uint32_t)(sorted[mid] >> 32) < c) lo = mid + 1; else hi = mid;
+    if (label_of(sorted[mid]) < c) lo = mid + 1; else hi = mid;
   }
   starts[c] = (uint32_t)lo;
 }
@@ -220,6 +250,24 @@ update_centres_kernel(const float* __restrict__ x, uint32_t width, uint32_t d,
   if (tid < d) centre[(uint64_t)c * kClusterDim + tid] = s / (double)(e - b);
 }
 
+// Sorts (key, value) pairs by the key's low `bits` (stable).
+template <class Key>
+void sort_pairs(const Key* key, Key* key_out, const uint32_t* val, uint32_t* val_out, uint64_t n,
+                int bits, cudaStream_t s) {
+  size_t temp = 0;
+  KG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp, key, key_out, val, val_out, (int)n, 0, bits,
+                                          s));
+  DeviceBuffer<unsigned char> scratch(temp, s);
+  KG_CUDA(cub::DeviceRadixSort::SortPairs(scratch.ptr, temp, key, key_out, val, val_out, (int)n, 0,
+                                          bits, s));
+}
+
+int label_bits(uint32_t K) {
+  int bits = 1;
+  while (bits < 32 && (1ull << bits) <= (uint64_t)K) ++bits;
+  return bits;
+}
+
 // The rows by (cluster, first component): perm and the clusters' starts.
 void order_by_cluster(const float* x, uint64_t n, uint32_t width, const uint32_t* label,
                       uint32_t K, DeviceBuffer<uint32_t>& perm, DeviceBuffer<uint32_t>& start,
@@ -229,14 +277,7 @@ void order_by_cluster(const float* x, uint64_t n, uint32_t width, const uint32_t
   order_key_kernel<<<blocks_for(n, 256), 256, 0, s>>>(x, n, width, label, key.ptr, iota.ptr);
   KG_LAUNCH_CHECK();
   perm.alloc(n, s);
-  int bits = 33;
-  while (bits < 64 && (1ull << (bits - 32)) <= (uint64_t)K) ++bits;
-  size_t temp = 0;
-  KG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp, key.ptr, key_sorted.ptr, iota.ptr,
-                                          perm.ptr, (int)n, 0, bits, s));
-  DeviceBuffer<unsigned char> scratch(temp, s);
-  KG_CUDA(cub::DeviceRadixSort::SortPairs(scratch.ptr, temp, key.ptr, key_sorted.ptr, iota.ptr,
-                                          perm.ptr, (int)n, 0, bits, s));
+  sort_pairs(key.ptr, key_sorted.ptr, iota.ptr, perm.ptr, n, 32 + label_bits(K), s);
   start.alloc((uint64_t)K + 1, s);
   key_starts_kernel<<<blocks_for((uint64_t)K + 1, 256), 256, 0, s>>>(key_sorted.ptr, n, K,
                                                                     start.ptr);
@@ -274,18 +315,30 @@ void cluster_rows(const float* x, uint64_t n, uint32_t width, uint32_t d, uint32
   seed_centres_kernel<<<blocks_for((uint64_t)K * kClusterDim, 256), 256, 0, s>>>(
       xs.ptr, m, d, K, out.centre.ptr);
   KG_LAUNCH_CHECK();
-  DeviceBuffer<uint32_t> lab(m, s);
+  // The sample by its first component, once: a round then sorts by the cluster alone, one or two
+  // passes that keep each cluster's rows in that order (by both, five passes a round, 45 us).
+  DeviceBuffer<uint32_t> key(m, s), key_sorted(m, s), iota(m, s), order(m, s), starts(K + 1ull, s);
+  DeviceBuffer<float> sorted(m * d, s);
+  component_key_kernel<<<blocks_for(m, 256), 256, 0, s>>>(xs.ptr, m, d, key.ptr, iota.ptr);
+  KG_LAUNCH_CHECK();
+  sort_pairs(key.ptr, key_sorted.ptr, iota.ptr, order.ptr, m, 32, s);
+  permute_rows_kernel<<<blocks_for(m * d, 256), 256, 0, s>>>(xs.ptr, m, d, order.ptr, sorted.ptr);
+  KG_LAUNCH_CHECK();
   for (uint32_t it = 0; it < iters; ++it) {
-    centres_f32_kernel<<<blocks_for(K, 128), 128, 0, s>>>(out.centre.ptr, K, cf.ptr, cn.ptr);
+    centres_f32_kernel<<<(K + kCentresABlock - 1) / kCentresABlock, kCentresABlock * kClusterDim, 0,
+                       s>>>(out.centre.ptr, K, cf.ptr, cn.ptr);
     KG_LAUNCH_CHECK();
-    nearest_centres(xs.ptr, m, d, d, cf.ptr, cn.ptr, K, lab.ptr, s);
-    DeviceBuffer<uint32_t> order, starts;
-    order_by_cluster(xs.ptr, m, d, lab.ptr, K, order, starts, s);
-    update_centres_kernel<<<K, kUcThreads, 0, s>>>(xs.ptr, d, d, order.ptr, starts.ptr,
+    nearest_centres(sorted.ptr, m, d, d, cf.ptr, cn.ptr, K, key.ptr, s);
+    sort_pairs(key.ptr, key_sorted.ptr, iota.ptr, order.ptr, m, label_bits(K), s);
+    key_starts_kernel<<<blocks_for((uint64_t)K + 1, 256), 256, 0, s>>>(key_sorted.ptr, m, K,
+                                                                       starts.ptr);
+    KG_LAUNCH_CHECK();
+    update_centres_kernel<<<K, kUcThreads, 0, s>>>(sorted.ptr, d, d, order.ptr, starts.ptr,
                                                     out.centre.ptr);
     KG_LAUNCH_CHECK();
   }
-  centres_f32_kernel<<<blocks_for(K, 128), 128, 0, s>>>(out.centre.ptr, K, cf.ptr, cn.ptr);
+  centres_f32_kernel<<<(K + kCentresABlock - 1) / kCentresABlock, kCentresABlock * kClusterDim, 0,
+                       s>>>(out.centre.ptr, K, cf.ptr, cn.ptr);
   KG_LAUNCH_CHECK();
   out.label.alloc(n, s);
   nearest_centres(x, n, width, d, cf.ptr, cn.ptr, K, out.label.ptr, s);

@@ -261,7 +261,10 @@ void spatial_order(const float* x, uint64_t n, uint32_t width, uint32_t d, const
 // group row from it, rounded up) and box (each component's smallest and largest centred
 // value) of each group of `size` consecutive slots; component j of group g is written at
 // g * g_stride + j * j_stride of each per-component array (component-major: g_stride 1,
-// j_stride n_groups; group-major: 64 and 1). One 64-thread block per group.
+// j_stride n_groups; group-major: 64 and 1). One 64-thread block per group, waiting for its
+// rows: kBallAhead of them at a time are on their way.
+constexpr int kBallAhead = 16;
+
 __global__ void __launch_bounds__(64)
 group_balls_kernel(const float* x, uint32_t width, uint32_t d, const double* mean,
                    const uint32_t* rows, uint64_t n, uint32_t size, uint64_t g_stride,
@@ -277,11 +280,20 @@ group_balls_kernel(const float* x, uint32_t width, uint32_t d, const double* mea
     double sum = 0.0;
     lo = INFINITY;
     hi = -INFINITY;
-    for (uint64_t sl = s0; sl < s1; ++sl) {
-      const double v = (double)x[(uint64_t)rows[sl] * width + j] - mean[j];
-      sum += v;
-      lo = fmin(lo, v);
-      hi = fmax(hi, v);
+    const double mu = mean[j];
+    for (uint64_t sl = s0; sl < s1; sl += kBallAhead) {  // (in slot order)
+      float v[kBallAhead];
+#pragma unroll
+      for (int i = 0; i < kBallAhead; ++i)
+        v[i] = x[(uint64_t)rows[min(sl + i, s1 - 1)] * width + j];
+#pragma unroll
+      for (int i = 0; i < kBallAhead; ++i)
+        if (sl + i < s1) {
+          const double t = (double)v[i] - mu;
+          sum += t;
+          lo = fmin(lo, t);
+          hi = fmax(hi, t);
+        }
     }
     c[j] = sum / (double)(s1 - s0);
   }
@@ -314,17 +326,19 @@ group_balls_kernel(const float* x, uint32_t width, uint32_t d, const double* mea
 // boxes' sqrt(sum_j gap_j^2) (gap_j: how far apart the two boxes are in component j). The
 // larger, less a margin for the rounding of the centred rows and at least 0, is kept as a
 // scaled squared distance rounded down, packed with the centre distance into the sort key
-// (bound, then centre distance); the tile as the value. kBoundBlocks query blocks per CTA
-// share each tile's reads.
+// (bound, then centre distance); the tile as the value. B query blocks per CTA share each tile's
+// reads where that leaves two CTAs an SM, else one: the f64 arithmetic bounds it, and eight blocks
+// a CTA took 85 us for 60,000 rows on 30 CTAs, one a CTA 35.
 constexpr int kBoundBlocks = 8;
+template <int B>
 __global__ void __launch_bounds__(256)
 ball_bounds_kernel(const double* bc_t, const double* blo_t, const double* bhi_t,
                    const double* br, uint64_t n_blocks, const double* tc_t, const double* tlo_t,
                    const double* thi_t, const double* tr, uint32_t n_tiles, uint32_t d,
                    double s2, double margin, unsigned long long* key, uint32_t* tile) {
-  __shared__ double cb[kBoundBlocks][kDim], lb_[kBoundBlocks][kDim], hb[kBoundBlocks][kDim];
-  const uint64_t b0 = (uint64_t)blockIdx.x * kBoundBlocks;
-  for (uint32_t i = threadIdx.x; i < kBoundBlocks * kDim; i += blockDim.x) {
+  __shared__ double cb[B][kDim], lb_[B][kDim], hb[B][kDim];
+  const uint64_t b0 = (uint64_t)blockIdx.x * B;
+  for (uint32_t i = threadIdx.x; i < B * kDim; i += blockDim.x) {
     const uint32_t bb = i / kDim, j = i % kDim;
     const bool in = b0 + bb < n_blocks && j < d;
     const uint64_t at = (uint64_t)j * n_blocks + b0 + bb;
@@ -333,18 +347,18 @@ ball_bounds_kernel(const double* bc_t, const double* blo_t, const double* bhi_t,
     hb[bb][j] = in ? bhi_t[at] : 0.0;
   }
   __syncthreads();
-  double rb[kBoundBlocks];
+  double rb[B];
 #pragma unroll
-  for (int bb = 0; bb < kBoundBlocks; ++bb) rb[bb] = b0 + bb < n_blocks ? br[b0 + bb] : 0.0;
+  for (int bb = 0; bb < B; ++bb) rb[bb] = b0 + bb < n_blocks ? br[b0 + bb] : 0.0;
   for (uint32_t t = threadIdx.x; t < n_tiles; t += blockDim.x) {
-    double acc[kBoundBlocks], box[kBoundBlocks];
+    double acc[B], box[B];
 #pragma unroll
-    for (int bb = 0; bb < kBoundBlocks; ++bb) acc[bb] = box[bb] = 0.0;
+    for (int bb = 0; bb < B; ++bb) acc[bb] = box[bb] = 0.0;
     for (uint32_t j = 0; j < d; ++j) {
       const uint64_t at = (uint64_t)j * n_tiles + t;
       const double v = tc_t[at], tl = tlo_t[at], th = thi_t[at];
 #pragma unroll
-      for (int bb = 0; bb < kBoundBlocks; ++bb) {
+      for (int bb = 0; bb < B; ++bb) {
         const double u = cb[bb][j] - v;
         acc[bb] = fma(u, u, acc[bb]);
         const double gap = fmax(fmax(tl - hb[bb][j], lb_[bb][j] - th), 0.0);
@@ -353,7 +367,7 @@ ball_bounds_kernel(const double* bc_t, const double* blo_t, const double* bhi_t,
     }
     const double rt = tr[t];
 #pragma unroll
-    for (int bb = 0; bb < kBoundBlocks; ++bb) {
+    for (int bb = 0; bb < B; ++bb) {
       if (b0 + bb >= n_blocks) break;
       const double dist = sqrt(acc[bb]);
       const double ball = dist * (1.0 - 0x1p-40) - rb[bb] - rt;
@@ -381,8 +395,8 @@ __global__ void key_bounds_kernel(const unsigned long long* key, uint64_t count,
 // unused in the library's pool, or three times free on the device (asked for only then:
 // cudaMemGetInfo takes 0.1 to 1.8 ms).
 bool bounded_scan(const float* x, uint64_t n, uint32_t width, uint32_t d, const double* mean,
-                  double scale, double max_norm, uint32_t qblock, bool skip, ScanPlan& sp,
-                  cudaStream_t s, Trace& trace) {
+                  double scale, double max_norm, uint32_t qblock, bool skip, int sm_count,
+                  ScanPlan& sp, cudaStream_t s, Trace& trace) {
   const uint64_t n_blocks = (n + qblock - 1) / qblock;
   const uint32_t n_tiles = (uint32_t)((n + kTile - 1) / kTile);
   const uint64_t entries = n_blocks * n_tiles;
@@ -412,9 +426,15 @@ bool bounded_scan(const float* x, uint64_t n, uint32_t width, uint32_t d, const 
   sp.list_tiles.alloc(entries, s);
   // Margin: the centred rows' f64 rounding, far below any bound that prunes.
   const double margin = 0x1p-30 * max_norm;
-  ball_bounds_kernel<<<(unsigned)((n_blocks + kBoundBlocks - 1) / kBoundBlocks), 256, 0, s>>>(
-      bc.ptr, blo.ptr, bhi.ptr, br.ptr, n_blocks, tc.ptr, tlo.ptr, thi.ptr, tr.ptr, n_tiles, d,
-      scale * scale, margin, key.ptr, tile.ptr);
+  const uint64_t shared_ctas = (n_blocks + kBoundBlocks - 1) / kBoundBlocks;
+  if (shared_ctas >= 2ull * sm_count)
+    ball_bounds_kernel<kBoundBlocks><<<(unsigned)shared_ctas, 256, 0, s>>>(
+        bc.ptr, blo.ptr, bhi.ptr, br.ptr, n_blocks, tc.ptr, tlo.ptr, thi.ptr, tr.ptr, n_tiles, d,
+        scale * scale, margin, key.ptr, tile.ptr);
+  else
+    ball_bounds_kernel<1><<<(unsigned)n_blocks, 256, 0, s>>>(
+        bc.ptr, blo.ptr, bhi.ptr, br.ptr, n_blocks, tc.ptr, tlo.ptr, thi.ptr, tr.ptr, n_tiles, d,
+        scale * scale, margin, key.ptr, tile.ptr);
   KG_LAUNCH_CHECK();
   trace.mark("scan bounds");
   DeviceBuffer<int> off(n_blocks + 1, s);
@@ -1496,7 +1516,7 @@ void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t 
       bool listed = false;
       if (order != "morton") {
         listed = bounded_scan(x, n, width, d, mean.ptr, scale, std::sqrt(h_largest),
-                              filter_query_block(kind), order != "cluster", sp, s, trace);
+                              filter_query_block(kind), order != "cluster", ctx->sm_count, sp, s, trace);
       }
       if (!listed) spatial_order(x, n, width, d, mean.ptr, lo_hi.ptr, sp.qrows, s);
       trace.mark("scan order");
