@@ -778,7 +778,12 @@ void Mlp::adam(float lr, cudaStream_t s) {
 // takes the warp's best of those (ties to the lower part) and only the lane that gave it
 // looks again. Parts, probabilities and sums come out in the same order and bits as
 // top_parts_kernel's.
+//
+// The instructions bound it: a round costs about 50, a look at every slot 900 with four held.
+// Six held make the first look dearer and the later ones, one for every lane that has given
+// more than it held, rare (64 rounds: 5 a row with four held, 0.5 with six).
 constexpr uint32_t kRegParts = 32;  // parts a lane holds
+constexpr int kTopHeld = 6;
 __device__ __forceinline__ uint32_t order_key(float v) {
   const uint32_t b = __float_as_uint(v);
   return b ^ ((b >> 31) ? 0xFFFFFFFFu : 0x80000000u);  // unsigned order = float order
@@ -812,14 +817,14 @@ top_parts_reg_kernel(const float* z, uint64_t rows, uint32_t parts, uint32_t pro
     return sum;
   };
   const float sum0 = n_mass ? lane_sum(temps[0]) : 0.0f;
-  // The lane's four best parts not yet taken, best first (value, then the lower slot on
+  // The lane's kTopHeld best parts not yet taken, best first (value, then the lower slot on
   // ties), kept sorted; refilled from every slot when they run out.
   uint32_t taken = 0;
-  float cv[4];
-  uint32_t cj[4];
+  float cv[kTopHeld];
+  uint32_t cj[kTopHeld];
   auto refill = [&]() {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < kTopHeld; ++i) {
       cv[i] = -INFINITY;
       cj[i] = 0xFFFFFFFFu;
     }
@@ -830,7 +835,7 @@ top_parts_reg_kernel(const float* z, uint64_t rows, uint32_t parts, uint32_t pro
       uint32_t xj = j;
       // Insert (strictly greater moves ahead: an earlier slot stays ahead on ties).
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < kTopHeld; ++i) {
         const bool ahead = cj[i] == 0xFFFFFFFFu || x > cv[i];
         const float tv = cv[i];
         const uint32_t tj = cj[i];
@@ -868,19 +873,20 @@ top_parts_reg_kernel(const float* z, uint64_t rows, uint32_t parts, uint32_t pro
     }
     if (t < probe) {
 #pragma unroll
-      for (uint32_t i = 0; i < kMaxTemps; ++i)
-        if (i < n_temps) picked[i] += __expf(temps[i] * (bv - m));
+      for (uint32_t i = 0; i < kMaxTemps; ++i) {
+        if (i >= n_temps) break;
+        picked[i] += __expf(temps[i] * (bv - m));
+      }
     }
     if (bp % 32 == lane) {
       taken |= 1u << (bp / 32);
-      cv[0] = cv[1];
-      cj[0] = cj[1];
-      cv[1] = cv[2];
-      cj[1] = cj[2];
-      cv[2] = cv[3];
-      cj[2] = cj[3];
-      cv[3] = -INFINITY;
-      cj[3] = 0xFFFFFFFFu;
+#pragma unroll
+      for (int i = 0; i + 1 < kTopHeld; ++i) {
+        cv[i] = cv[i + 1];
+        cj[i] = cj[i + 1];
+      }
+      cv[kTopHeld - 1] = -INFINITY;
+      cj[kTopHeld - 1] = 0xFFFFFFFFu;
       if (cj[0] == 0xFFFFFFFFu) refill();
     }
   }
