@@ -170,6 +170,28 @@ __device__ __forceinline__ uint2 map_entry(uint2 e, const ValueMap& vm, float me
                     *reinterpret_cast<const uint32_t*>(&sl) & held);
 }
 
+// C's value `c` at (row, column j): less the column's offset into the outputs that are wanted
+// (fp16 parts of the next product's D^T, f32 rows); the value as the next product sees it.
+__device__ __forceinline__ double row_output(const SpmmOut& out, uint64_t row, bool live, int j,
+                                             double c, double t_mul, double t_inv) {
+  const double cval = live && j < (int)out.width ? c - out.offsets[j] : 0.0;
+  double seen = cval;
+  if (out.t) {
+    const double y = cval * t_mul;
+    const __half hi = __double2half(y);
+    const __half lo = __double2half(y - (double)__half2float(hi));
+    seen = ((double)__half2float(hi) + (double)__half2float(lo)) * t_inv;
+    if (live) {
+      uint16_t* t = out.t + (row / 32) * 64 + (row % 32) + (uint64_t)j * out.ld_t;
+      t[0] = __half_as_ushort(hi);
+      t[32] = __half_as_ushort(lo);
+    }
+  }
+  if (live && out.rows_f32 && j < (int)out.width)
+    out.rows_f32[row * (uint64_t)out.width + j] = (float)cval;
+  return seen;
+}
+
 // One CTA per SM, 18 warps: the register file is split over the SM's four sub-partitions
 // (five warps on two of them), so 96 registers a thread; each drain warp keeps 32 f64
 // sums, and two expand warps per sub-partition hide each other's latency.
@@ -331,25 +353,10 @@ spmm_tc_kernel(const __grid_constant__ CUtensorMap tmap_dt, const uint64_t* __re
         // tile's column sums (fixed tree: warp shuffles, then the 4 quarters in order).
         const bool live = row < rows;
         const double t_mul = ldexp(1.0, out.t_scale), t_inv = ldexp(1.0, -out.t_scale);
-        uint16_t* t_row = out.t ? out.t + (row / 32) * 64 + (row % 32) : nullptr;
 #pragma unroll
         for (int jj = 0; jj < kH; ++jj) {
           const int j = (int)half * kH + jj;
-          const double cval =
-              live && j < (int)out.width ? acc[jj] * out_scale - out.offsets[j] : 0.0;
-          double seen = cval;
-          if (out.t) {
-            const double y = cval * t_mul;
-            const __half hi = __double2half(y);
-            const __half lo = __double2half(y - (double)__half2float(hi));
-            seen = ((double)__half2float(hi) + (double)__half2float(lo)) * t_inv;
-            if (live) {
-              t_row[(uint64_t)j * out.ld_t] = __half_as_ushort(hi);
-              t_row[(uint64_t)j * out.ld_t + 32] = __half_as_ushort(lo);
-            }
-          }
-          if (live && out.rows_f32 && j < (int)out.width)
-            out.rows_f32[row * (uint64_t)out.width + j] = (float)cval;
+          const double seen = row_output(out, row, live, j, acc[jj] * out_scale, t_mul, t_inv);
           if (out.colsum_partial) {
             double sv = seen;
             for (int o = 16; o; o >>= 1) sv += __shfl_xor_sync(0xFFFFFFFFu, sv, o);
@@ -847,10 +854,54 @@ sum_groups_kernel(const float* __restrict__ groups, uint32_t n_groups, uint32_t 
   partial[blockIdx.y * plane + at] = acc * out_scale;
 }
 
+// kOutRows from the groups of the product's f32 sums: each value's groups added in f64 in order,
+// then the product's own epilogue (column sums: lanes, then the tile's quarters in order). A CTA a
+// tile, a warp 32 rows and 16 columns, a lane a row.
+__global__ void __launch_bounds__(512)
+rows_of_groups_kernel(const float* __restrict__ groups, uint32_t n_groups, uint64_t rows,
+                      double out_scale, SpmmOut out) {
+  __shared__ double colsum[4][kN];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t quad = warp & 3u, j0 = (warp >> 2) * 16;
+  const uint64_t row = blockIdx.x * (uint64_t)kRows + quad * 32 + lane;
+  const bool live = row < rows;
+  double acc[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) acc[j] = 0.0;
+  for (uint32_t g = 0; g < n_groups && live; ++g) {
+    const float4* from = reinterpret_cast<const float4*>(groups + (g * rows + row) * kN + j0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float4 v = from[k];
+      acc[4 * k] += (double)v.x;
+      acc[4 * k + 1] += (double)v.y;
+      acc[4 * k + 2] += (double)v.z;
+      acc[4 * k + 3] += (double)v.w;
+    }
+  }
+  const double t_mul = ldexp(1.0, out.t_scale), t_inv = ldexp(1.0, -out.t_scale);
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    double sv = row_output(out, row, live, (int)j0 + j, acc[j] * out_scale, t_mul, t_inv);
+    if (out.colsum_partial) {
+      for (int o = 16; o; o >>= 1) sv += __shfl_xor_sync(0xFFFFFFFFu, sv, o);
+      if (lane == 0) colsum[quad][j0 + j] = sv;
+    }
+  }
+  if (!out.colsum_partial) return;
+  __syncthreads();
+  if (threadIdx.x < kN) {
+    const uint32_t j = threadIdx.x;
+    out.colsum_partial[blockIdx.x * (uint64_t)kN + j] =
+        ((colsum[0][j] + colsum[1][j]) + colsum[2][j]) + colsum[3][j];
+  }
+}
+
 // Whether `items` whole segments leave too much of the chip idle: up to three rounds of one item
-// an SM with a fifth or more of them empty. 50,000 cells x 2,000 genes have 64 segments: 340 us
-// whole, 158 and 11 us for the sums in groups. (Where the last of many rounds is the ragged one,
-// the groups, 256 bytes a row and 512 columns, cost more than it does.)
+// an SM with a fifth or more of them empty. X^T of 50,000 cells x 2,000 genes has 64 segments: 340
+// us whole, 158 and 11 us for the sums in groups; X of 2,700 cells has 22 tiles: 57 us, 20 and 12.
+// (Where the last of many rounds is the ragged one, the groups, 256 bytes a row and 512 columns,
+// cost more than it does.)
 bool split_groups(uint64_t items, int sm_count) {
   const uint64_t rounds = (items + sm_count - 1) / sm_count;
   return rounds <= 3 && items * 5 < rounds * sm_count * 4;
@@ -883,7 +934,7 @@ void spmm_tc(const SpmmArgs& a, cudaStream_t s) {
   SpmmOut to = a.out;
   DeviceBuffer<float> groups;
   const uint32_t n_groups = (geo.n_chunks + kFlushChunks - 1) / kFlushChunks;
-  if (a.out.mode == kOutPartial && (seg_chunks % kFlushChunks == 0 || geo.n_segs == 1) &&
+  if (n_groups > geo.n_segs && (seg_chunks % kFlushChunks == 0 || geo.n_segs == 1) &&
       split_groups((uint64_t)geo.n_tiles * geo.n_segs, a.sm_count)) {
     uint32_t part = kFlushChunks;
     while (part * 2 < seg_chunks &&
@@ -917,7 +968,10 @@ void spmm_tc(const SpmmArgs& a, cudaStream_t s) {
   spmm_tc_kernel<<<grid, kSpThreads, kSpSmemBytes, s>>>(m, b.off.ptr, b.data.ptr, b.rows, geo, vm,
                                                         a.row_means, out_scale, to, a.error);
   KG_LAUNCH_CHECK();
-  if (to.mode == kOutGroups) {
+  if (to.mode == kOutGroups && a.out.mode == kOutRows) {
+    rows_of_groups_kernel<<<b.n_tiles, 512, 0, s>>>(groups.ptr, n_groups, b.rows, out_scale, a.out);
+    KG_LAUNCH_CHECK();
+  } else if (to.mode == kOutGroups) {
     const uint32_t segs = (uint32_t)((geo.n_chunks + seg_chunks - 1) / seg_chunks);
     sum_groups_kernel<<<dim3(blocks_for(b.rows * kN, 256), segs), 256, 0, s>>>(
         groups.ptr, n_groups, (uint32_t)((seg_chunks + kFlushChunks - 1) / kFlushChunks), b.rows, out_scale,

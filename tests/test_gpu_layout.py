@@ -57,3 +57,21 @@ def test_split_work_items_keep_the_bits(n):
     m = np.zeros((n, few))
     m[rows[keep.ravel()], idx[keep]] = val[keep]
     assert np.all(np.abs(part - m.T @ d) <= (m.T @ np.abs(d)) * 2.0**-15 + 1e-300)
+
+
+@pytest.mark.parametrize("n", [60, 127, 128, 129, 2500])
+@pytest.mark.parametrize("g", [512, 513, 1030])
+def test_rows_from_split_work_items(n, g):
+    # Few tiles of cells: their rows come from work items of 512 columns. Each is (x - mean) V to
+    # the product's bar, 2^-15 of |x| |V| (and of the means' part), and its f32 rounding.
+    rng = np.random.default_rng(n * 7 + g)
+    x = (rng.gamma(1.0, 1.0, (n, g)) * (rng.random((n, g)) < 0.3)).astype(np.float32)
+    x[:, g - 1] = 1.0
+    rows, idx = np.nonzero(x)
+    indptr = np.zeros(n + 1, dtype=np.uint64)
+    indptr[1:] = np.cumsum(np.bincount(rows, minlength=n))
+    res = K.pca(indptr, idx.astype(np.uint32), x[rows, idx], g, 5)
+    m, v = x.astype(np.float64), res.loadings.astype(np.float64)
+    ref = (m - m.mean(0)) @ v
+    bar = ((np.abs(m) + np.abs(m).mean(0)) @ np.abs(v)) * (2.0**-15 + 2.0**-22)
+    assert np.all(np.abs(res.embedding - ref) <= bar)
