@@ -408,7 +408,7 @@ bool bounded_scan(const float* x, uint64_t n, uint32_t width, uint32_t d, const 
   }
   Clusters cl;
   const uint32_t parts = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(n / 1024, 1), 4096);
-  cluster_rows(x, n, width, d, parts, 5, 131072, cl, s);
+  cluster_rows(x, n, width, d, parts, 5, 131072, false, cl, s);
   trace.mark("scan parts");
   DeviceBuffer<double> bc((uint64_t)kDim * n_blocks, s), blo((uint64_t)kDim * n_blocks, s),
       bhi((uint64_t)kDim * n_blocks, s), br(n_blocks, s);
