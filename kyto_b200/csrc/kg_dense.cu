@@ -5,6 +5,7 @@
 
 #include "kg_dense.cuh"
 #include "kg_internal.cuh"
+#include "kg_order.cuh"
 
 namespace kg {
 
@@ -238,13 +239,10 @@ __device__ __forceinline__ int jacobi_square(JacobiShared& sh, uint32_t w, doubl
     const double n = sh.norms[c];
     uint32_t rank = 0;
     for (uint32_t o = 0; o < w; ++o) {
-      const double m = sh.norms[o];
-      rank += (m > n || (!(m < n) && o < c)) ? 1u : 0u;
+      rank += column_before(sh.norms[o], o, n, c) ? 1u : 0u;
     }
-    if (rank < w) {
-      sh.order[rank] = c;
-      sigma[rank] = n;
-    }
+    sh.order[rank] = c;  // the ranks are a permutation of 0 .. w - 1
+    sigma[rank] = n;
   }
   __syncthreads();
   return sweep >= 60 ? 1 : 0;
@@ -278,6 +276,10 @@ small_svd_kernel(const double* r, uint32_t w, const double* block, uint64_t n, c
   if (blockIdx.x == 1) {
     const double t = squares_sum(block, n, sh.norms);
     if (threadIdx.x == 0) out[w] = sqrt(t);
+    return;
+  }
+  if (*status) {  // a factor was not written (the same for every thread)
+    if (threadIdx.x == 0) out[w + 1] = 1.0;
     return;
   }
   const uint32_t tid = threadIdx.x, tx = tid & 15u, ty = tid >> 4;
@@ -327,7 +329,7 @@ small_svd_kernel(const double* r, uint32_t w, const double* block, uint64_t n, c
     const double nv = sh.norms[sh.order[c]];
     u_r[x] = nv > 0.0 ? sh.a[sh.order[c]][jacobi_row(i)] / nv : 0.0;
   }
-  if (tid == 0) out[w + 1] = failed || *status ? 1.0 : 0.0;
+  if (tid == 0) out[w + 1] = failed ? 1.0 : 0.0;
 }
 
 __global__ void __launch_bounds__(1024)

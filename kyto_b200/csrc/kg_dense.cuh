@@ -23,8 +23,9 @@ void cholesky_step(const double* gram, uint32_t w, double shift, double* r, int*
 // The SVD of R = R_3 R_2 R_1, the steps' factors one after another in r (w x w upper
 // triangular, column-major, w <= 64): out[0 .. w) the singular values (descending, ties to
 // the lower column), u_r (w x w: column c the unit left singular vector of out[c]; zero for
-// 0), out[w] = the Frobenius norm of `block` (n values), out[w + 1] = 0, or 1 if *status
-// was set or Jacobi did not converge.
+// 0), out[w] = the Frobenius norm of `block` (n values), out[w + 1] = 0, or 1 if Jacobi did
+// not converge or *status is set: then a step's factor is not there, r is not read, and the
+// singular values and u_r are left as they are.
 void small_svd(const double* r, uint32_t w, const double* block, uint64_t n, const int* status,
                double* u_r, double* out, cudaStream_t s);
 
