@@ -41,7 +41,10 @@ __device__ __forceinline__ float exp2_approx(float x) {
 
 // The rows' checks, sigmas and memberships, a CTA's blockDim.x rows at a time (their entries
 // are one run). Sets *bad on a violation of the graph's shape: 1 when row r does not hold
-// entries [r k, (r + 1) k), 2 when its columns do not increase strictly below n.
+// entries [r k, (r + 1) k), 2 when its columns do not increase strictly below n. A CTA reads its
+// rows' entries only after all its rows' indptr has passed (a graph of another k may hold fewer),
+// and the kernels after this one return on *bad: what a CTA left out is not written, and a column
+// out of range would take a merge past its rows.
 //
 // A thread a row (connectivities.rs:90-104, 133-176): the distances ranked by (distance,
 // column), a stable insertion sort in shared memory (equal distances keep the input order,
@@ -73,12 +76,15 @@ __global__ void graph_rows_kernel(const uint64_t* indptr, const uint32_t* __rest
   const uint32_t rows = (uint32_t)min((uint64_t)blockDim.x, n - r0);
   const uint32_t entries = rows * k;
   const uint64_t e0 = r0 * k;
+  const uint64_t r = r0 + threadIdx.x;
+  if (__syncthreads_or(threadIdx.x < rows && (indptr[r] != r * k || indptr[r + 1] != (r + 1) * k))) {
+    if (threadIdx.x == 0) atomicExch(bad, 1);
+    return;
+  }
   for (uint32_t x = threadIdx.x; x < entries; x += blockDim.x)
     sorted[(x / k) * ld + x % k] = distances[e0 + x];
   __syncthreads();
   if (threadIdx.x < rows) {
-    const uint64_t r = r0 + threadIdx.x;
-    if (indptr[r] != r * k || (r + 1 == n && indptr[n] != n * k)) atomicExch(bad, 1);
     float* row = sorted + threadIdx.x * ld;
     for (uint32_t j = 1; j < k; ++j) {
       const float v = row[j];
@@ -198,11 +204,12 @@ __device__ __forceinline__ float union_weight(float wf, float wt) {
 __global__ void union_rows_kernel(const uint32_t* __restrict__ indices,
                                   const float* __restrict__ w, uint64_t n, uint32_t k,
                                   const uint32_t* __restrict__ tentry,
-                                  const uint32_t* __restrict__ tstart, uint64_t* counts,
-                                  uint32_t* __restrict__ out_idx, float* __restrict__ out_w) {
+                                  const uint32_t* __restrict__ tstart, const int* bad,
+                                  uint64_t* counts, uint32_t* __restrict__ out_idx,
+                                  float* __restrict__ out_w) {
   const uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-  if (r >= n) return;
+  if (r >= n || *bad) return;
   const bool own = lane < k;
   const uint32_t col = own ? indices[r * k + lane] : 0xFFFFFFFFu;
   const float wf = own ? w[r * k + lane] : 0.0f;
@@ -264,9 +271,10 @@ __global__ void union_rows_kernel(const uint32_t* __restrict__ indices,
 // Any k: a thread a row, the two runs merged.
 __global__ void union_merge_kernel(const uint32_t* indices, const float* w, uint64_t n, uint32_t k,
                                    const uint32_t* tentry, const uint32_t* tstart,
-                                   uint64_t* counts, uint32_t* out_idx, float* out_w) {
+                                   const int* bad, uint64_t* counts, uint32_t* out_idx,
+                                   float* out_w) {
   const uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (r >= n) return;
+  if (r >= n || *bad) return;
   uint64_t f = r * k;
   const uint64_t f_end = f + k;
   uint32_t b = tstart[r];
@@ -385,10 +393,12 @@ extern "C" kg_status kg_connectivities(kg_ctx* ctx, const uint64_t* indptr,
     KG_CUDA(cudaMemsetAsync(ptr.ptr + n_rows, 0, 8, s));
     if (k <= 32)
       union_rows_kernel<<<blocks_for(n_rows * 32, 256), 256, 0, s>>>(
-          d_idx, w.ptr, n_rows, k, tentry_sorted.ptr, tstart.ptr, ptr.ptr, oi.ptr, ow.ptr);
+          d_idx, w.ptr, n_rows, k, tentry_sorted.ptr, tstart.ptr, bad.ptr, ptr.ptr, oi.ptr,
+          ow.ptr);
     else
       union_merge_kernel<<<blocks_for(n_rows, 128), 128, 0, s>>>(
-          d_idx, w.ptr, n_rows, k, tentry_sorted.ptr, tstart.ptr, ptr.ptr, oi.ptr, ow.ptr);
+          d_idx, w.ptr, n_rows, k, tentry_sorted.ptr, tstart.ptr, bad.ptr, ptr.ptr, oi.ptr,
+          ow.ptr);
     KG_LAUNCH_CHECK();
     size_t temp2 = 0;
     KG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp2, ptr.ptr, ptr.ptr, n_rows + 1, s));
