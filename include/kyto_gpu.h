@@ -172,7 +172,9 @@ KG_API kg_status kg_pca_begin(kg_ctx* ctx, const kg_pca_params* params, kg_pca**
  * is copied to the device, normalized/log1p'd/gene-selected there in one kernel and
  * held in HBM for every pass (kyto's held input, held_input.rs). cells: each row's
  * table position (Omega's seed input); NULL numbers the rows on from the last
- * block. */
+ * block. Each row's genes are distinct, in increasing order as kyto's store holds them; rows
+ * in another order are taken too, but send the whole run to the f64 products, which are
+ * several times slower. */
 KG_API kg_status kg_pca_push_block(kg_pca* pca, const uint64_t* indptr, const uint32_t* indices,
                             const void* values, kg_dtype dtype, uint64_t n_rows,
                             const uint64_t* cells);

@@ -749,14 +749,15 @@ struct TcHeld {
   DeviceBuffer<int> error;     // set by a product whose bounded wait ran out
   int sm = 148;
 
-  void build(const uint64_t* indptr, const uint32_t* col, const float* val, uint64_t n_rows,
+  // False when a row's columns do not strictly increase (the layouts need them to).
+  bool build(const uint64_t* indptr, const uint32_t* col, const float* val, uint64_t n_rows,
              uint32_t n_genes, uint64_t nnz, int sm_count, cudaStream_t s, Trace& trace) {
     n = n_rows;
     g = n_genes;
     this->nnz = nnz;
     sm = sm_count;
     counts.alloc(g, s);
-    build_blocked(indptr, col, val, n, g, nnz, bx, &bxt, counts.ptr, s);
+    if (!build_blocked(indptr, col, val, n, g, nnz, bx, &bxt, counts.ptr, s)) return false;
     trace.mark("blocked X, X^T");
     dt.alloc(64 * dense_ld(n), s);
     dt.zero();
@@ -764,6 +765,7 @@ struct TcHeld {
     qt.zero();
     error.alloc(1, s);
     error.zero();
+    return true;
   }
 
   // Whether a product gave up waiting (reads the flag: synchronises the stream).
@@ -1219,7 +1221,8 @@ void kg_pca::run() {
   Trace trace(s, "pca");
   // The products run on the tensor cores (fp16 hi/lo parts of both operands, about 2^-22
   // each; f32 sums of at most 512 terms flushed into f64) when the genes fit 16-bit
-  // positions, the block one 64-column tile, the values span at most 2^30, and no gene's
+  // positions, the block one 64-column tile, every row's genes increase (kyto's do; the
+  // layouts' builder finds out), the values span at most 2^30, and no gene's
   // mean dwarfs its spread (the rows are centred after the product, so the products'
   // relative error is scaled by |mean| / sd: at most 64, about 2^-16); else on the SIMT
   // pipes in f64 (kyto's arithmetic, any data).
@@ -1237,11 +1240,14 @@ void kg_pca::run() {
                                  " holds a value that is not finite (NaN or infinity)");
   };
   DeviceBuffer<double> omega_sums(l, s), sketch1((uint64_t)g * l, s);
+  if (tc && !th.build(indptr.ptr, col.ptr, val.ptr, n, g, nnz, c->sm_count, s, trace)) {
+    tc = false;
+    th = TcHeld();
+  }
   if (tc) {
     // Pass 0's sketch X^T Omega (pca.rs:588-622) and gene means (its sums, pca.rs:707-717, with
     // the sketch), and the centred sums of squares over the stored values (the last pass's,
     // pca.rs:664-676), as products with a column of ones; the stored counts from the layout.
-    th.build(indptr.ptr, col.ptr, val.ptr, n, g, nnz, c->sm_count, s, trace);
     trace.mark("operand buffers");
     DeviceBuffer<double> sums(g, s), sq(g, s);
     th.sketch(cells.ptr, l, seed, sketch1.ptr, omega_sums.ptr, sums.ptr, s);
@@ -1752,7 +1758,9 @@ kg_status kg_diag_spmm(kg_ctx* ctx, const uint64_t* indptr, const uint32_t* indi
     const uint32_t* d_idx = device_view(indices, nnz, hi_idx, s);
     const float* d_val = device_view(values, nnz, hv, s);
     Blocked bx, bxt;
-    build_blocked(d_ptr, d_idx, d_val, n_rows, n_cols, nnz, bx, transposed ? &bxt : nullptr, nullptr, s);
+    if (!build_blocked(d_ptr, d_idx, d_val, n_rows, n_cols, nnz, bx, transposed ? &bxt : nullptr,
+                       nullptr, s))
+      fail(KG_ERR_INVALID, "kg_diag_spmm: a row's columns must increase strictly");
     const Blocked* sp = transposed ? &bxt : &bx;
     const uint64_t rows = sp->rows, K = sp->K, ld = dense_ld(K);
     DeviceBuffer<double> hd;

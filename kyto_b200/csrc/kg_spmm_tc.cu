@@ -568,15 +568,36 @@ constexpr int kLayRows = 32 / kLayWarps;    // CSR rows a warp
 constexpr uint32_t kMaskCols = 512;         // columns a window of masks_kernel
 constexpr uint32_t kValueCols = 256;        // and of values_kernel
 
+// This warp's rows: each row's entries still to come, and the least column the next may have.
+struct WalkRows {
+  uint64_t at[kLayRows], end[kLayRows];
+  uint32_t least[kLayRows];
+};
+
+__device__ __forceinline__ WalkRows walk_start(const uint64_t* __restrict__ ptr, uint64_t n_rows) {
+  WalkRows w;
+#pragma unroll
+  for (int k = 0; k < kLayRows; ++k) {
+    const uint64_t r = blockIdx.x * 32ull + (threadIdx.x >> 5) * kLayRows + k;
+    w.at[k] = r < n_rows ? ptr[r] : 0;
+    w.end[k] = r < n_rows ? ptr[r + 1] : 0;
+    w.least[k] = 0;
+  }
+  return w;
+}
+
 // Calls f(row, column - c0, value) for the entries of this warp's rows in columns [c0, c_end)
-// that it has not passed yet (`at` to `end`: each row's entries still to come). The value is 0
-// without `Values`.
+// that it has not passed yet. The value is 0 without `Values`. Returns (without `Values`) whether
+// this lane met a column that does not follow the one before it: the entries it then calls f for
+// are not the window's, but every column it passes lies inside the window, whatever the rows hold.
 template <bool Values, class F>
-__device__ __forceinline__ void walk_window(const uint32_t* __restrict__ col,
-                                            const float* __restrict__ val, uint64_t (&at)[kLayRows],
-                                            const uint64_t (&end)[kLayRows], uint32_t c0,
+__device__ __forceinline__ bool walk_window(const uint32_t* __restrict__ col,
+                                            const float* __restrict__ val, WalkRows& w, uint32_t c0,
                                             uint32_t c_end, F&& f) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint64_t(&at)[kLayRows] = w.at;
+  const uint64_t(&end)[kLayRows] = w.end;
+  bool unsorted = false;
   for (;;) {
     uint32_t c[kLayRows];
     float v[kLayRows];
@@ -589,42 +610,47 @@ __device__ __forceinline__ void walk_window(const uint32_t* __restrict__ col,
     bool more = false;
 #pragma unroll
     for (int k = 0; k < kLayRows; ++k) {
-      const bool in = c[k] < c_end;
+      const bool in = c[k] - c0 < c_end - c0;
       if (in) f(warp * kLayRows + k, c[k] - c0, v[k]);
       const uint32_t n = __popc(__ballot_sync(0xFFFFFFFFu, in));  // increasing: the first n
+      if (!Values) {
+        const uint32_t before = __shfl_up_sync(0xFFFFFFFFu, c[k], 1);
+        unsorted |= at[k] + lane < end[k] && (lane ? c[k] <= before : c[k] < w.least[k]);
+        const uint32_t last = __shfl_sync(0xFFFFFFFFu, c[k], n - 1);
+        if (n) w.least[k] = last + 1;
+      }
       at[k] += n;
       more = more || n == 32;
     }
     if (!more) break;
   }
+  return unsorted;
 }
 
 // Header masks of X (masks, words of 64 a block) and, if masks_t, of X^T: a byte an entry in
 // shared memory, gathered into words by ballots. Every word of both layouts is written. `groups`:
 // groups of 32 columns to pass, at least X's chunks and four times X^T's tiles. With X^T each
-// column's entries are counted too (counts, if given: whole numbers, so any order).
+// column's entries are counted too (counts, if given: whole numbers, so any order). *unsorted is
+// set when a row's columns do not strictly increase: the masks are then of no use.
 __global__ void __launch_bounds__(kLayWarps * 32)
 masks_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint64_t n_rows,
              uint32_t n_chunks, uint32_t n_tiles_t, uint32_t n_chunks_t, uint32_t groups,
-             uint32_t* masks, uint32_t* masks_t, unsigned long long* counts) {
+             uint32_t* masks, uint32_t* masks_t, unsigned long long* counts,
+             unsigned long long* unsorted) {
   constexpr uint32_t kLd = kMaskCols / 4 + 1;  // words a row: an odd stride
   __shared__ uint32_t flags[32][kLd];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint64_t rb = blockIdx.x, tile = rb / 4, q = rb % 4;
-  uint64_t at[kLayRows], end[kLayRows];
-#pragma unroll
-  for (int k = 0; k < kLayRows; ++k) {
-    const uint64_t r = rb * 32 + warp * kLayRows + k;
-    at[k] = r < n_rows ? ptr[r] : 0;
-    end[k] = r < n_rows ? ptr[r + 1] : 0;
-  }
+  WalkRows rows = walk_start(ptr, n_rows);
+  bool out_of_order = false;
   for (uint32_t g0 = 0; g0 < groups; g0 += kMaskCols / 32) {
     for (uint32_t i = threadIdx.x; i < 32 * kLd; i += kLayWarps * 32) (&flags[0][0])[i] = 0;
     __syncthreads();
     const uint32_t c0 = g0 * 32;
-    walk_window<false>(col, nullptr, at, end, c0, c0 + kMaskCols, [&](uint32_t row, uint32_t c, float) {
-      reinterpret_cast<unsigned char*>(flags[row])[c] = 1;
-    });
+    out_of_order |= walk_window<false>(col, nullptr, rows, c0, c0 + kMaskCols,
+                                       [&](uint32_t row, uint32_t c, float) {
+                                         reinterpret_cast<unsigned char*>(flags[row])[c] = 1;
+                                       });
     __syncthreads();
     for (uint32_t g = warp; g < kMaskCols / 32 && g0 + g < groups; g += kLayWarps) {
       if (g0 + g < n_chunks) {  // lane = row
@@ -657,6 +683,7 @@ masks_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col,
     }
     __syncthreads();
   }
+  if (__any_sync(0xFFFFFFFFu, out_of_order) && lane == 0) *unsorted = 1;
 }
 
 // A layout as values_kernel writes it.
@@ -699,18 +726,12 @@ values_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col
   __shared__ uint32_t tile[32][kValueCols + 1];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint64_t rb = blockIdx.x;
-  uint64_t at[kLayRows], end[kLayRows];
-#pragma unroll
-  for (int k = 0; k < kLayRows; ++k) {
-    const uint64_t r = rb * 32 + warp * kLayRows + k;
-    at[k] = r < n_rows ? ptr[r] : 0;
-    end[k] = r < n_rows ? ptr[r + 1] : 0;
-  }
+  WalkRows rows = walk_start(ptr, n_rows);
   for (uint32_t g0 = 0; g0 < groups; g0 += kValueCols / 32) {
     for (uint32_t i = threadIdx.x; i < 32 * (kValueCols + 1); i += kLayWarps * 32)
       (&tile[0][0])[i] = kAbsentHi;
     __syncthreads();
-    walk_window<true>(col, val, at, end, g0 * 32, g0 * 32 + kValueCols,
+    walk_window<true>(col, val, rows, g0 * 32, g0 * 32 + kValueCols,
                       [&](uint32_t row, uint32_t c, float v) { tile[row][c] = stored_parts(v, scale); });
     __syncthreads();
     for (uint32_t g = warp; g < kValueCols / 32 && g0 + g < groups; g += kLayWarps) {
@@ -789,21 +810,20 @@ struct Building {
 
 }  // namespace
 
-void build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val, uint64_t n_rows,
+bool build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val, uint64_t n_rows,
                    uint64_t n_cols, uint64_t nnz, Blocked& out, Blocked* twin,
                    unsigned long long* col_counts, cudaStream_t s) {
   if (col_counts) KG_CUDA(cudaMemsetAsync(col_counts, 0, n_cols * sizeof *col_counts, s));
   // The values' range (the scale of their fp16 parts) and the largest row norm.
-  DeviceBuffer<unsigned long long> st(3, s);
-  const unsigned long long init[3] = {0ull, 0ull, 0x7FF0000000000000ull};  // 0, 0, +inf
+  // And whether a row's columns are out of order.
+  DeviceBuffer<unsigned long long> st(4, s);
+  const unsigned long long init[4] = {0ull, 0ull, 0x7FF0000000000000ull, 0ull};  // 0, 0, +inf
   KG_CUDA(cudaMemcpyAsync(st.ptr, init, sizeof init, cudaMemcpyHostToDevice, s));
   if (nnz) {
     csr_stats_kernel<<<std::min<unsigned>(blocks_for(n_rows * 32, 256), 2048), 256, 0, s>>>(
         ptr, val, n_rows, st.ptr, st.ptr + 1, st.ptr + 2);
     KG_LAUNCH_CHECK();
   }
-  unsigned long long h_st[3];
-  KG_CUDA(cudaMemcpyAsync(h_st, st.ptr, sizeof h_st, cudaMemcpyDeviceToHost, s));
   Building x, t;
   x.start(out, n_rows, n_cols, s);
   if (twin) t.start(*twin, n_cols, n_rows, s);
@@ -812,12 +832,16 @@ void build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val, u
   const unsigned grid = out.n_tiles * 4;
   if (grid) {
     masks_kernel<<<grid, kLayWarps * 32, 0, s>>>(ptr, col, n_rows, out.n_chunks, tiles_t, chunks_t,
-                                                 groups, x.masks.ptr, t.masks.ptr, col_counts);
+                                                 groups, x.masks.ptr, t.masks.ptr, col_counts,
+                                                 st.ptr + 3);
     KG_LAUNCH_CHECK();
   }
   x.offsets(s);
   if (twin) t.offsets(s);
+  unsigned long long h_st[4];
+  KG_CUDA(cudaMemcpyAsync(h_st, st.ptr, sizeof h_st, cudaMemcpyDeviceToHost, s));
   KG_CUDA(cudaStreamSynchronize(s));
+  if (h_st[3]) return false;
   double d[3];
   std::memcpy(d, h_st, sizeof d);
   out.max_row_norm = std::sqrt(d[0]);
@@ -832,10 +856,11 @@ void build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val, u
   }
   const LayoutOut xo = x.layout(s);
   const LayoutOut to = twin ? t.layout(s) : LayoutOut{nullptr, nullptr, nullptr, nullptr, 0};
-  if (!x.units) return;
+  if (!x.units) return true;
   values_kernel<<<grid, kLayWarps * 32, 0, s>>>(ptr, col, val, n_rows, tiles_t, groups, out.scale, xo,
                                                 to);
   KG_LAUNCH_CHECK();
+  return true;
 }
 
 namespace {
