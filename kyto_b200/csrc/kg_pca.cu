@@ -749,7 +749,7 @@ struct TcHeld {
   DeviceBuffer<int> error;     // set by a product whose bounded wait ran out
   int sm = 148;
 
-  // False when a row's columns do not strictly increase (the layouts need them to).
+  // False, with nothing to use, when the rows' order does not allow the layouts.
   bool build(const uint64_t* indptr, const uint32_t* col, const float* val, uint64_t n_rows,
              uint32_t n_genes, uint64_t nnz, int sm_count, cudaStream_t s, Trace& trace) {
     n = n_rows;
@@ -1221,8 +1221,8 @@ void kg_pca::run() {
   Trace trace(s, "pca");
   // The products run on the tensor cores (fp16 hi/lo parts of both operands, about 2^-22
   // each; f32 sums of at most 512 terms flushed into f64) when the genes fit 16-bit
-  // positions, the block one 64-column tile, every row's genes increase (kyto's do; the
-  // layouts' builder finds out), the values span at most 2^30, and no gene's
+  // positions, the block one 64-column tile, every row's genes increase (kyto's do; rows
+  // that do not show in the layouts' counts), the values span at most 2^30, and no gene's
   // mean dwarfs its spread (the rows are centred after the product, so the products'
   // relative error is scaled by |mean| / sd: at most 64, about 2^-16); else on the SIMT
   // pipes in f64 (kyto's arithmetic, any data).
@@ -1267,6 +1267,7 @@ void kg_pca::run() {
     th.mean_norm = std::sqrt(mn);
     colptr[0] = 0;
     for (uint32_t i = 0; i < g; ++i) colptr[i + 1] = colptr[i] + (uint64_t)h_cnt[i];
+    const bool distinct = colptr[g] == nnz;  // (a gene twice in a row counts once)
     double worst_ratio = 0.0;
     for (uint32_t i = 0; i < g; ++i) {
       uint64_t stored = colptr[i + 1] - colptr[i];
@@ -1278,7 +1279,7 @@ void kg_pca::run() {
     // comfortable range, goes to the f64 path.
     const bool range_ok = th.bx.min_abs == 0.0 || th.bx.max_abs / th.bx.min_abs <= 0x1p30;
     const bool scale_ok = th.bx.scale >= -100 && th.bx.scale <= 100;
-    if (worst_ratio > 4096.0 || !range_ok || !scale_ok) {
+    if (!distinct || worst_ratio > 4096.0 || !range_ok || !scale_ok) {
       tc = false;
       th.clock.release();
       th = TcHeld();

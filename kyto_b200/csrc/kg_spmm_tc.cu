@@ -562,16 +562,15 @@ __device__ __forceinline__ uint2 make_entry(uint32_t w0, uint32_t w1) {
 // chunk of X^T's columns, through a window of columns at a time in shared memory, a warp four
 // rows, the lanes over each row's entries. Reading the entries and writing both layouts bounds
 // it. (Each layout by itself, a lane writing where its entry goes, every entry a sector:
-// masks 3.8 and values 11.0 ms for 1M rows of 570 entries, now 1.4 and 3.8, 3.3 TB/s.)
+// masks 3.8 and values 11.0 ms for 1M rows of 570 entries, now 1.75 and 3.8.)
 constexpr int kLayWarps = 8;                // a CTA
 constexpr int kLayRows = 32 / kLayWarps;    // CSR rows a warp
 constexpr uint32_t kMaskCols = 512;         // columns a window of masks_kernel
 constexpr uint32_t kValueCols = 256;        // and of values_kernel
 
-// This warp's rows: each row's entries still to come, and the least column the next may have.
+// This warp's rows: each row's entries still to come.
 struct WalkRows {
   uint64_t at[kLayRows], end[kLayRows];
-  uint32_t least[kLayRows];
 };
 
 __device__ __forceinline__ WalkRows walk_start(const uint64_t* __restrict__ ptr, uint64_t n_rows) {
@@ -581,23 +580,26 @@ __device__ __forceinline__ WalkRows walk_start(const uint64_t* __restrict__ ptr,
     const uint64_t r = blockIdx.x * 32ull + (threadIdx.x >> 5) * kLayRows + k;
     w.at[k] = r < n_rows ? ptr[r] : 0;
     w.end[k] = r < n_rows ? ptr[r + 1] : 0;
-    w.least[k] = 0;
   }
   return w;
 }
 
-// Calls f(row, column - c0, value) for the entries of this warp's rows in columns [c0, c_end)
-// that it has not passed yet. The value is 0 without `Values`. Returns (without `Values`) whether
-// this lane met a column that does not follow the one before it: the entries it then calls f for
-// are not the window's, but every column it passes lies inside the window, whatever the rows hold.
-template <bool Values, class F>
-__device__ __forceinline__ bool walk_window(const uint32_t* __restrict__ col,
+// Calls f(row, column - c0, value) for the entries of this warp's rows in columns [c0, c0 + Cols)
+// that it has not passed yet. The value is 0 without `Values`. With `Checked`, f's columns lie inside
+// the window whatever the rows hold, and *jumped becomes not 0 when an entry stands behind one of
+// a later run of kValueCols columns: where that is so for no window, each entry is passed once, in
+// its own window, in windows of Cols and of kValueCols columns alike (within a run the order does
+// not matter: the tiles are filled by column). Rows without a jump need no check of the window's
+// lower end (0.5 ms of values_kernel's 3.8 for the check; masks_kernel's take 0.35 of 1.75).
+template <bool Values, bool Checked, uint32_t Cols, class F>
+__device__ __forceinline__ void walk_window(const uint32_t* __restrict__ col,
                                             const float* __restrict__ val, WalkRows& w, uint32_t c0,
-                                            uint32_t c_end, F&& f) {
+                                            uint32_t* jumped, F&& f) {
+  static_assert(Cols == kValueCols || Cols == 2 * kValueCols, "a window is one or two runs");
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   uint64_t(&at)[kLayRows] = w.at;
   const uint64_t(&end)[kLayRows] = w.end;
-  bool unsorted = false;
+  uint32_t second = 0;  // bit k: row k is in the window's second run
   for (;;) {
     uint32_t c[kLayRows];
     float v[kLayRows];
@@ -610,29 +612,38 @@ __device__ __forceinline__ bool walk_window(const uint32_t* __restrict__ col,
     bool more = false;
 #pragma unroll
     for (int k = 0; k < kLayRows; ++k) {
-      const bool in = c[k] - c0 < c_end - c0;
+      const bool in = Checked ? c[k] - c0 < Cols : c[k] < c0 + Cols;
       if (in) f(warp * kLayRows + k, c[k] - c0, v[k]);
-      const uint32_t n = __popc(__ballot_sync(0xFFFFFFFFu, in));  // increasing: the first n
-      if (!Values) {
-        const uint32_t before = __shfl_up_sync(0xFFFFFFFFu, c[k], 1);
-        unsorted |= at[k] + lane < end[k] && (lane ? c[k] <= before : c[k] < w.least[k]);
-        const uint32_t last = __shfl_sync(0xFFFFFFFFu, c[k], n - 1);
-        if (n) w.least[k] = last + 1;
+      const uint32_t held = __ballot_sync(0xFFFFFFFFu, in);  // in order: the first n
+      const uint32_t n = __popc(held);
+      if (Checked) {
+        const uint32_t run = __ballot_sync(0xFFFFFFFFu, c[k] - c0 < kValueCols);
+        *jumped |= (held & (held + 1u)) | (run & (run + 1u)) | (run & (0u - (second >> k & 1u)));
+        second |= (held != run ? 1u : 0u) << k;
       }
       at[k] += n;
       more = more || n == 32;
     }
     if (!more) break;
   }
-  return unsorted;
+}
+
+// Whether every entry of this warp's rows was passed: one that comes behind an entry of a later
+// window holds its row up before its end.
+__device__ __forceinline__ bool walk_ended(const WalkRows& w) {
+  bool all = true;
+#pragma unroll
+  for (int k = 0; k < kLayRows; ++k) all = all && w.at[k] == w.end[k];
+  return all;
 }
 
 // Header masks of X (masks, words of 64 a block) and, if masks_t, of X^T: a byte an entry in
 // shared memory, gathered into words by ballots. Every word of both layouts is written. `groups`:
 // groups of 32 columns to pass, at least X's chunks and four times X^T's tiles. With X^T each
-// column's entries are counted too (counts, if given: whole numbers, so any order). *unsorted is
-// set when a row's columns do not strictly increase: the masks are then of no use.
-__global__ void __launch_bounds__(kLayWarps * 32)
+// column's entries are counted too (counts, if given: whole numbers, so any order; a column twice
+// in a row counts once). *unsorted is set when a row's entries do not come run by run of kValueCols
+// columns, and without `counts` when a row holds a column twice: the masks are then of no use.
+__global__ void __launch_bounds__(kLayWarps * 32, 5)
 masks_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint64_t n_rows,
              uint32_t n_chunks, uint32_t n_tiles_t, uint32_t n_chunks_t, uint32_t groups,
              uint32_t* masks, uint32_t* masks_t, unsigned long long* counts,
@@ -642,15 +653,15 @@ masks_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col,
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint64_t rb = blockIdx.x, tile = rb / 4, q = rb % 4;
   WalkRows rows = walk_start(ptr, n_rows);
-  bool out_of_order = false;
+  uint32_t held_x = 0, jumped = 0;
   for (uint32_t g0 = 0; g0 < groups; g0 += kMaskCols / 32) {
     for (uint32_t i = threadIdx.x; i < 32 * kLd; i += kLayWarps * 32) (&flags[0][0])[i] = 0;
     __syncthreads();
     const uint32_t c0 = g0 * 32;
-    out_of_order |= walk_window<false>(col, nullptr, rows, c0, c0 + kMaskCols,
-                                       [&](uint32_t row, uint32_t c, float) {
-                                         reinterpret_cast<unsigned char*>(flags[row])[c] = 1;
-                                       });
+    walk_window<false, true, kMaskCols>(col, nullptr, rows, c0, &jumped,
+                                        [&](uint32_t row, uint32_t c, float) {
+                                          reinterpret_cast<unsigned char*>(flags[row])[c] = 1;
+                                        });
     __syncthreads();
     for (uint32_t g = warp; g < kMaskCols / 32 && g0 + g < groups; g += kLayWarps) {
       if (g0 + g < n_chunks) {  // lane = row
@@ -662,6 +673,7 @@ masks_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col,
           const uint32_t odd = __ballot_sync(0xFFFFFFFFu, w >> 16);
           if (lane == 2 * k) mine = even;
           if (lane == 2 * k + 1) mine = odd;
+          if (!counts) held_x += __popc(w);  // (a byte an entry, 0 or 1)
         }
         if (lane < 16) masks[(tile * n_chunks + g0 + g) * 64 + q * 16 + lane] = mine;
       }
@@ -683,7 +695,16 @@ masks_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col,
     }
     __syncthreads();
   }
-  if (__any_sync(0xFFFFFFFFu, out_of_order) && lane == 0) *unsorted = 1;
+  if (jumped || !walk_ended(rows)) *unsorted = 1;
+  if (!counts) {
+    __shared__ uint32_t held_all;
+    if (threadIdx.x == 0) held_all = 0;
+    __syncthreads();
+    atomicAdd(&held_all, held_x);
+    __syncthreads();
+    const uint64_t first = min(rb * 32, n_rows), past = min(rb * 32 + 32, n_rows);
+    if (threadIdx.x == 0 && held_all != ptr[past] - ptr[first]) *unsorted = 1;
+  }
 }
 
 // A layout as values_kernel writes it.
@@ -718,7 +739,8 @@ __device__ __forceinline__ void write_quarter(const LayoutOut& o, uint64_t b, ui
   }
 }
 
-// Headers and entries of X and, if wanted, of X^T. `groups` as in masks_kernel.
+// Headers and entries of X and, if wanted, of X^T, of rows that masks_kernel has passed. `groups` as
+// there.
 __global__ void __launch_bounds__(kLayWarps * 32)
 values_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col,
               const float* __restrict__ val, uint64_t n_rows, uint32_t n_tiles_t, uint32_t groups,
@@ -731,8 +753,9 @@ values_kernel(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ col
     for (uint32_t i = threadIdx.x; i < 32 * (kValueCols + 1); i += kLayWarps * 32)
       (&tile[0][0])[i] = kAbsentHi;
     __syncthreads();
-    walk_window<true>(col, val, rows, g0 * 32, g0 * 32 + kValueCols,
-                      [&](uint32_t row, uint32_t c, float v) { tile[row][c] = stored_parts(v, scale); });
+    walk_window<true, false, kValueCols>(
+        col, val, rows, g0 * 32, nullptr,
+        [&](uint32_t row, uint32_t c, float v) { tile[row][c] = stored_parts(v, scale); });
     __syncthreads();
     for (uint32_t g = warp; g < kValueCols / 32 && g0 + g < groups; g += kLayWarps) {
       if (g0 + g < x.n_chunks)
@@ -815,9 +838,9 @@ bool build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val, u
                    unsigned long long* col_counts, cudaStream_t s) {
   if (col_counts) KG_CUDA(cudaMemsetAsync(col_counts, 0, n_cols * sizeof *col_counts, s));
   // The values' range (the scale of their fp16 parts) and the largest row norm.
-  // And whether a row's columns are out of order.
+  // And the masks' verdict on the rows' order.
   DeviceBuffer<unsigned long long> st(4, s);
-  const unsigned long long init[4] = {0ull, 0ull, 0x7FF0000000000000ull, 0ull};  // 0, 0, +inf
+  const unsigned long long init[4] = {0ull, 0ull, 0x7FF0000000000000ull, 0ull};  // 0, 0, +inf, 0
   KG_CUDA(cudaMemcpyAsync(st.ptr, init, sizeof init, cudaMemcpyHostToDevice, s));
   if (nnz) {
     csr_stats_kernel<<<std::min<unsigned>(blocks_for(n_rows * 32, 256), 2048), 256, 0, s>>>(

@@ -39,11 +39,13 @@ struct Blocked {
 
 // The blocked layout of a CSR matrix (n_rows x n_cols, u32 column indices, each row's columns
 // strictly increasing) and, if `twin`, of its transpose with the same scale and value range, and
-// then each column's number of entries if `col_counts` (n_cols). Waits for the stream once. False,
-// with no layout, when a row's columns do not strictly increase.
-[[nodiscard]] bool build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val, uint64_t n_rows,
-                   uint64_t n_cols, uint64_t nnz, Blocked& out, Blocked* twin,
-                   unsigned long long* col_counts, cudaStream_t s);
+// then each column's number of entries if `col_counts` (n_cols). Waits for the stream once.
+// False, with no layout, when a row's columns jump back so far that the builder would miss some,
+// or (without `col_counts`) when one is there twice; with col_counts the caller sees columns that
+// are there twice by a sum short of nnz.
+[[nodiscard]] bool build_blocked(const uint64_t* ptr, const uint32_t* col, const float* val,
+                                 uint64_t n_rows, uint64_t n_cols, uint64_t nnz, Blocked& out,
+                                 Blocked* twin, unsigned long long* col_counts, cudaStream_t s);
 
 // The dense operand D (K x 64) as the products read it: D^T, 64 rows of fp16 parts of
 // each value times 2^scale, interleaved by chunk: for chunk c, row j holds the 32 high
