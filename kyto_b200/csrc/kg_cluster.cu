@@ -6,7 +6,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 
 namespace kg {
 
@@ -331,12 +330,7 @@ void nearest_centres(const float* x, uint64_t n, uint32_t width, uint32_t d,
                      cudaStream_t s) {
   if (!n) return;
   if (d > kClusterDim) fail(KG_ERR_INVALID, "clusters: more than 64 components");
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    KG_CUDA(cudaFuncSetAttribute(nearest_centres_kernel,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(NcShared)));
-  });
+  allow_dynamic_smem(nearest_centres_kernel, sizeof(NcShared));
   nearest_centres_kernel<<<(unsigned)((n + kNcRows - 1) / kNcRows), 256, sizeof(NcShared), s>>>(
       x, n, width, d, centres, cn, K, labels);
   KG_LAUNCH_CHECK();

@@ -12,7 +12,6 @@
 
 #include <cfloat>
 #include <cmath>
-#include <mutex>
 #include <vector>
 
 #include "kg_internal.cuh"
@@ -362,11 +361,7 @@ extern "C" kg_status kg_connectivities(kg_ctx* ctx, const uint64_t* indptr,
     DeviceBuffer<uint32_t> tcol(m, s), tentry(m, s), tcol_sorted(m, s), tentry_sorted(m, s);
     const unsigned threads = k <= 192 ? 128 : 64;
     const size_t smem = threads * ((k | 1u) + 2) * sizeof(float);
-    static std::once_flag attr;
-    std::call_once(attr, [] {
-      KG_CUDA(cudaFuncSetAttribute(graph_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(128 * 195 * sizeof(float))));
-    });
+    allow_dynamic_smem(graph_rows_kernel, 128 * 195 * sizeof(float));
     graph_rows_kernel<<<blocks_for(n_rows, threads), threads, smem, s>>>(
         d_ptr, d_idx, d_dist, n_rows, k, n_neighbors, std::log2((double)n_neighbors), w.ptr,
         tcol.ptr, tentry.ptr, bad.ptr);

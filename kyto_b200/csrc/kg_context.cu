@@ -1,5 +1,6 @@
 // The context entry points of the C ABI: open/close, errors, cancel flag, progress.
 #include "kg_internal.cuh"
+#include "kg_once.cuh"
 
 namespace kg {
 std::atomic<uint64_t> g_launches{0};
@@ -33,6 +34,15 @@ uint64_t pool_unused() {
   KG_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
   KG_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
   return reserved > used ? reserved - used : 0;
+}
+
+void allow_dynamic_smem(const void* kernel, size_t bytes) {
+  static OncePerDevice once;
+  int device = 0;
+  KG_CUDA(cudaGetDevice(&device));
+  once(kernel, device, [&] {
+    KG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  });
 }
 
 thread_local bool g_stage_pageable = false;

@@ -1,7 +1,6 @@
 // The PCA's dense FP64 steps on narrow blocks (kg_dense.cuh). Every sum runs in a fixed
 // order: the same bits on every run, whatever the thread layout.
 #include <cmath>
-#include <mutex>
 
 #include "kg_dense.cuh"
 #include "kg_internal.cuh"
@@ -437,11 +436,7 @@ void cholesky_step(const double* gram, uint32_t w, double shift, double* r, int*
 
 void small_svd(const double* r, uint32_t w, const double* block, uint64_t n, const int* status,
                double* u_r, double* out, cudaStream_t s) {
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    KG_CUDA(cudaFuncSetAttribute(small_svd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(SvdShared)));
-  });
+  allow_dynamic_smem(small_svd_kernel, sizeof(SvdShared));
   small_svd_kernel<<<2, kJacobiThreads, sizeof(SvdShared), s>>>(r, w, block, n, status, u_r, out);
   KG_LAUNCH_CHECK();
 }

@@ -6,7 +6,6 @@
 
 #include <cfloat>
 #include <cmath>
-#include <mutex>
 
 #include "kg_dense.cuh"
 #include "kg_internal.cuh"
@@ -630,10 +629,8 @@ bool leading_eigenpairs(cublasHandle_t cublas, const double* a, uint32_t m, uint
   // A cluster of 16 CTAs is past the portable size: asked for, and used only where it fits.
   KG_CUDA(cudaFuncSetAttribute(tridiagonalise_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed,
                                1));
-  KG_CUDA(cudaFuncSetAttribute(tridiagonalise_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(kTriKept * kMaxM * sizeof(double))));
-  KG_CUDA(cudaFuncSetAttribute(orthonormalise_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(kMaxTake * kMaxM * sizeof(double))));
+  allow_dynamic_smem(tridiagonalise_kernel, kTriKept * kMaxM * sizeof(double));
+  allow_dynamic_smem(orthonormalise_kernel, kMaxTake * kMaxM * sizeof(double));
   cudaLaunchAttribute at;
   cudaLaunchConfig_t cfg = tri_config(&at, s);
   int fit = 0;

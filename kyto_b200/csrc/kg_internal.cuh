@@ -98,6 +98,14 @@ cudaMemPool_t device_pool(int device);
 // Bytes the library's pool on the current device holds and no buffer uses.
 uint64_t pool_unused();
 
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device (needed past 48 KB; the
+// attribute is a device's, so it is set once on each).
+void allow_dynamic_smem(const void* kernel, size_t bytes);
+template <class... A>
+void allow_dynamic_smem(void (*kernel)(A...), size_t bytes) {
+  allow_dynamic_smem(reinterpret_cast<const void*>(kernel), bytes);
+}
+
 // Allocation failures injected for tests (kg_diag_fail_allocations): after `n` more
 // allocations every allocation fails as out of memory, until the count is reset.
 extern std::atomic<uint64_t> g_allocs_left;

@@ -1101,12 +1101,7 @@ void launch_filter(unsigned grid, cudaStream_t s, const CUtensorMap& mq, const C
                    const FilterScan& scan, uint32_t k, const float* slack2, uint32_t idesc,
                    uint32_t cap, float* cand_key, uint32_t* cand_row, uint32_t* cand_count,
                    float* threshold, int* err) {
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    KG_CUDA(cudaFuncSetAttribute(knn_filter_tc_kernel<KR, SUBS, AM>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)tc_smem_bytes<KR, SUBS>()));
-  });
+  allow_dynamic_smem(knn_filter_tc_kernel<KR, SUBS, AM>, tc_smem_bytes<KR, SUBS>());
   knn_filter_tc_kernel<KR, SUBS, AM><<<grid, kTcThreads, tc_smem_bytes<KR, SUBS>(), s>>>(
       mq, mp, scan, k, slack2, idesc, cap, cand_key, cand_row, cand_count, threshold, err);
 }

@@ -658,11 +658,7 @@ kg_status kg_knn_learned(kg_ctx* ctx, const float* embedding, uint64_t n, uint32
       const size_t smem = (size_t)((n_tiles + 31) / 32 + pwords) * 4;
       if (smem > 200 * 1024)
         fail(KG_ERR_INVALID, "kg_knn_learned: too many rows for the tile bitmap");
-      static std::once_flag attr;
-      std::call_once(attr, [] {
-        KG_CUDA(cudaFuncSetAttribute(probe_tiles_kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      });
+      allow_dynamic_smem(probe_tiles_kernel, 200 * 1024);
       DeviceBuffer<uint64_t> len(n_blocks + 1, s);
       len.zero();
       probe_tiles_kernel<<<(unsigned)n_blocks, kProbeThreads, smem, s>>>(

@@ -443,15 +443,8 @@ bool moments_by_group(const uint64_t* indptr, const uint32_t* idx, const V* valu
       std::min(kGroupGenes, ((n_genes + sm_count - 1) / sm_count + 31) / 32 * 32);
   const uint32_t groups = (n_genes + gg - 1) / gg;
   if (groups > kGroupsMax) return false;
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    KG_CUDA(cudaFuncSetAttribute(seurat_rows_kernel<V>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(kGroupsMax * 33 * 4)));
-    KG_CUDA(cudaFuncSetAttribute(group_moments_kernel,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)((kRing * kTileRows + 2) * kGroupGenes * 4)));
-  });
+  allow_dynamic_smem(seurat_rows_kernel<V>, kGroupsMax * 33 * 4);
+  allow_dynamic_smem(group_moments_kernel, (kRing * kTileRows + 2) * kGroupGenes * 4);
   DeviceBuffer<float> t(nnz, s);
   DeviceBuffer<uint32_t> bounds((uint64_t)(groups - 1) * n_rows, s);
   seurat_rows_kernel<V><<<blocks_for(n_rows, 32), kSeuratThreads, (groups - 1) * 33 * 4, s>>>(

@@ -5,7 +5,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 #include <type_traits>
 
 #include "kg_sm100.cuh"
@@ -383,11 +382,7 @@ void mlp_tc_gemm(int M, int N, int K, const __nv_bfloat16* A, int lda, const __n
   const int tn = N < kTcNMax ? N : kTcNMax;
   if (K % kTcKBox || K > kTcKMax || tn % 32 || N % tn)
     fail(KG_ERR_INVALID, "MLP layer: shape outside the tensor-core tiles");
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    KG_CUDA(cudaFuncSetAttribute(mlp_tc_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kMlpTcSmemBytes));
-  });
+  allow_dynamic_smem(mlp_tc_kernel<EPI>, kMlpTcSmemBytes);
   const CUtensorMap ta = tma_map_2d_16bit(A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (uint64_t)K,
                                           (uint64_t)M, (uint64_t)lda * 2, kTcKBox, kTcRows);
   const CUtensorMap tb = tma_map_2d_16bit(W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (uint64_t)K,

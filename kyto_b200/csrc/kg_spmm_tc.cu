@@ -37,7 +37,6 @@
 #include <cmath>
 #include <cstddef>
 #include <cstring>
-#include <mutex>
 
 #include "kg_internal.cuh"
 #include "kg_sm100.cuh"
@@ -960,11 +959,7 @@ bool split_groups(uint64_t items, int sm_count) {
 void spmm_tc(const SpmmArgs& a, cudaStream_t s) {
   const Blocked& b = *a.s;
   if (b.K == 0 || b.rows == 0) return;
-  static std::once_flag attr;
-  std::call_once(attr, [] {
-    KG_CUDA(cudaFuncSetAttribute(spmm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSpSmemBytes));
-  });
+  allow_dynamic_smem(spmm_tc_kernel, kSpSmemBytes);
   if (a.ld_t != dense_ld(b.K)) fail(KG_ERR_INVALID, "spmm: D^T row length must be dense_ld(K)");
   if (a.out.mode == kOutRows && a.out.t && a.out.ld_t != dense_ld(b.rows))
     fail(KG_ERR_INVALID, "spmm: the output D^T row length must be dense_ld(rows)");
