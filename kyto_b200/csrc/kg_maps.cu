@@ -428,11 +428,24 @@ void gene_moments(const uint64_t* colptr, const float* t, uint32_t n_genes, doub
   KG_LAUNCH_CHECK();
 }
 
+// Whether `groups` groups of `group_genes` genes suit a block. A group's CTA passes every row of the
+// block, stored values or none, so its time goes by the rows (16 ns a row for groups of 32 genes, 21
+// for 160; as often as the groups go over the SMs); the sort's goes by the values, after some 30
+// us more of launches. Measured, group / sort: 60,000 rows of 285 values of 2,000 genes 1.21 /
+// 1.20 ms, of 95 values 1.02 / 0.64; 16,000 rows of 427 of 20,000 genes 0.44 / 0.52, of 285 0.43 /
+// 0.35; 250,000 rows of 95 of 20,000 genes 5.3 / 1.9; 4,000 rows of 190 of 2,000 genes 0.14 / 0.18;
+// 60,000 rows of 380 of 32,000 genes (two rounds of groups) 2.7 / 1.3. The rule also keeps the groups'
+// bounds, 4 bytes a row and group, below the sort's own scratch.
+bool groups_suit(uint64_t n_rows, uint64_t nnz, uint32_t group_genes, uint32_t groups, int sm_count) {
+  const uint64_t passes = n_rows * ((groups + sm_count - 1) / sm_count);
+  return passes <= 4096 || nnz / passes >= 220 + group_genes * 5 / 4;
+}
+
 // The moments of a block whose rows hold their genes in strictly increasing order, without a
 // sort; false (and nothing queued) for a shape outside the kernels' (more groups of genes than
-// their bounds' tile holds). The flags are read by the caller once its work is queued: a
-// block with an index out of range or an unsorted row leaves the moments meaningless (every
-// access stays inside the arrays).
+// their bounds' tile holds) or that the sort suits better. The flags are read by the caller once
+// its work is queued: a block with an index out of range or an unsorted row leaves the moments
+// meaningless (every access stays inside the arrays).
 template <class V>
 bool moments_by_group(const uint64_t* indptr, const uint32_t* idx, const V* values,
                       uint64_t n_rows, uint64_t nnz, uint32_t n_genes, double target_sum,
@@ -442,7 +455,7 @@ bool moments_by_group(const uint64_t* indptr, const uint32_t* idx, const V* valu
   const uint32_t gg =
       std::min(kGroupGenes, ((n_genes + sm_count - 1) / sm_count + 31) / 32 * 32);
   const uint32_t groups = (n_genes + gg - 1) / gg;
-  if (groups > kGroupsMax) return false;
+  if (groups > kGroupsMax || !groups_suit(n_rows, nnz, gg, groups, sm_count)) return false;
   allow_dynamic_smem(seurat_rows_kernel<V>, kGroupsMax * 33 * 4);
   allow_dynamic_smem(group_moments_kernel, (kRing * kTileRows + 2) * kGroupGenes * 4);
   DeviceBuffer<float> t(nnz, s);
