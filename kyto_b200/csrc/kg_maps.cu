@@ -138,7 +138,7 @@ seurat_rows_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
   const uint64_t rb = blockIdx.x * 32ull;
   for (uint32_t rr = warp; rr < 32 && rb + rr < n_rows; rr += kSeuratThreads / 32) {
     const uint64_t r = rb + rr;
-    const uint64_t s = indptr[r], e = indptr[r + 1];
+    const uint64_t s = indptr[r], e = max(indptr[r + 1], s);  // (a row that ends before it starts)
     RowMap map{tables[warp], 1.0f, normalize != 0, do_log1p != 0};
     if (normalize) map.divisor = warp_row_divisor(values, s, e, target32);
     __syncwarp();
@@ -152,7 +152,7 @@ seurat_rows_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
     const V* row_values = values + s;
     float* row_t = t + s;
     const uint32_t len = (uint32_t)(e - s), at = (uint32_t)s;
-    bool unsorted = false, wide = false;
+    bool unsorted = indptr[r + 1] < s, wide = false;
     uint32_t worst = 0, carry = 0;  // carry: the gene before the chunk's first
     for (uint32_t j0 = 0; j0 < len; j0 += 128) {
       uint32_t gene[4];
