@@ -136,6 +136,8 @@ seurat_rows_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
   extern __shared__ uint32_t crossing[];  // [groups - 1][33]
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint64_t rb = blockIdx.x * 32ull;
+  // The block will be sorted: nothing here is used any more.
+  if (__syncthreads_or(threadIdx.x == 0 && *(volatile unsigned int*)(flags + kFlagUnsorted))) return;
   for (uint32_t rr = warp; rr < 32 && rb + rr < n_rows; rr += kSeuratThreads / 32) {
     const uint64_t r = rb + rr;
     const uint64_t s = indptr[r], e = max(indptr[r + 1], s);  // (a row that ends before it starts)
@@ -225,6 +227,7 @@ group_moments_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
                      const unsigned int* flags, double* sums, double* squares,
                      uint64_t* positives) {
   extern __shared__ float tiles[];  // [kRing][kTileRows][group_genes], then two counts a gene
+  if (flags[kFlagUnsorted]) return;
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t k = blockIdx.x, g0 = k * group_genes;
   const uint32_t genes = min(group_genes, n_genes - g0);
@@ -599,7 +602,7 @@ kg_status kg_hvg_moments(kg_ctx* ctx, const uint64_t* indptr, const uint32_t* in
     DeviceBuffer<double> dsum(n_genes, s), dsq(n_genes, s);
     DeviceBuffer<uint64_t> dpos(n_genes, s);
     // Rows of strictly increasing genes (kyto's) need no sort; a block with any other row,
-    // found on the way, is sorted.
+    // found on the way, is sorted: what is left of the rows' pass then ends at once.
     bool sorted = nnz > 0 && n_genes > 0 && nnz <= (uint64_t)std::numeric_limits<int>::max();
     if (sorted) {
       DeviceBuffer<unsigned int> flags(kFlags, s);
@@ -616,8 +619,8 @@ kg_status kg_hvg_moments(kg_ctx* ctx, const uint64_t* indptr, const uint32_t* in
         unsigned int h[kFlags] = {};
         KG_CUDA(cudaMemcpyAsync(h, flags.ptr, sizeof h, cudaMemcpyDeviceToHost, s));
         wait_stream(ctx, s);
-        check_worst_index(h[kFlagWorst], n_genes);
         sorted = h[kFlagUnsorted] == 0;
+        if (sorted) check_worst_index(h[kFlagWorst], n_genes);  // (else not every row was read)
       }
     }
     if (!sorted) {

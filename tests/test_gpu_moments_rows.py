@@ -1,6 +1,7 @@
 """Gene moments of blocks whose offsets step back: such a row is empty, and the block goes to the sort,
 which takes each stored value once. Bit for bit the sorting form's (kg_hvg_moments_noalloc). No
-normalization, which would depend on the row a value is in."""
+normalization, which would depend on the row a value is in. And blocks of many rows with one out of
+gene order, wherever it stands, with and without a gene out of range after it."""
 
 import ctypes
 import math
@@ -42,3 +43,22 @@ def test_offsets_that_step_back(n_genes, rows, at, back):
     want = _moments("kg_hvg_moments_noalloc", indptr, idx, values, n_genes)
     for a, b in zip(got, want):
         assert np.array_equal(a.view(np.uint64), b.view(np.uint64))
+
+
+@pytest.mark.parametrize("where", [0, 1500, 2999])
+@pytest.mark.parametrize("n_genes", [300, 9000])
+def test_one_row_out_of_order(where, n_genes):
+    rows, per_row = 3000, 300
+    rng = np.random.default_rng(where + n_genes)
+    idx = np.sort(np.argsort(rng.random((rows, n_genes)), 1)[:, :per_row], 1).astype(np.uint32)
+    values = rng.integers(1, 90, idx.size).astype(np.uint32)
+    idx[where, 3:5] = idx[where, 4:2:-1]
+    indptr = np.arange(rows + 1, dtype=np.uint64) * np.uint64(per_row)
+    idx = idx.reshape(-1)
+    got = _moments("kg_hvg_moments", indptr, idx, values, n_genes)
+    want = _moments("kg_hvg_moments_noalloc", indptr, idx, values, n_genes)
+    for a, b in zip(got, want):
+        assert np.array_equal(a.view(np.uint64), b.view(np.uint64))
+    idx[-1], idx[5] = n_genes + 7, n_genes + 2  # the largest is named, wherever it stands
+    with pytest.raises(K.KytoError, match=f"gene index {n_genes + 7} but has {n_genes} genes"):
+        _moments("kg_hvg_moments", indptr, idx, values, n_genes)
