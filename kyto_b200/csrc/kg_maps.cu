@@ -46,28 +46,57 @@ void check_indices(const uint32_t* d_idx, uint64_t nnz, uint32_t n_genes, cudaSt
 // loads in flight a lane. HBM-bound: 8 bytes a value (the second read of a row comes from
 // L2); 8,192 rows of 1,900 counts: 39 us, 3.2 TB/s (eight threads a row with a log1p a value
 // and a rounding pass before: 296 us).
+// Short rows leave a warp's lanes idle, and the instructions bound it. Where a block of kShortRows
+// or more holds kShortRow values a row or fewer, eight lanes take a row and map value by value (the
+// offsets tell, so no host waits for them): 1M rows of 30 counts 200 us, a warp a row 400; with
+// 8,000 rows of 30 both take 16. So they do where a block of kManyRows or more holds f32 values that
+// are no counts: a row's divisor is then eight chains of additions, which a warp a row computes
+// four times over (100,000 rows of 200: 105 us, a warp a row 139; with fewer rows the warps are
+// what is short).
 constexpr int kMapWarps = 8;
+constexpr unsigned kMapBlocks = 8192;  // at most: warps go on to further rows
+constexpr uint64_t kShortRow = 64, kShortRows = 16384, kManyRows = 32768;
 template <class V>
 __global__ void __launch_bounds__(kMapWarps * 32)
 normalize_log1p_kernel(const uint64_t* indptr, const V* __restrict__ values, uint64_t n_rows,
                        float target32, int normalize, int do_log1p, float* __restrict__ out) {
   __shared__ float tables[kMapWarps][kMapTable];
-  const uint64_t row = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const unsigned lane = threadIdx.x & 31u;
-  if (row >= n_rows) return;  // whole warps leave together
-  const uint64_t s = indptr[row], e = indptr[row + 1];
-  RowMap map{tables[threadIdx.x >> 5], 1.0f, normalize != 0, do_log1p != 0};
-  if (normalize) map.divisor = warp_row_divisor(values, s, e, target32);
-  map.fill();
-  uint64_t i = s + lane;
-  for (; i + 96 < e; i += 128) {
-    const V a = values[i], b = values[i + 32], c = values[i + 64], d = values[i + 96];
-    out[i] = map.at(a);
-    out[i + 32] = map.at(b);
-    out[i + 64] = map.at(c);
-    out[i + 96] = map.at(d);
+  const uint64_t first = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t warps = gridDim.x * (uint64_t)kMapWarps;
+  bool eight = false;
+  if (n_rows >= kShortRows) {
+    const uint64_t s0 = indptr[0], end = indptr[n_rows];
+    eight = end - s0 <= kShortRow * n_rows;
+    if (!eight && normalize && n_rows >= kManyRows) eight = !row_of_counts(values, s0, end);
   }
-  for (; i < e; i += 32) out[i] = map.at(values[i]);
+  if (eight) {
+    for (uint64_t row4 = 4 * first; row4 < n_rows; row4 += 4 * warps) {  // whole warps
+      const uint64_t row = row4 + lane / 8;
+      const uint64_t s = row < n_rows ? indptr[row] : 0, e = row < n_rows ? indptr[row + 1] : 0;
+      // (A u32 count that is not an f32 enters its row's sum rounded: whole_value.)
+      const float divisor = normalize ? row_divisor(values, s, e, target32, true) : 1.0f;
+      for (uint64_t i = s + (lane & 7u); i < e; i += 8)
+        out[i] = mapped_f32(to_f32(values[i]), normalize != 0, divisor, do_log1p != 0);
+    }
+    return;
+  }
+  for (uint64_t row = first; row < n_rows; row += warps) {
+    const uint64_t s = indptr[row], e = indptr[row + 1];
+    RowMap map{tables[threadIdx.x >> 5], 1.0f, normalize != 0, do_log1p != 0};
+    const bool counts = row_of_counts(values, s, e);
+    if (normalize) map.divisor = warp_row_divisor(values, s, e, target32, counts);
+    map.fill(e - s, counts);
+    uint64_t i = s + lane;
+    for (; i + 96 < e; i += 128) {
+      const V a = values[i], b = values[i + 32], c = values[i + 64], d = values[i + 96];
+      out[i] = map.at(a);
+      out[i + 32] = map.at(b);
+      out[i + 64] = map.at(c);
+      out[i + 96] = map.at(d);
+    }
+    for (; i < e; i += 32) out[i] = map.at(values[i]);
+  }
 }
 
 // Device f32 map outputs of a (device) CSR block.
@@ -76,7 +105,7 @@ void map_block(const uint64_t* d_indptr, const void* d_values, kg_dtype dtype,
                cudaStream_t stream) {
   if (!n_rows) return;
   const int normalize = std::isnan(target_sum) ? 0 : 1;
-  const unsigned blocks = blocks_for(n_rows, kMapWarps);
+  const unsigned blocks = std::min(blocks_for(n_rows, kMapWarps), kMapBlocks);
   if (dtype == KG_U32)
     normalize_log1p_kernel<uint32_t><<<blocks, kMapWarps * 32, 0, stream>>>(
         d_indptr, (const uint32_t*)d_values, n_rows, (float)target_sum, normalize, do_log1p,
@@ -142,11 +171,15 @@ seurat_rows_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
     const uint64_t r = rb + rr;
     const uint64_t s = indptr[r], e = max(indptr[r + 1], s);  // (a row that ends before it starts)
     RowMap map{tables[warp], 1.0f, normalize != 0, do_log1p != 0};
-    if (normalize) map.divisor = warp_row_divisor(values, s, e, target32);
-    __syncwarp();
-    for (uint32_t c = lane; c < kMapTable; c += 32)
-      map.table[c] = seurat_value(mapped_f32((float)c, map.normalize, map.divisor, map.do_log1p));
-    __syncwarp();
+    const bool counts = row_of_counts(values, s, e);
+    if (normalize) map.divisor = warp_row_divisor(values, s, e, target32, counts);
+    const bool tabled = RowMap::tabled(e - s, counts);
+    if (tabled) {
+      __syncwarp();
+      for (uint32_t c = lane; c < kMapTable; c += 32)
+        map.table[c] = seurat_value(mapped_f32((float)c, map.normalize, map.divisor, map.do_log1p));
+      __syncwarp();
+    }
     // gene / group_genes: exact for genes below 2^24 (magic = ceil(2^32 / group_genes), a
     // divisor of at most 2^8); a gene out of range may land in any group.
     auto group_of = [&](uint32_t gene) { return min(__umulhi(gene, magic), groups - 1); };
@@ -178,7 +211,7 @@ seurat_rows_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
         const uint32_t to = group_of(gene[m]);
         for (uint32_t k = j > 0 ? group_of(before) : 0; k < to; ++k) crossing[k * 33 + rr] = at + j;
         uint32_t c;
-        const float x = map_tabled(v[m], c)
+        const float x = tabled && map_tabled(v[m], c)
                             ? map.table[c]
                             : seurat_value(mapped_f32(to_f32(v[m]), map.normalize, map.divisor,
                                                       map.do_log1p));

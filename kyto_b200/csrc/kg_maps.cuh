@@ -84,12 +84,23 @@ __device__ __forceinline__ bool whole_value(float v, unsigned long long& out) {
   return v >= 0.0f && v <= 16777216.0f && (float)(uint32_t)v == v;
 }
 
+// Whether the row [s, e) looks like counts, by its first values: if not, the integer sum and the
+// table would be for nothing. (For the whole warp.)
+__device__ __forceinline__ bool row_of_counts(const uint32_t*, uint64_t, uint64_t) { return true; }
+__device__ __forceinline__ bool row_of_counts(const float* values, uint64_t s, uint64_t e) {
+  const uint64_t i = s + (threadIdx.x & 31u);
+  unsigned long long w;
+  return __all_sync(0xFFFFFFFFu, i >= e || whole_value(values[i], w));
+}
+
 // The normalize divisor of the row [s, e), by a whole warp (every lane gets it). Whole
-// numbers whose sum stays below 2^53 add up exactly in any order, so the lanes sum integers;
-// any other row takes kyto's order (row_divisor: eight chains of dependent f64 additions).
+// numbers whose sum stays below 2^53 add up exactly in any order, so the lanes sum integers (a
+// row of `counts`: row_of_counts); any other row takes kyto's order (row_divisor: eight chains of
+// dependent f64 additions).
 template <class V>
 __device__ __forceinline__ float warp_row_divisor(const V* values, uint64_t s, uint64_t e,
-                                                  float target32) {
+                                                  float target32, bool counts) {
+  if (!counts) return row_divisor(values, s, e, target32, true);
   const unsigned lane = threadIdx.x & 31u;
   unsigned long long sum = 0;
   bool whole = true;
@@ -111,13 +122,21 @@ __device__ __forceinline__ float warp_row_divisor(const V* values, uint64_t s, u
   return divisor == 0.0f ? 1.0f : divisor;
 }
 
-// A row's maps by a warp: fill() makes the table (kMapTable floats of the warp's own), at()
-// maps a value.
+// A row's maps by a warp: fill() makes the table (kMapTable floats of the warp's own) for a row of
+// counts (row_of_counts) of more values than the table has, at() maps a value. (A lane makes two of
+// the table's entries: a shorter row's lanes have two values at most.)
 struct RowMap {
   float* table;
   float divisor;
   bool normalize, do_log1p;
-  __device__ __forceinline__ void fill() const {
+  __device__ __forceinline__ static bool tabled(uint64_t n, bool counts) {
+    return counts && n > kMapTable;
+  }
+  __device__ __forceinline__ void fill(uint64_t n, bool counts) {
+    if (!tabled(n, counts)) {
+      table = nullptr;
+      return;
+    }
     __syncwarp();
     for (uint32_t c = threadIdx.x & 31u; c < kMapTable; c += 32)
       table[c] = mapped_f32((float)c, normalize, divisor, do_log1p);
@@ -126,7 +145,7 @@ struct RowMap {
   template <class V>
   __device__ __forceinline__ float at(V v) const {
     uint32_t c;
-    return map_tabled(v, c) ? table[c] : mapped_f32(to_f32(v), normalize, divisor, do_log1p);
+    return table && map_tabled(v, c) ? table[c] : mapped_f32(to_f32(v), normalize, divisor, do_log1p);
   }
 };
 

@@ -79,7 +79,7 @@ count_kept_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
   for (int o = 16; o; o >>= 1) count += __shfl_down_sync(0xFFFFFFFFu, count, o);
   if (lane == 0) kept[row] = count;
   if (divisor) {
-    const float d = warp_row_divisor(values, s, e, target32);
+    const float d = warp_row_divisor(values, s, e, target32, row_of_counts(values, s, e));
     if (lane == 0) divisor[row] = d;
   }
 }
@@ -98,10 +98,10 @@ write_kept_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
   if (row >= n_rows) return;
   const uint64_t s = indptr[row], e = indptr[row + 1];
   uint64_t base = out_ptr[row];
-  const RowMap map{tables[threadIdx.x >> 5], divisor ? divisor[row] : 1.0f, divisor != nullptr,
-                   do_log1p != 0};
+  RowMap map{tables[threadIdx.x >> 5], divisor ? divisor[row] : 1.0f, divisor != nullptr,
+             do_log1p != 0};
   const bool maps = divisor != nullptr || do_log1p;
-  if (maps) map.fill();
+  if (maps) map.fill(out_ptr[row + 1] - base, row_of_counts(values, s, e));
   for (uint64_t i0 = s; i0 < e; i0 += 128) {
     uint32_t p[4];
 #pragma unroll
@@ -140,8 +140,9 @@ pack_rows_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
   const uint64_t s = indptr[row], e = indptr[row + 1];
   RowMap map{tables[threadIdx.x >> 5], 1.0f, normalize != 0, do_log1p != 0};
   const bool maps = normalize || do_log1p;
-  if (normalize) map.divisor = warp_row_divisor(values, s, e, target32);
-  if (maps) map.fill();
+  const bool counts = maps && row_of_counts(values, s, e);
+  if (normalize) map.divisor = warp_row_divisor(values, s, e, target32, counts);
+  if (maps) map.fill(e - s, counts);
   auto put = [&](uint64_t i, uint32_t gene, V v) {
     gene_ok(gene, n_genes, worst);
     col[i] = gene;
