@@ -154,13 +154,14 @@ __device__ __forceinline__ float seurat_value(float mapped) { return (float)expm
 // + row] = the row's first entry of a gene in group k >= 1 (group_genes genes each) or later;
 // flags: [kFlagWorst] the largest gene index at or past n_genes (0: none), [kFlagUnsorted]
 // set by a row whose genes do not increase strictly, [kFlagWide] set by a seurat value that
-// is not 0 nor of a magnitude in [2^-28, 2^60). HBM-bound: 8 bytes a value in, 4 out.
+// is not 0 nor of a magnitude in [least, 2^60). HBM-bound: 8 bytes a value in, 4 out.
 template <class V>
 __global__ void __launch_bounds__(kSeuratThreads, 5)
 seurat_rows_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
                    const V* __restrict__ values, uint64_t n_rows, uint32_t n_genes,
                    uint32_t magic, uint32_t groups, int normalize,
-                   float target32, int do_log1p, float* __restrict__ t, uint32_t* bounds, unsigned int* flags) {
+                   float target32, int do_log1p, float least, float* __restrict__ t,
+                   uint32_t* bounds, unsigned int* flags) {
   __shared__ float tables[kSeuratThreads / 32][kMapTable];
   extern __shared__ uint32_t crossing[];  // [groups - 1][33]
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -215,7 +216,7 @@ seurat_rows_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
                             ? map.table[c]
                             : seurat_value(mapped_f32(to_f32(v[m]), map.normalize, map.divisor,
                                                       map.do_log1p));
-        wide |= x != 0.0f && !(fabsf(x) >= 0x1p-28f && fabsf(x) < 0x1p60f);
+        wide |= x != 0.0f && !(fabsf(x) >= least && fabsf(x) < 0x1p60f);
         row_t[j] = x;
       }
     }
@@ -238,9 +239,10 @@ seurat_rows_kernel(const uint64_t* indptr, const uint32_t* __restrict__ idx,
 // gene a lane, then add a tile's rows in order.
 // The chains' instructions bound it: per row and lane two dependent f64 additions and the
 // conversions before them, one through the conversion unit (16 lanes a clock an SM), the
-// square's by shifting its bits. That shift reads an f32 zero as 2^-127, which any real
-// square added to it swallows while every nonzero value is at least 2^-28 (a gene of no
-// nonzero value is put right at the end); a block with other values converts both.
+// square's by shifting its bits. That shift reads an f32 zero as 2^-127. A gene's zeros before its
+// first real square add up to less than n_rows of those, which that square swallows while it is
+// large enough (least_value; a gene of no nonzero value is put right at the end); a block with
+// other values converts both.
 constexpr int kTileRows = 32;
 constexpr int kRing = 7;               // two named barriers a slot, 15 in all
 constexpr int kTeamWarps = 2;
@@ -464,6 +466,14 @@ void gene_moments(const uint64_t* colptr, const float* t, uint32_t n_genes, doub
   KG_LAUNCH_CHECK();
 }
 
+// The least magnitude, a power of two 2^b, of the nonzero values whose squares may be widened by their
+// bits: n_rows 2^-127 has to be below half an ulp of the smallest square, 2^(2 b - 53).
+float least_value(uint64_t n_rows) {
+  int b = -28;
+  while (std::ldexp((double)n_rows, -(2 * b + 74)) >= 1.0) ++b;
+  return (float)std::ldexp(1.0, b);
+}
+
 // Whether `groups` groups of `group_genes` genes suit a block. A group's CTA passes every row of the
 // block, stored values or none, so its time goes by the rows (16 ns a row for groups of 32 genes, 21
 // for 160; as often as the groups go over the SMs); the sort's goes by the values, after some 30
@@ -498,7 +508,8 @@ bool moments_by_group(const uint64_t* indptr, const uint32_t* idx, const V* valu
   DeviceBuffer<uint32_t> bounds((uint64_t)(groups - 1) * n_rows, s);
   seurat_rows_kernel<V><<<blocks_for(n_rows, 32), kSeuratThreads, (groups - 1) * 33 * 4, s>>>(
       indptr, idx, values, n_rows, n_genes, (uint32_t)(((1ull << 32) + gg - 1) / gg), groups,
-      std::isnan(target_sum) ? 0 : 1, (float)target_sum, do_log1p, t.ptr, bounds.ptr, flags);
+      std::isnan(target_sum) ? 0 : 1, (float)target_sum, do_log1p, least_value(n_rows), t.ptr,
+      bounds.ptr, flags);
   KG_LAUNCH_CHECK();
   group_moments_kernel<<<groups, kLoadWarps * 32 + gg, (kRing * kTileRows + 2) * gg * 4, s>>>(
       indptr, idx, t.ptr, n_rows, n_genes, gg, groups, bounds.ptr, flags, sums, squares,
