@@ -485,10 +485,11 @@ KG_API kg_status kg_diag_kernel_launches(uint64_t* count);
 KG_API kg_status kg_diag_pool_usage(int device, uint64_t* reserved, uint64_t* used,
                                     uint64_t* used_high, int32_t reset_high);
 
-/* Test hook: after `after` more device allocations by this library, every allocation fails
- * as out of memory (the call returns KG_ERR_OOM and frees what it allocated); UINT64_MAX
- * turns the injection off. No kyto counterpart (tests the KG_ERR_OOM path without
- * exhausting a GPU). */
+/* Test hook: after `after` more attempts by this library to allocate device memory, every
+ * one fails as out of memory (the call returns KG_ERR_OOM and frees what it allocated);
+ * UINT64_MAX turns the injection off. With bit 63 set, one attempt fails, after the lower
+ * bits' number of others (a call may then succeed another way). No kyto counterpart (tests
+ * the KG_ERR_OOM path without exhausting a GPU). */
 KG_API kg_status kg_diag_fail_allocations(uint64_t after);
 
 /* One of the PCA's tensor-core products on a caller's CSR matrix (n_rows x n_cols, f32

@@ -36,6 +36,51 @@ uint64_t pool_unused() {
   return reserved > used ? reserved - used : 0;
 }
 
+namespace {
+
+// Whether this attempt is to fail (kg_diag_fail_allocations).
+bool injected_failure() {
+  uint64_t left = g_allocs_left.load(std::memory_order_relaxed);
+  while (left != UINT64_MAX) {
+    const uint64_t more = left & ~kOneFailure;
+    if (!more && !(left & kOneFailure)) return true;
+    const uint64_t next = more ? left - 1 : UINT64_MAX;
+    if (g_allocs_left.compare_exchange_weak(left, next)) return !more;
+  }
+  return false;
+}
+
+cudaError_t pool_attempt(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t s) {
+  if (injected_failure()) return cudaErrorMemoryAllocation;
+  return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
+}  // namespace
+
+void* pool_alloc(size_t bytes, cudaStream_t s) {
+  int device = 0;
+  KG_CUDA(cudaGetDevice(&device));
+  cudaMemPool_t pool = device_pool(device);
+  const auto t0 = std::chrono::steady_clock::now();
+  void* p = nullptr;
+  const size_t rounded = pool_bytes(bytes);
+  cudaError_t e = pool_attempt(&p, rounded, pool, s);
+  if (e == cudaErrorMemoryAllocation && rounded != bytes) {
+    (void)cudaGetLastError();
+    e = pool_attempt(&p, bytes, pool, s);
+  }
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();  // reported here; no later launch check is to find it
+    fail_cuda(e, "cudaMallocFromPoolAsync", __FILE__, __LINE__);
+  }
+  if (trace_on()) {
+    const double ms =
+        std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    if (ms > 2.0) trace_slow_alloc(bytes, ms);
+  }
+  return p;
+}
+
 void allow_dynamic_smem(const void* kernel, size_t bytes) {
   static OncePerDevice once;
   int device = 0;

@@ -106,20 +106,25 @@ void allow_dynamic_smem(void (*kernel)(A...), size_t bytes) {
   allow_dynamic_smem(reinterpret_cast<const void*>(kernel), bytes);
 }
 
-// Allocation failures injected for tests (kg_diag_fail_allocations): after `n` more
-// allocations every allocation fails as out of memory, until the count is reset.
+// Allocation failures injected for tests (kg_diag_fail_allocations): after `n` more attempts
+// every one fails as out of memory, until the count is reset; with kOneFailure set in `n`, one does.
 extern std::atomic<uint64_t> g_allocs_left;
+constexpr uint64_t kOneFailure = 1ull << 63;
 
 // The bytes asked of the pool for `bytes`: from 1 MB on rounded up to an eighth of the
 // power of two below (at most 64 MB more). Calls on inputs of slightly different sizes then
 // ask for the same blocks in the same order and find them free; unrounded, a pool with
-// little to spare moves memory to fit them, which stalls the host for 10 to 240 ms.
+// little to spare moves memory to fit them, which stalls the host for 10 to 240 ms. (Where the
+// rounded size does not fit, pool_alloc asks for the bytes themselves.)
 inline size_t pool_bytes(size_t bytes) {
   if (bytes < (1u << 20)) return bytes;
   size_t unit = 1u << 17;
   while (unit < (64u << 20) && unit * 16 <= bytes) unit <<= 1;
   return (bytes + unit - 1) / unit * unit;
 }
+
+// `bytes` (> 0) of the library's pool on the current device, stream-ordered; throws KG_ERR_OOM.
+void* pool_alloc(size_t bytes, cudaStream_t s);
 
 // A device allocation, stream-ordered (cudaMallocFromPoolAsync on the library's pool /
 // cudaFreeAsync).
@@ -149,28 +154,9 @@ struct DeviceBuffer {
   void alloc(size_t n, cudaStream_t s) {
     reset();
     stream = s;
-    count = n;
     if (!n) return;
-    if (g_allocs_left.load(std::memory_order_relaxed) != UINT64_MAX) {
-      uint64_t left = g_allocs_left.load();
-      while (left != UINT64_MAX && left > 0 && !g_allocs_left.compare_exchange_weak(left, left - 1)) {
-      }
-      if (left == 0) {
-        count = 0;
-        fail_cuda(cudaErrorMemoryAllocation, "an injected allocation failure", __FILE__, __LINE__);
-      }
-    }
-    int device = 0;
-    KG_CUDA(cudaGetDevice(&device));
-    cudaMemPool_t pool = device_pool(device);
-    if (!trace_on()) {
-      KG_CUDA(cudaMallocFromPoolAsync((void**)&ptr, pool_bytes(n * sizeof(T)), pool, s));
-      return;
-    }
-    auto t0 = std::chrono::steady_clock::now();
-    KG_CUDA(cudaMallocFromPoolAsync((void**)&ptr, pool_bytes(n * sizeof(T)), pool, s));
-    double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    if (ms > 2.0) trace_slow_alloc(n * sizeof(T), ms);
+    ptr = static_cast<T*>(pool_alloc(n * sizeof(T), s));
+    count = n;
   }
   void reset() noexcept {
     if (ptr) cudaFreeAsync(ptr, stream);

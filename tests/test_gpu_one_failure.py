@@ -1,0 +1,42 @@
+"""One allocation attempt that fails, where there is another way: a size that was rounded up is asked
+for as it is. (Failures that stay are in test_gpu_errors.)"""
+
+import numpy as np
+import pytest
+
+import kyto_b200 as K
+
+pytestmark = pytest.mark.gpu
+
+ONE = 1 << 63
+
+
+@pytest.fixture(autouse=True)
+def _off():
+    yield
+    K.fail_allocations(None)
+
+
+@pytest.mark.parametrize("count", [262_144, 262_145, 300_001, 5_000_003])
+def test_a_rounded_size_is_asked_for_as_it_is(count):
+    """Host arrays: the offsets (small, never rounded), the values and the output (from 1 MB on)."""
+    values = np.arange(count, dtype=np.uint32) % 50
+    indptr = np.array([0, count // 3, count], dtype=np.uint64)
+    want = K.normalize_log1p(indptr, values)
+    unit = 1 << 17
+    while unit < 64 << 20 and unit * 16 <= 4 * count:
+        unit <<= 1
+    rounded = 4 * count % unit != 0
+    for attempt in (1, 2):
+        K.fail_allocations(ONE | attempt)
+        if rounded:
+            assert np.array_equal(K.normalize_log1p(indptr, values), want)
+        else:
+            with pytest.raises(K.KytoError) as err:
+                K.normalize_log1p(indptr, values)
+            assert err.value.status == K.KG_ERR_OOM
+    K.fail_allocations(ONE)  # the offsets
+    with pytest.raises(K.KytoError) as err:
+        K.normalize_log1p(indptr, values)
+    assert err.value.status == K.KG_ERR_OOM
+    assert np.array_equal(K.normalize_log1p(indptr, values), want)
