@@ -1426,11 +1426,11 @@ FilterChoice tune_filter_kind(kg_ctx* ctx, cudaStream_t s, const float* x, uint6
   return best;
 }
 
-// The exact search on device rows: every row's k nearest other rows by (kyto key, row)
-// into out.key / out.row (n x k). `plan` chooses the tensor-core filter's scan (NULL:
-// the rows in a spatial order, each query block scanning every tile from its own).
-void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t d, uint32_t k,
-              const PlanBuilder* plan, KnnResult& out, Trace& trace, const KnnBatch* batch) {
+// knn_core's search. Without a plan or batch, `lists` lets it take the bounded scan; *listed tells
+// whether it did.
+void knn_search(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t d, uint32_t k,
+                const PlanBuilder* plan, KnnResult& out, Trace& trace, const KnnBatch* batch,
+                bool lists, bool* listed) {
   cudaStream_t s = ctx->stream;
   DeviceBuffer<double> mean(d, s), largest(1, s);
   DeviceBuffer<float> lo_hi(6, s);
@@ -1531,12 +1531,14 @@ void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t 
       // when the lists would not fit).
       const char* ord = std::getenv("KYTO_GPU_KNN_ORDER");
       const std::string order = ord ? ord : "bounded";
-      bool listed = false;
-      if (order != "morton") {
-        listed = bounded_scan(x, n, width, d, mean.ptr, scale, std::sqrt(h_largest),
-                              filter_query_block(kind), order != "cluster", ctx->sm_count, sp, s, trace);
+      bool got = false;
+      if (lists && order != "morton") {
+        *listed = true;  // (also when it runs out of memory half-way)
+        got = bounded_scan(x, n, width, d, mean.ptr, scale, std::sqrt(h_largest),
+                           filter_query_block(kind), order != "cluster", ctx->sm_count, sp, s, trace);
+        *listed = got;
       }
-      if (!listed) spatial_order(x, n, width, d, mean.ptr, lo_hi.ptr, sp.qrows, s);
+      if (!got) spatial_order(x, n, width, d, mean.ptr, lo_hi.ptr, sp.qrows, s);
       trace.mark("scan order");
     }
     FilterScan scan;
@@ -1762,6 +1764,24 @@ void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t 
   out.rows_full = h_full;
   out.filter_ms = filter_ms;
   out.rank_ms = rank_ms;
+}
+
+// The exact search on device rows: every row's k nearest other rows by (kyto key, row)
+// into out.key / out.row (n x k). `plan` chooses the tensor-core filter's scan (NULL:
+// the rows in a spatial order, each query block scanning every tile from its own).
+// The bounded scan's lists are taken where twice their size is to be had, but the memory is other
+// sessions' too: a listed search that runs out of it is done again without them.
+void knn_core(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_t d, uint32_t k,
+              const PlanBuilder* plan, KnnResult& out, Trace& trace, const KnnBatch* batch) {
+  bool listed = false;
+  try {
+    knn_search(ctx, x, n, width, d, k, plan, out, trace, batch, true, &listed);
+    return;
+  } catch (const Error& e) {
+    if (e.status != KG_ERR_OOM || !listed) throw;
+  }
+  out = KnnResult();
+  knn_search(ctx, x, n, width, d, k, plan, out, trace, batch, false, &listed);
 }
 
 // n_neighbors and n_components checked as neighbors::search does (neighbors.rs:226-312);

@@ -40,3 +40,26 @@ def test_a_rounded_size_is_asked_for_as_it_is(count):
         K.normalize_log1p(indptr, values)
     assert err.value.status == K.KG_ERR_OOM
     assert np.array_equal(K.normalize_log1p(indptr, values), want)
+
+
+def test_a_search_out_of_memory_for_its_lists_goes_without():
+    """Each attempt of a search fails once: the answer is the graph or KG_ERR_OOM, and the graph
+    wherever the scan's lists had been begun (all but the few attempts before them and the output's
+    after)."""
+    x = np.random.default_rng(0).normal(size=(6000, 20)).astype(np.float32)
+    want = K.neighbors(x, 10)
+    out_of_memory = []
+    for attempt in range(200):  # more than a search makes
+        K.fail_allocations(ONE | attempt)
+        try:
+            got = K.neighbors(x, 10)
+        except K.KytoError as err:
+            assert err.status == K.KG_ERR_OOM
+            out_of_memory.append(attempt)
+        else:
+            assert np.array_equal(got.indices, want.indices)
+            assert np.array_equal(got.distances, want.distances)
+    assert max(out_of_memory) < 199
+    listed = [a for a in range(max(out_of_memory)) if a not in out_of_memory]
+    # The lists' own attempts come one after another, from the clustering to the filter's end.
+    assert len(listed) >= 40 and listed == list(range(listed[0], listed[-1] + 1))
