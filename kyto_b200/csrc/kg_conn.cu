@@ -399,8 +399,9 @@ extern "C" kg_status kg_connectivities(kg_ctx* ctx, const uint64_t* indptr,
     KG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp2, ptr.ptr, ptr.ptr, n_rows + 1, s));
     DeviceBuffer<unsigned char> scratch2(temp2, s);
     KG_CUDA(cub::DeviceScan::ExclusiveSum(scratch2.ptr, temp2, ptr.ptr, ptr.ptr, n_rows + 1, s));
-    const bool dev_out = is_device_pointer(out_indptr) && is_device_pointer(out_indices) &&
-                         is_device_pointer(out_weights);
+    const bool dev_out = is_writable_here(out_indptr, ctx->device) &&
+                         is_writable_here(out_indices, ctx->device) &&
+                         is_writable_here(out_weights, ctx->device);
     DeviceBuffer<uint64_t> hp_out;
     DeviceBuffer<uint32_t> hi_out;
     DeviceBuffer<float> hw_out;

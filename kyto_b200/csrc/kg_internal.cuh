@@ -182,6 +182,18 @@ inline bool is_device_pointer(const void* p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// Whether kernels on `device` may write T's at p: this device's memory (or managed), aligned. A
+// copy takes any other pointer too.
+template <class T>
+bool is_writable_here(const T* p, int device) {
+  cudaPointerAttributes a{};
+  if (reinterpret_cast<uintptr_t>(p) % alignof(T) || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeManaged || (a.type == cudaMemoryTypeDevice && a.device == device);
+}
+
 // Whether p is ordinary (pageable) host memory: neither the device's nor page-locked.
 inline bool is_pageable_host(const void* p) {
   if (!p) return false;
