@@ -54,8 +54,38 @@ struct TileStarts {
 
 constexpr unsigned kTileThreads = 256;
 
+// Past kOneByOne tiles a row's segments are short and a warp takes 32 tiles of a row, a lane a
+// tile's offsets, then the segments' entries as one run. (A warp a tile sums every tile's offsets
+// for each: 4,096 rows x 512 tiles of 2 entries 1.15 ms and 0.49 for the checks, in runs 75 us and 49; one
+// warp for the whole row, its tiles one after another, had taken 0.69 for both. Up to 32 tiles that
+// sum is one read a lane, and a warp a tile has the more warps: 39 and 36 us for 32 tiles of 37.)
+constexpr uint32_t kOneByOne = 32;
+
+// Segments of up to 32 tiles, a lane a tile: this lane's length and where it starts in the run.
+struct SegmentRun {
+  uint64_t end, total;  // this lane's segment's end in the run; the run's length
+  __device__ __forceinline__ explicit SegmentRun(uint64_t len) : end(len) {
+    const unsigned lane = threadIdx.x & 31u;
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+      const uint64_t v = __shfl_up_sync(0xFFFFFFFFu, end, o);
+      if (lane >= (unsigned)o) end += v;
+    }
+    total = __shfl_sync(0xFFFFFFFFu, end, 31);
+  }
+  // The lane whose segment holds entry x (< total) of the run: the first whose end is past it.
+  __device__ __forceinline__ unsigned find(uint64_t x) const {
+    unsigned at = 0;
+#pragma unroll
+    for (unsigned step = 16; step; step /= 2)
+      if (__shfl_sync(0xFFFFFFFFu, end, at + step - 1) <= x) at += step;
+    return at;
+  }
+};
+
 // Blocks [0, shard_blocks): a thread per value i of the shard (tile g = i / (C + 1), row r =
 // i % (C + 1)). The others: a warp per (tile, row).
+template <bool Runs>
 __global__ void __launch_bounds__(kTileThreads)
 tile_check_kernel(const uint32_t* __restrict__ shard, uint32_t n_gb, uint64_t row_len,
                   uint32_t rows, const __grid_constant__ TileStarts start,
@@ -78,6 +108,32 @@ tile_check_kernel(const uint32_t* __restrict__ shard, uint32_t n_gb, uint64_t ro
   const unsigned lane = threadIdx.x & 31u;
   const uint64_t warps = (gridDim.x - shard_blocks) * (kTileThreads / 32);
   uint64_t wq = ((blockIdx.x - shard_blocks) * (uint64_t)kTileThreads + threadIdx.x) >> 5;
+  if (Runs) {  // a warp per (32 tiles, row)
+    for (; wq < (uint64_t)((n_gb + 31) / 32) * rows; wq += warps) {
+      const uint32_t g = (uint32_t)(wq / rows) * 32 + lane, r = (uint32_t)(wq % rows);
+      uint64_t from = 0, len = 0;
+      if (g < n_gb) {
+        const uint64_t nnz = start[g + 1] - start[g];
+        const uint64_t a = min((uint64_t)shard[g * row_len + r], nnz);
+        const uint64_t e = min((uint64_t)shard[g * row_len + r + 1], nnz);
+        from = start[g] + a;
+        len = e > a ? e - a : 0;
+      }
+      const SegmentRun run(len);
+      for (uint64_t x0 = 0; x0 < run.total; x0 += 32) {
+        const uint64_t x = min(x0 + lane, run.total - 1);  // (the last again: the same verdict)
+        const unsigned at = run.find(x);
+        const uint64_t in = x - (__shfl_sync(0xFFFFFFFFu, run.end, at) - __shfl_sync(0xFFFFFFFFu, len, at));
+        const uint32_t* t = idx + __shfl_sync(0xFFFFFFFFu, from, at) + in;
+        const uint32_t tile = g - lane + at, v = *t;
+        if (v >= min(gene_block, n_genes - tile * gene_block))
+          atomicMin(problem, problem_key(tile, kRow, r, 0));
+        else if (in && v <= t[-1])
+          atomicMin(problem, problem_key(tile, kRow, r, 1));
+      }
+    }
+    return;
+  }
   for (; wq < (uint64_t)n_gb * rows; wq += warps) {
     const uint32_t g = (uint32_t)(wq / rows), r = (uint32_t)(wq % rows);
     const uint64_t nnz = start[g + 1] - start[g];
@@ -108,9 +164,10 @@ tile_check_kernel(const uint32_t* __restrict__ shard, uint32_t n_gb, uint64_t ro
   }
 }
 
-// A warp per (row, tile). Writes nothing when the checks found a problem (the caller's
+// A warp per (row, tile) or (row, 32 tiles). Writes nothing when the checks found a problem (the caller's
 // outputs stay as they were): every thread reads the verdict, final once the checks ran
 // before it on the stream.
+template <bool Runs>
 __global__ void __launch_bounds__(kTileThreads)
 tile_join_kernel(const uint32_t* __restrict__ shard, uint32_t n_gb, uint64_t row_len,
                  uint32_t rows, const __grid_constant__ TileStarts start,
@@ -124,6 +181,34 @@ tile_join_kernel(const uint32_t* __restrict__ shard, uint32_t n_gb, uint64_t row
   if (n_gb == 0) {  // a layer without genes: empty rows
     for (; wq <= rows; wq += warps)
       if (lane == 0) out_ptr[wq] = 0;
+    return;
+  }
+  if (Runs) {  // a warp per (32 tiles, row)
+    for (; wq < (uint64_t)((n_gb + 31) / 32) * rows; wq += warps) {
+      const uint32_t g0 = (uint32_t)(wq / rows) * 32, g = g0 + lane, r = (uint32_t)(wq % rows);
+      uint64_t dst = 0, from = 0, len = 0;
+      for (uint32_t h = lane; h < n_gb; h += 32) dst += shard[h * row_len + r + (h < g0 ? 1 : 0)];
+      for (int o = 16; o; o >>= 1) dst += __shfl_xor_sync(0xFFFFFFFFu, dst, o);
+      if (g < n_gb) {
+        const uint64_t a = shard[g * row_len + r];
+        len = shard[g * row_len + r + 1] - a;
+        from = start[g] + a;
+      }
+      const SegmentRun run(len);
+      if (lane == 0) {
+        if (g0 + 32 >= n_gb) out_ptr[r + 1] = dst + run.total;
+        if (r == 0 && g0 == 0) out_ptr[0] = 0;
+      }
+      for (uint64_t x0 = 0; x0 < run.total; x0 += 32) {
+        const uint64_t x = min(x0 + lane, run.total - 1);
+        const unsigned at = run.find(x);
+        const uint64_t in = x - (__shfl_sync(0xFFFFFFFFu, run.end, at) - __shfl_sync(0xFFFFFFFFu, len, at));
+        const uint64_t src = __shfl_sync(0xFFFFFFFFu, from, at) + in;
+        if (x0 + lane >= run.total) continue;
+        out_idx[dst + x] = (uint32_t)((g0 + at) * gene_block) + idx[src];
+        out_val[dst + x] = val[src];
+      }
+    }
     return;
   }
   for (; wq < (uint64_t)n_gb * rows; wq += warps) {
@@ -157,8 +242,10 @@ tile_join_kernel(const uint32_t* __restrict__ shard, uint32_t n_gb, uint64_t row
   }
 }
 
-// Blocks of a warp per (tile, row), the warps going on from the grid's end past 2^25 of them.
-unsigned row_blocks_for(uint64_t pairs) {
+// Blocks of a warp per (tile, row) or (32 tiles, row), the warps going on from the grid's end past
+// 2^25 of them.
+unsigned row_blocks_for(uint64_t tiles, uint64_t rows) {
+  const uint64_t pairs = (tiles > kOneByOne ? (tiles + 31) / 32 : std::max<uint64_t>(tiles, 1)) * rows;
   return (unsigned)std::min<uint64_t>((pairs + kTileThreads / 32 - 1) / (kTileThreads / 32), 1u << 22);
 }
 
@@ -226,17 +313,19 @@ void join_tiles(kg_ctx* ctx, cudaStream_t s, const kg_tile_block* tb, const Tile
   }
   DeviceBuffer<unsigned long long> problem(1, s);
   KG_CUDA(cudaMemsetAsync(problem.ptr, 0xFF, 8, s));
+  const bool runs = n_gb > kOneByOne;
+  const unsigned row_blocks = row_blocks_for(n_gb, rows);
   if (n_gb) {
     const uint64_t shard_blocks = blocks_for((uint64_t)n_gb * row_len, kTileThreads);
-    const uint64_t row_blocks = row_blocks_for((uint64_t)n_gb * rows);
-    tile_check_kernel<<<(unsigned)(shard_blocks + row_blocks), kTileThreads, 0, s>>>(
-        shard, n_gb, row_len, rows, start, idx, tb->gene_block_size, tb->n_genes, shard_blocks,
-        problem.ptr);
+    (runs ? tile_check_kernel<true> : tile_check_kernel<false>)
+        <<<(unsigned)(shard_blocks + row_blocks), kTileThreads, 0, s>>>(
+            shard, n_gb, row_len, rows, start, idx, tb->gene_block_size, tb->n_genes, shard_blocks,
+            problem.ptr);
     KG_LAUNCH_CHECK();
   }
   // The join is queued before the verdict is read (one wait a call); it writes only when the
   // checks passed.
-  tile_join_kernel<<<row_blocks_for(std::max<uint64_t>(n_gb, 1) * rows), kTileThreads, 0, s>>>(
+  (runs ? tile_join_kernel<true> : tile_join_kernel<false>)<<<row_blocks, kTileThreads, 0, s>>>(
       shard, n_gb, row_len, rows, start, idx, val, tb->gene_block_size, problem.ptr, d_indptr,
       d_indices, d_values);
   KG_LAUNCH_CHECK();
