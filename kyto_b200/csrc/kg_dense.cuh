@@ -39,8 +39,8 @@ void frobenius(const double* m, uint64_t n, double* out, cudaStream_t s);
 // The `take` largest eigenvalues of the symmetric m x m matrix `a` (column-major, both halves),
 // descending, into `values`, and their orthonormal vectors into `vectors` (m x take,
 // column-major) (kg_eigen.cu). False, with both undefined and `a` as it was, where it does not
-// apply (m past 544, take past 50, no room for a cluster of 16 CTAs) or where the pairs fail their check (residuals and orthonormality within 16 m 2^-52 of
-// the norm). Waits for the stream.
+// apply (m past 544, take past 50, no room for a cluster of 16 CTAs) or where the pairs fail their
+// check (residuals of the norm and orthonormality within (16 + m / 8) 2^-52). Waits for the stream.
 bool leading_eigenpairs(cublasHandle_t cublas, const double* a, uint32_t m, uint32_t take,
                         double* vectors, std::vector<double>& values, cudaStream_t s);
 
