@@ -69,10 +69,7 @@ void* pool_alloc(size_t bytes, cudaStream_t s) {
     (void)cudaGetLastError();
     e = pool_attempt(&p, bytes, pool, s);
   }
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();  // reported here; no later launch check is to find it
-    fail_cuda(e, "cudaMallocFromPoolAsync", __FILE__, __LINE__);
-  }
+  if (e != cudaSuccess) fail_cuda(e, "cudaMallocFromPoolAsync", __FILE__, __LINE__);
   if (trace_on()) {
     const double ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

@@ -34,6 +34,7 @@ struct Error {
 
 [[noreturn]] inline void fail_cuda(cudaError_t e, const char* what, const char* file,
                                    int line) {
+  (void)cudaGetLastError();  // reported here; no later launch check is to find it
   kg_status s = (e == cudaErrorMemoryAllocation) ? KG_ERR_OOM : KG_ERR_DEVICE;
   std::string msg = std::string("CUDA error ") + cudaGetErrorName(e) + " (" +
                     cudaGetErrorString(e) + ") in " + what + " at " + file + ":" +
@@ -362,9 +363,12 @@ struct Trace {
   }
 };
 
+// Every call begins without an error that somebody else's CUDA call left in this thread: the launch
+// checks (cudaGetLastError) would report it as their own.
 template <class F>
 kg_status guarded(F&& body) {
   try {
+    (void)cudaGetLastError();
     body();
     return KG_OK;
   } catch (const Error& e) {
