@@ -218,8 +218,8 @@ typedef struct kg_tile_block {
  * decreases and is flat over padding rows; each row's local indices strictly increase
  * below the block width). Replaces decode_cell_block and its checks
  * (crates/kyto-store/src/tile_decode.rs:74-196); the first problem, in kyto's order (tile,
- * then check, then row), returns KG_ERR_CORRUPT with kyto's wording, and no entry is
- * read through an indptr that failed its check. Outputs (host or device): indptr
+ * then check, then row), returns KG_ERR_CORRUPT with kyto's wording, the outputs are left
+ * as they were, and no entry is read outside its tile, whatever the indptr holds. Outputs (host or device): indptr
  * rows + 1 values from 0; indices and values tile_offsets[last] - tile_offsets[0]
  * entries, each row's genes in increasing order. */
 KG_API kg_status kg_tiles_to_csr(kg_ctx* ctx, const kg_tile_block* block, uint64_t* indptr,

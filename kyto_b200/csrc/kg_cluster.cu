@@ -273,12 +273,12 @@ join_centres_kernel(const double* partial, uint32_t parts, const uint32_t* start
 
 // The centres of the clusters' rows. A large cluster's chain of additions is what a call waits
 // for (8,000 rows: 36 us), so unless the sums are to be in slot order throughout (`ordered`) a
-// cluster is cut into up to 16 parts where the clusters alone leave the chip idle: 50 us a round of
+// cluster is cut into up to 16 parts while there are fewer than four an SM: 50 us a round of
 // 58 clusters of 60,000 rows, in parts 11 and 5 to join them.
 void update_centres(const float* x, uint32_t width, uint32_t d, const uint32_t* order,
-                    const uint32_t* starts, uint32_t K, bool ordered, double* centre,
+                    const uint32_t* starts, uint32_t K, bool ordered, int sm_count, double* centre,
                     cudaStream_t s) {
-  const uint32_t parts = ordered ? 1 : std::min(16u, std::max(1u, 592u / K));
+  const uint32_t parts = ordered ? 1 : std::min(16u, std::max(1u, 4u * (uint32_t)sm_count / K));
   DeviceBuffer<double> partial(parts > 1 ? (uint64_t)K * parts * kClusterDim : 0, s);
   update_centres_kernel<<<dim3(K, parts), kUcThreads, 0, s>>>(x, width, d, order, starts, centre,
                                                               partial.ptr);
@@ -337,7 +337,8 @@ void nearest_centres(const float* x, uint64_t n, uint32_t width, uint32_t d,
 }
 
 void cluster_rows(const float* x, uint64_t n, uint32_t width, uint32_t d, uint32_t K,
-                  uint32_t iters, uint64_t sample, bool ordered, Clusters& out, cudaStream_t s) {
+                  uint32_t iters, uint64_t sample, bool ordered, int sm_count, Clusters& out,
+                  cudaStream_t s) {
   if (d > kClusterDim) fail(KG_ERR_INVALID, "clusters: more than 64 components");
   K = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(K, n));
   out.K = K;
@@ -367,7 +368,7 @@ void cluster_rows(const float* x, uint64_t n, uint32_t width, uint32_t d, uint32
     key_starts_kernel<<<blocks_for((uint64_t)K + 1, 256), 256, 0, s>>>(key_sorted.ptr, m, K,
                                                                        starts.ptr);
     KG_LAUNCH_CHECK();
-    update_centres(sorted.ptr, d, d, order.ptr, starts.ptr, K, ordered, out.centre.ptr, s);
+    update_centres(sorted.ptr, d, d, order.ptr, starts.ptr, K, ordered, sm_count, out.centre.ptr, s);
   }
   centres_f32_kernel<<<(K + kCentresABlock - 1) / kCentresABlock, kCentresABlock * kClusterDim, 0,
                        s>>>(out.centre.ptr, K, cf.ptr, cn.ptr);
@@ -375,7 +376,7 @@ void cluster_rows(const float* x, uint64_t n, uint32_t width, uint32_t d, uint32
   out.label.alloc(n, s);
   nearest_centres(x, n, width, d, cf.ptr, cn.ptr, K, out.label.ptr, s);
   order_by_cluster(x, n, width, out.label.ptr, K, out.perm, out.start, s);
-  update_centres(x, width, d, out.perm.ptr, out.start.ptr, K, ordered, out.centre.ptr, s);
+  update_centres(x, width, d, out.perm.ptr, out.start.ptr, K, ordered, sm_count, out.centre.ptr, s);
 }
 
 }  // namespace kg

@@ -25,7 +25,8 @@ struct Clusters {
 // all rows. Deterministic: fixed-order sums (a centre's rows one after another if `ordered`, else in
 // parts added in order), ties to the lower centre.
 void cluster_rows(const float* x, uint64_t n, uint32_t width, uint32_t d, uint32_t K,
-                  uint32_t iters, uint64_t sample, bool ordered, Clusters& out, cudaStream_t s);
+                  uint32_t iters, uint64_t sample, bool ordered, int sm_count, Clusters& out,
+                  cudaStream_t s);
 
 // labels[r] = the centre (of K, K x kClusterDim f32, squared norms cn) nearest to row r
 // of x (f32 distances; ties to the lower centre).

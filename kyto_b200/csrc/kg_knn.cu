@@ -426,7 +426,7 @@ bool bounded_scan(const float* x, uint64_t n, uint32_t width, uint32_t d, const 
   }
   Clusters cl;
   const uint32_t parts = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(n / 1024, 1), 4096);
-  cluster_rows(x, n, width, d, parts, 5, 131072, false, cl, s);
+  cluster_rows(x, n, width, d, parts, 5, 131072, false, sm_count, cl, s);
   trace.mark("scan parts");
   DeviceBuffer<double> bc((uint64_t)kDim * n_blocks, s), blo((uint64_t)kDim * n_blocks, s),
       bhi((uint64_t)kDim * n_blocks, s), br(n_blocks, s);
@@ -838,10 +838,11 @@ __device__ __forceinline__ uint32_t count_before(uint32_t count, const RankCandi
 // candidate, lane j with the components j, j + 8, ..., which is the partial sum j of
 // exact_key; sixteen candidates' reads are in flight a warp, and a read is one sector a
 // candidate. Latency bounds it: a lane that read a candidate's row by itself touched a sector
-// a component, waited for each and then merged its ranked list (0.69 ms for 60,000 rows of 50
-// components and 70 candidates each, 10 ms for 1M rows with 63; now 0.43 and 6.4 ms). Past 64 candidates those beyond the k-th smallest of the 32 lanes' smallest keys are
-// dropped (at least k lie at or before it; k <= 32). A candidate's rank is the number of
-// candidates before it. More candidates: ranked lists a lane, merged (warp_merge).
+// a component, waited for each and then merged its ranked list (0.69 ms for 60,013 rows of 30
+// components, 30 neighbours and 70 candidates each, 10 ms for 1M rows with 63; now 0.43 and 6.4
+// ms). Past 64 candidates those beyond the k-th smallest of the 32 lanes' smallest keys are dropped
+// (at least k lie at or before it; k <= 32). A candidate's rank is the number of candidates before
+// it. More candidates: ranked lists a lane, merged (warp_merge).
 __global__ void __launch_bounds__(kRankWarps * 32)
 rank_kernel(const float* __restrict__ x, uint32_t width, uint32_t d,
                             uint64_t q_begin, uint64_t q_end, uint32_t k, uint32_t cap,

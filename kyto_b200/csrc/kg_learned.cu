@@ -487,7 +487,7 @@ kg_status kg_knn_learned(kg_ctx* ctx, const float* embedding, uint64_t n, uint32
     knn_core(ctx, xs.ptr, m, d, d, k, nullptr, sg, trace);
     trace.mark("sample graph");
     Clusters cl;
-    cluster_rows(xs.ptr, m, d, d, std::min<uint32_t>(parts, (uint32_t)m), 10, m, true, cl, s);
+    cluster_rows(xs.ptr, m, d, d, std::min<uint32_t>(parts, (uint32_t)m), 10, m, true, ctx->sm_count, cl, s);
     DeviceBuffer<uint32_t> labels(m * L, s);
     target_labels_kernel<<<blocks_for(m, 256), 256, 0, s>>>(cl.label.ptr, sg.row.ptr, m, k,
                                                             labels.ptr);
