@@ -561,7 +561,7 @@ __device__ __forceinline__ uint2 make_entry(uint32_t w0, uint32_t w1) {
 // chunk of X^T's columns, through a window of columns at a time in shared memory, a warp four
 // rows, the lanes over each row's entries. Reading the entries and writing both layouts bounds
 // it. (Each layout by itself, a lane writing where its entry goes, every entry a sector:
-// masks 3.8 and values 11.0 ms for 1M rows of 570 entries, now 1.75 and 3.8.)
+// masks 3.8 and values 11.0 ms for 1M rows of 570 entries, now 1.8 and 3.8.)
 constexpr int kLayWarps = 8;                // a CTA
 constexpr int kLayRows = 32 / kLayWarps;    // CSR rows a warp
 constexpr uint32_t kMaskCols = 512;         // columns a window of masks_kernel
@@ -589,7 +589,7 @@ __device__ __forceinline__ WalkRows walk_start(const uint64_t* __restrict__ ptr,
 // a later run of kValueCols columns: where that is so for no window, each entry is passed once, in
 // its own window, in windows of Cols and of kValueCols columns alike (within a run the order does
 // not matter: the tiles are filled by column). Rows without a jump need no check of the window's
-// lower end (0.5 ms of values_kernel's 3.8 for the check; masks_kernel's take 0.35 of 1.75).
+// lower end (0.5 ms of values_kernel's 3.8 for the check; masks_kernel's checks take 0.4 of 1.8).
 template <bool Values, bool Checked, uint32_t Cols, class F>
 __device__ __forceinline__ void walk_window(const uint32_t* __restrict__ col,
                                             const float* __restrict__ val, WalkRows& w, uint32_t c0,
