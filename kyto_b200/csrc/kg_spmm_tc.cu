@@ -972,20 +972,28 @@ void spmm_tc(const SpmmArgs& a, cudaStream_t s) {
   if (a.out.mode == kOutRows && geo.n_segs != 1)
     fail(KG_ERR_INVALID, "spmm: row output needs one K segment");
   // A chip that one segment a tile leaves idle: shorter work items whose f32 groups are added
-  // afterwards in the segments' order.
+  // afterwards in the segments' order. (Whole segments give the same bits, and take no memory.)
   const uint64_t seg_chunks = geo.seg_chunks;
   SpmmOut to = a.out;
   DeviceBuffer<float> groups;
   const uint32_t n_groups = (geo.n_chunks + kFlushChunks - 1) / kFlushChunks;
+  auto room = [&] {
+    try {
+      groups.alloc((uint64_t)n_groups * b.rows * kN, s);
+      return true;
+    } catch (const Error& e) {
+      if (e.status != KG_ERR_OOM) throw;
+      return false;
+    }
+  };
   if (n_groups > geo.n_segs && (seg_chunks % kFlushChunks == 0 || geo.n_segs == 1) &&
-      split_groups((uint64_t)geo.n_tiles * geo.n_segs, a.sm_count)) {
+      split_groups((uint64_t)geo.n_tiles * geo.n_segs, a.sm_count) && room()) {
     uint32_t part = kFlushChunks;
     while (part * 2 < seg_chunks &&
            (uint64_t)geo.n_tiles * (geo.n_chunks / (part * 2)) >= 4ull * a.sm_count)
       part *= 2;
     geo.seg_chunks = part;
     geo.n_segs = (geo.n_chunks + part - 1) / part;
-    groups.alloc((uint64_t)n_groups * b.rows * kN, s);
     to.mode = kOutGroups;
     to.groups = groups.ptr;
   }

@@ -63,3 +63,35 @@ def test_a_search_out_of_memory_for_its_lists_goes_without():
     listed = [a for a in range(max(out_of_memory)) if a not in out_of_memory]
     # The lists' own attempts come one after another, from the clustering to the filter's end.
     assert len(listed) >= 40 and listed == list(range(listed[0], listed[-1] + 1))
+
+
+def test_a_product_out_of_memory_for_its_groups_goes_without():
+    """A product's groups (300 rows x 4 groups x 256 bytes: never rounded) are worth having, not
+    needed: the whole segments give the same bits. Eleven passes, a product of X in ten of them."""
+    rng = np.random.default_rng(1)
+    rows, genes, per_row = 300, 2000, 200
+    idx = np.sort(np.argsort(rng.random((rows, genes)), 1)[:, :per_row], 1).astype(np.uint32)
+    indptr = np.arange(rows + 1, dtype=np.uint64) * np.uint64(per_row)
+    values = rng.uniform(0.5, 2.0, idx.size).astype(np.float32)
+
+    def run():
+        sess = K.PcaSession(5, genes)
+        sess.push(indptr, idx.reshape(-1), values)
+        sess.run()
+        assert sess.stats().product_launches > 0
+        return sess.results()
+
+    want = run()
+    out_of_memory = []
+    for attempt in range(600):  # more than a run makes
+        K.fail_allocations(ONE | attempt)
+        try:
+            got = run()
+        except K.KytoError as err:
+            assert err.status == K.KG_ERR_OOM
+            out_of_memory.append(attempt)
+        else:
+            assert np.array_equal(got.variance, want.variance)
+            assert np.array_equal(got.embedding, want.embedding)
+    assert max(out_of_memory) < 599
+    assert max(out_of_memory) + 1 - len(out_of_memory) >= 10
