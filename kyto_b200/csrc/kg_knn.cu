@@ -825,6 +825,129 @@ __device__ __forceinline__ uint32_t count_before(uint32_t count, const RankCandi
   return t;
 }
 
+// The candidates of cand[0 .. m) that keep(c) says, for c = 32 j + lane, moved to the front in
+// order; how many. (For the whole warp, as the functions below.)
+template <class F>
+__device__ __forceinline__ uint32_t keep_candidates(RankCandidate* cand, uint32_t m, F&& keep) {
+  const unsigned lane = threadIdx.x & 31u;
+  uint32_t left = 0;
+  for (uint32_t c0 = 0; c0 < m; c0 += 32) {
+    RankCandidate o;
+    const uint32_t c = c0 + lane;
+    const bool in = c < m && keep(c);
+    if (in) o = cand[c];
+    const unsigned ballot = __ballot_sync(0xFFFFFFFFu, in);
+    __syncwarp();
+    if (in) cand[left + __popc(ballot & ((1u << lane) - 1u))] = o;
+    left += __popc(ballot);
+    __syncwarp();
+  }
+  return left;
+}
+
+// What a query's candidates are measured against.
+struct RankQuery {
+  const float* x;
+  const float* row;  // the query's own
+  uint32_t width, d;
+  double inv_s2, shift, slack;
+};
+
+// Exact keys of cand[from .. kept); whether this lane met one farther from its approximate key than
+// the slack.
+__device__ __forceinline__ bool candidate_keys(const RankQuery& q, RankCandidate* cand,
+                                               uint32_t from, uint32_t kept) {
+  const unsigned lane = threadIdx.x & 31u;
+  const uint32_t part = lane & 7u, group = lane >> 3;
+  double query[kDim / 8];
+#pragma unroll
+  for (uint32_t i = 0; i < kDim / 8; ++i)
+    query[i] = 8 * i + part < q.d ? (double)q.row[8 * i + part] : 0.0;
+  bool bad = false;
+  __syncwarp();
+  for (uint32_t c0 = from; c0 < kept; c0 += 16) {
+    float b[4][kDim / 8];
+#pragma unroll
+    for (uint32_t g = 0; g < 4; ++g) {
+      const float* pr =
+          q.x + (uint64_t)cand[min(c0 + 4 * g + group, kept - 1)].row * q.width + part;
+#pragma unroll
+      for (uint32_t i = 0; i < kDim / 8; ++i) b[g][i] = 8 * i + part < q.d ? pr[8 * i] : 0.0f;
+    }
+#pragma unroll
+    for (uint32_t g = 0; g < 4; ++g) {
+      // exact_key's operations in its order (a component past d adds +0 to a sum >= 0).
+      double e = 0;
+#pragma unroll
+      for (uint32_t i = 0; i < kDim / 8; ++i) {
+        const double diff = __dsub_rn(query[i], (double)b[g][i]);
+        e = __dadd_rn(e, __dmul_rn(diff, diff));
+      }
+#pragma unroll
+      for (int o = 4; o; o >>= 1) e = __dadd_rn(e, __shfl_xor_sync(0xFFFFFFFFu, e, o));
+      const uint32_t c = c0 + 4 * g + group;
+      if (part == 0 && c < kept) {
+        if (fabs(e - ((double)cand[c].approx * q.inv_s2 + q.shift)) > q.slack) bad = true;
+        cand[c].key = e;
+      }
+    }
+  }
+  __syncwarp();
+  return bad;
+}
+
+// Past 64 candidates (k <= 32): those beyond the k-th smallest of the lanes' smallest keys dropped (at
+// least k lie at or before it); how many are left.
+__device__ __forceinline__ uint32_t drop_far(RankCandidate* cand, uint32_t m, uint32_t k) {
+  const unsigned lane = threadIdx.x & 31u;
+  if (m <= 64 || k > 32) return m;
+  RankCandidate least = cand[lane];
+  for (uint32_t c = lane + 32; c < m; c += 32) {
+    const RankCandidate o = cand[c];
+    if (count_before(0, o, least)) least = o;
+  }
+  uint32_t at = 0;
+  for (int o = 0; o < 32; ++o) {
+    RankCandidate other;
+    other.key = __shfl_sync(0xFFFFFFFFu, least.key, o);
+    other.row = __shfl_sync(0xFFFFFFFFu, least.row, o);
+    at = count_before(at, other, least);
+  }
+  const int kth = __ffs(__ballot_sync(0xFFFFFFFFu, at == k - 1)) - 1;
+  RankCandidate line;
+  line.key = __shfl_sync(0xFFFFFFFFu, least.key, kth);
+  line.row = __shfl_sync(0xFFFFFFFFu, least.row, kth);
+  return keep_candidates(cand, m, [&](uint32_t c) { return count_before(0, line, cand[c]) == 0; });
+}
+
+// put(rank, candidate, index) for this lane's candidates among cand[0 .. m): four a lane at a time
+// (past the end: the last, its rank unused).
+template <class F>
+__device__ __forceinline__ void rank_candidates(const RankCandidate* cand, uint32_t m, F&& put) {
+  for (uint32_t c0 = threadIdx.x & 31u; c0 < m; c0 += 128) {
+    RankCandidate own[4];
+    uint32_t rank[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      own[i] = cand[min(c0 + 32 * i, m - 1)];
+      rank[i] = 0;
+    }
+    const uint32_t in_use = (m - c0 + 31) / 32;
+    for (uint32_t o = 0; o < m; ++o) {
+      const RankCandidate other = cand[o];
+      rank[0] = count_before(rank[0], other, own[0]);
+      rank[1] = count_before(rank[1], other, own[1]);
+      if (in_use > 2) {
+        rank[2] = count_before(rank[2], other, own[2]);
+        rank[3] = count_before(rank[3], other, own[3]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (c0 + 32 * i < m) put(rank[i], own[i], c0 + 32 * i);
+  }
+}
+
 // One warp per query: exact keys of its candidates, the k best by (key, row). A row
 // that overflowed, holds fewer than k candidates or has a candidate outside its slack
 // is flagged for a full search (kyto's rank, neighbors_exact.rs:318-340).
@@ -834,7 +957,7 @@ __device__ __forceinline__ uint32_t count_before(uint32_t count, const RankCandi
 // With `perm`, the filter ran on the rows in scan order: its query position qp and its
 // candidates' rows are positions there, row perm[.] of x (ranks and outputs use x's).
 //
-// Up to kRankKept candidates within the threshold (nearly every query): eight lanes a
+// Up to kRankKept candidates within the threshold (nearly every query) are one batch: eight lanes a
 // candidate, lane j with the components j, j + 8, ..., which is the partial sum j of
 // exact_key; sixteen candidates' reads are in flight a warp, and a read is one sector a
 // candidate. Latency bounds it: a lane that read a candidate's row by itself touched a sector
@@ -842,175 +965,152 @@ __device__ __forceinline__ uint32_t count_before(uint32_t count, const RankCandi
 // components, 30 neighbours and 70 candidates each, 10 ms for 1M rows with 63; now 0.43 and 6.4
 // ms). Past 64 candidates those beyond the k-th smallest of the 32 lanes' smallest keys are dropped
 // (at least k lie at or before it; k <= 32). A candidate's rank is the number of candidates before
-// it. More candidates: ranked lists a lane, merged (warp_merge).
-__global__ void __launch_bounds__(kRankWarps * 32)
-rank_kernel(const float* __restrict__ x, uint32_t width, uint32_t d,
-                            uint64_t q_begin, uint64_t q_end, uint32_t k, uint32_t cap,
-                            const float* __restrict__ cand_key,
-                            const uint32_t* __restrict__ cand_row,
-                            const uint32_t* cand_count, const float* threshold,
-                            const double* slack, double inv_s2, const double* qn2,
-                            const uint32_t* qperm, const uint32_t* pperm, double* out_key,
-                            uint32_t* out_row, uint32_t* full_flag,
-                            unsigned long long* n_candidates) {
-  __shared__ RankCandidate shared[kRankWarps][kRankKept];
-  uint64_t qi = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  unsigned lane = threadIdx.x & 31u;
-  uint64_t qp = q_begin + qi;
-  if (qp >= q_end) return;
-  uint64_t q = qperm ? qperm[qp] : qp;
-  uint32_t count = cand_count[qi];
-  if (count == kOverflow) {
-    if (lane == 0) full_flag[q] = 1;
-    return;
+// it. A query with more candidates is left to rank_many_kernel, its count marked with kMany.
+struct RankArgs {
+  const float* x;
+  uint32_t width, d;
+  uint64_t q_begin, q_end;
+  uint32_t k, cap;
+  const float* cand_key;
+  const uint32_t* cand_row;
+  uint32_t* cand_count;
+  const float* threshold;
+  const double* slack;
+  double inv_s2;
+  const double* qn2;
+  const uint32_t *qperm, *pperm;
+  double* out_key;
+  uint32_t *out_row, *full_flag;
+  unsigned long long* n_candidates;
+  uint8_t* overflowed;  // or null: per query, 1 where its candidates overflowed
+  __device__ __forceinline__ uint64_t row(uint64_t qi) const {
+    return qperm ? qperm[q_begin + qi] : q_begin + qi;
   }
-  float th = threshold[qi];
-  double sl = slack[qp];
-  double shift = qn2 ? qn2[qp] : 0.0;
-  const float* qrow = x + q * width;
-  RankCandidate* const cand = shared[threadIdx.x >> 5];
-  uint32_t kept = 0;
-  for (uint32_t c0 = 0; c0 < count; c0 += 32) {
+  __device__ __forceinline__ RankQuery query(uint64_t qi, uint64_t q) const {
+    return {x, x + q * width, width, d, inv_s2, qn2 ? qn2[q_begin + qi] : 0.0, slack[q_begin + qi]};
+  }
+  __device__ __forceinline__ void put(uint64_t q, uint32_t rank, const RankCandidate& c) const {
+    if (rank >= k) return;
+    out_key[q * (uint64_t)k + rank] = c.key;
+    out_row[q * (uint64_t)k + rank] = c.row;
+  }
+  // (For the whole warp.)
+  __device__ __forceinline__ void done(uint64_t q, uint32_t seen, bool bad) const {
+    const bool any_bad = __any_sync(0xFFFFFFFFu, bad);
+    if ((threadIdx.x & 31u) == 0) {
+      atomicAdd(n_candidates, (unsigned long long)seen);
+      full_flag[q] = (any_bad || seen < k) ? 1u : 0u;
+    }
+  }
+  // Slots c0 .. c0 + 31 of query qi: those within the threshold to cand from `kept` on, as far as
+  // they fit; their number.
+  __device__ __forceinline__ uint32_t gather(uint64_t qi, uint32_t c0, uint32_t count, float th,
+                                             RankCandidate* cand, uint32_t kept) const {
+    const unsigned lane = threadIdx.x & 31u;
     const uint32_t c = c0 + lane;
-    const float ak = c < count ? cand_key[qi * (uint64_t)cap + c] : INFINITY;
+    const float ak = c < count ? __ldg(cand_key + qi * (uint64_t)cap + c) : INFINITY;
     const bool pass = c < count && ak <= th;
     const unsigned ballot = __ballot_sync(0xFFFFFFFFu, pass);
     const uint32_t at = kept + __popc(ballot & ((1u << lane) - 1u));
     if (pass && at < kRankKept) {
-      const uint32_t p = cand_row[qi * (uint64_t)cap + c];
+      const uint32_t p = __ldg(cand_row + qi * (uint64_t)cap + c);
       cand[at].approx = ak;
       cand[at].row = pperm ? pperm[p] : p;
     }
-    kept += __popc(ballot);
-    if (kept > kRankKept) break;
+    return __popc(ballot);
   }
-  if (kept <= kRankKept) {
-    const uint32_t part = lane & 7u, group = lane >> 3;
-    double query[kDim / 8];
-#pragma unroll
-    for (uint32_t i = 0; i < kDim / 8; ++i)
-      query[i] = 8 * i + part < d ? (double)qrow[8 * i + part] : 0.0;
-    bool bad = false;
-    __syncwarp();
-    for (uint32_t c0 = 0; c0 < kept; c0 += 16) {
-      float b[4][kDim / 8];
-#pragma unroll
-      for (uint32_t g = 0; g < 4; ++g) {
-        const float* pr = x + (uint64_t)cand[min(c0 + 4 * g + group, kept - 1)].row * width + part;
-#pragma unroll
-        for (uint32_t i = 0; i < kDim / 8; ++i) b[g][i] = 8 * i + part < d ? pr[8 * i] : 0.0f;
-      }
-#pragma unroll
-      for (uint32_t g = 0; g < 4; ++g) {
-        // exact_key's operations in its order (a component past d adds +0 to a sum >= 0).
-        double e = 0;
-#pragma unroll
-        for (uint32_t i = 0; i < kDim / 8; ++i) {
-          const double diff = __dsub_rn(query[i], (double)b[g][i]);
-          e = __dadd_rn(e, __dmul_rn(diff, diff));
-        }
-#pragma unroll
-        for (int o = 4; o; o >>= 1) e = __dadd_rn(e, __shfl_xor_sync(0xFFFFFFFFu, e, o));
-        const uint32_t c = c0 + 4 * g + group;
-        if (part == 0 && c < kept) {
-          if (fabs(e - ((double)cand[c].approx * inv_s2 + shift)) > sl) bad = true;
-          cand[c].key = e;
-        }
-      }
-    }
-    __syncwarp();
-    uint32_t m = kept;  // candidates still to rank
-    if (m > 64 && k <= 32) {
-      RankCandidate least = cand[lane];
-      for (uint32_t c = lane + 32; c < m; c += 32) {
-        const RankCandidate o = cand[c];
-        if (count_before(0, o, least)) least = o;
-      }
-      uint32_t at = 0;
-      for (int o = 0; o < 32; ++o) {
-        RankCandidate other;
-        other.key = __shfl_sync(0xFFFFFFFFu, least.key, o);
-        other.row = __shfl_sync(0xFFFFFFFFu, least.row, o);
-        at = count_before(at, other, least);
-      }
-      const int kth = __ffs(__ballot_sync(0xFFFFFFFFu, at == k - 1)) - 1;
-      RankCandidate line;
-      line.key = __shfl_sync(0xFFFFFFFFu, least.key, kth);
-      line.row = __shfl_sync(0xFFFFFFFFu, least.row, kth);
-      uint32_t left = 0;
-      for (uint32_t c0 = 0; c0 < m; c0 += 32) {
-        RankCandidate o;
-        const bool in = c0 + lane < m;
-        if (in) o = cand[c0 + lane];
-        const bool keep = in && count_before(0, line, o) == 0;
-        const unsigned ballot = __ballot_sync(0xFFFFFFFFu, keep);
-        __syncwarp();
-        if (keep) cand[left + __popc(ballot & ((1u << lane) - 1u))] = o;
-        left += __popc(ballot);
-        __syncwarp();
-      }
-      m = left;
-    }
-    for (uint32_t c0 = lane; c0 < m; c0 += 128) {
-      // Four candidates a lane at a time (past the end: the last, its rank unused).
-      RankCandidate own[4];
-      uint32_t rank[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        own[i] = cand[min(c0 + 32 * i, m - 1)];
-        rank[i] = 0;
-      }
-      const uint32_t in_use = (m - c0 + 31) / 32;
-      for (uint32_t o = 0; o < m; ++o) {
-        const RankCandidate other = cand[o];
-        rank[0] = count_before(rank[0], other, own[0]);
-        rank[1] = count_before(rank[1], other, own[1]);
-        if (in_use > 2) {
-          rank[2] = count_before(rank[2], other, own[2]);
-          rank[3] = count_before(rank[3], other, own[3]);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (c0 + 32 * i < m && rank[i] < k) {
-          out_key[q * (uint64_t)k + rank[i]] = own[i].key;
-          out_row[q * (uint64_t)k + rank[i]] = own[i].row;
-        }
-    }
-    const bool any_bad = __any_sync(0xFFFFFFFFu, bad);
-    if (lane == 0) {
-      atomicAdd(n_candidates, (unsigned long long)kept);
-      full_flag[q] = (any_bad || kept < k) ? 1u : 0u;
-    }
+};
+constexpr uint32_t kMany = 1u << 31;  // in cand_count: left to rank_many_kernel (kOverflow holds it too)
+
+__global__ void __launch_bounds__(kRankWarps * 32)
+rank_kernel(const __grid_constant__ RankArgs a) {
+  __shared__ RankCandidate shared[kRankWarps][kRankKept];
+  const uint64_t qi = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const unsigned lane = threadIdx.x & 31u;
+  if (a.q_begin + qi >= a.q_end) return;
+  const uint64_t q = a.row(qi);
+  const uint32_t count = a.cand_count[qi];
+  if (count == kOverflow) {
+    if (lane == 0) a.full_flag[q] = 1;
     return;
   }
-  double keys[kMaxK];
-  uint32_t idx[kMaxK];
-  uint32_t len = 0;
-  bool bad = false;
-  uint32_t used = 0;
-  for (uint32_t c = lane; c < count; c += 32) {
-    float ak = cand_key[qi * (uint64_t)cap + c];
-    if (ak > th) continue;
-    uint32_t p = cand_row[qi * (uint64_t)cap + c];
-    if (pperm) p = pperm[p];
-    double e = exact_key(qrow, x + (uint64_t)p * width, d);
-    if (fabs(e - ((double)ak * inv_s2 + shift)) > sl) bad = true;
-    offer(keys, idx, len, k, e, p);
-    ++used;
+  const float th = a.threshold[qi];
+  const RankQuery query = a.query(qi, q);
+  RankCandidate* const cand = shared[threadIdx.x >> 5];
+  uint32_t kept = 0;
+  for (uint32_t c0 = 0; c0 < count; c0 += 32) {
+    kept += a.gather(qi, c0, count, th, cand, kept);
+    if (kept > kRankKept) {
+      if (lane == 0) a.cand_count[qi] = count | kMany;
+      return;
+    }
   }
-  for (int o = 16; o; o >>= 1) used += __shfl_xor_sync(0xFFFFFFFFu, used, o);
-  bool any_bad = __any_sync(0xFFFFFFFFu, bad);
-  __shared__ uint32_t merged_len[kRankWarps];
-  unsigned w = threadIdx.x >> 5;
-  double* ok = out_key + q * (uint64_t)k;
-  uint32_t* orow = out_row + q * (uint64_t)k;
-  warp_merge(keys, idx, len, k, ok, orow, &merged_len[w]);
-  __syncwarp();
-  if (lane == 0) {
-    atomicAdd(n_candidates, (unsigned long long)used);
-    full_flag[q] = (any_bad || merged_len[w] != k) ? 1u : 0u;
+  const bool bad = candidate_keys(query, cand, 0, kept);
+  rank_candidates(cand, drop_far(cand, kept, a.k),
+                  [&](uint32_t rank, const RankCandidate& c, uint32_t) { a.put(q, rank, c); });
+  a.done(q, kept, bad);
+}
+
+// Which queries overflowed, and the queries that rank_kernel left: their candidates come in batches of what `cand` holds, behind
+// the k best of the batches before. A warp takes every warps'th query. (A kernel of its own: its
+// registers in rank_kernel, in line or in a call, cost that 2 to 5%. A search with bf16 operands of
+// 200,000 rows of 50 components and 29 neighbours: 87 ms with a sorted list a lane, merged, in
+// rank_kernel, 51 so.)
+__global__ void __launch_bounds__(kRankWarps * 32)
+rank_many_kernel(const __grid_constant__ RankArgs a) {
+  __shared__ RankCandidate shared[kRankWarps][kRankKept];
+  const unsigned lane = threadIdx.x & 31u;
+  const uint64_t first = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t warps = gridDim.x * (uint64_t)kRankWarps, n = a.q_end - a.q_begin;
+  RankCandidate* const cand = shared[threadIdx.x >> 5];
+  if (a.overflowed)
+    for (uint64_t i = first * 32 + lane; i < n; i += 32 * warps)
+      a.overflowed[i] = a.cand_count[i] == kOverflow ? 1 : 0;
+  for (uint64_t r0 = first; r0 < n; r0 += 32 * warps) {
+    const uint64_t mine = r0 + lane * warps;
+    const uint32_t counts = mine < n ? a.cand_count[mine] : 0;
+    unsigned left = __ballot_sync(0xFFFFFFFFu, counts != kOverflow && (counts & kMany));
+    while (left) {
+      const int turn = __ffs(left) - 1;
+      left &= left - 1;
+      const uint64_t qi = r0 + turn * warps, q = a.row(qi);
+      const uint32_t count = __shfl_sync(0xFFFFFFFFu, counts, turn) & ~kMany;
+      const float th = a.threshold[qi];
+      const RankQuery query = a.query(qi, q);
+      uint32_t held = 0, c0 = 0, seen = 0;
+      bool bad = false;
+      for (;;) {
+        uint32_t kept = held;
+        __syncwarp();
+        for (; c0 < count && kept + 32 <= kRankKept; c0 += 32)
+          kept += a.gather(qi, c0, count, th, cand, kept);
+        seen += kept - held;
+        bad |= candidate_keys(query, cand, held, kept);
+        const uint32_t m = drop_far(cand, kept, a.k);
+        if (c0 >= count) {
+          rank_candidates(cand, m, [&](uint32_t rank, const RankCandidate& c, uint32_t) {
+            a.put(q, rank, c);
+          });
+          break;
+        }
+        uint32_t best = 0;  // bit j: candidate 32 j + lane is among the k best
+        rank_candidates(cand, m, [&](uint32_t rank, const RankCandidate&, uint32_t c) {
+          if (rank < a.k) best |= 1u << (c / 32);
+        });
+        __syncwarp();
+        held = keep_candidates(cand, m, [&](uint32_t c) { return ((best >> (c / 32)) & 1u) != 0; });
+      }
+      a.done(q, seen, bad);
+    }
   }
+}
+
+void launch_rank(const RankArgs& a, int sm_count, cudaStream_t s) {
+  const unsigned blocks = blocks_for((a.q_end - a.q_begin) * 32, kRankWarps * 32);
+  rank_kernel<<<blocks, kRankWarps * 32, 0, s>>>(a);
+  KG_LAUNCH_CHECK();
+  rank_many_kernel<<<std::min(blocks, 4u * (unsigned)sm_count), kRankWarps * 32, 0, s>>>(a);
+  KG_LAUNCH_CHECK();
 }
 
 // One CTA per flagged row: every other row's exact key, the k best by (key, row).
@@ -1129,12 +1229,6 @@ __global__ void compact_flags_kernel(const uint32_t* flag, uint64_t n, uint32_t*
                                      unsigned int* count) {
   uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (r < n && flag[r]) list[atomicAdd(count, 1u)] = (uint32_t)r;
-}
-
-// Whether each query slot's candidates overflowed (1) or not (0).
-__global__ void overflow_flags_kernel(const uint32_t* cand_count, uint64_t n, uint8_t* flag) {
-  uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (q < n) flag[q] = cand_count[q] == kOverflow ? 1 : 0;
 }
 
 // Slots whose list does not cover their row: marked overflowed, so they are searched
@@ -1585,11 +1679,10 @@ void knn_search(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_
     }
     check_cancel(ctx);
     Timer tr(s);
-    rank_kernel<<<blocks_for(n * 32, kRankWarps * 32), kRankWarps * 32, 0, s>>>(
-        x, width, d, 0, n, k, cap, cand_key, cand_row, cand_count.ptr, thr.ptr,
-        slack_d.ptr, 1.0 / (scale * scale), qn2.ptr, sp.qrows.ptr, prows, out.key.ptr,
-        out.row.ptr, full_flag.ptr, n_cand.ptr);
-    KG_LAUNCH_CHECK();
+    DeviceBuffer<uint8_t> oflag(n, s);
+    launch_rank({x, width, d, 0, n, k, cap, cand_key, cand_row, cand_count.ptr, thr.ptr,
+                 slack_d.ptr, 1.0 / (scale * scale), qn2.ptr, sp.qrows.ptr, prows, out.key.ptr,
+                 out.row.ptr, full_flag.ptr, n_cand.ptr, oflag.ptr}, ctx->sm_count, s);
     rank_ms += tr.stop_ms();
     // Queries whose candidates overflowed (more than the slots hold within the slack of
     // their k-th: dense regions) get a second filter pass with room for kTcRetryCap
@@ -1601,9 +1694,6 @@ void knn_search(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_
     {
       // The overflowed slots in slot order (a stable compaction: the retry's blocks, and
       // with them every count the search reports, are the same run to run).
-      DeviceBuffer<uint8_t> oflag(n, s);
-      overflow_flags_kernel<<<blocks_for(n, 256), 256, 0, s>>>(cand_count.ptr, n, oflag.ptr);
-      KG_LAUNCH_CHECK();
       cub::CountingInputIterator<uint32_t> slots(0);
       size_t tb = 0;
       KG_CUDA(cub::DeviceSelect::Flagged(nullptr, tb, slots, oflag.ptr, over.ptr, n_over.ptr,
@@ -1674,7 +1764,7 @@ void knn_search(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_
       DeviceBuffer<uint32_t> m_row, m_count;
       const float* use_key = r_key.ptr;
       const uint32_t* use_row = r_row.ptr;
-      const uint32_t* use_count = r_count.ptr;
+      uint32_t* use_count = r_count.ptr;
       const float* use_thr = r_thr.ptr;
       if (nc > 1) {
         m_key.alloc(m * kTcRetryCap, s);
@@ -1690,11 +1780,10 @@ void knn_search(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_
         use_count = m_count.ptr;
         use_thr = m_thr.ptr;
       }
-      rank_kernel<<<blocks_for(m * 32, kRankWarps * 32), kRankWarps * 32, 0, s>>>(
-          x, width, d, 0, m, k, nc > 1 ? kTcRetryCap : copy_cap, use_key, use_row, use_count,
-          use_thr, r_slack.ptr, 1.0 / (scale * scale), r_qn2.ptr, r_qrows.ptr, prows,
-          out.key.ptr, out.row.ptr, full_flag.ptr, n_cand.ptr);
-      KG_LAUNCH_CHECK();
+      launch_rank({x, width, d, 0, m, k, nc > 1 ? kTcRetryCap : copy_cap, use_key, use_row,
+                   use_count, use_thr, r_slack.ptr, 1.0 / (scale * scale), r_qn2.ptr, r_qrows.ptr,
+                   prows, out.key.ptr, out.row.ptr, full_flag.ptr, n_cand.ptr, nullptr},
+                  ctx->sm_count, s);
       rank_ms += trr.stop_ms();
     }
     out.retried = h_over;
@@ -1724,11 +1813,9 @@ void knn_search(kg_ctx* ctx, const float* x, uint64_t n, uint32_t width, uint32_
       KG_LAUNCH_CHECK();
       filter_ms += tf.stop_ms();
       Timer tr(s);
-      rank_kernel<<<blocks_for((q1 - q0) * 32, kRankWarps * 32), kRankWarps * 32, 0, s>>>(
-          x, width, d, q0, q1, k, cap, cand_key.ptr, cand_row.ptr, cand_count.ptr, thr.ptr,
-          slack.ptr, 1.0, nullptr, nullptr, nullptr, out.key.ptr, out.row.ptr, full_flag.ptr,
-          n_cand.ptr);
-      KG_LAUNCH_CHECK();
+      launch_rank({x, width, d, q0, q1, k, cap, cand_key.ptr, cand_row.ptr, cand_count.ptr, thr.ptr,
+                   slack.ptr, 1.0, nullptr, nullptr, nullptr, out.key.ptr, out.row.ptr,
+                   full_flag.ptr, n_cand.ptr, nullptr}, ctx->sm_count, s);
       rank_ms += tr.stop_ms();
       ctx->done = q1;
     }
