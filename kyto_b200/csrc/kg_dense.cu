@@ -247,15 +247,28 @@ __device__ __forceinline__ int jacobi_square(JacobiShared& sh, uint32_t w, doubl
   return sweep >= 60 ? 1 : 0;
 }
 
-// The CTA's sum of squares of m's n values, to every thread (a fixed order).
-__device__ double squares_sum(const double* m, uint64_t n, double* part) {
+// A part's sum of squares: values [n part / parts, n (part + 1) / parts) of m, to thread 0 (a fixed
+// order). Waiting for the reads is what it does: eight are on their way a thread, and the parts
+// spread over the chip. (One CTA, a read at a time, behind a block of 60,000 genes x 40: 4.1 ms; now
+// the parts end long before the SVD beside them.)
+__device__ double squares_part(const double* m, uint64_t n, uint32_t part, uint32_t parts,
+                               double* warp_sums) {
+  constexpr int kAhead = 8;
+  const uint64_t end = n * (part + 1) / parts;
   double ss = 0.0;
-  for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) ss = fma(m[i], m[i], ss);
+  for (uint64_t i = n * part / parts + threadIdx.x; i < end; i += kAhead * (uint64_t)blockDim.x) {
+    double v[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      v[k] = i + k * (uint64_t)blockDim.x < end ? m[i + k * (uint64_t)blockDim.x] : 0.0;
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) ss = fma(v[k], v[k], ss);
+  }
   for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-  if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = ss;
+  if ((threadIdx.x & 31u) == 0) warp_sums[threadIdx.x >> 5] = ss;
   __syncthreads();
   double t = 0.0;
-  for (uint32_t i = 0; i < blockDim.x / 32; ++i) t += part[i];
+  for (uint32_t i = 0; i < blockDim.x / 32; ++i) t += warp_sums[i];
   return t;
 }
 
@@ -264,21 +277,21 @@ struct SvdShared {
   double f[2][kW][kW + 1];  // two factors by row
 };
 
-// CTA 0: the SVD of R = R_3 R_2 R_1. CTA 1 meanwhile: |block|_F (the host needs both at
-// once).
+// CTA 0: the SVD of R = R_3 R_2 R_1. The others meanwhile: the block's sums of squares (the host
+// needs both at once).
 __global__ void __launch_bounds__(kJacobiThreads, 1)
 small_svd_kernel(const double* r, uint32_t w, const double* block, uint64_t n, const int* status,
                  double* u_r, double* out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SvdShared& sm = *reinterpret_cast<SvdShared*>(smem_raw);
   JacobiShared& sh = sm.jac;
-  if (blockIdx.x == 1) {
-    const double t = squares_sum(block, n, sh.norms);
-    if (threadIdx.x == 0) out[w] = sqrt(t);
+  if (blockIdx.x > 0) {
+    const double t = squares_part(block, n, blockIdx.x - 1, gridDim.x - 1, sh.norms);
+    if (threadIdx.x == 0) out[w + blockIdx.x] = t;
     return;
   }
   if (*status) {  // a factor was not written (the same for every thread)
-    if (threadIdx.x == 0) out[w + 1] = 1.0;
+    if (threadIdx.x == 0) out[w] = 1.0;
     return;
   }
   const uint32_t tid = threadIdx.x, tx = tid & 15u, ty = tid >> 4;
@@ -328,14 +341,14 @@ small_svd_kernel(const double* r, uint32_t w, const double* block, uint64_t n, c
     const double nv = sh.norms[sh.order[c]];
     u_r[x] = nv > 0.0 ? sh.a[sh.order[c]][jacobi_row(i)] / nv : 0.0;
   }
-  if (tid == 0) out[w + 1] = failed ? 1.0 : 0.0;
+  if (tid == 0) out[w] = failed ? 1.0 : 0.0;
 }
 
-__global__ void __launch_bounds__(1024)
-frobenius_kernel(const double* m, uint64_t n, double* out) {
-  __shared__ double part[32];
-  const double t = squares_sum(m, n, part);
-  if (threadIdx.x == 0) *out = sqrt(t);
+__global__ void __launch_bounds__(kJacobiThreads)
+squares_kernel(const double* m, uint64_t n, double* out) {
+  __shared__ double warp_sums[kJacobiThreads / 32];
+  const double t = squares_part(m, n, blockIdx.x, gridDim.x, warp_sums);
+  if (threadIdx.x == 0) out[blockIdx.x] = t;
 }
 
 // ------------------------------------------------ Householder QR + Jacobi -----------
@@ -401,7 +414,7 @@ qr_svd_kernel(double* b, uint32_t g, uint32_t w, double* u, double* out) {
   }
   __syncthreads();
   const int failed = jacobi_square(sh, w, out);
-  if (threadIdx.x == 0) out[w + 1] = failed ? 1.0 : 0.0;
+  if (threadIdx.x == 0) out[w] = failed ? 1.0 : 0.0;
   // U = Q [U_R; 0]: start from U_R's unit columns, apply H_{w-1}, ..., H_0.
   for (uint64_t x = threadIdx.x; x < (uint64_t)g * w; x += blockDim.x) {
     uint32_t c = (uint32_t)(x / g), r = (uint32_t)(x % g);
@@ -437,7 +450,7 @@ void cholesky_step(const double* gram, uint32_t w, double shift, double* r, int*
 void small_svd(const double* r, uint32_t w, const double* block, uint64_t n, const int* status,
                double* u_r, double* out, cudaStream_t s) {
   allow_dynamic_smem(small_svd_kernel, sizeof(SvdShared));
-  small_svd_kernel<<<2, kJacobiThreads, sizeof(SvdShared), s>>>(r, w, block, n, status, u_r, out);
+  small_svd_kernel<<<1 + squares_parts(n), kJacobiThreads, sizeof(SvdShared), s>>>(r, w, block, n, status, u_r, out);
   KG_LAUNCH_CHECK();
 }
 
@@ -446,8 +459,8 @@ void qr_svd(double* b, uint32_t g, uint32_t w, double* u, double* out, cudaStrea
   KG_LAUNCH_CHECK();
 }
 
-void frobenius(const double* m, uint64_t n, double* out, cudaStream_t s) {
-  frobenius_kernel<<<1, 1024, 0, s>>>(m, n, out);
+void squares(const double* m, uint64_t n, double* out, cudaStream_t s) {
+  squares_kernel<<<squares_parts(n), kJacobiThreads, 0, s>>>(m, n, out);
   KG_LAUNCH_CHECK();
 }
 

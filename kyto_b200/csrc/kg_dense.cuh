@@ -4,6 +4,7 @@
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 
@@ -20,21 +21,26 @@ constexpr uint32_t kQrMaxCols = 64;
 void cholesky_step(const double* gram, uint32_t w, double shift, double* r, int* status,
                    cudaStream_t s);
 
+// The parts that a block's n values' sum of squares comes in.
+inline uint32_t squares_parts(uint64_t n) {
+  return (uint32_t)std::min<uint64_t>(128, n / 16384 + 1);
+}
+
 // The SVD of R = R_3 R_2 R_1, the steps' factors one after another in r (w x w upper
 // triangular, column-major, w <= 64): out[0 .. w) the singular values (descending, ties to
 // the lower column), u_r (w x w: column c the unit left singular vector of out[c]; zero for
-// 0), out[w] = the Frobenius norm of `block` (n values), out[w + 1] = 0, or 1 if Jacobi did
-// not converge or *status is set: then a step's factor is not there, r is not read, and the
-// singular values and u_r are left as they are.
+// 0), out[w] = 0, or 1 if Jacobi did not converge or *status is set: then a step's factor is not
+// there, r is not read, and the singular values and u_r are left as they are. And from out[w + 1]
+// on: the squares_parts(n) parts of the sum of squares of `block` (n values).
 void small_svd(const double* r, uint32_t w, const double* block, uint64_t n, const int* status,
                double* u_r, double* out, cudaStream_t s);
 
 // The thin SVD of the g x w column-major block `b` (overwritten): u the left singular
-// vectors, out[0 .. w) and out[w + 1] as above (out[w] is left as it is).
+// vectors, out[0 .. w] as above.
 void qr_svd(double* b, uint32_t g, uint32_t w, double* u, double* out, cudaStream_t s);
 
-// *out = the Frobenius norm of m (n values).
-void frobenius(const double* m, uint64_t n, double* out, cudaStream_t s);
+// The squares_parts(n) parts of the sum of squares of m (n values).
+void squares(const double* m, uint64_t n, double* out, cudaStream_t s);
 
 // The `take` largest eigenvalues of the symmetric m x m matrix `a` (column-major, both halves),
 // descending, into `values`, and their orthonormal vectors into `vectors` (m x take,

@@ -1122,9 +1122,10 @@ struct Dense {
                               proj.ptr, m, &one, rest.ptr, g));
       }
     }
-    // Singular values, |block|_F, status.
-    DeviceBuffer<double> out(w + 2, s);
-    std::vector<double> h(w + 2);
+    // Singular values, status, the parts of |block|_F^2.
+    const uint32_t parts = squares_parts((uint64_t)g * w);
+    DeviceBuffer<double> out(w + 1 + parts, s);
+    std::vector<double> h(w + 1 + parts);
     auto read_back = [&]() {
       KG_CUDA(cudaMemcpyAsync(h.data(), out.ptr, out.bytes(), cudaMemcpyDeviceToHost, s));
       KG_CUDA(cudaStreamSynchronize(s));
@@ -1155,21 +1156,23 @@ struct Dense {
       read_back();
     } else {
       order.alloc(w, s);
-      frobenius(block, (uint64_t)g * w, out.ptr + w, s);
-      jacobi_svd_kernel<<<1, 1024, 0, s>>>(rest.ptr, g, w, out.ptr, order.ptr, out.ptr + w + 1);
+      squares(block, (uint64_t)g * w, out.ptr + w + 1, s);
+      jacobi_svd_kernel<<<1, 1024, 0, s>>>(rest.ptr, g, w, out.ptr, order.ptr, out.ptr + w);
       KG_LAUNCH_CHECK();
       read_back();
     }
-    const double scale = h[w];
+    double scale = 0.0;
+    for (uint32_t i = 0; i < parts; ++i) scale += h[w + 1 + i];
+    scale = std::sqrt(scale);
     if (!(scale > 0.0)) {
       if (std::isnan(scale)) fail(KG_ERR_INVALID, "pca: the Krylov block is not finite");
       return none;
     }
-    if (narrow && h[w + 1] != 0.0) {
+    if (narrow && h[w] != 0.0) {
       qr_svd(saved.ptr, g, w, u.ptr, out.ptr, s);
       read_back();
     }
-    if (h[w + 1] != 0.0)
+    if (h[w] != 0.0)
       fail(KG_ERR_INVALID, "pca: orthonormalising a Krylov block did not converge");
     uint32_t keep = 0;
     while (keep < w && h[keep] > kDropTolerance * scale) ++keep;
