@@ -347,6 +347,9 @@ extern "C" kg_status kg_connectivities(kg_ctx* ctx, const uint64_t* indptr,
     DeviceBuffer<uint64_t> hp;
     DeviceBuffer<uint32_t> hi;
     DeviceBuffer<float> hd;
+    // (Host arrays are copied whole: their offsets are looked at first.)
+    if (!is_device_pointer(indptr) && indptr[n_rows] != m)
+      fail(KG_ERR_INVALID, "kg_connectivities: every row must hold n_neighbors - 1 entries");
     const uint64_t* d_ptr = device_view(indptr, n_rows + 1, hp, s);
     const uint32_t* d_idx = device_view(indices, m, hi, s);
     const float* d_dist = device_view(distances, m, hd, s);

@@ -73,3 +73,18 @@ def test_a_row_out_of_shape(k, fault):
     assert status == K.KG_OK and nnz == want[1].size
     assert np.array_equal(out[0].cpu().numpy().view(np.uint64), want[0])
     assert np.array_equal(out[1][:nnz].cpu().numpy().view(np.uint32), want[1])
+
+
+@pytest.mark.parametrize("k,neighbors", [(9, 15), (14, 10)])
+def test_host_arrays_of_another_number_of_neighbors(k, neighbors):
+    """Host arrays as long as the graph they hold."""
+    n = 500
+    graph = _graph(n, k)
+    most = 2 * n * max(k, neighbors)
+    out = np.zeros(n + 1, dtype=np.uint64), np.zeros(most, dtype=np.uint32), np.zeros(most, np.float32)
+    nnz = ctypes.c_uint64(7)
+    status = K.library().kg_connectivities(
+        K.default_context().handle, *(a.ctypes.data for a in graph), n, neighbors,
+        *(a.ctypes.data for a in out), ctypes.byref(nnz))
+    assert status == K.KG_ERR_INVALID and nnz.value == 7
+    assert not any(a.any() for a in out)
